@@ -95,12 +95,24 @@ void with_all_contexts_idle(mynah_b200_model *h, F fn) {
     for (int i = 0; i < h->n_ctx(); i++) fn(h->ctx(i));
 }
 }  // namespace
+// A resident weight and the buffers of its products. Allocating them per call cost 0.48 ms of a 16 us product: the
+// stream-ordered pool gives its memory back at every synchronisation and maps it anew at the next allocation.
+//   block  device [status, 256 B | QMAT_SMALL out | QMAT_SMALL x], pinned twin `host`: small calls move the rows in with
+//          one copy and the result with the status word out with one copy
+//   ws     device workspace of larger calls, kept up to QMAT_KEEP bytes (a larger one is freed when its call ends)
+// One lock per handle: products of one weight share these and run one after the other on the handle's stream.
 struct mynah_b200_qmat {
     QWeight w;
     std::vector<void *> owned;
     cudaStream_t stream = nullptr;
-    int *status = nullptr;
+    int *status = nullptr;               // = the first word of the block
+    mutable std::mutex mu;
+    mutable uint8_t *host = nullptr;     // from the pinned pool, taken by the first call
+    mutable uint8_t *ws = nullptr;
+    mutable size_t ws_cap = 0;
 };
+static constexpr size_t QMAT_HEAD = 256, QMAT_SMALL = 128 << 10, QMAT_BLOCK = QMAT_HEAD + 2 * QMAT_SMALL;
+static constexpr size_t QMAT_KEEP = 64 << 20;
 struct mynah_b200_batch {
     int batch = 0;
     std::vector<float *> audio;          // device
@@ -124,6 +136,67 @@ QmatView qmat_view(const void *handle) {
     return QmatView{&q->w, q->stream};
 }
 }  // namespace mb
+
+namespace {
+// Pinned twins of the handles' blocks. Pinning costs more than a product, so up to POOL_MAX blocks outlive their handle
+// and serve the next one.
+class PinnedPool {
+public:
+    uint8_t *take() {
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (!free_.empty()) { uint8_t *p = free_.back(); free_.pop_back(); return p; }
+        }
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, QMAT_BLOCK, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        return (uint8_t *)p;
+    }
+    void give(uint8_t *p) {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (free_.size() < POOL_MAX) { free_.push_back(p); return; }
+        }
+        cudaFreeHost(p);
+    }
+
+private:
+    static constexpr size_t POOL_MAX = 32;
+    std::mutex mu_;
+    std::vector<uint8_t *> free_;
+};
+PinnedPool &pinned_pool() { static PinnedPool *p = new PinnedPool(); return *p; }   // alive until the process ends
+
+// `bytes` of device workspace on a handle whose lock is held: the kept one, or (above QMAT_KEEP) a stream-ordered
+// allocation that ends with the call.
+class QmatScratch {
+public:
+    QmatScratch(const mynah_b200_qmat *q, size_t bytes) : q_(q) {
+        if (bytes <= q->ws_cap) { p_ = q->ws; return; }
+        if (bytes > QMAT_KEEP) {
+            if (cudaMallocAsync(&own_, bytes, q->stream) != cudaSuccess) { cudaGetLastError(); own_ = nullptr; }
+            p_ = (uint8_t *)own_;
+            return;
+        }
+        if (q->ws) cudaFree(q->ws);                              // waits for the products that use it
+        q->ws = nullptr; q->ws_cap = 0;
+        size_t cap = 1 << 20;
+        while (cap < bytes) cap <<= 1;
+        if (cudaMalloc((void **)&q->ws, cap) != cudaSuccess) { cudaGetLastError(); q->ws = nullptr; return; }
+        q->ws_cap = cap;
+        p_ = q->ws;
+    }
+    ~QmatScratch() { if (own_) cudaFreeAsync(own_, q_->stream); }
+    uint8_t *get() const { return p_; }
+    QmatScratch(const QmatScratch &) = delete;
+    QmatScratch &operator=(const QmatScratch &) = delete;
+
+private:
+    const mynah_b200_qmat *q_;
+    uint8_t *p_ = nullptr;
+    void *own_ = nullptr;
+};
+}  // namespace
 
 static int internal_fmt(int fmt) {
     switch (fmt) {
@@ -1115,9 +1188,9 @@ mynah_b200_qmat *mynah_b200_qmat_create(int fmt, const void *data, const float *
     if (cudaStreamCreateWithFlags(&tmp.stream, cudaStreamNonBlocking) != cudaSuccess) { set_error("cudaStreamCreate failed"); return nullptr; }
     mynah_b200_qmat *q = new mynah_b200_qmat();
     const bool planes = (k % 64) == 0;
-    tmp.status = q->status = (int *)tmp.dev_alloc(sizeof(int));
+    tmp.status = q->status = (int *)tmp.dev_alloc(QMAT_BLOCK);
     if (!q->status) { delete q; return nullptr; }
-    cudaMemset(q->status, 0, sizeof(int));
+    cudaMemset(q->status, 0, QMAT_HEAD);
     cudaDeviceSynchronize();
     if (tmp.upload_weight(q->w, f, data, scales, n, k, planes, false)) { delete q; return nullptr; }
     cudaDeviceSynchronize();
@@ -1135,32 +1208,46 @@ mynah_b200_qmat *mynah_b200_qmat_create(int fmt, const void *data, const float *
 
 void mynah_b200_qmat_free(mynah_b200_qmat *q) {
     if (!q) return;
-    for (void *p : q->owned) cudaFree(p);
+    for (void *p : q->owned) cudaFree(p);                       // waits for the handle's products
+    if (q->ws) cudaFree(q->ws);
     if (q->stream) cudaStreamDestroy(q->stream);
+    pinned_pool().give(q->host);
     delete q;
 }
+
+// device bytes of temporaries that a product of T rows needs beside its input and output
+static size_t qmat_temp_bytes(const QWeight &w, int T, int flags) {
+    if (flags & MYNAH_B200_A8)
+        return w.fmt == FMT_MYNAH_Q8 && T > 16 && w.k % 128 == 0 ? align_up((size_t)T * w.k, 256) + (size_t)T * 4 : 0;
+    if (T <= 16 && w.k <= 8192 && !(flags & MYNAH_B200_FEW_ROWS)) return 0;
+    return 2 * align_up((size_t)T * w.k * 2, 256);
+}
+
+static int qmat_mul_locked(const mynah_b200_qmat *q, const float *x, float *out, int T, int flags, uint8_t *temp);
 
 int mynah_b200_qmat_mul_device(const mynah_b200_qmat *q, const float *x, float *out, int T, int flags) {
     if (!q || !x || !out || T < 0) { set_error("qmat_mul: bad argument"); return -1; }
     if (T == 0) return 0;
+    std::lock_guard<std::mutex> lk(q->mu);
+    const size_t bytes = qmat_temp_bytes(q->w, T, flags);
+    QmatScratch s(q, bytes);
+    if (bytes && !s.get()) { set_error("qmat_mul: device allocation failed"); return -1; }
+    return qmat_mul_locked(q, x, out, T, flags, s.get());
+}
+
+static int qmat_mul_locked(const mynah_b200_qmat *q, const float *x, float *out, int T, int flags, uint8_t *temp) {
     const QWeight &w = q->w;
     if (flags & MYNAH_B200_A8) {
         if (w.fmt == FMT_MYNAH_Q8 && T > 16 && w.k % 128 == 0) {
             // many rows: the same integers on the tensor cores (bit-identical to the row-dot kernel below)
-            int8_t *qx = nullptr;
-            float *sx = nullptr;
-            MB_CUDA(cudaMallocAsync(&qx, (size_t)T * w.k, q->stream));
-            if (cudaMallocAsync(&sx, (size_t)T * sizeof(float), q->stream) != cudaSuccess) {
-                cudaGetLastError(); cudaFreeAsync(qx, q->stream); set_error("qmat_mul: device allocation failed"); return -1;
-            }
+            int8_t *qx = (int8_t *)temp;
+            float *sx = (float *)(temp + align_up((size_t)T * w.k, 256));
             GemmEpilogue e;
             memset(&e, 0, sizeof(e));
             e.mode = OUT_F32; e.act = ACT_NONE; e.alpha = 1.f; e.out = out; e.ldo = w.n;
             int rc = act_quant_rows(x, qx, sx, T, w.k, q->stream);
             if (rc == 0) rc = gemm_i8(qx, w.k, sx, reinterpret_cast<const int8_t *>(w.raw), w.k, w.scales, e, T, w.n, w.k, q->status, q->stream);
             if (rc == 0) note_launch(2);
-            cudaFreeAsync(qx, q->stream);
-            cudaFreeAsync(sx, q->stream);
             return rc;
         }
         const int rc = qgemv_a8(w, x, out, T, nullptr, nullptr, q->stream);
@@ -1186,11 +1273,7 @@ int mynah_b200_qmat_mul_device(const mynah_b200_qmat *q, const float *x, float *
         return rc;
     }
     if (!w.hi) { set_error("qmat_mul: the many-row path needs k %% 64 == 0 (k=%d) and weights below the fp16 operand limit 65504", w.k); return -1; }
-    __half *hi = nullptr, *lo = nullptr;
-    MB_CUDA(cudaMallocAsync(&hi, (size_t)T * w.k * 2, q->stream));
-    if (cudaMallocAsync(&lo, (size_t)T * w.k * 2, q->stream) != cudaSuccess) {
-        cudaGetLastError(); cudaFreeAsync(hi, q->stream); set_error("qmat_mul: device allocation failed"); return -1;
-    }
+    __half *hi = (__half *)temp, *lo = (__half *)(temp + align_up((size_t)T * w.k * 2, 256));
     int rc = split_to_h16(x, hi, lo, (size_t)T * w.k, q->stream, q->status);
     GemmEpilogue e;
     memset(&e, 0, sizeof(e));
@@ -1199,9 +1282,16 @@ int mynah_b200_qmat_mul_device(const mynah_b200_qmat *q, const float *x, float *
     if (rc == 0) rc = (flags & MYNAH_B200_FEW_ROWS) ? gemm_skinny(A, B, e, T, w.n, w.k, (flags & MYNAH_B200_FAST) ? 1 : 3, q->status, q->stream)
                                                     : gemm_tc(A, B, e, T, w.n, w.k, (flags & MYNAH_B200_FAST) ? 1 : 3, q->status, q->stream);
     if (rc == 0) note_launch(2);
-    cudaFreeAsync(hi, q->stream);
-    cudaFreeAsync(lo, q->stream);
     return rc;
+}
+
+static int qmat_status(const mynah_b200_qmat *q, int st) {
+    if (st == 0) return 0;
+    if (st == ST_RANGE) set_error("qmat: a value reached the fp16 operand range (|v| >= 65504) or was not finite");
+    else set_error("qmat: a bounded wait inside the contraction kernel ran out (code %d)", st);
+    cudaMemsetAsync(q->status, 0, sizeof(int), q->stream);
+    cudaStreamSynchronize(q->stream);
+    return -1;
 }
 
 int mynah_b200_qmat_sync(const mynah_b200_qmat *q) {
@@ -1209,31 +1299,32 @@ int mynah_b200_qmat_sync(const mynah_b200_qmat *q) {
     int st = 0;
     MB_CUDA(cudaMemcpyAsync(&st, q->status, sizeof(int), cudaMemcpyDeviceToHost, q->stream));
     MB_CUDA(cudaStreamSynchronize(q->stream));
-    if (st != 0) {
-        if (st == ST_RANGE) set_error("qmat: a value reached the fp16 operand range (|v| >= 65504) or was not finite");
-        else set_error("qmat: a bounded wait inside the contraction kernel ran out (code %d)", st);
-        cudaMemsetAsync(q->status, 0, sizeof(int), q->stream);
-        cudaStreamSynchronize(q->stream);
-        return -1;
-    }
-    return 0;
+    return qmat_status(q, st);
 }
 
 int mynah_b200_qmat_mul(const mynah_b200_qmat *q, const float *x, float *out, int T, int flags) {
     if (!q || !x || !out || T < 0) { set_error("qmat_mul: bad argument"); return -1; }
     if (T == 0) return 0;
-    float *xd = nullptr, *od = nullptr;
-    MB_CUDA(cudaMallocAsync(&xd, (size_t)T * q->w.k * 4, q->stream));
-    if (cudaMallocAsync(&od, (size_t)T * q->w.n * 4, q->stream) != cudaSuccess) {
-        cudaGetLastError(); cudaFreeAsync(xd, q->stream); set_error("qmat_mul: device allocation failed"); return -1;
-    }
-    int rc = 0;
-    if (cudaMemcpyAsync(xd, x, (size_t)T * q->w.k * 4, cudaMemcpyHostToDevice, q->stream) != cudaSuccess) { set_error("qmat_mul: H2D copy failed"); rc = -1; }
-    if (rc == 0) rc = mynah_b200_qmat_mul_device(q, xd, od, T, flags);
-    if (rc == 0 && cudaMemcpyAsync(out, od, (size_t)T * q->w.n * 4, cudaMemcpyDeviceToHost, q->stream) != cudaSuccess) { set_error("qmat_mul: D2H copy failed"); rc = -1; }
-    cudaFreeAsync(xd, q->stream);
-    cudaFreeAsync(od, q->stream);
-    if (mynah_b200_qmat_sync(q)) return -1;
+    std::lock_guard<std::mutex> lk(q->mu);
+    if (!q->host && !(q->host = pinned_pool().take())) { set_error("qmat_mul: host allocation failed"); return -1; }
+    const size_t nx = (size_t)T * q->w.k * 4, no = (size_t)T * q->w.n * 4;
+    uint8_t *block = (uint8_t *)q->status;
+    const bool small_x = nx <= QMAT_SMALL, small_out = no <= QMAT_SMALL;
+    const size_t nt = align_up(qmat_temp_bytes(q->w, T, flags), 256), nxw = small_x ? 0 : align_up(nx, 256);
+    QmatScratch s(q, nt + nxw + (small_out ? 0 : no));
+    if (nt + nxw + (small_out ? 0 : no) && !s.get()) { set_error("qmat_mul: device allocation failed"); return -1; }
+    float *xd = (float *)(small_x ? block + QMAT_HEAD + QMAT_SMALL : s.get() + nt);
+    float *od = (float *)(small_out ? block + QMAT_HEAD : s.get() + nt + nxw);
+    const void *src = x;
+    if (small_x) src = memcpy(q->host + QMAT_HEAD + QMAT_SMALL, x, nx);
+    if (cudaMemcpyAsync(xd, src, nx, cudaMemcpyHostToDevice, q->stream) != cudaSuccess) { cudaGetLastError(); set_error("qmat_mul: H2D copy failed"); return -1; }
+    const int rc = qmat_mul_locked(q, xd, od, T, flags, s.get());
+    bool copied = true;
+    if (rc == 0 && !small_out) copied = cudaMemcpyAsync(out, od, no, cudaMemcpyDeviceToHost, q->stream) == cudaSuccess;
+    copied = cudaMemcpyAsync(q->host, block, QMAT_HEAD + (small_out ? no : 0), cudaMemcpyDeviceToHost, q->stream) == cudaSuccess && copied;
+    if (cudaStreamSynchronize(q->stream) != cudaSuccess || !copied) { cudaGetLastError(); set_error("qmat_mul: D2H copy failed"); return -1; }
+    if (qmat_status(q, *(const int *)q->host)) return -1;
+    if (rc == 0 && small_out) memcpy(out, q->host + QMAT_HEAD, no);
     return rc;
 }
 
