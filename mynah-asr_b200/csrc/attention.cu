@@ -30,6 +30,7 @@ struct AttnDev {
     __half *ctx_hi, *ctx_lo;
     const int *seg_off, *seg_len, *rk_off;
     int d, H, left, right;
+    int ldkv, ldrk;                  // row strides of k / v and rk
     float scaling;
 };
 
@@ -46,12 +47,14 @@ __device__ __forceinline__ void window(const AttnDev &a, int t, int len, int &jl
 // tests as an on-device cross-check.
 __global__ void __launch_bounds__(128)
 attn_plain_kernel(AttnDev a, int max_len) {
+    chain_trigger();
+    chain_wait();
     const int b = blockIdx.z, h = blockIdx.y;
     const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int len = a.seg_len[b];
     if (t >= len) return;
     const int off = a.seg_off[b], dk = a.d / a.H, ho = h * dk;
-    const __half *rk = a.rk + (size_t)a.rk_off[b] * a.d;
+    const __half *rk = a.rk + (size_t)a.rk_off[b] * a.ldrk;
     const int per = dk / 32;   // dk in {32,64,96,128}
     float qu[4], qv[4], acc[4] = {0, 0, 0, 0};
     for (int i = 0; i < per; i++) {
@@ -63,14 +66,14 @@ attn_plain_kernel(AttnDev a, int max_len) {
     window(a, t, len, jlo, jhi);
     float m = -3.0e38f, l = 0.0f;
     for (int j = jlo; j < jhi; j++) {
-        const __half *kr = a.k + (size_t)(off + j) * a.d + ho + lane * per;
-        const __half *pr = rk + (size_t)(len - 1 + j - t) * a.d + ho + lane * per;
+        const __half *kr = a.k + (size_t)(off + j) * a.ldkv + ho + lane * per;
+        const __half *pr = rk + (size_t)(len - 1 + j - t) * a.ldrk + ho + lane * per;
         float s = 0.0f;
         for (int i = 0; i < per; i++) s += qu[i] * __half2float(kr[i]) + qv[i] * __half2float(pr[i]);
         s = warp_sum(s) * a.scaling;
         const float mn = fmaxf(m, s), corr = expf(m - mn), p = expf(s - mn);
         const float ph = __half2float(__float2half_rn(p));
-        const __half *vr = a.v + (size_t)(off + j) * a.d + ho + lane * per;
+        const __half *vr = a.v + (size_t)(off + j) * a.ldkv + ho + lane * per;
         l = l * corr + p;
         for (int i = 0; i < per; i++) acc[i] = acc[i] * corr + ph * __half2float(vr[i]);
         m = mn;
@@ -120,6 +123,8 @@ static constexpr int AT_Q = 64, AT_K = 64, AT_BDW = 80, AT_BDS = 81;
 template <int DK>
 __global__ void __launch_bounds__(128, 2)
 attn_tiled_kernel(AttnDev a) {
+    chain_trigger();
+    chain_wait();
     constexpr int LD = DK + 8;                       // padded fp16 row (conflict-free fragment loads)
     extern __shared__ __align__(16) uint8_t smem_at[];
     __half *Ks = reinterpret_cast<__half *>(smem_at);
@@ -131,7 +136,7 @@ attn_tiled_kernel(AttnDev a) {
     const int len = a.seg_len[b];
     if (tq0 >= len) return;
     const int off = a.seg_off[b], ho = h * DK;
-    const __half *rkg = a.rk + (size_t)a.rk_off[b] * a.d;
+    const __half *rkg = a.rk + (size_t)a.rk_off[b] * a.ldrk;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     float *BDw = BD + warp * 16 * AT_BDS;
 
@@ -183,18 +188,18 @@ attn_tiled_kernel(AttnDev a) {
         for (int i = threadIdx.x; i < AT_K * CPR; i += 128) {
             const int r = i / CPR, c = (i % CPR) * 8;
             const bool ok = j0 + r < len;
-            cp_async16_zfill(Ks + r * LD + c, a.k + (size_t)(off + (ok ? j0 + r : 0)) * a.d + ho + c, ok);
+            cp_async16_zfill(Ks + r * LD + c, a.k + (size_t)(off + (ok ? j0 + r : 0)) * a.ldkv + ho + c, ok);
         }
         for (int i = threadIdx.x; i < 128 * CPR; i += 128) {
             const int r = i / CPR, c = (i % CPR) * 8, p = pbase + r;
             const bool ok = p >= 0 && p <= 2 * len - 2;
-            cp_async16_zfill(Rs + r * LD + c, rkg + (size_t)(ok ? p : 0) * a.d + ho + c, ok);
+            cp_async16_zfill(Rs + r * LD + c, rkg + (size_t)(ok ? p : 0) * a.ldrk + ho + c, ok);
         }
         cp_async_commit();
         for (int i = threadIdx.x; i < AT_K * CPR; i += 128) {
             const int r = i / CPR, c = (i % CPR) * 8;
             const bool ok = j0 + r < len;
-            cp_async16_zfill(Vs + r * LD + c, a.v + (size_t)(off + (ok ? j0 + r : 0)) * a.d + ho + c, ok);
+            cp_async16_zfill(Vs + r * LD + c, a.v + (size_t)(off + (ok ? j0 + r : 0)) * a.ldkv + ho + c, ok);
         }
         cp_async_commit();
         cp_async_wait<1>();
@@ -323,7 +328,7 @@ attn_tiled_kernel(AttnDev a) {
 }
 
 template <int DK>
-static int launch_tiled(const AttnDev &dv, int batch, int max_len, cudaStream_t st) {
+static int launch_tiled(const AttnDev &dv, int batch, int max_len, cudaStream_t st, bool chain) {
     constexpr int LD = DK + 8;
     const int smem = (2 * AT_K + 128) * LD * 2 + 4 * 16 * AT_BDS * 4;
     static PerDevice configured = {};
@@ -333,8 +338,7 @@ static int launch_tiled(const AttnDev &dv, int batch, int max_len, cudaStream_t 
         configured.record(dev, (size_t)smem);
     }
     dim3 grid(cdiv(max_len, AT_Q), dv.H, batch);
-    attn_tiled_kernel<DK><<<grid, 128, smem, st>>>(dv);
-    MB_CUDA(cudaGetLastError());
+    MB_CUDA(launch_kernel(attn_tiled_kernel<DK>, grid, dim3(128), (size_t)smem, st, chain, 1, dv));
     return 0;
 }
 
@@ -346,16 +350,16 @@ int attention_forward(const AttnArgs &a, int impl, cudaStream_t st) {
     dv.bias_u = a.bias_u; dv.bias_v = a.bias_v; dv.ctx_f32 = a.ctx_f32;
     dv.ctx_hi = a.ctx_h.hi; dv.ctx_lo = a.ctx_h.lo;
     dv.seg_off = a.seg_off; dv.seg_len = a.seg_len; dv.rk_off = a.rk_off;
+    dv.ldkv = a.ldkv ? a.ldkv : a.d; dv.ldrk = a.ldrk ? a.ldrk : a.d;
     dv.d = a.d; dv.H = a.H; dv.left = a.left; dv.right = a.right;
     dv.scaling = 1.0f / sqrtf((float)dk);
     if (impl == 0 && attention_tc_eligible(a)) return attention_tc(a, st);
-    if ((impl == 0 || impl == 2) && (dk == 64 || dk == 128) && (a.ldq % 2) == 0 && (a.d % 8) == 0) {
-        return dk == 64 ? launch_tiled<64>(dv, a.batch, a.max_len, st) : launch_tiled<128>(dv, a.batch, a.max_len, st);
+    if ((impl == 0 || impl == 2) && (dk == 64 || dk == 128) && (a.ldq % 2) == 0 && (a.d % 8) == 0 && (a.ldkv % 8) == 0 && (a.ldrk % 8) == 0) {
+        return dk == 64 ? launch_tiled<64>(dv, a.batch, a.max_len, st, a.chain) : launch_tiled<128>(dv, a.batch, a.max_len, st, a.chain);
     }
     if (dk % 32 != 0 || dk > 128) { set_error("attention: head dim %d unsupported", dk); return -1; }
     dim3 grid(cdiv(a.max_len, 4), a.H, a.batch);
-    attn_plain_kernel<<<grid, 128, 0, st>>>(dv, a.max_len);
-    MB_CUDA(cudaGetLastError());
+    MB_CUDA(launch_kernel(attn_plain_kernel, grid, dim3(128), 0, st, a.chain, 1, dv, a.max_len));
     return 0;
 }
 

@@ -109,6 +109,7 @@ __global__ void __launch_bounds__(TA_THREADS, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                const __grid_constant__ CUtensorMap tmR, const AttnTcDev a) {
     const int b = blockIdx.z, h = blockIdx.y, t0 = blockIdx.x * TA_Q;
+    chain_wait();
     const int len = a.seg_len[b];
     if (t0 >= len) return;                                   // the whole CTA leaves before any barrier exists
     extern __shared__ uint8_t ta_smem_raw[];
@@ -151,6 +152,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_trigger();
 
     if (warp == TA_W_TMA) {
         if (lane == 0) {
@@ -429,8 +431,8 @@ typedef CUresult (*TaEncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, v
                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// fp16 [rows, d] row-major: boxes of 64 rows x 64 columns, 128-byte swizzle, zeros outside the tensor
-static int ta_make_map(CUtensorMap *m, const __half *base, long long rows, int d) {
+// fp16 [rows, d] row-major, row stride ld: boxes of 64 rows x 64 columns, 128-byte swizzle, zeros outside the tensor
+static int ta_make_map(CUtensorMap *m, const __half *base, long long rows, int d, int ld) {
     static TaEncodeFn fn = nullptr;
     if (!fn) {
         void *p = nullptr;
@@ -440,7 +442,7 @@ static int ta_make_map(CUtensorMap *m, const __half *base, long long rows, int d
     }
     if (!fn) { set_error("cuTensorMapEncodeTiled entry point unavailable"); return -1; }
     cuuint64_t dims[2] = {(cuuint64_t)d, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)d * 2};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
     cuuint32_t box[2] = {64, (cuuint32_t)TA_K};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(base), dims, strides, box, estr,
@@ -451,14 +453,15 @@ static int ta_make_map(CUtensorMap *m, const __half *base, long long rows, int d
 }
 
 bool attention_tc_eligible(const AttnArgs &a) {
-    return a.left < 0 && a.H > 0 && a.d / a.H == TA_DK && a.d % 8 == 0 && a.ldq % 4 == 0 && a.rows > 0 && a.rk_rows > 0 &&
+    return a.left < 0 && a.H > 0 && a.d / a.H == TA_DK && a.d % 8 == 0 && a.ldkv % 8 == 0 && a.ldrk % 8 == 0 && a.ldq % 4 == 0 && a.rows > 0 && a.rk_rows > 0 &&
            a.status != nullptr && (reinterpret_cast<uintptr_t>(a.k) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.v) & 15) == 0 &&
            (reinterpret_cast<uintptr_t>(a.rk) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.q) & 15) == 0;
 }
 
 int attention_tc(const AttnArgs &a, cudaStream_t st) {
     CUtensorMap tk, tv, tr;
-    if (ta_make_map(&tk, a.k, a.rows, a.d) || ta_make_map(&tv, a.v, a.rows, a.d) || ta_make_map(&tr, a.rk, a.rk_rows, a.d)) return -1;
+    const int ldkv = a.ldkv ? a.ldkv : a.d, ldrk = a.ldrk ? a.ldrk : a.d;
+    if (ta_make_map(&tk, a.k, a.rows, a.d, ldkv) || ta_make_map(&tv, a.v, a.rows, a.d, ldkv) || ta_make_map(&tr, a.rk, a.rk_rows, a.d, ldrk)) return -1;
     static PerDevice configured = {};
     int dev = 0;
     if (configured.below((size_t)TA_SMEM, &dev)) {
@@ -471,8 +474,7 @@ int attention_tc(const AttnArgs &a, cudaStream_t st) {
     dv.seg_off = a.seg_off; dv.seg_len = a.seg_len; dv.rk_off = a.rk_off;
     dv.d = a.d; dv.scale2 = 1.4426950408889634f / sqrtf((float)TA_DK); dv.status = a.status;
     dim3 grid(cdiv(a.max_len, TA_Q), a.H, a.batch);
-    attn_tc_kernel<<<grid, TA_THREADS, TA_SMEM, st>>>(tk, tv, tr, dv);
-    MB_CUDA(cudaGetLastError());
+    MB_CUDA(launch_kernel(attn_tc_kernel, grid, dim3(TA_THREADS), (size_t)TA_SMEM, st, a.chain, 1, tk, tv, tr, dv));
     return 0;
 }
 

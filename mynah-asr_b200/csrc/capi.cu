@@ -76,7 +76,8 @@ private:
         for (int i = 0; i < Model::DEC_LANES; i++) { c->lane[i] = nullptr; c->lane_done[i] = nullptr; }
         c->lane_fork = nullptr;
         c->prof_spans.clear(); c->prof_used = 0; c->prof_on = false;
-        c->ws = Arena();
+        c->ws = Arena(); c->host_stage = HostStage();
+        c->copy = nullptr; c->copy_ev.clear();
         c->stream = nullptr; c->status = nullptr;
         if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); delete c; return nullptr; }
         c->status = (int *)c->dev_alloc(sizeof(int));
@@ -339,6 +340,47 @@ static int lin(Model &m, QWeight &w, const std::string &wname, bool planes, bool
     return err ? -1 : 0;
 }
 
+// q, k and v of a layer read the same rows: their operands (planes, or natively quantised bytes and scales) get one block,
+// so that L.qkv is all three as one [3 d, d] weight and q_w, k_w, v_w are parts of it
+static int place_qkv(Model &m, EncLayer &L, const std::string &p) {
+    const char *names[3] = {"q_proj", "k_proj", "v_proj"};
+    const int d = m.d_model;
+    const size_t dd = (size_t)d * d;
+    bool native8 = true;
+    for (const char *nm : names) {
+        const HostTensor *t = find(m, p + "self_attn." + nm + ".weight");
+        if (!t || t->shape.empty()) { set_error("missing tensor '%sself_attn.%s.weight'", p.c_str(), nm); return -1; }
+        if (t->shape[0] != d || t->nelem() != dd) { set_error("'%sself_attn.%s.weight' is not [%d, %d]", p.c_str(), nm, d, d); return -1; }
+        native8 = native8 && t->fmt == FMT_MYNAH_Q8;
+    }
+    QWeight &w = L.qkv;
+    w.n = 3 * d; w.k = d;
+    w.hi = (__half *)m.dev_alloc(3 * dd * 2); w.lo = (__half *)m.dev_alloc(3 * dd * 2);
+    if (!w.hi || !w.lo) return -1;
+    if (native8) {
+        w.fmt = FMT_MYNAH_Q8;
+        w.raw = (uint8_t *)m.dev_alloc(3 * dd + 64); w.scales = (float *)m.dev_alloc(3 * (size_t)d * 4);
+        if (!w.raw || !w.scales) return -1;
+    }
+    QWeight *parts[3] = {&L.q_w, &L.k_w, &L.v_w};
+    for (int i = 0; i < 3; i++) {
+        parts[i]->hi = w.hi + i * dd; parts[i]->lo = w.lo + i * dd;
+        if (native8) { parts[i]->raw = w.raw + i * dd; parts[i]->scales = w.scales + (size_t)i * d; }
+    }
+    return 0;
+}
+static int finish_qkv(Model &m, EncLayer &L) {
+    const int d = m.d_model;
+    const float *b[3] = {L.q_w.bias, L.k_w.bias, L.v_w.bias};
+    if (!b[0] && !b[1] && !b[2]) return 0;
+    L.qkv.bias = (float *)m.dev_alloc(3 * (size_t)d * 4);
+    if (!L.qkv.bias) return -1;
+    MB_CUDA(cudaMemsetAsync(L.qkv.bias, 0, 3 * (size_t)d * 4, m.stream));
+    for (int i = 0; i < 3; i++)
+        if (b[i]) MB_CUDA(cudaMemcpyAsync(L.qkv.bias + (size_t)i * d, b[i], (size_t)d * 4, cudaMemcpyDeviceToDevice, m.stream));
+    return 0;
+}
+
 // several linears over the same input, stored one below the other: [sum n, k] with the biases concatenated
 // (block formats keep whole rows of blocks, so the stored bytes concatenate as they are)
 static int lin_cat(Model &m, QWeight &w, const float **bias, const std::vector<std::string> &prefixes) {
@@ -414,6 +456,10 @@ int mynah_b200_model_finalize(mynah_b200_model *h) {
     m.n_layers = nl;
     m.layers.resize(nl);
     const bool bn = find(m, "encoder.layers.0.conv.norm.running_mean") != nullptr;
+    // the layers' rel-pos projections sit one below the other ([layers d, d]): one contraction makes the keys of all layers
+    const size_t dd = (size_t)m.d_model * m.d_model;
+    __half *relk_hi = (__half *)m.dev_alloc(nl * dd * 2), *relk_lo = (__half *)m.dev_alloc(nl * dd * 2);
+    if (!relk_hi || !relk_lo) return -1;
     for (int li = 0; li < nl; li++) {
         EncLayer &L = m.layers[li];
         const std::string p = "encoder.layers." + std::to_string(li) + ".";
@@ -441,12 +487,15 @@ int mynah_b200_model_finalize(mynah_b200_model *h) {
             L.cnorm_shift = m.upload_f32(sh.data(), m.d_model);
             if (!L.cnorm_scale || !L.cnorm_shift) return -1;
         }
+        L.relk.hi = relk_hi + li * dd; L.relk.lo = relk_lo + li * dd;
+        if (place_qkv(m, L, p)) return -1;
         if (lin(m, L.ff1_w1, p + "feed_forward1.linear1.weight", true, false) || lin(m, L.ff1_w2, p + "feed_forward1.linear2.weight", true, false) ||
             lin(m, L.ff2_w1, p + "feed_forward2.linear1.weight", true, false) || lin(m, L.ff2_w2, p + "feed_forward2.linear2.weight", true, false) ||
             lin(m, L.q_w, p + "self_attn.q_proj.weight", true, false) || lin(m, L.k_w, p + "self_attn.k_proj.weight", true, false) ||
             lin(m, L.v_w, p + "self_attn.v_proj.weight", true, false) || lin(m, L.o_w, p + "self_attn.o_proj.weight", true, false) ||
             lin(m, L.relk, p + "self_attn.relative_k_proj.weight", true, false) ||
-            lin(m, L.pw1_w, p + "conv.pointwise_conv1.weight", true, false) || lin(m, L.pw2_w, p + "conv.pointwise_conv2.weight", true, false))
+            lin(m, L.pw1_w, p + "conv.pointwise_conv1.weight", true, false) || lin(m, L.pw2_w, p + "conv.pointwise_conv2.weight", true, false) ||
+            finish_qkv(m, L))
             return -1;
     }
     m.ffn_dim = m.layers[0].ff1_w1.n;
@@ -626,37 +675,16 @@ void mynah_b200_model_load_stats(const mynah_b200_model *h, double *seconds, dou
 }  // extern "C"
 
 // -------------------------------------------------------------- workspace sizes
-static size_t ss_bytes(const Model &m, int t_mel) {
-    const int C = m.channels;
-    const size_t T1 = Model::sub_len(t_mel, m.causal), F1 = Model::sub_len(m.cfg.n_mels, m.causal);
-    const size_t T2 = Model::sub_len((int)T1, m.causal), F2 = Model::sub_len((int)F1, m.causal);
-    const size_t T3 = Model::sub_len((int)T2, m.causal), F3 = Model::sub_len((int)F2, m.causal);
-    return T1 * F1 * C * 4 + T2 * F2 * C * 8 + T3 * F3 * C * 8 + (1 << 16);
-}
-static size_t enc_bytes(const Model &m, size_t M, size_t rk_rows) {
-    return M * ((size_t)m.d_model * 44 + (size_t)m.ffn_dim * 4) + rk_rows * m.d_model * 6 + (1 << 20) +
+static size_t enc_bytes(const Model &m, size_t M, size_t max_len) {
+    const size_t rk_rows = 2 * max_len + 1;
+    return M * ((size_t)m.d_model * 44 + (size_t)m.ffn_dim * 4) +
+           rk_rows * m.d_model * (4 + 2 * (size_t)m.rk_layers((int)rk_rows, m.n_layers)) + (1 << 20) +
            (m.a8_layers ? M * ((size_t)m.d_model + 5 * (size_t)m.ffn_dim + 64) + 4096 : 0);
 }
+static size_t stage_bytes(int batch) { return (size_t)batch * (sizeof(FrontItem) + 16) + 4096; }
 static size_t dec_bytes(const Model &m, int max_len) {
     const size_t B = DEC_MAX_B;
     return (size_t)max_len * m.cfg.max_symbols * B * 8 + B * 148 * 8 * 16 + 4 * (size_t)DEC_MAX_LAYERS * B * 1024 * 4 + B * (size_t)m.pred_hidden * 4 + (1 << 20);
-}
-
-// Full device pipeline for a packed batch whose mel features are already on the
-// device: subsampling per item, layer stack on the packed rows, projector.
-// x_out receives [sum T, d_model]; returns lens.
-static int encode_batch_dev(Model &m, const std::vector<const float *> &feats_dev, const std::vector<int> &t_mel, int left,
-                            int right, float *x, std::vector<int> &lens) {
-    const int B = (int)t_mel.size();
-    lens.resize(B);
-    int off = 0;
-    for (int b = 0; b < B; b++) {
-        int t = 0;
-        if (t_mel[b] > 0 && m.subsample_item(feats_dev[b], t_mel[b], x + (size_t)off * m.d_model, &t)) return -1;
-        lens[b] = t;
-        off += t;
-    }
-    return m.encoder_layers(x, lens, left, right, 0, m.n_layers);
 }
 
 extern "C" {
@@ -685,12 +713,12 @@ float *mynah_b200_subsampling_forward(mynah_b200_model *h, const float *feats, i
     Lease lease(h);
     Model &m = lease.model();
     const int T3 = m.enc_len(T);
-    if (m.ws.reserve(ss_bytes(m, T) + (size_t)T * n_mels * 4 + (size_t)T3 * m.d_model * 4 + (1 << 20))) return nullptr;
+    if (m.ws.reserve(m.front_bytes(nullptr, &T, 1, false, true) + (size_t)T3 * m.d_model * 4 + (1 << 20)) || m.host_stage.begin(stage_bytes(1))) return nullptr;
     m.ws.reset();
-    float *f = m.ws.get<float>((size_t)T * n_mels), *x = m.ws.get<float>((size_t)T3 * m.d_model);
-    MB_CUDA_NULL(cudaMemcpyAsync(f, feats, (size_t)T * n_mels * 4, cudaMemcpyHostToDevice, m.stream));
-    int t = 0;
-    if (m.subsample_item(f, T, x, &t) || m.check_status("subsampling")) return nullptr;
+    float *x = m.ws.get<float>((size_t)T3 * m.d_model);
+    std::vector<int> lens;
+    if (!x || m.front_end(nullptr, nullptr, &feats, &T, 1, true, x, lens) || m.check_status("subsampling")) return nullptr;
+    const int t = lens[0];
     float *out = (float *)malloc((size_t)t * m.d_model * sizeof(float));
     if (!out) { set_error("out of host memory"); return nullptr; }
     MB_CUDA_NULL(cudaMemcpyAsync(out, x, (size_t)t * m.d_model * 4, cudaMemcpyDeviceToHost, m.stream));
@@ -703,7 +731,7 @@ int mynah_b200_encoder_layer(mynah_b200_model *h, int li, float *x, int T, int l
     if (!h || !h->m.finalized || !x || T <= 0 || li < 0 || li >= h->m.n_layers) { set_error("encoder_layer: bad argument"); return -1; }
     Lease lease(h);
     Model &m = lease.model();
-    if (m.ws.reserve(enc_bytes(m, T, 2 * T - 1) + (size_t)T * m.d_model * 4)) return -1;
+    if (m.ws.reserve(enc_bytes(m, T, T) + (size_t)T * m.d_model * 4) || m.host_stage.begin(stage_bytes(1))) return -1;
     m.ws.reset();
     float *xd = m.ws.get<float>((size_t)T * m.d_model);
     MB_CUDA(cudaMemcpyAsync(xd, x, (size_t)T * m.d_model * 4, cudaMemcpyHostToDevice, m.stream));
@@ -719,25 +747,20 @@ int mynah_b200_encoder_forward_batch(mynah_b200_model *h, const float *const *fe
     if (!h || !h->m.finalized || batch <= 0 || n_mels != h->m.cfg.n_mels) { set_error("encoder_forward_batch: bad argument"); return -1; }
     Lease lease(h);
     Model &m = lease.model();
-    size_t M = 0, rk = 0, fbytes = 0, ssmax = 0;
+    size_t M = 0, max_len = 0;
     for (int b = 0; b < batch; b++) {
         const size_t t = t_mel[b] > 0 ? m.enc_len(t_mel[b]) : 0;
-        M += t; rk += 2 * t; fbytes += align_up((size_t)t_mel[b] * n_mels * 4, 256) + 256;
-        if (t_mel[b] > 0 && ss_bytes(m, t_mel[b]) > ssmax) ssmax = ss_bytes(m, t_mel[b]);
+        M += t;
+        if (t > max_len) max_len = t;
     }
-    if (m.ws.reserve(fbytes + ssmax + enc_bytes(m, M, rk) + M * ((size_t)m.d_model + m.d_out) * 4 + (1 << 20))) return -1;
+    if (m.ws.reserve(m.front_bytes(nullptr, t_mel, batch, false, true) + enc_bytes(m, M, max_len) + M * ((size_t)m.d_model + m.d_out) * 4 + (1 << 20)) ||
+        m.host_stage.begin(stage_bytes(batch)))
+        return -1;
     m.ws.reset();
-    std::vector<const float *> fd(batch);
-    std::vector<int> tm(t_mel, t_mel + batch), lens;
-    for (int b = 0; b < batch; b++) {
-        float *f = m.ws.get<float>((size_t)(t_mel[b] > 0 ? t_mel[b] : 1) * n_mels);
-        if (!f) return -1;
-        if (t_mel[b] > 0) MB_CUDA(cudaMemcpyAsync(f, feats[b], (size_t)t_mel[b] * n_mels * 4, cudaMemcpyHostToDevice, m.stream));
-        fd[b] = f;
-    }
+    std::vector<int> lens;
     float *x = m.ws.get<float>((M ? M : 1) * m.d_model), *y = m.ws.get<float>((M ? M : 1) * m.d_out);
     if (!x || !y) return -1;
-    if (encode_batch_dev(m, fd, tm, left, right, x, lens)) return -1;
+    if (m.front_end(nullptr, nullptr, feats, t_mel, batch, true, x, lens) || m.encoder_layers(x, lens, left, right, 0, m.n_layers)) return -1;
     if (m.encoder_post(x, lens, prompt_ids, y) || m.check_status("encoder_forward_batch")) return -1;
     size_t off = 0;
     for (int b = 0; b < batch; b++) {
@@ -757,14 +780,14 @@ static float *forward_one(mynah_b200_model *h, const float *feats, int t_mel, in
     Lease lease(h);
     Model &m = lease.model();
     const size_t M = m.enc_len(t_mel);
-    if (m.ws.reserve((size_t)t_mel * n_mels * 4 + ss_bytes(m, t_mel) + enc_bytes(m, M, 2 * M) + M * ((size_t)m.d_model + m.d_out) * 4 + (1 << 20))) return nullptr;
+    if (m.ws.reserve(m.front_bytes(nullptr, &t_mel, 1, false, true) + enc_bytes(m, M, M) + M * ((size_t)m.d_model + m.d_out) * 4 + (1 << 20)) ||
+        m.host_stage.begin(stage_bytes(1)))
+        return nullptr;
     m.ws.reset();
-    float *f = m.ws.get<float>((size_t)t_mel * n_mels), *x = m.ws.get<float>(M * m.d_model), *y = m.ws.get<float>(M * m.d_out);
-    if (!f || !x || !y) return nullptr;
-    MB_CUDA_NULL(cudaMemcpyAsync(f, feats, (size_t)t_mel * n_mels * 4, cudaMemcpyHostToDevice, m.stream));
-    std::vector<const float *> fd{f};
-    std::vector<int> tm{t_mel}, lens;
-    if (encode_batch_dev(m, fd, tm, left, right, x, lens)) return nullptr;
+    float *x = m.ws.get<float>(M * m.d_model), *y = m.ws.get<float>(M * m.d_out);
+    if (!x || !y) return nullptr;
+    std::vector<int> lens;
+    if (m.front_end(nullptr, nullptr, &feats, &t_mel, 1, true, x, lens) || m.encoder_layers(x, lens, left, right, 0, m.n_layers)) return nullptr;
     const int wout = raw ? m.d_model : m.d_out;
     if (!raw && m.encoder_post(x, lens, &prompt_id, y)) return nullptr;
     if (m.check_status("encoder_forward")) return nullptr;
@@ -1043,47 +1066,31 @@ void mynah_b200_batch_free(mynah_b200_batch *bt) {
 // on the hot path). Caller holds the model lock.
 static int run_batch_locked(Model &m, mynah_b200_batch *bt, const float *const *audio_dev, const float *const *audio_host,
                             int decoder) {
-    const int B = bt->batch, nm = m.cfg.n_mels, hop = m.cfg.hop_length;
-    size_t M = 0, rk = 0, fbytes = 0, ssmax = 0, abytes = 0;
+    const int B = bt->batch, hop = m.cfg.hop_length;
+    size_t M = 0;
     int max_len = 0;
-    std::vector<int> tmel(B), valid(B);
+    std::vector<int> valid(B);
     for (int b = 0; b < B; b++) {
-        tmel[b] = 1 + (int)(bt->n_samples[b] / hop); valid[b] = (int)(bt->n_samples[b] / hop);
+        valid[b] = (int)(bt->n_samples[b] / hop);
         const int t = valid[b] > 0 ? m.enc_len(valid[b]) : 0;
-        M += t; rk += 2 * (size_t)t; if (t > max_len) max_len = t;
-        fbytes += align_up((size_t)tmel[b] * nm * 4, 256) + 256;
-        abytes += align_up(bt->n_samples[b] * 4, 256) + 256;
-        if (valid[b] > 0 && ss_bytes(m, valid[b]) > ssmax) ssmax = ss_bytes(m, valid[b]);
+        M += t; if (t > max_len) max_len = t;
     }
     if (decoder == 2 && (!m.has_aed || bt->aed_prompt.empty())) { set_error("batch_run: AED decoding needs an AED model and mynah_b200_batch_set_aed"); return -1; }
     int aed_len = (int)bt->aed_prompt.size() + max_len + bt->aed_delta;
     if (decoder == 2 && aed_len > m.aed_max_seq) aed_len = m.aed_max_seq;
     const size_t decb = decoder == 1 ? M * ((size_t)m.d_model * 4 + (size_t)m.ctc_vocab * 4 + 8)
                       : decoder == 2 ? m.aed_bytes((int)M, B, aed_len) : dec_bytes(m, max_len);
-    if (m.ws.reserve((audio_host ? abytes : 0) + fbytes + ssmax + enc_bytes(m, M, rk) + M * ((size_t)m.d_model + m.d_out) * 4 +
-                     decb + (4 << 20))) return -1;
+    if (m.ws.reserve(m.front_bytes(bt->n_samples.data(), valid.data(), B, true, audio_host != nullptr) + enc_bytes(m, M, max_len) +
+                     M * ((size_t)m.d_model + m.d_out) * 4 + decb + (4 << 20)) ||
+        m.host_stage.begin(stage_bytes(B)))
+        return -1;
     m.ws.reset();
-    std::vector<const float *> ad(B), fd(B);
-    for (int b = 0; b < B; b++) {
-        if (audio_host) {
-            float *a = m.ws.get<float>(bt->n_samples[b] ? bt->n_samples[b] : 1);
-            if (!a) return -1;
-            MB_CUDA(cudaMemcpyAsync(a, audio_host[b], bt->n_samples[b] * sizeof(float), cudaMemcpyHostToDevice, m.stream));
-            ad[b] = a;
-        } else {
-            ad[b] = audio_dev[b];
-        }
-    }
-    for (int b = 0; b < B; b++) {
-        float *f = m.ws.get<float>((size_t)tmel[b] * nm);
-        if (!f) return -1;
-        if (m.log_mel(ad[b], bt->n_samples[b], f, tmel[b], valid[b])) return -1;
-        fd[b] = f;
-    }
     float *x = m.ws.get<float>((M ? M : 1) * m.d_model), *y = m.ws.get<float>((M ? M : 1) * m.d_out);
     if (!x || !y) return -1;
     std::vector<int> lens;
-    if (encode_batch_dev(m, fd, valid, m.cfg.left_ctx, m.cfg.right_ctx, x, lens)) return -1;
+    if (m.front_end(audio_host ? audio_host : audio_dev, bt->n_samples.data(), nullptr, valid.data(), B, audio_host != nullptr, x, lens) ||
+        m.encoder_layers(x, lens, m.cfg.left_ctx, m.cfg.right_ctx, 0, m.n_layers))
+        return -1;
     bt->tokens.assign(B, {}); bt->frames.assign(B, {});
     if (decoder == 1) {
         size_t off = 0;

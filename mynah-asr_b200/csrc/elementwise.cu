@@ -125,6 +125,8 @@ glu_dw_kernel(const float *__restrict__ h2, const float *__restrict__ dw_w, cons
               __half *__restrict__ hi, __half *__restrict__ lo, const int *__restrict__ seg_off,
               const int *__restrict__ seg_len, int d, int k, int pad_left) {
     __shared__ float4 g[(DW_TT + DW_KMAX - 1) * (DW_CH / 4)];
+    chain_trigger();
+    chain_wait();
     const int b = blockIdx.z;
     const int len = seg_len[b], off = seg_off[b];
     const int t0 = blockIdx.y * DW_TT;
@@ -192,18 +194,13 @@ glu_dw_kernel(const float *__restrict__ h2, const float *__restrict__ dw_w, cons
 
 int glu_dwconv(const float *h2, const float *dw_w, const float *dw_b, const float *scale, const float *shift,
                float *out_f32, H16 out_h, const int *seg_off, const int *seg_len, int batch, int max_len, int d,
-               int k, int pad_left, cudaStream_t st) {
+               int k, int pad_left, cudaStream_t st, bool chain) {
     if (batch <= 0 || max_len <= 0) return 0;
     if (k > DW_KMAX) { set_error("glu_dwconv: kernel width %d > %d", k, DW_KMAX); return -1; }
     if (d % 4) { set_error("glu_dwconv: d=%d must be a multiple of 4", d); return -1; }
     dim3 grid(cdiv(d, DW_CH), cdiv(max_len, DW_TT), batch);
-    if (k == 9)
-        glu_dw_kernel<9><<<grid, dim3(32, DW_TY), 0, st>>>(h2, dw_w, dw_b, scale, shift, out_f32, out_h.hi, out_h.lo, seg_off,
-                                                 seg_len, d, k, pad_left);
-    else
-        glu_dw_kernel<0><<<grid, dim3(32, DW_TY), 0, st>>>(h2, dw_w, dw_b, scale, shift, out_f32, out_h.hi, out_h.lo, seg_off,
-                                                 seg_len, d, k, pad_left);
-    MB_CUDA(cudaGetLastError());
+    MB_CUDA(launch_kernel(k == 9 ? glu_dw_kernel<9> : glu_dw_kernel<0>, grid, dim3(32, DW_TY), 0, st, chain, 1, h2, dw_w, dw_b, scale, shift,
+                          out_f32, out_h.hi, out_h.lo, seg_off, seg_len, d, k, pad_left));
     return 0;
 }
 

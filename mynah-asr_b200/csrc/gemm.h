@@ -29,6 +29,10 @@ struct GemmEpilogue {
     __half *out_hi;      // fp16 planes (OUT_H16 / OUT_F32_H16)
     __half *out_lo;
     int ldh;
+    // Column split (0 = none, else a multiple of 32): columns from n_split on leave as fp16 planes, column n at
+    // out_hi[m, n - n_split], whatever `mode` (OUT_F32) does with the columns before. q | k | v of one attention as one
+    // contraction: q stays f32, k and v become the operands of the attention kernel.
+    int n_split = 0;
     // Optional LayerNorm of the finished rows (few-row kernel only; the other kernels ignore it): when the last tile of
     // row m has been written to `out`, that row (ldo == N, one of ln_row's widths) is normalised by the CTA that
     // completed it — the LayerNorm that follows a residual update, without a launch of its own.
@@ -48,6 +52,10 @@ struct GemmEpilogue {
 static constexpr int GEMM_BM = 128;      // rows of an output tile (one tcgen05.mma M)
 
 #ifdef __CUDACC__
+// what happens to the 32 columns from nb on, and where column nb's planes start
+__device__ __forceinline__ int gemm_mode(const GemmEpilogue &ep, int nb) { return ep.n_split && nb >= ep.n_split ? (int)OUT_H16 : ep.mode; }
+__device__ __forceinline__ int gemm_plane_col(const GemmEpilogue &ep, int nb) { return ep.n_split ? nb - ep.n_split : nb; }
+
 // Work units of the persistent loop. Whole waves of gridDim.x tiles come first; the tiles of the last, partial
 // wave are cut into 2 or 4 column strips when that still fits one wave, so that the tail costs a half or a
 // quarter of a tile time instead of a whole one (752 tiles on 148 CTAs: 5.25 instead of 6 tile times). A strip
@@ -79,7 +87,7 @@ struct GemmUnits {
 // Returns false if a value written as fp16 planes was out of their range (see split_h16).
 __device__ __forceinline__ bool gemm_epilogue_row(const GemmEpilogue &ep, float (&v)[32], int m, int nb, int N) {
     bool fits = true;
-    const int nvalid = N - nb < 32 ? N - nb : 32;
+    const int nvalid = N - nb < 32 ? N - nb : 32, mode = gemm_mode(ep, nb), nh = gemm_plane_col(ep, nb);
 #pragma unroll
     for (int j = 0; j < 32; j++) {
         float x = v[j];
@@ -88,10 +96,10 @@ __device__ __forceinline__ bool gemm_epilogue_row(const GemmEpilogue &ep, float 
         else if (ep.act == ACT_RELU) x = fmaxf(x, 0.0f);
         v[j] = x;
     }
-    if (ep.mode != OUT_H16) {
+    if (mode != OUT_H16) {
         float *o = ep.out + (size_t)m * ep.ldo + nb;
         const bool vec = nvalid == 32 && ((reinterpret_cast<uintptr_t>(o) & 15) == 0);
-        if (ep.mode == OUT_RESID) {
+        if (mode == OUT_RESID) {
             if (vec) {
 #pragma unroll
                 for (int j = 0; j < 32; j += 4) {
@@ -115,9 +123,9 @@ __device__ __forceinline__ bool gemm_epilogue_row(const GemmEpilogue &ep, float 
             }
         }
     }
-    if (ep.mode == OUT_H16 || ep.mode == OUT_F32_H16) {
-        __half *ph = ep.out_hi + (size_t)m * ep.ldh + nb;
-        __half *pl = ep.out_lo ? ep.out_lo + (size_t)m * ep.ldh + nb : nullptr;
+    if (mode == OUT_H16 || mode == OUT_F32_H16) {
+        __half *ph = ep.out_hi + (size_t)m * ep.ldh + nh;
+        __half *pl = ep.out_lo ? ep.out_lo + (size_t)m * ep.ldh + nh : nullptr;
         const bool vec = nvalid == 32 && ((reinterpret_cast<uintptr_t>(ph) & 15) == 0);
         if (vec) {
 #pragma unroll
@@ -154,7 +162,7 @@ static constexpr int GEMM_BLOCK_STAGE_FLOATS = 32 * 32;           // shared memo
 __device__ __forceinline__ bool gemm_block_ok(const GemmEpilogue &ep) {
     bool ok = !ep.bias || (reinterpret_cast<uintptr_t>(ep.bias) & 15) == 0;
     if (ep.mode != OUT_H16) ok = ok && (reinterpret_cast<uintptr_t>(ep.out) & 15) == 0 && (ep.ldo & 3) == 0;
-    if (ep.mode == OUT_H16 || ep.mode == OUT_F32_H16)
+    if (ep.mode == OUT_H16 || ep.mode == OUT_F32_H16 || ep.n_split)
         ok = ok && (reinterpret_cast<uintptr_t>(ep.out_hi) & 7) == 0 && (reinterpret_cast<uintptr_t>(ep.out_lo) & 7) == 0 && (ep.ldh & 3) == 0;
     return ok;
 }
@@ -187,7 +195,7 @@ __device__ __forceinline__ bool gemm_block_store(const GemmEpilogue &ep, const f
                                                  int nb, float *stage, int lane) {
     float4 *s4 = reinterpret_cast<float4 *>(stage);
     __syncwarp();
-    const int q = lane & 7, r0 = lane >> 3, col = nb + q * 4;
+    const int q = lane & 7, r0 = lane >> 3, col = nb + q * 4, mode = gemm_mode(ep, nb), hcol = gemm_plane_col(ep, nb) + q * 4;
     const float4 b = ep.bias ? *reinterpret_cast<const float4 *>(ep.bias + col) : make_float4(0.f, 0.f, 0.f, 0.f);
     bool fits = true;
 #pragma unroll
@@ -197,9 +205,9 @@ __device__ __forceinline__ bool gemm_block_store(const GemmEpilogue &ep, const f
         if (ep.bias) { t.x += b.x; t.y += b.y; t.z += b.z; t.w += b.w; }
         t.x = gemm_act(ep, t.x); t.y = gemm_act(ep, t.y); t.z = gemm_act(ep, t.z); t.w = gemm_act(ep, t.w);
         if (m >= M) continue;
-        if (ep.mode != OUT_H16) {
+        if (mode != OUT_H16) {
             float4 *o = reinterpret_cast<float4 *>(ep.out + (size_t)m * ep.ldo + col);
-            if (ep.mode == OUT_RESID) {
+            if (mode == OUT_RESID) {
                 float4 a = res[i];
                 a.x += ep.alpha * t.x; a.y += ep.alpha * t.y; a.z += ep.alpha * t.z; a.w += ep.alpha * t.w;
                 *o = a;
@@ -207,13 +215,13 @@ __device__ __forceinline__ bool gemm_block_store(const GemmEpilogue &ep, const f
                 *o = t;
             }
         }
-        if (ep.mode == OUT_H16 || ep.mode == OUT_F32_H16) {
+        if (mode == OUT_H16 || mode == OUT_F32_H16) {
             __half h0, h1, h2, h3, l0, l1, l2, l3;
             fits &= split_h16(t.x, h0, l0);
             fits &= split_h16(t.y, h1, l1);
             fits &= split_h16(t.z, h2, l2);
             fits &= split_h16(t.w, h3, l3);
-            const size_t off = (size_t)m * ep.ldh + col;
+            const size_t off = (size_t)m * ep.ldh + hcol;
             const __half2 ha = __halves2half2(h0, h1), hb = __halves2half2(h2, h3), la = __halves2half2(l0, l1), lb = __halves2half2(l2, l3);
             *reinterpret_cast<uint2 *>(ep.out_hi + off) = make_uint2(*reinterpret_cast<const uint32_t *>(&ha), *reinterpret_cast<const uint32_t *>(&hb));
             if (ep.out_lo) *reinterpret_cast<uint2 *>(ep.out_lo + off) = make_uint2(*reinterpret_cast<const uint32_t *>(&la), *reinterpret_cast<const uint32_t *>(&lb));
@@ -227,8 +235,10 @@ __device__ __forceinline__ bool gemm_block_store(const GemmEpilogue &ep, const f
 // C = A * B^T on tcgen05 tensor cores; nterms 1 (hi*hi) or 3 (hi*hi + lo*hi + hi*lo).
 // K must be a multiple of 64. status: device int receiving a non-zero code if a
 // bounded wait inside the kernel ran out.
+// chain: launched as a chained kernel (common.cuh): its first B tiles (weights) are requested while the kernel before it
+// still runs.
 int gemm_tc(const GemmOperand &A, const GemmOperand &B, const GemmEpilogue &ep, int M, int N, int K, int nterms,
-            int *status, cudaStream_t stream);
+            int *status, cudaStream_t stream, bool chain = false);
 
 // The same contraction for a handful of rows (a decoder position): gemm_skinny.cu. X: [M, K] activation planes, W: [N, K]
 // weight planes; K slices over the CTAs of a cluster, added in slice order (the count depends on N and K alone).
@@ -244,6 +254,6 @@ int gemm_skinny(const GemmOperand &X, const GemmOperand &W, const GemmEpilogue &
 // a: [M, K] int8 row-major (activation rows quantised by quantize_act_int8's rule), b: [N, K] int8 row-major
 // (reference-native per-row int8 weights). K must be a multiple of 128; lda / ldb in bytes, multiples of 16.
 int gemm_i8(const int8_t *a, int lda, const float *row_scale, const int8_t *b, int ldb, const float *col_scale,
-            const GemmEpilogue &ep, int M, int N, int K, int *status, cudaStream_t stream);
+            const GemmEpilogue &ep, int M, int N, int K, int *status, cudaStream_t stream, bool chain = false);
 
 }  // namespace mb

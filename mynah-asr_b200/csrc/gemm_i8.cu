@@ -91,11 +91,23 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_trigger();       // not before the allocation: a successor placed on this SM must not be first to take tensor memory
 
     if (warp == 0 && lane == 0) {
         // ---------------------------------------------------------- TMA producer
         int it = 0;
         bool ok = true;
+        int ahead = 0;                                 // B tiles (weights) asked for before the kernels in front have finished
+        if (blockIdx.x < total) {
+            int m0, n0, width;
+            units.at(blockIdx.x, BN, m0, n0, width);
+            ahead = num_k < Cfg::STAGES ? num_k : Cfg::STAGES;
+            for (int s = 0; s < ahead; s++) {
+                mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
+                tma_load_2d(tiles + s * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmB, s * I8_BK, n0, &full_bar[s]);
+            }
+        }
+        chain_wait();
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
             int m0, n0, width;
             units.at(tile, BN, m0, n0, width);               // a strip still loads BN rows of B: the MMAs read the first `width`
@@ -104,9 +116,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const uint32_t ph = (it / Cfg::STAGES) & 1;
                 if (!mbar_wait(&empty_bar[s], ph ^ 1)) { ok = false; break; }
                 uint8_t *st = tiles + s * Cfg::STAGE_BYTES;
-                mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
+                if (it >= ahead) mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
                 tma_load_2d(st, &tmA, kb * I8_BK, m0, &full_bar[s]);
-                tma_load_2d(st + Cfg::A_BYTES, &tmB, kb * I8_BK, n0, &full_bar[s]);
+                if (it >= ahead) tma_load_2d(st + Cfg::A_BYTES, &tmB, kb * I8_BK, n0, &full_bar[s]);
             }
         }
         if (!ok) {
@@ -151,6 +163,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int row = lg * 32 + lane;
         int lt = 0;
         bool fits = true;
+        chain_wait();                                  // row scales, the residual and the outputs belong to the kernels in front
         // the block form pays when a CTA walks several tiles (stores set the pace); with one tile per CTA the run is
         // latency-bound and the shorter row form is used. Both produce the same bits.
         const bool blk_ok = Cfg::BLOCK_EPILOGUE && gemm_block_ok(ep) && total > (int)gridDim.x;
@@ -252,7 +265,7 @@ static int i8_make_map(CUtensorMap *m, const int8_t *base, int rows, int K, int 
 
 template <int BN>
 static int i8_launch(const int8_t *a, int lda, const float *row_scale, const int8_t *b, int ldb, const float *col_scale,
-                     const GemmEpilogue &ep, int M, int N, int K, int *status, cudaStream_t stream) {
+                     const GemmEpilogue &ep, int M, int N, int K, int *status, cudaStream_t stream, bool chain) {
     using Cfg = I8Cfg<BN>;
     CUtensorMap ta, tb;
     if (i8_make_map(&ta, a, M, K, lda, GEMM_BM)) return -1;
@@ -267,13 +280,13 @@ static int i8_launch(const int8_t *a, int lda, const float *row_scale, const int
     // fewer tiles than SMs: the kernel cuts them into column strips (GemmUnits) when the grid leaves room
     const int total = cdiv(N, BN) * cdiv(M, GEMM_BM), strips = BN % 128 == 0 ? 4 : BN % 64 == 0 ? 2 : 1;
     dim3 grid(total >= sms ? sms : total * strips <= sms ? total * strips : total * 2 <= sms && strips >= 2 ? total * 2 : total);
-    gemm_i8_kernel<BN><<<grid, I8_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, ep, row_scale, col_scale, M, N, K, status);
-    MB_CUDA(cudaGetLastError());
+    MB_CUDA(launch_kernel(gemm_i8_kernel<BN>, grid, dim3(I8_THREADS), Cfg::SMEM_BYTES, stream, chain, 1, ta, tb, ep, row_scale, col_scale,
+                          M, N, K, status));
     return 0;
 }
 
 int gemm_i8(const int8_t *a, int lda, const float *row_scale, const int8_t *b, int ldb, const float *col_scale,
-            const GemmEpilogue &ep, int M, int N, int K, int *status, cudaStream_t stream) {
+            const GemmEpilogue &ep, int M, int N, int K, int *status, cudaStream_t stream, bool chain) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % I8_BK != 0) { set_error("gemm_i8: K=%d must be a positive multiple of %d", K, I8_BK); return -1; }
     if (!row_scale || !col_scale) { set_error("gemm_i8: scales missing"); return -1; }
@@ -287,10 +300,10 @@ int gemm_i8(const int8_t *a, int lda, const float *row_scale, const int8_t *b, i
         const long cost = (long)cdiv(tm * cdiv(N, cand), sms) * (cand + 48);
         if (best < 0 || cost < best) { best = cost; bn = cand; }
     }
-    if (bn == 256) return i8_launch<256>(a, lda, row_scale, b, ldb, col_scale, ep, M, N, K, status, stream);
-    if (bn == 128) return i8_launch<128>(a, lda, row_scale, b, ldb, col_scale, ep, M, N, K, status, stream);
-    if (bn == 64) return i8_launch<64>(a, lda, row_scale, b, ldb, col_scale, ep, M, N, K, status, stream);
-    return i8_launch<32>(a, lda, row_scale, b, ldb, col_scale, ep, M, N, K, status, stream);
+    if (bn == 256) return i8_launch<256>(a, lda, row_scale, b, ldb, col_scale, ep, M, N, K, status, stream, chain);
+    if (bn == 128) return i8_launch<128>(a, lda, row_scale, b, ldb, col_scale, ep, M, N, K, status, stream, chain);
+    if (bn == 64) return i8_launch<64>(a, lda, row_scale, b, ldb, col_scale, ep, M, N, K, status, stream, chain);
+    return i8_launch<32>(a, lda, row_scale, b, ldb, col_scale, ep, M, N, K, status, stream, chain);
 }
 
 }  // namespace mb

@@ -33,19 +33,25 @@ static constexpr int EPI_WARPS = 8;
 static constexpr int GEMM_THREADS = (2 + EPI_WARPS) * 32;   // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
 static constexpr int SMEM_LIMIT = 232448;  // 227 KB
 
-template <int BN, int NTERMS>
+// AR: rows of an A tile that shared memory holds and TMA loads. The MMA always reads 128 rows; with at most 64 rows in
+// all (AR = 64) the upper half of what it reads is whatever follows in the stage, and the accumulator rows it makes are
+// never stored. A stage is then a third smaller and two CTAs fit one SM: a chained successor sets up, and asks for its
+// weights, under its predecessor.
+template <int BN, int NTERMS, int AR>
 struct GemmCfg {
     static constexpr int NPLANES = NTERMS == 1 ? 1 : 2;
-    static constexpr int A_BYTES = BM * BK * 2;
+    static constexpr int A_BYTES = AR * BK * 2;
     static constexpr int B_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = NPLANES * (A_BYTES + B_BYTES);
     // the epilogue warps' turning buffers: only the wide tiles have them — the narrow ones serve contractions with few
     // rows, which are latency-bound and want every stage of the operand ring instead
     static constexpr bool BLOCK_EPILOGUE = BN >= 128;
     static constexpr int EPI_BYTES = BLOCK_EPILOGUE ? EPI_WARPS * GEMM_BLOCK_STAGE_FLOATS * 4 : 0;
-    static constexpr int STAGES_RAW = (SMEM_LIMIT - 2048 - EPI_BYTES) / STAGE_BYTES;
+    static constexpr int PER_SM = AR < BM ? 2 : 1;
+    static constexpr int TAIL_BYTES = (BM - AR) * BK * 2;         // what the last stage's MMAs may read past its end
+    static constexpr int STAGES_RAW = (SMEM_LIMIT / PER_SM - 2048 - 1024 * (PER_SM - 1) - TAIL_BYTES - EPI_BYTES) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 6 ? 6 : STAGES_RAW;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 2048;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + TAIL_BYTES + EPI_BYTES + 2048;
     // NTERMS == 3 keeps a second accumulator for the cross terms (lo*hi + hi*lo);
     // everything is double-buffered so the epilogue of tile i overlaps the MMAs of tile i+1
     static constexpr int ACC_COLS = NTERMS == 1 ? BN : 2 * BN;
@@ -55,17 +61,17 @@ struct GemmCfg {
 
 // Persistent kernel: one CTA per SM walks the output tiles (n fastest, so the CTAs in
 // flight share a few A row-blocks while B stays L2-resident).
-template <int BN, int NTERMS>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+template <int BN, int NTERMS, int AR>
+__global__ void __launch_bounds__(GEMM_THREADS, (AR < BM ? 2 : 1))
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CUtensorMap tmA_lo,
                const __grid_constant__ CUtensorMap tmB_hi, const __grid_constant__ CUtensorMap tmB_lo,
-               const GemmEpilogue ep, const int M, const int N, const int K, int *status) {
-    using Cfg = GemmCfg<BN, NTERMS>;
+               const GemmEpilogue ep, const int M, const int N, const int K, const uint32_t stage_tx, int *status) {
+    using Cfg = GemmCfg<BN, NTERMS, AR>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *tiles = smem;
-    float *epi_stage = reinterpret_cast<float *>(smem + Cfg::STAGES * Cfg::STAGE_BYTES);
-    uint64_t *full_bar = reinterpret_cast<uint64_t *>(smem + Cfg::STAGES * Cfg::STAGE_BYTES + Cfg::EPI_BYTES);
+    float *epi_stage = reinterpret_cast<float *>(smem + Cfg::STAGES * Cfg::STAGE_BYTES + Cfg::TAIL_BYTES);
+    uint64_t *full_bar = reinterpret_cast<uint64_t *>(smem + Cfg::STAGES * Cfg::STAGE_BYTES + Cfg::TAIL_BYTES + Cfg::EPI_BYTES);
     uint64_t *empty_bar = full_bar + Cfg::STAGES;
     uint64_t *acc_full = empty_bar + Cfg::STAGES;      // [2] MMA -> epilogue
     uint64_t *acc_empty = acc_full + 2;                // [2] epilogue -> MMA
@@ -89,11 +95,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_trigger();       // not before the allocation: a successor placed on this SM must not be first to take tensor memory
 
     if (warp == 0 && lane == 0) {
         // ---------------------------------------------------------- TMA producer
         int it = 0;                                    // k-blocks issued so far (ring position)
         bool ok = true;
+        // the first ring of B tiles (weights) is asked for before the kernels in front have finished
+        int ahead = 0;
+        if (blockIdx.x < total) {
+            int m0, n0, width;
+            units.at(blockIdx.x, BN, m0, n0, width);
+            ahead = num_k < Cfg::STAGES ? num_k : Cfg::STAGES;
+            for (int s = 0; s < ahead; s++) {
+                uint8_t *bt = tiles + s * Cfg::STAGE_BYTES + Cfg::NPLANES * Cfg::A_BYTES;
+                mbar_expect_tx(&full_bar[s], stage_tx);
+                tma_load_2d(bt, &tmB_hi, s * BK, n0, &full_bar[s]);
+                if (NTERMS > 1) tma_load_2d(bt + Cfg::B_BYTES, &tmB_lo, s * BK, n0, &full_bar[s]);
+            }
+        }
+        chain_wait();
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
             int m0, n0, width;
             units.at(tile, BN, m0, n0, width);               // a strip still loads BN rows of B: the MMAs read the first `width`
@@ -102,9 +123,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
                 const uint32_t ph = (it / Cfg::STAGES) & 1;
                 if (!mbar_wait(&empty_bar[s], ph ^ 1)) { ok = false; break; }
                 uint8_t *st = tiles + s * Cfg::STAGE_BYTES;
-                mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
+                if (it >= ahead) mbar_expect_tx(&full_bar[s], stage_tx);
                 tma_load_2d(st, &tmA_hi, kb * BK, m0, &full_bar[s]);
                 if (NTERMS > 1) tma_load_2d(st + Cfg::A_BYTES, &tmA_lo, kb * BK, m0, &full_bar[s]);
+                if (it < ahead) continue;
                 uint8_t *bt = st + Cfg::NPLANES * Cfg::A_BYTES;
                 tma_load_2d(bt, &tmB_hi, kb * BK, n0, &full_bar[s]);
                 if (NTERMS > 1) tma_load_2d(bt + Cfg::B_BYTES, &tmB_lo, kb * BK, n0, &full_bar[s]);
@@ -160,6 +182,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
         const int row = lg * 32 + lane;
         int lt = 0;
         bool fits = true;
+        chain_wait();                                  // the residual is read and outputs are written only after the kernels in front
         // the block form pays when a CTA walks several tiles (stores set the pace); with one tile per CTA the run is
         // latency-bound and the shorter row form is used. Both produce the same bits.
         const bool blk_ok = Cfg::BLOCK_EPILOGUE && gemm_block_ok(ep) && total > (int)gridDim.x;
@@ -266,15 +289,17 @@ static int make_map(CUtensorMap *m, const __half *base, int rows, int K, int ld,
     return 0;
 }
 
-template <int BN, int NTERMS>
+template <int BN, int NTERMS, int AR>
 static int launch(const GemmOperand &A, const GemmOperand &B, const GemmEpilogue &ep, int M, int N, int K,
-                  int *status, cudaStream_t stream) {
-    using Cfg = GemmCfg<BN, NTERMS>;
+                  int *status, cudaStream_t stream, bool chain) {
+    using Cfg = GemmCfg<BN, NTERMS, AR>;
     CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
-    if (make_map(&ta_hi, A.hi, M, K, A.ld, BM)) return -1;
+    // a single row tile loads the rows there are (in eights, the swizzle atom): rows of zeros cost shared-memory writes
+    const int a_rows = M < AR ? (int)align_up((size_t)M, 8) : AR;
+    if (make_map(&ta_hi, A.hi, M, K, A.ld, a_rows)) return -1;
     if (make_map(&tb_hi, B.hi, N, K, B.ld, BN)) return -1;
     if (NTERMS > 1) {
-        if (make_map(&ta_lo, A.lo, M, K, A.ld, BM)) return -1;
+        if (make_map(&ta_lo, A.lo, M, K, A.ld, a_rows)) return -1;
         if (make_map(&tb_lo, B.lo, N, K, B.ld, BN)) return -1;
     } else {
         ta_lo = ta_hi; tb_lo = tb_hi;
@@ -282,7 +307,7 @@ static int launch(const GemmOperand &A, const GemmOperand &B, const GemmEpilogue
     static PerDevice configured = {};
     int dev = 0;
     if (configured.below(Cfg::SMEM_BYTES, &dev)) {
-        MB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<BN, NTERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        MB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<BN, NTERMS, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      Cfg::SMEM_BYTES));
         configured.record(dev, Cfg::SMEM_BYTES);
     }
@@ -290,14 +315,14 @@ static int launch(const GemmOperand &A, const GemmOperand &B, const GemmEpilogue
     // fewer tiles than SMs: the kernel cuts them into column strips (GemmUnits) when the grid leaves room
     const int total = cdiv(N, BN) * cdiv(M, BM), strips = BN % 128 == 0 ? 4 : BN % 64 == 0 ? 2 : 1;
     dim3 grid(total >= sms ? sms : total * strips <= sms ? total * strips : total * 2 <= sms && strips >= 2 ? total * 2 : total);
-    gemm_tc_kernel<BN, NTERMS><<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta_hi, ta_lo, tb_hi, tb_lo, ep, M,
-                                                                               N, K, status);
-    MB_CUDA(cudaGetLastError());
+    const uint32_t stage_tx = Cfg::NPLANES * (uint32_t)(a_rows * BK * 2 + Cfg::B_BYTES);
+    MB_CUDA(launch_kernel(gemm_tc_kernel<BN, NTERMS, AR>, grid, dim3(GEMM_THREADS), Cfg::SMEM_BYTES, stream, chain, 1,
+                          ta_hi, ta_lo, tb_hi, tb_lo, ep, M, N, K, stage_tx, status));
     return 0;
 }
 
 int gemm_tc(const GemmOperand &A, const GemmOperand &B, const GemmEpilogue &ep, int M, int N, int K, int nterms,
-            int *status, cudaStream_t stream) {
+            int *status, cudaStream_t stream, bool chain) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % BK != 0) { set_error("gemm_tc: K=%d must be a positive multiple of %d", K, BK); return -1; }
     if (nterms != 1 && (!A.lo || !B.lo)) { set_error("gemm_tc: 3-term mode needs lo planes"); return -1; }
@@ -313,16 +338,16 @@ int gemm_tc(const GemmOperand &A, const GemmOperand &B, const GemmEpilogue &ep, 
         const long cost = (long)cdiv(tm * cdiv(N, cand), sms) * (cand + 48);
         if (best < 0 || cost < best) { best = cost; bn = cand; }
     }
+    const bool low = M <= 64;                        // one half-height row tile
+#define GEMM_GO(BN_, NT_) (low ? launch<BN_, NT_, 64>(A, B, ep, M, N, K, status, stream, chain) : launch<BN_, NT_, 128>(A, B, ep, M, N, K, status, stream, chain))
     if (nterms == 1) {
-        if (bn == 128 && N >= 256) return launch<256, 1>(A, B, ep, M, N, K, status, stream);
-        if (bn == 128) return launch<128, 1>(A, B, ep, M, N, K, status, stream);
-        if (bn == 64) return launch<64, 1>(A, B, ep, M, N, K, status, stream);
-        return launch<32, 1>(A, B, ep, M, N, K, status, stream);
+        if (bn == 128 && N >= 256) return launch<256, 1, 128>(A, B, ep, M, N, K, status, stream, chain);
+        if (bn == 128) return launch<128, 1, 128>(A, B, ep, M, N, K, status, stream, chain);
+        return bn == 64 ? GEMM_GO(64, 1) : GEMM_GO(32, 1);
     }
-    if (!A.lo || !B.lo) { set_error("gemm_tc: 3-term mode needs lo planes"); return -1; }
-    if (bn == 128) return launch<128, 3>(A, B, ep, M, N, K, status, stream);
-    if (bn == 64) return launch<64, 3>(A, B, ep, M, N, K, status, stream);
-    return launch<32, 3>(A, B, ep, M, N, K, status, stream);
+    if (bn == 128) return launch<128, 3, 128>(A, B, ep, M, N, K, status, stream, chain);
+    return bn == 64 ? GEMM_GO(64, 3) : GEMM_GO(32, 3);
+#undef GEMM_GO
 }
 
 }  // namespace mb

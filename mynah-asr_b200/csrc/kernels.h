@@ -39,7 +39,7 @@ int layer_norm_q8(const float *x, const float *w, const float *b, float *out_f32
 // receives the same values as the planes (either may be null).
 int glu_dwconv(const float *h2, const float *dw_w, const float *dw_b, const float *scale, const float *shift,
                float *out_f32, H16 out_h, const int *seg_off, const int *seg_len, int batch, int max_len, int d,
-               int k, int pad_left, cudaStream_t st);
+               int k, int pad_left, cudaStream_t st, bool chain = false);
 int scale_inplace(float *x, size_t n, float s, cudaStream_t st);
 int pos_emb(H16 pe, int T, int d, cudaStream_t st);            // [2T-1, d] planes
 
@@ -55,6 +55,8 @@ struct AttnArgs {
     const int *seg_off, *seg_len, *rk_off;   // device arrays [batch]
     int batch, max_len, d, H;
     int left, right;            // left < 0: full attention
+    int ldkv = 0, ldrk = 0;     // row strides of k / v and of rk in halves, multiples of 8; 0: d
+    bool chain = false;         // launched as a chained kernel (common.cuh)
     long long rows = 0, rk_rows = 0;   // rows of k / v and of rk (bounds of the TMA descriptors); 0: unknown
     int *status = nullptr;      // device status word for the bounded waits of the tcgen05 kernel
 };
@@ -68,10 +70,13 @@ int attention_tc(const AttnArgs &a, cudaStream_t st);
 // ---- subsampling.cu
 int conv_in_relu(const float *feats, const float *w, const float *b, float *out, int T, int F, int C, int To, int Fo,
                  int pl, cudaStream_t st);                         // [T,F] -> [To,Fo,C]
-int conv_in_dw_fused(const float *feats, const float *w0, const float *b0, const float *w1, const float *b1, H16 out,
-                     int T, int F, int C, int T1, int F1, int T2, int F2, int pl, cudaStream_t st);   // [T,F] -> planes [T2*F2, C]
-int dwconv3x3_s2(const float *x, const float *w, const float *b, H16 out, int T, int F, int C, int To, int Fo, int pl,
-                 cudaStream_t st);                                 // [T,F,C] -> planes [To*Fo, C]
+struct FrontItem;                                                  // model.h
+// a group of utterances at once (items on the device): features -> planes [sum T2 * F2, C] of stage 1
+int conv_in_dw_fused(const FrontItem *items, int n_items, int rows2, const float *w0, const float *b0, const float *w1, const float *b1,
+                     H16 out, int F, int C, int F1, int F2, int pl, cudaStream_t st);
+// x [sum T2, F2, C] -> planes [sum T3 * F3, C] of stage 2
+int dwconv3x3_s2(const FrontItem *items, int n_items, int rows3, const float *x, const float *w, const float *b, H16 out, int F, int C,
+                 int Fo, int pl, cudaStream_t st);
 
 // ---- mel.cu
 struct MelCfg {
@@ -82,6 +87,10 @@ struct MelCfg {
 int log_mel_device(const MelCfg &c, const float *audio, size_t n_samples, const float *mel_fb, const int *mel_lo,
                    const int *mel_hi, const double *win, const double *twiddle, float *feats, int T, int valid,
                    cudaStream_t st);
+
+// a group of utterances at once (items on the device), frames [0, t_mel) of each; max_t: the longest
+int log_mel_group(const MelCfg &c, const FrontItem *items, int n_items, int max_t, const float *mel_fb, const int *mel_lo,
+                  const int *mel_hi, const double *win, const double *twiddle, cudaStream_t st);
 
 int log_mel_stream_device(const MelCfg &c, const float *tail, long long base, long long total, long long sig_stride, int n_sig,
                           const float *mel_fb, const int *mel_lo, const int *mel_hi, const double *win, const double *twiddle,
@@ -101,7 +110,7 @@ int qstream_tc(const QWeight &w, const float *x, int ldx, float *out, int ldo, c
                cudaStream_t st);
 // int8 activation rows by the reference's rule (quantize_act_int8, src/qmat.c:186-202): per row scale = amax / 127,
 // q = round-half-away(x * 127 / amax) clamped to +-127; x [T, k] f32 -> qx [T, k] int8, sx [T]
-int act_quant_rows(const float *x, int8_t *qx, float *sx, int T, int k, cudaStream_t st);
+int act_quant_rows(const float *x, int8_t *qx, float *sx, int T, int k, cudaStream_t st, bool chain = false);
 int qgemv_a8(const QWeight &w, const float *x, float *out, int T, int32_t *block_dots, float *sx_out, cudaStream_t st);
 
 // ---- align.cu : CTC forced alignment (mynah_asr_align_ctc, src/align.c) with the scores resident

@@ -10,6 +10,7 @@
 // at ~0.14 GFLOP per minute of audio it costs nothing), twiddles come from an exact
 // host table. Frames >= valid stay zero, as in the reference.
 #include "kernels.h"
+#include "model.h"
 
 namespace mb {
 
@@ -18,17 +19,24 @@ static constexpr int MEL_MAX_FFT = 1024;
 // blockIdx.y selects one of several signals (streams of a lock-step group): signal y starts at
 // audio + y * sig_stride and its frames go to feats + y * feat_stride. `base` is the absolute sample index
 // of audio[0] (streaming keeps only the tail of the signal; 0 offline), t0 the first frame of this launch.
+// With `items` the signals are the utterances of a batch, each with its own place and length.
 __global__ void __launch_bounds__(128)
 mel_frame_kernel(const float *__restrict__ audio_all, long long S, const double *__restrict__ win,
                  const double *__restrict__ tw, const float *__restrict__ fb, const int *__restrict__ mlo,
                  const int *__restrict__ mhi, float *__restrict__ feats_all, int n_fft, int log2n, int hop, int n_mels,
-                 double preemph, double guard, long long base, int t0, long long sig_stride, long long feat_stride) {
+                 double preemph, double guard, long long base, int t0, long long sig_stride, long long feat_stride,
+                 const FrontItem *__restrict__ items) {
     // one double of padding after every 16: the bit-reversed stores and the small-stride stages would
     // otherwise pile a warp's accesses onto one bank pair
 #define PD(i) ((i) + ((i) >> 4))
     __shared__ double re[MEL_MAX_FFT + MEL_MAX_FFT / 16], im[MEL_MAX_FFT + MEL_MAX_FFT / 16];
     const float *audio = audio_all + blockIdx.y * sig_stride - base;      // audio[s] is sample s of the signal
     float *feats = feats_all + blockIdx.y * feat_stride - (long long)t0 * n_mels;
+    if (items) {
+        const FrontItem &it = items[blockIdx.y];
+        if ((int)blockIdx.x >= it.t_mel) return;
+        audio = it.audio; S = it.n_samples; feats = it.feats;
+    }
     const int t = t0 + blockIdx.x;
     const long long start = (long long)t * hop - n_fft / 2;      // index into the unpadded signal
     for (int i = threadIdx.x; i < n_fft; i += blockDim.x) {
@@ -77,10 +85,11 @@ __device__ __forceinline__ double mel_norm_reduce(double v, double (*red)[MN_BX]
 }
 
 __global__ void __launch_bounds__(MN_BX * MN_BY)
-mel_norm_kernel(float *feats, int valid, int n_mels) {
+mel_norm_kernel(float *feats, int valid, int n_mels, const FrontItem *__restrict__ items) {
     __shared__ double red[MN_BY][MN_BX];
     const int x = threadIdx.x, y = threadIdx.y, m = blockIdx.x * MN_BX + x;
     const bool on = m < n_mels;
+    if (items) { feats = items[blockIdx.y].feats; valid = items[blockIdx.y].t_mel; if (valid < 2) return; }
     double s = 0.0;
     if (on) for (int t = y; t < valid; t += MN_BY) s += (double)feats[(size_t)t * n_mels + m];
     const double mu = mel_norm_reduce(s, red, x, y) / valid;
@@ -102,10 +111,26 @@ int log_mel_device(const MelCfg &c, const float *audio, size_t n_samples, const 
     int log2n = 0;
     while ((1 << log2n) < c.n_fft) log2n++;
     mel_frame_kernel<<<valid, 128, 0, st>>>(audio, (long long)n_samples, win, twiddle, mel_fb, mel_lo, mel_hi, feats,
-                                            c.n_fft, log2n, c.hop, c.n_mels, c.preemph, c.guard, 0, 0, 0, 0);
+                                            c.n_fft, log2n, c.hop, c.n_mels, c.preemph, c.guard, 0, 0, 0, 0, nullptr);
     MB_CUDA(cudaGetLastError());
     if (c.normalize && valid > 1) {
-        mel_norm_kernel<<<cdiv(c.n_mels, MN_BX), dim3(MN_BX, MN_BY), 0, st>>>(feats, valid, c.n_mels);
+        mel_norm_kernel<<<cdiv(c.n_mels, MN_BX), dim3(MN_BX, MN_BY), 0, st>>>(feats, valid, c.n_mels, nullptr);
+        MB_CUDA(cudaGetLastError());
+    }
+    return 0;
+}
+
+int log_mel_group(const MelCfg &c, const FrontItem *items, int n_items, int max_t, const float *mel_fb, const int *mel_lo,
+                  const int *mel_hi, const double *win, const double *twiddle, cudaStream_t st) {
+    if (c.n_fft > MEL_MAX_FFT || (c.n_fft & (c.n_fft - 1))) { set_error("log_mel: n_fft %d unsupported", c.n_fft); return -1; }
+    if (n_items <= 0 || max_t <= 0) return 0;
+    int log2n = 0;
+    while ((1 << log2n) < c.n_fft) log2n++;
+    mel_frame_kernel<<<dim3(max_t, n_items), 128, 0, st>>>(nullptr, 0, win, twiddle, mel_fb, mel_lo, mel_hi, nullptr, c.n_fft, log2n, c.hop,
+                                                           c.n_mels, c.preemph, c.guard, 0, 0, 0, 0, items);
+    MB_CUDA(cudaGetLastError());
+    if (c.normalize) {
+        mel_norm_kernel<<<dim3(cdiv(c.n_mels, MN_BX), n_items), dim3(MN_BX, MN_BY), 0, st>>>(nullptr, 0, c.n_mels, items);
         MB_CUDA(cudaGetLastError());
     }
     return 0;
@@ -122,7 +147,7 @@ int log_mel_stream_device(const MelCfg &c, const float *tail, long long base, lo
     int log2n = 0;
     while ((1 << log2n) < c.n_fft) log2n++;
     mel_frame_kernel<<<dim3(n_frames, n_sig), 128, 0, st>>>(tail, total, win, twiddle, mel_fb, mel_lo, mel_hi, feats, c.n_fft, log2n,
-                                                            c.hop, c.n_mels, c.preemph, c.guard, base, t0, sig_stride, feat_stride);
+                                                            c.hop, c.n_mels, c.preemph, c.guard, base, t0, sig_stride, feat_stride, nullptr);
     MB_CUDA(cudaGetLastError());
     return 0;
 }

@@ -34,6 +34,17 @@ void *Arena::take(size_t bytes) {
 }
 void Arena::release() { if (base) cudaFree(base); base = nullptr; cap = off = 0; }
 
+int HostStage::begin(size_t bytes) {
+    off = 0;
+    if (bytes <= cap) return 0;
+    release();
+    const size_t want = align_up(bytes, 64 << 10);
+    MB_CUDA(cudaMallocHost((void **)&base, want));
+    cap = want;
+    return 0;
+}
+void HostStage::release() { if (base) cudaFreeHost(base); base = nullptr; cap = off = 0; }
+
 // -------------------------------------------------------------------- model
 static constexpr size_t SLAB_BYTES = 256u << 20;
 static constexpr size_t STAGE_BYTES = 32u << 20;
@@ -43,6 +54,9 @@ Model::~Model() {
     for (void *p : owned) cudaFree(p);
     for (auto &s : prof_spans) { cudaEventDestroy(s.a); cudaEventDestroy(s.b); }
     ws.release();
+    host_stage.release();
+    for (cudaEvent_t e : copy_ev) cudaEventDestroy(e);
+    if (copy) cudaStreamDestroy(copy);
     for (int i = 0; i < DEC_LANES; i++) {
         if (lane_done[i]) cudaEventDestroy(lane_done[i]);
         if (lane[i]) cudaStreamDestroy(lane[i]);
@@ -157,15 +171,15 @@ int Model::upload_weight(QWeight &w, int fmt, const void *data, const float *sca
     if (k % blk) { set_error("weight [%d,%d]: k not a multiple of the %d-element block", n, k, blk); return -1; }
     w.raw_bytes = format_bytes(fmt, n, k);
     if (!w.raw_bytes) { set_error("unknown weight format %d", fmt); return -1; }
-    w.raw = (uint8_t *)dev_alloc(w.raw_bytes + 64);          // slack for aligned over-reads
+    if (!w.raw) w.raw = (uint8_t *)dev_alloc(w.raw_bytes + 64);          // slack for aligned over-reads
     if (!w.raw) return -1;
     if (upload_bytes(w.raw, data, w.raw_bytes)) return -1;
     MB_CUDA(cudaMemsetAsync(w.raw + w.raw_bytes, 0, 64, stream));
     if (fmt == FMT_MYNAH_Q8 || fmt == FMT_MYNAH_Q4) {
         if (!scales) { set_error("native quantised weight without scales"); return -1; }
         const size_t ns = fmt == FMT_MYNAH_Q8 ? (size_t)n : (size_t)n * (k / 32);
-        w.scales = upload_f32(scales, ns);
-        if (!w.scales) return -1;
+        if (!w.scales) w.scales = (float *)dev_alloc(ns * sizeof(float));
+        if (!w.scales || upload_bytes(w.scales, scales, ns * sizeof(float))) return -1;
     }
     if ((fmt == FMT_GGML_Q4_0 || fmt == FMT_GGML_Q8_0) && k % 128 == 0) {
         // re-tiled copy for the tensor-core small-T kernel (same bytes per parameter)
@@ -208,8 +222,9 @@ int Model::upload_weight(QWeight &w, int fmt, const void *data, const float *sca
         cudaFree(perm_dev);
     }
     if (rc == 0 && want_planes) {
-        w.hi = (__half *)dev_alloc((size_t)n * k * 2);
-        w.lo = (__half *)dev_alloc((size_t)n * k * 2);
+        // a caller may have given the planes a place beside those of a related weight
+        if (!w.hi) w.hi = (__half *)dev_alloc((size_t)n * k * 2);
+        if (!w.lo) w.lo = (__half *)dev_alloc((size_t)n * k * 2);
         if (!w.hi || !w.lo) rc = -1;
         else { rc = split_to_h16(permuted ? permuted : tmp, w.hi, w.lo, (size_t)n * k, stream, status); note_launch(); }
     }
@@ -247,12 +262,12 @@ int Model::check_status(const char *where) {
     return 0;
 }
 
-int Model::gemm(const H16 &a, int lda, const QWeight &w, const GemmEpilogue &ep, int M, bool few_rows) {
+int Model::gemm(const H16 &a, int lda, const QWeight &w, const GemmEpilogue &ep, int M, bool few_rows, bool chain) {
     if (!w.hi) { set_error("contraction on a weight without operand planes"); return -1; }
     GemmOperand A{a.hi, a.lo, lda}, B{w.hi, w.lo, w.k};
     const int sp = prof_begin_span(PROF_GEMM);
     const int rc = few_rows ? gemm_skinny(A, B, ep, M, w.n, w.k, cfg.strict ? 3 : 1, status, stream, true)
-                            : gemm_tc(A, B, ep, M, w.n, w.k, cfg.strict ? 3 : 1, status, stream);
+                            : gemm_tc(A, B, ep, M, w.n, w.k, cfg.strict ? 3 : 1, status, stream, chain);
     prof_end_span(sp);
     if (sp >= 0) {
         prof_flops[PROF_GEMM] += 2.0 * M * (double)w.n * w.k;
@@ -266,10 +281,10 @@ int Model::gemm(const H16 &a, int lda, const QWeight &w, const GemmEpilogue &ep,
     return rc;
 }
 
-int Model::gemm_q8(const int8_t *qa, const float *sx, const QWeight &w, const GemmEpilogue &ep, int M) {
+int Model::gemm_q8(const int8_t *qa, const float *sx, const QWeight &w, const GemmEpilogue &ep, int M, bool chain) {
     if (!a8_ok(w)) { set_error("int8-activation contraction on a weight that is not reference-native int8 with k %% 128 == 0"); return -1; }
     const int sp = prof_begin_span(PROF_GEMM);
-    const int rc = gemm_i8(qa, w.k, sx, reinterpret_cast<const int8_t *>(w.raw), w.k, w.scales, ep, M, w.n, w.k, status, stream);
+    const int rc = gemm_i8(qa, w.k, sx, reinterpret_cast<const int8_t *>(w.raw), w.k, w.scales, ep, M, w.n, w.k, status, stream, chain);
     prof_end_span(sp);
     if (sp >= 0) {
         prof_flops[PROF_GEMM] += 2.0 * M * (double)w.n * w.k;
@@ -289,30 +304,127 @@ static GemmEpilogue epi(int mode, int act, float alpha, const float *bias, float
     return e;
 }
 
-// ---------------------------------------------------------------- subsampling
-// feats [t_mel, n_mels] on the device -> x_out [T3, d_model]; scratch from the arena
+// ---------------------------------------------------------------- front end
+// A group of utterances: feats [t_mel, n_mels] on the device -> x_out [sum T3, d_model]; scratch from the arena
 // (released on return: later kernels are ordered behind these on the same stream).
-int Model::subsample_item(const float *feats, int t_mel, float *x_out, int *t_out) {
+int Model::subsample_group(const FrontItem *items_dev, const FrontItem *items, int n, float *x_out) {
     const int C = channels, pl = causal ? 2 : 1, F0 = cfg.n_mels;
-    const int T1 = sub_len(t_mel, causal), F1 = sub_len(F0, causal);
-    const int T2 = sub_len(T1, causal), F2 = sub_len(F1, causal);
-    const int T3 = sub_len(T2, causal), F3 = sub_len(F2, causal);
+    const int F1 = sub_len(F0, causal), F2 = sub_len(F1, causal), F3 = sub_len(F2, causal);
+    const int R2 = items[n - 1].off2 + items[n - 1].T2, R3 = items[n - 1].off3 + items[n - 1].T3;
     const size_t mark = ws.off;
-    H16 p1 = ws.planes((size_t)T2 * F2 * C);
-    float *a1 = ws.get<float>((size_t)T2 * F2 * C);
-    H16 p2 = ws.planes((size_t)T3 * F3 * C);
-    H16 flat = ws.planes((size_t)T3 * F3 * C);
+    H16 p1 = ws.planes((size_t)R2 * F2 * C);
+    float *a1 = ws.get<float>((size_t)R2 * F2 * C);
+    H16 p2 = ws.planes((size_t)R3 * F3 * C);
+    H16 flat = ws.planes((size_t)R3 * F3 * C);
     if (!p1.hi || !p1.lo || !a1 || !p2.hi || !p2.lo || !flat.hi || !flat.lo) return -1;
-    if (conv_in_dw_fused(feats, conv_in_w, conv_in_b, dw_w[0], dw_b[0], p1, t_mel, F0, C, T1, F1, T2, F2, pl, stream)) return -1;
-    if (gemm(p1, C, pw[0], epi(OUT_F32, ACT_RELU, 1.f, pw[0].bias, a1, C), T2 * F2)) return -1;
-    if (dwconv3x3_s2(a1, dw_w[1], dw_b[1], p2, T2, F2, C, T3, F3, pl, stream)) return -1;
-    if (gemm(p2, C, pw[1], epi(OUT_H16, ACT_RELU, 1.f, pw[1].bias, nullptr, 0, flat, C), T3 * F3)) return -1;
+    if (conv_in_dw_fused(items_dev, n, R2, conv_in_w, conv_in_b, dw_w[0], dw_b[0], p1, F0, C, F1, F2, pl, stream)) return -1;
+    if (gemm(p1, C, pw[0], epi(OUT_F32, ACT_RELU, 1.f, pw[0].bias, a1, C), R2 * F2)) return -1;
+    if (dwconv3x3_s2(items_dev, n, R3, a1, dw_w[1], dw_b[1], p2, F2, C, F3, pl, stream)) return -1;
+    if (gemm(p2, C, pw[1], epi(OUT_H16, ACT_RELU, 1.f, pw[1].bias, nullptr, 0, flat, C), R3 * F3)) return -1;
     // flat is [T3, F3*C]: the linear's columns were permuted to this order at load
-    if (gemm(flat, F3 * C, ss_lin, epi(OUT_F32, ACT_NONE, 1.f, ss_lin.bias, x_out, d_model), T3)) return -1;
+    if (gemm(flat, F3 * C, ss_lin, epi(OUT_F32, ACT_NONE, 1.f, ss_lin.bias, x_out, d_model), R3)) return -1;
     note_launch(2);
-    if (xscale != 1.0f) { if (scale_inplace(x_out, (size_t)T3 * d_model, xscale, stream)) return -1; note_launch(); }
+    if (xscale != 1.0f) { if (scale_inplace(x_out, (size_t)R3 * d_model, xscale, stream)) return -1; note_launch(); }
     ws.off = mark;
-    *t_out = T3;
+    return 0;
+}
+
+// Groups of about a minute: enough rows to fill the chip at every stage, few enough that the scratch of a group (130 MB)
+// passes through the L2 and that the copies of the next group hide behind its kernels.
+std::vector<int> Model::front_groups(const int *t_mel, int batch) const {
+    static constexpr long long GROUP_FRAMES = 6000;
+    std::vector<int> ends;
+    long long sum = 0;
+    for (int b = 0; b < batch; b++) {
+        sum += t_mel[b] > 0 ? t_mel[b] : 0;
+        if (sum >= GROUP_FRAMES || b + 1 == batch) { ends.push_back(b + 1); sum = 0; }
+    }
+    return ends;
+}
+
+size_t Model::front_bytes(const size_t *n_samples, const int *t_mel, int batch, bool audio, bool on_host) const {
+    const int C = channels, F1 = sub_len(cfg.n_mels, causal), F2 = sub_len(F1, causal), F3 = sub_len(F2, causal);
+    size_t in = 0, group = 0, most = 0;
+    int b = 0;
+    for (int e : front_groups(t_mel, batch)) {
+        for (group = 0; b < e; b++) {
+            const size_t t = t_mel[b] > 0 ? t_mel[b] : 0;
+            if (audio && on_host) in += align_up((n_samples[b] + 1) * 4, 256);
+            if (audio || on_host) in += align_up((t + 1) * cfg.n_mels * 4, 256);
+            const int T2 = sub_len(sub_len((int)t, causal), causal), T3 = sub_len(T2, causal);
+            if (t) group += (size_t)T2 * F2 * C * 8 + (size_t)T3 * F3 * C * 8;
+        }
+        if (group > most) most = group;
+    }
+    return in + most + (size_t)batch * sizeof(FrontItem) + (1 << 16);
+}
+
+int Model::front_end(const float *const *audio, const size_t *n_samples, const float *const *feats, const int *t_mel, int batch,
+                     bool on_host, float *x_out, std::vector<int> &lens) {
+    if (audio && !has_mel) { set_error("log_mel: mel filterbank not set"); return -1; }
+    if (on_host && !copy) MB_CUDA(cudaStreamCreateWithFlags(&copy, cudaStreamNonBlocking));
+    lens.assign(batch, 0);
+    const std::vector<int> ends = front_groups(t_mel, batch);
+    FrontItem *items = host_stage.get<FrontItem>(batch), *items_dev = ws.get<FrontItem>(batch);
+    if (!items || !items_dev) { set_error("front end: no room for the utterance table"); return -1; }
+    // utterances with at least one frame, packed group by group
+    struct Group { int first, n, max_t, b0, b1; };
+    std::vector<Group> groups;
+    int used = 0, b = 0;
+    for (int e : ends) {
+        Group g{used, 0, 0, b, e};
+        int off2 = 0, off3 = 0;
+        for (; b < e; b++) {
+            if (t_mel[b] <= 0) continue;
+            FrontItem it;
+            it.n_samples = audio ? (long long)n_samples[b] : 0;
+            it.audio = !audio ? nullptr : on_host ? ws.get<float>(n_samples[b]) : audio[b];
+            it.feats = audio || on_host ? ws.get<float>((size_t)t_mel[b] * cfg.n_mels) : const_cast<float *>(feats[b]);
+            if ((audio && !it.audio) || !it.feats) return -1;
+            it.t_mel = t_mel[b]; it.T1 = sub_len(it.t_mel, causal); it.T2 = sub_len(it.T1, causal); it.T3 = sub_len(it.T2, causal);
+            it.off2 = off2; it.off3 = off3;
+            off2 += it.T2; off3 += it.T3;
+            lens[b] = it.T3;
+            if (it.t_mel > g.max_t) g.max_t = it.t_mel;
+            items[used++] = it;
+            g.n++;
+        }
+        if (g.n) groups.push_back(g);
+    }
+    if (!used) return 0;
+    MB_CUDA(cudaMemcpyAsync(items_dev, items, (size_t)used * sizeof(FrontItem), cudaMemcpyHostToDevice, stream));
+    const MelCfg c{cfg.n_mels, cfg.n_fft, cfg.win_length, cfg.hop_length, cfg.preemphasis, cfg.log_zero_guard, cfg.normalize_per_feature};
+    float *x = x_out;
+    for (size_t gi = 0; gi < groups.size(); gi++) {
+        const Group &g = groups[gi];
+        if (on_host) {
+            int i = g.first;
+            for (int u = g.b0; u < g.b1; u++) {
+                if (t_mel[u] <= 0) continue;
+                const FrontItem &it = items[i++];
+                if (audio) MB_CUDA(cudaMemcpyAsync(const_cast<float *>(it.audio), audio[u], n_samples[u] * 4, cudaMemcpyHostToDevice, copy));
+                else MB_CUDA(cudaMemcpyAsync(it.feats, feats[u], (size_t)it.t_mel * cfg.n_mels * 4, cudaMemcpyHostToDevice, copy));
+            }
+            if (gi >= copy_ev.size()) {
+                cudaEvent_t e = nullptr;
+                MB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+                copy_ev.push_back(e);
+            }
+            MB_CUDA(cudaEventRecord(copy_ev[gi], copy));
+            MB_CUDA(cudaStreamWaitEvent(stream, copy_ev[gi], 0));
+        }
+        if (audio) {
+            const int sp = prof_begin_span(PROF_MEL);
+            const int rc = log_mel_group(c, items_dev + g.first, g.n, g.max_t, mel_fb, mel_lo, mel_hi, mel_win, mel_tw, stream);
+            prof_end_span(sp);
+            if (sp >= 0) prof_launches[PROF_MEL]++;
+            if (rc) return -1;
+            note_launch(c.normalize ? 2 : 1);
+        }
+        if (subsample_group(items_dev + g.first, items + g.first, g.n, x)) return -1;
+        const FrontItem &last = items[g.first + g.n - 1];
+        x += (size_t)(last.off3 + last.T3) * d_model;
+    }
     return 0;
 }
 
@@ -321,25 +433,16 @@ int Model::subsample_item(const float *feats, int t_mel, float *x_out, int *t_ou
 int Model::encoder_layers(float *x, const std::vector<int> &lens, int left, int right, int first_layer, int n_run) {
     const int d = d_model, F = ffn_dim, B = (int)lens.size();
     int M = 0, max_len = 0;
-    std::vector<int> seg_off(B), rk_off(B);
-    std::vector<int> distinct, rk_base;        // distinct lengths and the row offset of their rk block
-    int rk_rows = 0;
-    for (int b = 0; b < B; b++) {
-        seg_off[b] = M; M += lens[b];
-        if (lens[b] > max_len) max_len = lens[b];
-        int j = -1;
-        for (size_t i = 0; i < distinct.size(); i++) if (distinct[i] == lens[b]) j = (int)i;
-        if (j < 0) { distinct.push_back(lens[b]); rk_base.push_back(rk_rows); j = (int)distinct.size() - 1; rk_rows += 2 * lens[b] - 1; }
-        rk_off[b] = rk_base[j];
-    }
+    for (int l : lens) { M += l; if (l > max_len) max_len = l; }
     if (M == 0) return 0;
+    // one table of relative positions for all lengths: row r of a segment of T frames is row max_len - T + r of the longest's
+    const int rk_rows = 2 * max_len - 1;
     const size_t mark = ws.off;
-    int *meta = ws.get<int>(3 * (size_t)B);
+    int *meta = ws.get<int>(3 * (size_t)B), *hmeta = host_stage.get<int>(3 * (size_t)B);
     if (!meta) return -1;
-    std::vector<int> hmeta(3 * B);
-    for (int b = 0; b < B; b++) { hmeta[b] = seg_off[b]; hmeta[B + b] = lens[b]; hmeta[2 * B + b] = rk_off[b]; }
-    MB_CUDA(cudaMemcpyAsync(meta, hmeta.data(), hmeta.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
-    MB_CUDA(cudaStreamSynchronize(stream));      // hmeta is a stack-lifetime buffer
+    if (!hmeta) { set_error("encoder: no room for the segment table"); return -1; }
+    for (int b = 0, off = 0; b < B; off += lens[b], b++) { hmeta[b] = off; hmeta[B + b] = lens[b]; hmeta[2 * B + b] = max_len - lens[b]; }
+    MB_CUDA(cudaMemcpyAsync(meta, hmeta, 3 * (size_t)B * sizeof(int), cudaMemcpyHostToDevice, stream));
     const int *d_off = meta, *d_len = meta + B, *d_rk = meta + 2 * B;
 
     // the single-product mode never reads the lo planes: its producers do not write them (half the bytes of every
@@ -347,12 +450,13 @@ int Model::encoder_layers(float *x, const std::vector<int> &lens, int left, int 
     const bool with_lo = cfg.strict != 0;
     H16 hA = ws.planes((size_t)M * d, with_lo), hC = ws.planes((size_t)M * d, with_lo), hF = ws.planes((size_t)M * F, with_lo);
     float *qbuf = ws.get<float>((size_t)M * d);
-    H16 kbuf = ws.planes((size_t)M * d, false), vbuf = ws.planes((size_t)M * d, false);
+    H16 kv = ws.planes((size_t)M * 2 * d, false);            // [M, k | v]
     float *h2 = ws.get<float>((size_t)M * 2 * d);
     float *cbuf = ws.get<float>((size_t)M * d);
+    const int rkl = rk_layers(rk_rows, n_run);
     H16 pe = ws.planes((size_t)rk_rows * d);
-    H16 rk = ws.planes((size_t)rk_rows * d, false);
-    if (!hA.hi || !hC.hi || !hF.hi || (with_lo && (!hA.lo || !hC.lo || !hF.lo)) || !qbuf || !kbuf.hi || !vbuf.hi || !h2 || !cbuf || !pe.lo || !rk.hi) return -1;
+    H16 rk_all = ws.planes((size_t)rk_rows * d * rkl, false);
+    if (!hA.hi || !hC.hi || !hF.hi || (with_lo && (!hA.lo || !hC.lo || !hF.lo)) || !qbuf || !kv.hi || !h2 || !cbuf || !pe.lo || !rk_all.hi) return -1;
 
     // int8-activation mode: quantised rows of the LayerNorm outputs / attention context / conv middle (qA) and of
     // SiLU(FFN1) (qF), their scales, and the f32 values that get quantised
@@ -364,29 +468,37 @@ int Model::encoder_layers(float *x, const std::vector<int> &lens, int left, int 
         sxA = ws.get<float>(M); sxF = ws.get<float>(M); fF = ws.get<float>((size_t)M * F);
         if (!qA || !qF || !sxA || !sxF || !fF) return -1;
     }
-    for (size_t i = 0; i < distinct.size(); i++) {
-        H16 p{pe.hi + (size_t)rk_base[i] * d, pe.lo + (size_t)rk_base[i] * d};
-        if (pos_emb(p, distinct[i], d, stream)) return -1;
-        note_launch();
-    }
+    if (pos_emb(pe, max_len, d, stream)) return -1;
+    note_launch();
+    // q (f32) and k | v (fp16) of a layer from one contraction
+    GemmEpilogue qkv_ep = epi(OUT_F32, ACT_NONE, 1.f, nullptr, qbuf, d, kv, 2 * d);
+    qkv_ep.n_split = d;
     const int pad_left = causal ? conv_k - 1 : (conv_k - 1) / 2;
+    // the kernels of a layer start as chained launches (common.cuh): set-up and first weight tiles overlap the kernel in
+    // front. With spans on, events between the launches keep them apart, so the figures of a span are its own.
+    const bool chain = !prof_on;
     const H16 none{nullptr, nullptr};
     for (int li = first_layer; li < first_layer + n_run; li++) {
         const EncLayer &L = layers[li];
+        const int rk_ld = rkl * d;                           // layer li's keys: columns [slot d, (slot + 1) d) of rk_all
+        __half *rk = rk_all.hi + (size_t)((li - first_layer) % rkl) * d;
+        if ((li - first_layer) % rkl == 0) {
+            QWeight w = L.relk;                              // the layers' projections sit one below the other
+            w.n = (first_layer + n_run - li < rkl ? first_layer + n_run - li : rkl) * d;
+            if (gemm(pe, d, w, epi(OUT_H16, ACT_NONE, 1.f, nullptr, nullptr, 0, rk_all, rk_ld), rk_rows)) return -1;
+        }
+        qkv_ep.bias = L.qkv.bias;
         if (a8) {
             // the same block with int8 activations into every linear (the reference with MYNAH_ASR_QGEMM=1:
             // qmat_mul quantises the input rows of each of the ten linears, src/qmat.c:615-618)
-            if (layer_norm_q8(x, L.ln_ff1_w, L.ln_ff1_b, nullptr, none, qA, sxA, M, d, ACT_NONE, stream)) return -1;
-            if (gemm_q8(qA, sxA, L.ff1_w1, epi(OUT_F32, ACT_SILU, 1.f, L.ff1_w1.bias, fF, F), M)) return -1;
-            if (act_quant_rows(fF, qF, sxF, M, F, stream)) return -1;
-            if (gemm_q8(qF, sxF, L.ff1_w2, epi(OUT_RESID, ACT_NONE, 0.5f, L.ff1_w2.bias, x, d), M)) return -1;
-            if (layer_norm_q8(x, L.ln_att_w, L.ln_att_b, nullptr, none, qA, sxA, M, d, ACT_NONE, stream)) return -1;
-            if (gemm_q8(qA, sxA, L.q_w, epi(OUT_F32, ACT_NONE, 1.f, L.q_w.bias, qbuf, d), M)) return -1;
-            if (gemm_q8(qA, sxA, L.k_w, epi(OUT_H16, ACT_NONE, 1.f, L.k_w.bias, nullptr, 0, kbuf, d), M)) return -1;
-            if (gemm_q8(qA, sxA, L.v_w, epi(OUT_H16, ACT_NONE, 1.f, L.v_w.bias, nullptr, 0, vbuf, d), M)) return -1;
-            if (gemm(pe, d, L.relk, epi(OUT_H16, ACT_NONE, 1.f, nullptr, nullptr, 0, rk, d), rk_rows)) return -1;
+            if (layer_norm_q8(x, L.ln_ff1_w, L.ln_ff1_b, nullptr, none, qA, sxA, M, d, ACT_NONE, stream, chain)) return -1;
+            if (gemm_q8(qA, sxA, L.ff1_w1, epi(OUT_F32, ACT_SILU, 1.f, L.ff1_w1.bias, fF, F), M, chain)) return -1;
+            if (act_quant_rows(fF, qF, sxF, M, F, stream, chain)) return -1;
+            if (gemm_q8(qF, sxF, L.ff1_w2, epi(OUT_RESID, ACT_NONE, 0.5f, L.ff1_w2.bias, x, d), M, chain)) return -1;
+            if (layer_norm_q8(x, L.ln_att_w, L.ln_att_b, nullptr, none, qA, sxA, M, d, ACT_NONE, stream, chain)) return -1;
+            if (gemm_q8(qA, sxA, L.qkv, qkv_ep, M, chain)) return -1;
             AttnArgs at;
-            at.q = qbuf; at.ldq = d; at.k = kbuf.hi; at.v = vbuf.hi; at.rk = rk.hi;
+            at.q = qbuf; at.ldq = d; at.k = kv.hi; at.v = kv.hi + d; at.rk = rk; at.ldkv = 2 * d; at.ldrk = rk_ld; at.chain = chain;
             at.bias_u = L.bias_u; at.bias_v = L.bias_v; at.ctx_f32 = cbuf; at.ctx_h = none;
             at.seg_off = d_off; at.seg_len = d_len; at.rk_off = d_rk;
             at.batch = B; at.max_len = max_len; at.d = d; at.H = n_heads; at.left = left; at.right = right;
@@ -396,40 +508,37 @@ int Model::encoder_layers(float *x, const std::vector<int> &lens, int left, int 
               prof_end_span(sp);
               if (sp >= 0) prof_launches[PROF_ATTN]++;
               if (rc) return -1; }
-            if (act_quant_rows(cbuf, qA, sxA, M, d, stream)) return -1;
-            if (gemm_q8(qA, sxA, L.o_w, epi(OUT_RESID, ACT_NONE, 1.f, L.o_w.bias, x, d), M)) return -1;
-            if (layer_norm_q8(x, L.ln_conv_w, L.ln_conv_b, nullptr, none, qA, sxA, M, d, ACT_NONE, stream)) return -1;
-            if (gemm_q8(qA, sxA, L.pw1_w, epi(OUT_F32, ACT_NONE, 1.f, L.pw1_w.bias, h2, 2 * d), M)) return -1;
+            if (act_quant_rows(cbuf, qA, sxA, M, d, stream, chain)) return -1;
+            if (gemm_q8(qA, sxA, L.o_w, epi(OUT_RESID, ACT_NONE, 1.f, L.o_w.bias, x, d), M, chain)) return -1;
+            if (layer_norm_q8(x, L.ln_conv_w, L.ln_conv_b, nullptr, none, qA, sxA, M, d, ACT_NONE, stream, chain)) return -1;
+            if (gemm_q8(qA, sxA, L.pw1_w, epi(OUT_F32, ACT_NONE, 1.f, L.pw1_w.bias, h2, 2 * d), M, chain)) return -1;
             if (L.cnorm_scale) {
                 if (glu_dwconv(h2, L.dw_w, L.dw_b, L.cnorm_scale, L.cnorm_shift, cbuf, none, d_off, d_len, B, max_len, d,
-                               conv_k, pad_left, stream)) return -1;
-                if (act_quant_rows(cbuf, qA, sxA, M, d, stream)) return -1;
+                               conv_k, pad_left, stream, chain)) return -1;
+                if (act_quant_rows(cbuf, qA, sxA, M, d, stream, chain)) return -1;
             } else {
                 if (glu_dwconv(h2, L.dw_w, L.dw_b, nullptr, nullptr, cbuf, none, d_off, d_len, B, max_len, d, conv_k,
-                               pad_left, stream)) return -1;
-                if (layer_norm_q8(cbuf, L.cnorm_w, L.cnorm_b, nullptr, none, qA, sxA, M, d, ACT_SILU, stream)) return -1;
+                               pad_left, stream, chain)) return -1;
+                if (layer_norm_q8(cbuf, L.cnorm_w, L.cnorm_b, nullptr, none, qA, sxA, M, d, ACT_SILU, stream, chain)) return -1;
             }
-            if (gemm_q8(qA, sxA, L.pw2_w, epi(OUT_RESID, ACT_NONE, 1.f, L.pw2_w.bias, x, d), M)) return -1;
-            if (layer_norm_q8(x, L.ln_ff2_w, L.ln_ff2_b, nullptr, none, qA, sxA, M, d, ACT_NONE, stream)) return -1;
-            if (gemm_q8(qA, sxA, L.ff2_w1, epi(OUT_F32, ACT_SILU, 1.f, L.ff2_w1.bias, fF, F), M)) return -1;
-            if (act_quant_rows(fF, qF, sxF, M, F, stream)) return -1;
-            if (gemm_q8(qF, sxF, L.ff2_w2, epi(OUT_RESID, ACT_NONE, 0.5f, L.ff2_w2.bias, x, d), M)) return -1;
-            if (layer_norm(x, L.ln_out_w, L.ln_out_b, x, none, M, d, ACT_NONE, stream)) return -1;
+            if (gemm_q8(qA, sxA, L.pw2_w, epi(OUT_RESID, ACT_NONE, 1.f, L.pw2_w.bias, x, d), M, chain)) return -1;
+            if (layer_norm_q8(x, L.ln_ff2_w, L.ln_ff2_b, nullptr, none, qA, sxA, M, d, ACT_NONE, stream, chain)) return -1;
+            if (gemm_q8(qA, sxA, L.ff2_w1, epi(OUT_F32, ACT_SILU, 1.f, L.ff2_w1.bias, fF, F), M, chain)) return -1;
+            if (act_quant_rows(fF, qF, sxF, M, F, stream, chain)) return -1;
+            if (gemm_q8(qF, sxF, L.ff2_w2, epi(OUT_RESID, ACT_NONE, 0.5f, L.ff2_w2.bias, x, d), M, chain)) return -1;
+            if (layer_norm(x, L.ln_out_w, L.ln_out_b, x, none, M, d, ACT_NONE, stream, chain)) return -1;
             note_launch(11);   // 5 LayerNorms + attention + glu_dwconv + 4 activation quantisations (the contractions count themselves)
             continue;
         }
         // half FFN 1 (src/encoder.c:464-482,495-496)
-        if (layer_norm(x, L.ln_ff1_w, L.ln_ff1_b, nullptr, hA, M, d, ACT_NONE, stream)) return -1;
-        if (gemm(hA, d, L.ff1_w1, epi(OUT_H16, ACT_SILU, 1.f, L.ff1_w1.bias, nullptr, 0, hF, F), M)) return -1;
-        if (gemm(hF, F, L.ff1_w2, epi(OUT_RESID, ACT_NONE, 0.5f, L.ff1_w2.bias, x, d), M)) return -1;
+        if (layer_norm(x, L.ln_ff1_w, L.ln_ff1_b, nullptr, hA, M, d, ACT_NONE, stream, chain)) return -1;
+        if (gemm(hA, d, L.ff1_w1, epi(OUT_H16, ACT_SILU, 1.f, L.ff1_w1.bias, nullptr, 0, hF, F), M, false, chain)) return -1;
+        if (gemm(hF, F, L.ff1_w2, epi(OUT_RESID, ACT_NONE, 0.5f, L.ff1_w2.bias, x, d), M, false, chain)) return -1;
         // rel-pos MHSA (src/encoder.c:315-410,501-503)
-        if (layer_norm(x, L.ln_att_w, L.ln_att_b, nullptr, hA, M, d, ACT_NONE, stream)) return -1;
-        if (gemm(hA, d, L.q_w, epi(OUT_F32, ACT_NONE, 1.f, L.q_w.bias, qbuf, d), M)) return -1;
-        if (gemm(hA, d, L.k_w, epi(OUT_H16, ACT_NONE, 1.f, L.k_w.bias, nullptr, 0, kbuf, d), M)) return -1;
-        if (gemm(hA, d, L.v_w, epi(OUT_H16, ACT_NONE, 1.f, L.v_w.bias, nullptr, 0, vbuf, d), M)) return -1;
-        if (gemm(pe, d, L.relk, epi(OUT_H16, ACT_NONE, 1.f, nullptr, nullptr, 0, rk, d), rk_rows)) return -1;
+        if (layer_norm(x, L.ln_att_w, L.ln_att_b, nullptr, hA, M, d, ACT_NONE, stream, chain)) return -1;
+        if (gemm(hA, d, L.qkv, qkv_ep, M, false, chain)) return -1;
         AttnArgs at;
-        at.q = qbuf; at.ldq = d; at.k = kbuf.hi; at.v = vbuf.hi; at.rk = rk.hi;
+        at.q = qbuf; at.ldq = d; at.k = kv.hi; at.v = kv.hi + d; at.rk = rk; at.ldkv = 2 * d; at.ldrk = rk_ld; at.chain = chain;
         at.bias_u = L.bias_u; at.bias_v = L.bias_v; at.ctx_f32 = nullptr; at.ctx_h = hC;
         at.seg_off = d_off; at.seg_len = d_len; at.rk_off = d_rk;
         at.batch = B; at.max_len = max_len; at.d = d; at.H = n_heads; at.left = left; at.right = right;
@@ -439,29 +548,36 @@ int Model::encoder_layers(float *x, const std::vector<int> &lens, int left, int 
           prof_end_span(sp);
           if (sp >= 0) prof_launches[PROF_ATTN]++;
           if (rc) return -1; }
-        if (gemm(hC, d, L.o_w, epi(OUT_RESID, ACT_NONE, 1.f, L.o_w.bias, x, d), M)) return -1;
+        if (gemm(hC, d, L.o_w, epi(OUT_RESID, ACT_NONE, 1.f, L.o_w.bias, x, d), M, false, chain)) return -1;
         // conv module (src/encoder.c:413-460,506-508)
-        if (layer_norm(x, L.ln_conv_w, L.ln_conv_b, nullptr, hA, M, d, ACT_NONE, stream)) return -1;
-        if (gemm(hA, d, L.pw1_w, epi(OUT_F32, ACT_NONE, 1.f, L.pw1_w.bias, h2, 2 * d), M)) return -1;
+        if (layer_norm(x, L.ln_conv_w, L.ln_conv_b, nullptr, hA, M, d, ACT_NONE, stream, chain)) return -1;
+        if (gemm(hA, d, L.pw1_w, epi(OUT_F32, ACT_NONE, 1.f, L.pw1_w.bias, h2, 2 * d), M, false, chain)) return -1;
         if (L.cnorm_scale) {
             if (glu_dwconv(h2, L.dw_w, L.dw_b, L.cnorm_scale, L.cnorm_shift, nullptr, hC, d_off, d_len, B, max_len, d,
-                           conv_k, pad_left, stream)) return -1;
+                           conv_k, pad_left, stream, chain)) return -1;
         } else {
             if (glu_dwconv(h2, L.dw_w, L.dw_b, nullptr, nullptr, cbuf, none, d_off, d_len, B, max_len, d, conv_k,
-                           pad_left, stream)) return -1;
-            if (layer_norm(cbuf, L.cnorm_w, L.cnorm_b, nullptr, hC, M, d, ACT_SILU, stream)) return -1;
+                           pad_left, stream, chain)) return -1;
+            if (layer_norm(cbuf, L.cnorm_w, L.cnorm_b, nullptr, hC, M, d, ACT_SILU, stream, chain)) return -1;
             note_launch();
         }
-        if (gemm(hC, d, L.pw2_w, epi(OUT_RESID, ACT_NONE, 1.f, L.pw2_w.bias, x, d), M)) return -1;
+        if (gemm(hC, d, L.pw2_w, epi(OUT_RESID, ACT_NONE, 1.f, L.pw2_w.bias, x, d), M, false, chain)) return -1;
         // half FFN 2 + output LayerNorm (src/encoder.c:510-516)
-        if (layer_norm(x, L.ln_ff2_w, L.ln_ff2_b, nullptr, hA, M, d, ACT_NONE, stream)) return -1;
-        if (gemm(hA, d, L.ff2_w1, epi(OUT_H16, ACT_SILU, 1.f, L.ff2_w1.bias, nullptr, 0, hF, F), M)) return -1;
-        if (gemm(hF, F, L.ff2_w2, epi(OUT_RESID, ACT_NONE, 0.5f, L.ff2_w2.bias, x, d), M)) return -1;
-        if (layer_norm(x, L.ln_out_w, L.ln_out_b, x, none, M, d, ACT_NONE, stream)) return -1;
+        if (layer_norm(x, L.ln_ff2_w, L.ln_ff2_b, nullptr, hA, M, d, ACT_NONE, stream, chain)) return -1;
+        if (gemm(hA, d, L.ff2_w1, epi(OUT_H16, ACT_SILU, 1.f, L.ff2_w1.bias, nullptr, 0, hF, F), M, false, chain)) return -1;
+        if (gemm(hF, F, L.ff2_w2, epi(OUT_RESID, ACT_NONE, 0.5f, L.ff2_w2.bias, x, d), M, false, chain)) return -1;
+        if (layer_norm(x, L.ln_out_w, L.ln_out_b, x, none, M, d, ACT_NONE, stream, chain)) return -1;
         note_launch(7);   // 5 LayerNorms + attention + glu_dwconv (the contractions count themselves)
     }
     ws.off = mark;
     return 0;
+}
+
+int Model::rk_layers(int rk_rows, int n_run) const {
+    static constexpr size_t RK_BYTES = 512u << 20;
+    const size_t per = (size_t)rk_rows * d_model * 2;
+    const size_t fit = per ? RK_BYTES / per : 1;
+    return fit < 1 ? 1 : fit < (size_t)n_run ? (int)fit : n_run;
 }
 
 // encoder_projector when present, else copy (src/encoder.c:573-590)

@@ -34,9 +34,29 @@ struct Arena {
     void release();
 };
 
+// Pinned host memory for the small tables of a call (and what they are copied from): taken in order, reset when the call
+// begins, which is after the previous one has waited for its stream.
+struct HostStage {
+    uint8_t *base = nullptr;
+    size_t cap = 0, off = 0;
+    int begin(size_t bytes);
+    template <typename T> T *get(size_t n) { const size_t o = align_up(off, 64); off = o + n * sizeof(T); return off <= cap ? reinterpret_cast<T *>(base + o) : nullptr; }
+    void release();
+};
+
+// One utterance of a batched front end. Offsets are rows of the packed tensors of its group.
+struct FrontItem {
+    const float *audio;          // device, n_samples; null: the features are given
+    long long n_samples;
+    float *feats;                // [t_mel, n_mels]
+    int t_mel, T1, T2, T3;       // frames before and after each stride-2 stage
+    int off2, off3;              // first stage-1 and stage-2 frame in the group
+};
+
 struct EncLayer {
     const float *ln_ff1_w, *ln_ff1_b, *ln_att_w, *ln_att_b, *ln_conv_w, *ln_conv_b, *ln_ff2_w, *ln_ff2_b, *ln_out_w, *ln_out_b;
     QWeight ff1_w1, ff1_w2, ff2_w1, ff2_w2, q_w, k_w, v_w, o_w, pw1_w, pw2_w, relk;
+    QWeight qkv;                 // q_w, k_w, v_w one below the other ([3 d, d]): their operands sit in one block
     const float *bias_u, *bias_v, *dw_w, *dw_b, *cnorm_w, *cnorm_b, *cnorm_scale, *cnorm_shift;
 };
 
@@ -95,6 +115,9 @@ struct Model {
     bool finalized = false;
     cudaStream_t stream = nullptr;                   // of this execution context (the weights are shared between contexts)
     Arena ws;
+    HostStage host_stage;
+    cudaStream_t copy = nullptr;                     // host-to-device copies that overlap the kernels of earlier utterances
+    std::vector<cudaEvent_t> copy_ev;
     int *status = nullptr;                           // device status word (bounded waits)
 
     // optional per-category device timing (CUDA events on `stream` around launches)
@@ -186,12 +209,21 @@ struct Model {
     int check_status(const char *where);
 
     // drivers (device pointers in / out, all on `stream`)
-    int gemm(const H16 &a, int lda, const QWeight &w, const GemmEpilogue &ep, int M, bool few_rows = false);   // few_rows: the decoder-position kernel (gemm_skinny.cu)
+    int gemm(const H16 &a, int lda, const QWeight &w, const GemmEpilogue &ep, int M, bool few_rows = false, bool chain = false);   // few_rows: the decoder-position kernel (gemm_skinny.cu)
     // int8-activation mode: qa [M, w.k] int8 rows with their scales sx [M] times a reference-native int8 weight
     bool a8_ok(const QWeight &w) const { return w.fmt == FMT_MYNAH_Q8 && w.k % 128 == 0 && w.scales != nullptr; }
     bool a8_layers = false;                          // cfg.a8 and every encoder-layer linear is a8_ok
-    int gemm_q8(const int8_t *qa, const float *sx, const QWeight &w, const GemmEpilogue &ep, int M);
-    int subsample_item(const float *feats_dev, int t_mel, float *x_out, int *t_out);
+    int gemm_q8(const int8_t *qa, const float *sx, const QWeight &w, const GemmEpilogue &ep, int M, bool chain = false);
+    // Audio (or features) of a batch -> packed encoder input x_out [sum T, d_model]; lens receives the frames. audio[b] /
+    // feats[b] may be host or device memory (`on_host`); exactly one of the two lists is given. Utterances go through in groups
+    // of about a minute of audio: one launch of every front-end kernel per group, the copies of the next group meanwhile.
+    int front_end(const float *const *audio, const size_t *n_samples, const float *const *feats, const int *t_mel, int batch,
+                  bool on_host, float *x_out, std::vector<int> &lens);
+    size_t front_bytes(const size_t *n_samples, const int *t_mel, int batch, bool audio, bool on_host) const;
+    std::vector<int> front_groups(const int *t_mel, int batch) const;          // end index of every group
+    int subsample_group(const FrontItem *items_dev, const FrontItem *items, int n, float *x_out);
+    // layers whose rel-pos key projections are made by one contraction: all of them unless that takes too much memory
+    int rk_layers(int rk_rows, int n_run) const;
     int encoder_layers(float *x, const std::vector<int> &lens, int left, int right, int first_layer, int n_run);
     // x [sum lens, d_model] -> out [sum lens, d_out]; prompt_ids (one per segment, may be null = all 0) select the
     // one-hot column of a prompt-conditioned model and are ignored otherwise

@@ -297,6 +297,12 @@ int qgemv(const QWeight &w, const float *x, int ldx, float *out, int ldo, const 
 // ------------------------------------------------------------------- A8 mode
 // One warp per (row t, weight row): lanes own one 32-block each per 1024 slice.
 // Activation rows are quantised once by act_quant_kernel.
+__device__ __forceinline__ int8_t act_quant_1(float x, float inv) {
+    const float v = __fmul_rn(x, inv);
+    int q = (int)(v >= 0.0f ? __fadd_rn(v, 0.5f) : __fsub_rn(v, 0.5f));
+    q = q > 127 ? 127 : (q < -127 ? -127 : q);
+    return (int8_t)q;
+}
 __global__ void __launch_bounds__(256)
 act_quant_kernel(const float *__restrict__ x, int8_t *__restrict__ qx, float *__restrict__ sx, int T, int k) {
     const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -305,19 +311,39 @@ act_quant_kernel(const float *__restrict__ x, int8_t *__restrict__ qx, float *__
     float amax = 0.0f;
     for (int i = lane; i < k; i += 32) amax = fmaxf(amax, fabsf(xr[i]));
     amax = warp_max(amax);
-    if (amax == 0.0f) {
-        for (int i = lane; i < k; i += 32) qx[(size_t)t * k + i] = 0;
-        if (lane == 0) sx[t] = 0.0f;
-        return;
-    }
-    const float inv = 127.0f / amax;
-    for (int i = lane; i < k; i += 32) {
-        const float v = __fmul_rn(xr[i], inv);
-        int q = (int)(v >= 0.0f ? __fadd_rn(v, 0.5f) : __fsub_rn(v, 0.5f));
-        q = q > 127 ? 127 : (q < -127 ? -127 : q);
-        qx[(size_t)t * k + i] = (int8_t)q;
-    }
+    const float inv = amax == 0.0f ? 0.0f : 127.0f / amax;
+    for (int i = lane; i < k; i += 32) qx[(size_t)t * k + i] = act_quant_1(xr[i], inv);
     if (lane == 0) sx[t] = amax / 127.0f;
+}
+// The same rows, bound by HBM: W warps hold a row in registers (k = W * NV * 128), so x is read once, in 16-byte pieces.
+template <int W, int NV>
+__global__ void __launch_bounds__(256)
+act_quant_vec_kernel(const float *__restrict__ x, int8_t *__restrict__ qx, float *__restrict__ sx, int T) {
+    constexpr int k = W * NV * 128, ROWS = 8 / W;
+    __shared__ float part[8];
+    chain_trigger();
+    chain_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x * ROWS + warp / W;
+    const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)(t < T ? t : 0) * k) + (warp % W) * NV * 32 + lane;
+    float4 v[NV];
+    float amax = 0.0f;
+#pragma unroll
+    for (int j = 0; j < NV; j++) v[j] = xr[32 * j];
+#pragma unroll
+    for (int j = 0; j < NV; j++) amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+    amax = warp_max(amax);
+    if (W > 1) {
+        if (lane == 0) part[warp] = amax;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < W; i++) amax = fmaxf(amax, part[warp / W * W + i]);
+    }
+    if (t >= T) return;
+    const float inv = amax == 0.0f ? 0.0f : 127.0f / amax;
+    char4 *q = reinterpret_cast<char4 *>(qx + (size_t)t * k) + (warp % W) * NV * 32 + lane;
+#pragma unroll
+    for (int j = 0; j < NV; j++) q[32 * j] = make_char4(act_quant_1(v[j].x, inv), act_quant_1(v[j].y, inv), act_quant_1(v[j].z, inv), act_quant_1(v[j].w, inv));
+    if (warp % W == 0 && lane == 0) sx[t] = amax / 127.0f;
 }
 
 template <int FMT>
@@ -392,8 +418,16 @@ qgemv_a8_kernel(const uint8_t *__restrict__ raw, const float *__restrict__ scale
     }
 }
 
-int act_quant_rows(const float *x, int8_t *qx, float *sx, int T, int k, cudaStream_t st) {
+int act_quant_rows(const float *x, int8_t *qx, float *sx, int T, int k, cudaStream_t st, bool chain) {
     if (T <= 0) return 0;
+    const bool al = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(qx) & 3) == 0;
+#define AQ_VEC(W, NV) MB_CUDA(launch_kernel(act_quant_vec_kernel<W, NV>, dim3(cdiv(T, 8 / W)), dim3(256), 0, st, chain, 1, x, qx, sx, T))
+    if (al && k == 512) AQ_VEC(1, 4);
+    else if (al && k == 1024) AQ_VEC(1, 8);
+    else if (al && k == 2048) AQ_VEC(4, 4);
+    else if (al && k == 4096) AQ_VEC(4, 8);
+    else
+#undef AQ_VEC
     act_quant_kernel<<<cdiv(T, 8), 256, 0, st>>>(x, qx, sx, T, k);
     MB_CUDA(cudaGetLastError());
     return 0;

@@ -12,6 +12,7 @@
 //     c*F'+f to f*C+c).
 // Zero padding: causal (2 left, 1 right) or symmetric (1, 1) on both axes.
 #include "kernels.h"
+#include "model.h"
 
 namespace mb {
 
@@ -59,12 +60,24 @@ int conv_in_relu(const float *feats, const float *w, const float *b, float *out,
 // Stage-0 positions outside [0,T1) x [0,F1) are the depthwise conv's own zero padding.
 static constexpr int FUSE_F2 = 8;      // stage-1 frequency positions per CTA
 
+// the utterance of a group that packed frame `row` of stage 1 (or 2) belongs to
+__device__ __forceinline__ int front_find(const FrontItem *__restrict__ items, int n, int row, bool stage2) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if ((stage2 ? items[mid].off3 : items[mid].off2) <= row) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
 __global__ void __launch_bounds__(256)
-conv_in_dw_kernel(const float *__restrict__ x, const float *__restrict__ w0, const float *__restrict__ b0,
+conv_in_dw_kernel(const FrontItem *__restrict__ items, int n_items, const float *__restrict__ w0, const float *__restrict__ b0,
                   const float *__restrict__ w1, const float *__restrict__ b1, __half *__restrict__ hi,
-                  __half *__restrict__ lo, int T, int F, int C, int T1, int F1, int T2, int F2, int pl) {
+                  __half *__restrict__ lo, int F, int C, int F1, int F2, int pl) {
     __shared__ __align__(16) float patch[7][4 * FUSE_F2 + 4];
-    const int t2 = blockIdx.y, f2base = blockIdx.x * FUSE_F2;
+    const FrontItem &item = items[front_find(items, n_items, blockIdx.y, false)];
+    const float *__restrict__ x = item.feats;
+    const int T = item.t_mel, T1 = item.T1, t2 = blockIdx.y - item.off2, f2base = blockIdx.x * FUSE_F2;
     // stage-0 rows 2*t2 - pl + {0,1,2} need input rows 2*(that) - pl + {0,1,2}
     const int trow0 = 2 * (2 * t2 - pl) - pl;           // first input row of the patch
     const int fcol0 = 2 * (2 * f2base - pl) - pl;       // first input column of the patch
@@ -112,31 +125,34 @@ conv_in_dw_kernel(const float *__restrict__ x, const float *__restrict__ w0, con
             }
             __half h, l;
             split_h16(bias1 + acc, h, l);
-            const size_t o = ((size_t)t2 * F2 + f2) * C + c;
+            const size_t o = ((size_t)blockIdx.y * F2 + f2) * C + c;
             hi[o] = h;
             lo[o] = l;
         }
     }
 }
 
-int conv_in_dw_fused(const float *feats, const float *w0, const float *b0, const float *w1, const float *b1, H16 out,
-                     int T, int F, int C, int T1, int F1, int T2, int F2, int pl, cudaStream_t st) {
-    if (T2 <= 0 || F2 <= 0) return 0;
-    dim3 grid(cdiv(F2, FUSE_F2), T2);
-    conv_in_dw_kernel<<<grid, 256, 0, st>>>(feats, w0, b0, w1, b1, out.hi, out.lo, T, F, C, T1, F1, T2, F2, pl);
+int conv_in_dw_fused(const FrontItem *items, int n_items, int rows2, const float *w0, const float *b0, const float *w1, const float *b1,
+                     H16 out, int F, int C, int F1, int F2, int pl, cudaStream_t st) {
+    if (rows2 <= 0 || F2 <= 0) return 0;
+    dim3 grid(cdiv(F2, FUSE_F2), rows2);
+    conv_in_dw_kernel<<<grid, 256, 0, st>>>(items, n_items, w0, b0, w1, b1, out.hi, out.lo, F, C, F1, F2, pl);
     MB_CUDA(cudaGetLastError());
     return 0;
 }
 
 // stages 1-2: depthwise 3x3 stride 2 + bias.   x [T,F,C] f32 -> (hi,lo) [To*Fo, C]
 __global__ void __launch_bounds__(256)
-dw3x3_kernel(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ b,
-             __half *__restrict__ hi, __half *__restrict__ lo, int T, int F, int C, int To, int Fo, int pl) {
-    const size_t total = (size_t)To * Fo * C;
+dw3x3_kernel(const FrontItem *__restrict__ items, int n_items, int rows3, const float *__restrict__ x_all, const float *__restrict__ w,
+             const float *__restrict__ b, __half *__restrict__ hi, __half *__restrict__ lo, int F, int C, int Fo, int pl) {
+    const size_t total = (size_t)rows3 * Fo * C;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const int c = (int)(i % C);
         const int fo = (int)((i / C) % Fo);
-        const int to = (int)(i / ((size_t)C * Fo));
+        const int row = (int)(i / ((size_t)C * Fo));
+        const FrontItem &item = items[front_find(items, n_items, row, true)];
+        const int to = row - item.off3, T = item.T2;
+        const float *x = x_all + (size_t)item.off2 * F * C;
         float acc = 0.0f;
 #pragma unroll
         for (int dt = 0; dt < 3; dt++) {
@@ -156,12 +172,12 @@ dw3x3_kernel(const float *__restrict__ x, const float *__restrict__ w, const flo
     }
 }
 
-int dwconv3x3_s2(const float *x, const float *w, const float *b, H16 out, int T, int F, int C, int To, int Fo, int pl,
-                 cudaStream_t st) {
-    const size_t total = (size_t)To * Fo * C;
+int dwconv3x3_s2(const FrontItem *items, int n_items, int rows3, const float *x, const float *w, const float *b, H16 out, int F, int C,
+                 int Fo, int pl, cudaStream_t st) {
+    const size_t total = (size_t)rows3 * Fo * C;
     if (total == 0) return 0;
     const unsigned blocks = (unsigned)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-    dw3x3_kernel<<<blocks, 256, 0, st>>>(x, w, b, out.hi, out.lo, T, F, C, To, Fo, pl);
+    dw3x3_kernel<<<blocks, 256, 0, st>>>(items, n_items, rows3, x, w, b, out.hi, out.lo, F, C, Fo, pl);
     MB_CUDA(cudaGetLastError());
     return 0;
 }
