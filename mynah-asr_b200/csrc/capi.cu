@@ -219,11 +219,11 @@ const char *mynah_b200_last_error(void) { return mb::last_error(); }
 int mynah_b200_available(void) {
     int n = 0;
     if (cudaGetDeviceCount(&n) != cudaSuccess || n <= 0) { cudaGetLastError(); return 0; }
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceProp p;
-    if (cudaGetDeviceProperties(&p, dev) != cudaSuccess) { cudaGetLastError(); return 0; }
-    return p.major == 10 && p.minor == 0 ? 1 : 0;      // the library holds sm_100a code only
+    int dev = 0, major = 0, minor = 0;
+    cudaGetDevice(&dev);                               // two attributes: the whole property block takes milliseconds to fill
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return major == 10 && minor == 0 ? 1 : 0;          // the library holds sm_100a code only
 }
 
 int mynah_b200_select_device(int index) {

@@ -10,8 +10,10 @@
 //   * vad_encode_kernel runs everything of the network that does not depend on the recurrent state for ALL frames
 //     at once (one CTA per frame): lookbehind | frame | reflect pad -> STFT as a product with the basis -> magnitude
 //     -> the conv + ReLU blocks -> the LSTM's input contribution b_ih + b_hh + W_ih x;
-//   * vad_lstm_kernel walks the frames in order with one CTA: thread r keeps row r of W_hh in registers, the state
-//     lives in shared memory, and the head (ReLU -> 1x1 conv -> sigmoid) gives the frame's probability;
+//     (vad_encode16_kernel for the geometry of the published models, vad_encode_kernel for any other);
+//   * vad_lstm_kernel walks the frames in order with one cluster of eight CTAs that hold W_hh in registers and exchange
+//     the state through distributed shared memory; vad_head_kernel (ReLU -> 1x1 conv -> sigmoid) then gives the
+//     probabilities of all frames at once;
 //   * window_energy_kernel forms the double-precision sum of squares of every candidate 20 ms window of a search
 //     range, one thread per window, in the reference's summation order (so the minimum falls on the same window);
 //   * the decisions that are integer / double logic over those numbers — hysteresis, padding, widening, merging,
@@ -19,6 +21,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <mutex>
 #include <vector>
 
 #include "../../include/mynah_b200.h"
@@ -36,17 +39,19 @@ struct VadDev {
     const float *basis, *enc_w[VAD_MAX_ENC], *enc_b[VAD_MAX_ENC], *w_ih, *w_hh, *b_ih, *b_hh, *head_w;
     float head_b;
     int act_max;                       // floats of the larger activation buffer
+    // the published geometry: weights with the output row fastest (vad_encode16_kernel), else null
+    const float *basis_t, *basis_ny, *enc_t[4], *w_ih_t;
 };
 
 __device__ __forceinline__ int conv_len(int t_in, int k, int stride, int pl, int pr) { return (t_in + pl + pr - k) / stride + 1; }
 
 // One CTA per frame. Shared memory: buf [context + frame + pad] | spec [2 n_bins stft_frames] | act0 | act1.
 __global__ void __launch_bounds__(256)
-vad_encode_kernel(const VadDev v, const float *__restrict__ audio, long long n_samples, float *__restrict__ xz) {
+vad_encode_kernel(const VadDev v, const float *__restrict__ audio, long long n_samples, int frame0, float *__restrict__ xz) {
     extern __shared__ float sm[];
     const int C = v.context, F = v.frame, P = v.pad, N = C + F, T0 = v.stft_frames, B = v.n_bins;
     float *buf = sm, *spec = buf + N + P, *act0 = spec + 2 * B * T0, *act1 = act0 + v.act_max;
-    const long long f = blockIdx.x, base = f * F;
+    const long long f = blockIdx.x, base = (frame0 + f) * F;
     for (int i = threadIdx.x; i < N; i += blockDim.x) {
         const long long s = base - C + i;        // the lookbehind is the tail of the previous frame (zeros before the signal)
         buf[i] = (s >= 0 && s < n_samples) ? audio[s] : 0.0f;
@@ -98,48 +103,357 @@ vad_encode_kernel(const VadDev v, const float *__restrict__ audio, long long n_s
     }
 }
 
+// The same for the published geometry (512-sample frames behind 64 samples of context, 256-point windows every 128
+// samples, four blocks of three taps with strides 1 2 2 1 and 128 64 64 128 channels), sixteen frames per CTA.
+// One frame per CTA reads every weight (0.9 MB) once per frame, one scalar at a time: 7.9 ms for five minutes of audio.
+// Here a lane owns output rows and a warp two frames: weights come in whole lines, with the output row fastest, and feed
+// all columns of the warp from a register; inputs are 16-byte broadcasts. Bound by the f32 FMA rate: 1.3 ms in pieces of
+// 64 CTAs under the recurrence, 0.17 at full rate. Every sum runs in the order of vad_encode_kernel, so the bits are the same.
+constexpr int VE_F = 16, VE_N = 576, VE_BUF = VE_N + 64 + 4, VE_THREADS = 256;
+constexpr int VE_MAG = 129 * 4 + 4;            // floats of one frame's magnitudes [bin][window], padded
+constexpr int VE_C0 = 128 * 4 + 4, VE_C1 = 64 * 2 + 4, VE_C2 = 64 + 4, VE_C3 = 128 + 4;
+constexpr int VE_SMEM = VE_F * (VE_BUF + VE_MAG + VE_C0) * 4;
+
+__global__ void __launch_bounds__(VE_THREADS, 2)
+vad_encode16_kernel(const VadDev v, const float *__restrict__ audio, long long n_samples, int frame0, int frames, float *__restrict__ xz) {
+    extern __shared__ __align__(16) float sm[];
+    float *buf = sm, *mag = buf + VE_F * VE_BUF, *c0 = mag + VE_F * VE_MAG, *c1 = buf, *c2 = c1 + VE_F * VE_C1, *c3 = c2 + VE_F * VE_C2;
+    const int f0 = frame0 + blockIdx.x * VE_F, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < VE_F * VE_N; i += VE_THREADS) {
+        const int f = i / VE_N, j = i % VE_N;
+        const long long s = (long long)(f0 + f) * 512 - 64 + j;
+        buf[f * VE_BUF + j] = (s >= 0 && s < n_samples) ? audio[s] : 0.0f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < VE_F * 64; i += VE_THREADS) {
+        const int f = i / 64, j = i % 64;
+        buf[f * VE_BUF + VE_N + j] = buf[f * VE_BUF + VE_N - 2 - j];
+    }
+    __syncthreads();
+    const int fa = 2 * warp;                                    // this warp's frames: fa, fa + 1
+    {   // bins 0..127: re and im rows of four bins per lane, eight windows
+        float re[4][8], im[4][8];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int c = 0; c < 8; c++) re[i][c] = im[i][c] = 0.0f;
+        const float *w = v.basis_t + lane;
+#pragma unroll 1
+        for (int k = 0; k < 256; k += 4) {
+            float4 x[8];
+#pragma unroll
+            for (int c = 0; c < 8; c++) x[c] = *reinterpret_cast<const float4 *>(buf + (fa + (c >> 2)) * VE_BUF + (c & 3) * 128 + k);
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) {
+                float wr[4], wi[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) { wr[i] = __ldg(w + (k + kk) * 256 + 32 * i); wi[i] = __ldg(w + (k + kk) * 256 + 128 + 32 * i); }
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    const float xv = kk == 0 ? x[c].x : kk == 1 ? x[c].y : kk == 2 ? x[c].z : x[c].w;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) { re[i][c] = fmaf(wr[i], xv, re[i][c]); im[i][c] = fmaf(wi[i], xv, im[i][c]); }
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float m[4];
+#pragma unroll
+                for (int t = 0; t < 4; t++) m[t] = sqrtf(re[i][4 * h + t] * re[i][4 * h + t] + im[i][4 * h + t] * im[i][4 * h + t]);
+                *reinterpret_cast<float4 *>(mag + (fa + h) * VE_MAG + (lane + 32 * i) * 4) = make_float4(m[0], m[1], m[2], m[3]);
+            }
+        // bin 128: a lane per window of this warp
+        if (lane < 8) {
+            const float *x = buf + (fa + (lane >> 2)) * VE_BUF + (lane & 3) * 128;
+            float r = 0.0f, q = 0.0f;
+            for (int k = 0; k < 256; k++) { r = fmaf(__ldg(v.basis_ny + k), x[k], r); q = fmaf(__ldg(v.basis_ny + 256 + k), x[k], q); }
+            mag[(fa + (lane >> 2)) * VE_MAG + 128 * 4 + (lane & 3)] = sqrtf(r * r + q * q);
+        }
+    }
+    __syncwarp();                                               // from here on a warp reads only what it wrote itself
+    {   // block 0: 129 -> 128 channels, four steps, taps t-1, t, t+1
+        float acc[4][8];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int c = 0; c < 8; c++) acc[i][c] = 0.0f;
+        const float *w = v.enc_t[0] + lane;
+#pragma unroll 1
+        for (int ci = 0; ci < 129; ci++) {
+            float x[2][4];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float4 q = *reinterpret_cast<const float4 *>(mag + (fa + h) * VE_MAG + ci * 4);
+                x[h][0] = q.x; x[h][1] = q.y; x[h][2] = q.z; x[h][3] = q.w;
+            }
+#pragma unroll
+            for (int kk = 0; kk < 3; kk++) {
+                float wv[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) wv[i] = __ldg(w + (ci * 3 + kk) * 128 + 32 * i);
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    const int s = (c & 3) - 1 + kk;
+                    if (s < 0 || s > 3) continue;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) acc[i][c] = fmaf(wv[i], x[c >> 2][s], acc[i][c]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float b = v.enc_b[0][lane + 32 * i];
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                *reinterpret_cast<float4 *>(c0 + (fa + h) * VE_C0 + (lane + 32 * i) * 4) =
+                    make_float4(fmaxf(acc[i][4 * h] + b, 0.0f), fmaxf(acc[i][4 * h + 1] + b, 0.0f), fmaxf(acc[i][4 * h + 2] + b, 0.0f), fmaxf(acc[i][4 * h + 3] + b, 0.0f));
+        }
+    }
+    __syncthreads();                                            // c1..c3 lie over the samples
+    {   // block 1: 128 -> 64, steps 0 and 1 at 2 t - 1 + kk
+        float acc[2][2][2];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) acc[i][h][0] = acc[i][h][1] = 0.0f;
+        const float *w = v.enc_t[1] + lane;
+#pragma unroll 2
+        for (int ci = 0; ci < 128; ci++) {
+            float x[2][4];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float4 q = *reinterpret_cast<const float4 *>(c0 + (fa + h) * VE_C0 + ci * 4);
+                x[h][0] = q.x; x[h][1] = q.y; x[h][2] = q.z; x[h][3] = q.w;
+            }
+#pragma unroll
+            for (int kk = 0; kk < 3; kk++) {
+                const float w0 = __ldg(w + (ci * 3 + kk) * 64), w1 = __ldg(w + (ci * 3 + kk) * 64 + 32);
+#pragma unroll
+                for (int t = 0; t < 2; t++) {
+                    const int s = 2 * t - 1 + kk;
+                    if (s < 0) continue;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) { acc[0][h][t] = fmaf(w0, x[h][s], acc[0][h][t]); acc[1][h][t] = fmaf(w1, x[h][s], acc[1][h][t]); }
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float b = v.enc_b[1][lane + 32 * i];
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                *reinterpret_cast<float2 *>(c1 + (fa + h) * VE_C1 + (lane + 32 * i) * 2) = make_float2(fmaxf(acc[i][h][0] + b, 0.0f), fmaxf(acc[i][h][1] + b, 0.0f));
+        }
+    }
+    __syncwarp();
+    {   // block 2: 64 -> 64, one step: taps 1 and 2 fall on steps 0 and 1
+        float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+        const float *w = v.enc_t[2] + lane;
+#pragma unroll 4
+        for (int ci = 0; ci < 64; ci++) {
+            const float2 xa = *reinterpret_cast<const float2 *>(c1 + fa * VE_C1 + ci * 2), xb = *reinterpret_cast<const float2 *>(c1 + (fa + 1) * VE_C1 + ci * 2);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const float w1 = __ldg(w + (ci * 3 + 1) * 64 + 32 * i), w2 = __ldg(w + (ci * 3 + 2) * 64 + 32 * i);
+                acc[i][0] = fmaf(w2, xa.y, fmaf(w1, xa.x, acc[i][0]));
+                acc[i][1] = fmaf(w2, xb.y, fmaf(w1, xb.x, acc[i][1]));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float b = v.enc_b[2][lane + 32 * i];
+            c2[fa * VE_C2 + lane + 32 * i] = fmaxf(acc[i][0] + b, 0.0f);
+            c2[(fa + 1) * VE_C2 + lane + 32 * i] = fmaxf(acc[i][1] + b, 0.0f);
+        }
+    }
+    __syncwarp();
+    {   // block 3: 64 -> 128, one step, the middle tap
+        float acc[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[i][0] = acc[i][1] = 0.0f;
+        const float *w = v.enc_t[3] + lane;
+#pragma unroll 4
+        for (int ci = 0; ci < 64; ci++) {
+            const float xa = c2[fa * VE_C2 + ci], xb = c2[(fa + 1) * VE_C2 + ci];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float wv = __ldg(w + (ci * 3 + 1) * 128 + 32 * i);
+                acc[i][0] = fmaf(wv, xa, acc[i][0]);
+                acc[i][1] = fmaf(wv, xb, acc[i][1]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float b = v.enc_b[3][lane + 32 * i];
+            c3[fa * VE_C3 + lane + 32 * i] = fmaxf(acc[i][0] + b, 0.0f);
+            c3[(fa + 1) * VE_C3 + lane + 32 * i] = fmaxf(acc[i][1] + b, 0.0f);
+        }
+    }
+    __syncthreads();
+    {   // the LSTM's input contribution: a warp takes 64 of the 512 rows for all sixteen frames
+        float acc[2][VE_F];
+#pragma unroll
+        for (int f = 0; f < VE_F; f++) acc[0][f] = acc[1][f] = 0.0f;
+        const int r = warp * 64 + lane;
+        const float *w = v.w_ih_t + r;
+#pragma unroll 1
+        for (int j = 0; j < 128; j += 4) {
+            float wv[4][2];
+#pragma unroll
+            for (int q = 0; q < 4; q++) { wv[q][0] = __ldg(w + (j + q) * 512); wv[q][1] = __ldg(w + (j + q) * 512 + 32); }
+#pragma unroll
+            for (int f = 0; f < VE_F; f++) {
+                const float4 x = *reinterpret_cast<const float4 *>(c3 + f * VE_C3 + j);
+#pragma unroll
+                for (int i = 0; i < 2; i++) acc[i][f] = fmaf(wv[3][i], x.w, fmaf(wv[2][i], x.z, fmaf(wv[1][i], x.y, fmaf(wv[0][i], x.x, acc[i][f]))));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float b = v.b_ih[r + 32 * i] + v.b_hh[r + 32 * i];
+#pragma unroll
+            for (int f = 0; f < VE_F; f++) if (f0 + f < frames) xz[(size_t)(f0 + f - frame0) * 512 + r + 32 * i] = b + acc[i][f];
+        }
+    }
+}
+
 __device__ __forceinline__ float vad_sigmoid(float x) {       // mynah_asr_sigmoid (src/qmat.h:31-35)
     if (x >= 0.0f) return 1.0f / (1.0f + expf(-x));
     const float e = expf(x);
     return e / (1.0f + e);
 }
 
-// One CTA of 4 H threads walks the frames: z = xz[f] + W_hh h, gates i f g o, head on ReLU(h).
-template <int H>
-__global__ void __launch_bounds__(4 * H)
-vad_lstm_kernel(const VadDev v, const float *__restrict__ xz, int frames, float *__restrict__ probs) {
-    // row r of W_hh: the first WR weights in registers, the rest in shared memory as [j][row] (conflict-free)
-    constexpr int WR = 96, WS = H - WR;
-    extern __shared__ float wsm[];
-    __shared__ float h[H], z[4 * H];
-    const int r = threadIdx.x;
-    float w[WR];
+// sigmoid(x) or tanh(x) without a branch: one exponential, one reciprocal. tanh is (1 - e) / (1 + e) with e = exp(-2 |x|), and
+// below 0.55, where 1 - e cancels, the fifth convergent of its continued fraction (relative error 3e-9 there).
+__device__ __forceinline__ float vl_gate(float x, bool is_tanh) {
+    const float ax = fabsf(x), e = expf(is_tanh ? -2.0f * ax : -ax), x2 = x * x;
+    const bool small = is_tanh && ax < 0.55f;
+    float num = is_tanh ? copysignf(1.0f - e, x) : x >= 0.0f ? 1.0f : e;
+    num = small ? x * fmaf(x2, x2 + 105.0f, 945.0f) : num;
+    const float den = small ? fmaf(x2, fmaf(x2, 15.0f, 420.0f), 945.0f) : 1.0f + e;
+    return num * __frcp_rn(den);
+}
+
+// The recurrence, frames [f0, f1): z = xz[f] + W_hh h, gates i f g o. A step is a chain of latencies, so everything is
+// laid out to shorten it (0.49 us a frame; 2.55 with one CTA that read h and part of W_hh from shared memory, waited at three
+// block barriers and had one thread add up the head's 128 terms):
+//   * a cluster of eight CTAs, sixteen hidden units each; eight lanes share a unit, a lane holds 16 columns of the
+//     unit's four gate rows in registers (64 weights) and reads its 16 values of h in four 16-byte loads;
+//   * the four sums are reduced by a halving exchange that leaves each lane pair with one gate, the pairs apply their
+//     non-linearities side by side, four shuffles bring the gates together, and all eight lanes of a unit go on with
+//     the same c and h: no barrier between the product and the new state;
+//   * lane k sends the unit's h to CTA k (st.async), whose mbarrier completes when all 128 values of the frame have
+//     arrived (readers that poll (value, frame number) pairs instead need 0.56 us a frame, against 0.49). Two h buffers suffice: frame f + 2 is sent only after every value of f + 1 has come, that is after every
+//     warp of the cluster has read f.
+// Waits are bounded; one that runs out sets the status word and the cluster unwinds together.
+constexpr int VL_CTAS = 8, VL_THREADS = 128, VL_H = 128;
+
+__device__ __forceinline__ void vl_send(uint32_t addr, float value, uint32_t bar, int cta) {
+    asm volatile(
+        "{\n\t.reg .b32 ra, rb;\n\t"
+        "mapa.shared::cluster.u32 ra, %0, %3;\n\t"
+        "mapa.shared::cluster.u32 rb, %2, %3;\n\t"
+        "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [ra], %1, [rb];\n\t}"
+        ::"r"(addr), "r"(__float_as_uint(value)), "r"(bar), "r"(cta)
+        : "memory");
+}
+__device__ __forceinline__ void vl_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(VL_CTAS, 1, 1) __launch_bounds__(VL_THREADS, 1)
+vad_lstm_kernel(const VadDev v, const float *__restrict__ xz, int f0, int f1, float *__restrict__ hist, float *__restrict__ c_state, int *status) {
+    __shared__ __align__(16) float h[2][VL_H + 8 * 4];            // eight slices of 16, four floats apart: no bank conflicts
+    __shared__ uint64_t bar[2];
+    const int lane = threadIdx.x & 31, part = lane & 7, u = blockIdx.x * 16 + (threadIdx.x >> 3);
+    float w[4][16];
 #pragma unroll
-    for (int j = 0; j < WR; j++) w[j] = v.w_hh[(size_t)r * H + j];
-    for (int j = 0; j < WS; j++) wsm[j * 4 * H + r] = v.w_hh[(size_t)r * H + WR + j];
-    float c = 0.0f;
-    if (r < H) h[r] = 0.0f;
+    for (int g = 0; g < 4; g++)
+#pragma unroll
+        for (int j = 0; j < 16; j++) w[g][j] = v.w_hh[(size_t)(g * VL_H + u) * VL_H + part * 16 + j];
+    for (int i = threadIdx.x; i < VL_H; i += VL_THREADS) h[(f0 & 1) ^ 1][(i >> 4) * 20 + (i & 15)] = f0 ? hist[(size_t)(f0 - 1) * VL_H + i] : 0.0f;
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < 2; b++) { mbar_init(&bar[b], 1); }
+        mbar_fence_init();
+        for (int b = 0; b < 2; b++) mbar_expect_tx(&bar[b], VL_H * 4);
+    }
+    float c = f0 ? c_state[u] : 0.0f;
     __syncthreads();
-    for (int f = 0; f < frames; f++) {
-        float acc = 0.0f;
+    vl_cluster_sync();
+    const int gate = ((part >> 2) & 1) * 2 + ((part >> 1) & 1);   // 0 i, 1 f, 2 g, 3 o
+    const float *xp = xz + (size_t)gate * VL_H + u;       // xz: rows of frames f0, f0 + 1, ..
+    const uint32_t dst = smem_u32(&h[0][(u >> 4) * 20 + (u & 15)]), dbar = smem_u32(&bar[0]);
+    constexpr int AHEAD = 4;                                      // input contributions asked for this many frames early
+    float xq[AHEAD];
 #pragma unroll
-        for (int j = 0; j < WR; j++) acc = fmaf(w[j], h[j], acc);
+    for (int i = 0; i < AHEAD; i++) xq[i] = f0 + i < f1 ? xp[(size_t)i * 4 * VL_H] : 0.0f;
+    bool ok = true;
+    for (int fb = f0; fb < f1 && ok; fb += AHEAD) {
 #pragma unroll
-        for (int j = 0; j < WS; j++) acc = fmaf(wsm[j * 4 * H + r], h[WR + j], acc);
-        z[r] = xz[(size_t)f * 4 * H + r] + acc;
-        __syncthreads();
-        if (r < H) {
-            const float ig = vad_sigmoid(z[r]), fg = vad_sigmoid(z[H + r]), gg = tanhf(z[2 * H + r]), og = vad_sigmoid(z[3 * H + r]);
+        for (int q = 0; q < AHEAD; q++) {
+            const int f = fb + q;
+            if (f >= f1 || !ok) break;
+            const int n = f - f0, buf = (f & 1) ^ 1;              // h of frame f - 1
+            if (n > 0) {
+                // the buffer's barrier: its k-th completion is the k-th frame of that parity
+                ok = __all_sync(0xffffffffu, mbar_wait(&bar[buf], (uint32_t)(((n - 1) >> 1) & 1)));
+                if (!ok) break;
+                if (threadIdx.x == 0) mbar_expect_tx(&bar[buf], VL_H * 4);
+            }
+            const float x0 = xq[q];
+            if (f + AHEAD < f1) xq[q] = xp[(size_t)(n + AHEAD) * 4 * VL_H];
+            float s[4][2];
+#pragma unroll
+            for (int g = 0; g < 4; g++) s[g][0] = s[g][1] = 0.0f;
+            const float4 *hp = reinterpret_cast<const float4 *>(&h[buf][part * 20]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float4 hv = hp[j];
+#pragma unroll
+                for (int g = 0; g < 4; g++) {
+                    s[g][0] = fmaf(w[g][4 * j], hv.x, s[g][0]); s[g][1] = fmaf(w[g][4 * j + 1], hv.y, s[g][1]);
+                    s[g][0] = fmaf(w[g][4 * j + 2], hv.z, s[g][0]); s[g][1] = fmaf(w[g][4 * j + 3], hv.w, s[g][1]);
+                }
+            }
+            // halving exchange: lane bit 2 picks gates {i, f} or {g, o}, bit 1 one of the two, bit 0 adds the last halves
+            const float t0 = s[0][0] + s[0][1], t1 = s[1][0] + s[1][1], t2 = s[2][0] + s[2][1], t3 = s[3][0] + s[3][1];
+            const bool hi2 = part & 4, hi1 = part & 2;
+            float a = (hi2 ? t2 : t0) + __shfl_xor_sync(0xffffffffu, hi2 ? t0 : t2, 4);
+            float b = (hi2 ? t3 : t1) + __shfl_xor_sync(0xffffffffu, hi2 ? t1 : t3, 4);
+            float z = (hi1 ? b : a) + __shfl_xor_sync(0xffffffffu, hi1 ? a : b, 2);
+            z += __shfl_xor_sync(0xffffffffu, z, 1);
+            z += x0;
+            const float y = vl_gate(z, gate == 2);
+            const int base = lane & 24;
+            const float ig = __shfl_sync(0xffffffffu, y, base), fg = __shfl_sync(0xffffffffu, y, base + 2), gg = __shfl_sync(0xffffffffu, y, base + 4),
+                        og = __shfl_sync(0xffffffffu, y, base + 6);
             c = fg * c + ig * gg;
-            h[r] = og * tanhf(c);
-        }
-        __syncthreads();
-        if (r == 0) {
-            float a = v.head_b;
-            for (int i = 0; i < H; i++) if (h[i] > 0.0f) a = fmaf(v.head_w[i], h[i], a);
-            probs[f] = vad_sigmoid(a);
+            const float hn = og * vl_gate(c, true);
+            vl_send(dst + (uint32_t)((f & 1) * sizeof(h[0])), hn, dbar + (uint32_t)((f & 1) * 8), part);
+            if (part == 0) hist[(size_t)f * VL_H + u] = hn;
         }
     }
+    // the last frame's values (and the one before, where a wait ran out) are still on their way into this CTA
+    if (ok && f1 > f0) ok = mbar_wait(&bar[(f1 - 1) & 1], (uint32_t)(((f1 - 1 - f0) >> 1) & 1));
+    if (!ok && lane == 0) atomicExch(status, ST_TIMEOUT_EPILOGUE);
+    if (part == 0) c_state[u] = c;
+    __syncthreads();
+    vl_cluster_sync();
+}
+
+// probability of every frame: head over ReLU(h), a warp per frame
+__global__ void __launch_bounds__(256)
+vad_head_kernel(const VadDev v, const float *__restrict__ hist, int frames, float *__restrict__ probs) {
+    const int f = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (f >= frames) return;
+    float a = 0.0f;
+#pragma unroll
+    for (int j = 0; j < VL_H / 32; j++) a = fmaf(v.head_w[lane + 32 * j], fmaxf(hist[(size_t)f * VL_H + lane + 32 * j], 0.0f), a);
+    a = warp_sum(a);
+    if (lane == 0) probs[f] = vad_sigmoid(v.head_b + a);
 }
 
 // e[j] = sum of squares (double) of the `win` samples from lo + j hop, added in order (find_split_point, src/mynah_asr.c:1183-1189)
@@ -154,15 +468,43 @@ __global__ void window_energy_kernel(const float *__restrict__ s, long long lo, 
 
 }  // namespace
 
+namespace {
+// Device buffers of one handle (or one call without a handle), kept from call to call and grown when needed. An audio
+// buffer above KEEP bytes is given back when its call ends.
+struct VadBuffers {
+    static constexpr size_t KEEP = 256u << 20;
+    float *audio = nullptr, *xz = nullptr, *hist = nullptr, *probs = nullptr;   // hist [frames][128]; xz: two chunks
+    double *energy = nullptr;
+    size_t audio_cap = 0, frame_cap = 0, energy_cap = 0;                        // in elements
+    template <typename T> static bool grow(T *&p, size_t &cap, size_t need, size_t per) {
+        if (need <= cap) return true;
+        if (p) cudaFree(p);
+        p = nullptr; cap = 0;
+        if (cudaMalloc((void **)&p, need * per * sizeof(T)) != cudaSuccess) { cudaGetLastError(); set_error("device allocation failed"); return false; }
+        cap = need;
+        return true;
+    }
+    void end_call() { if (audio_cap * sizeof(float) > KEEP) { cudaFree(audio); audio = nullptr; audio_cap = 0; } }
+    ~VadBuffers() { cudaFree(audio); cudaFree(xz); cudaFree(hist); cudaFree(probs); cudaFree(energy); }
+};
+}  // namespace
+
 struct mynah_b200_vad {
     mynah_b200_vad_config cfg;
     VadDev d;
     std::vector<void *> owned;
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr, copy = nullptr;
+    cudaEvent_t encoded = nullptr, walked[2] = {nullptr, nullptr};
     size_t smem = 0;
+    float *c_state = nullptr;
+    int *status = nullptr;
+    VadBuffers buf;
+    std::mutex mu;                       // calls on one handle share the buffers and run one after the other
 };
 
 namespace {
+
+constexpr int VAD_CHUNK = 1024;          // frames per piece of the copy -> encode -> recurrence pipeline; the first is a quarter
 
 float *vad_upload(mynah_b200_vad *v, const float *src, size_t n) {
     float *p = nullptr;
@@ -171,25 +513,65 @@ float *vad_upload(mynah_b200_vad *v, const float *src, size_t n) {
     if (cudaMemcpy(p, src, n * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
     return p;
 }
+// w [rows, cols] with the row index fastest
+float *vad_upload_t(mynah_b200_vad *v, const float *w, int rows, int cols) {
+    std::vector<float> t((size_t)rows * cols);
+    for (int r = 0; r < rows; r++) for (int c = 0; c < cols; c++) t[(size_t)c * rows + r] = w[(size_t)r * cols + c];
+    return vad_upload(v, t.data(), t.size());
+}
 
-// speech probabilities of the uploaded signal -> host vector
-int vad_probs_dev(mynah_b200_vad *v, const float *audio_dev, size_t n, std::vector<float> &probs) {
-    const int F = v->d.frame, H = v->d.hidden;
-    const int frames = (int)((n + F - 1) / F);
+bool vad_published_geometry(const VadDev &d) {
+    static const int cout[4] = {128, 64, 64, 128}, stride[4] = {1, 2, 2, 1};
+    bool ok = d.frame == 512 && d.context == 64 && d.pad == 64 && d.n_fft == 256 && d.hop == 128 && d.n_bins == 129 && d.n_enc == 4;
+    for (int i = 0; i < 4 && ok; i++) ok = d.cout[i] == cout[i] && d.k[i] == 3 && d.stride[i] == stride[i] && d.pl[i] == 1 && d.pr[i] == 1;
+    return ok;
+}
+
+// Host signal -> v->buf.audio and its speech probabilities. The recurrence sets the pace, so the signal goes up in pieces
+// on a second stream, where each piece is encoded too while the one before it is walked.
+int vad_run(mynah_b200_vad *v, const float *samples, size_t n, std::vector<float> &probs) {
+    const int F = v->d.frame, frames = (int)((n + F - 1) / F);
+    VadBuffers &b = v->buf;
     probs.assign((size_t)frames, 0.f);
+    size_t hist_cap = b.frame_cap;
+    if (!VadBuffers::grow(b.audio, b.audio_cap, n ? n : 1, 1)) return -1;
     if (frames == 0) return 0;
-    float *xz = nullptr, *pd = nullptr;
-    MB_CUDA(cudaMallocAsync((void **)&xz, (size_t)frames * 4 * H * sizeof(float), v->stream));
-    if (cudaMallocAsync((void **)&pd, (size_t)frames * sizeof(float), v->stream) != cudaSuccess) { cudaGetLastError(); cudaFreeAsync(xz, v->stream); set_error("vad: allocation failed"); return -1; }
-    vad_encode_kernel<<<frames, 256, v->smem, v->stream>>>(v->d, audio_dev, (long long)n, xz);
-    vad_lstm_kernel<128><<<1, 512, 32 * 512 * sizeof(float), v->stream>>>(v->d, xz, frames, pd);
-    note_launch(2);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(probs.data(), pd, (size_t)frames * sizeof(float), cudaMemcpyDeviceToHost, v->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(v->stream);
-    cudaFreeAsync(xz, v->stream);
-    cudaFreeAsync(pd, v->stream);
+    if (!VadBuffers::grow(b.hist, hist_cap, (size_t)frames, VL_H) || !VadBuffers::grow(b.probs, b.frame_cap, (size_t)frames, 1)) return -1;
+    const size_t nxz = (size_t)VAD_CHUNK * 4 * VL_H;
+    if (!b.xz && cudaMalloc((void **)&b.xz, 2 * nxz * sizeof(float)) != cudaSuccess) { cudaGetLastError(); b.xz = nullptr; set_error("vad: allocation failed"); return -1; }
+    cudaError_t e = cudaMemsetAsync(v->status, 0, sizeof(int), v->stream);
+    for (int f = 0, i = 0; f < frames && e == cudaSuccess; i++) {
+        const int end = f == 0 ? (frames < VAD_CHUNK / 4 ? frames : VAD_CHUNK / 4) : (frames - f < VAD_CHUNK ? frames : f + VAD_CHUNK);
+        const size_t s0 = (size_t)f * F, s1 = (size_t)end * F < n ? (size_t)end * F : n;
+        float *xz = b.xz + (i & 1) * nxz;
+        e = cudaMemcpyAsync(b.audio + s0, samples + s0, (s1 - s0) * sizeof(float), cudaMemcpyHostToDevice, v->copy);
+        if (e == cudaSuccess && i >= 2) e = cudaStreamWaitEvent(v->copy, v->walked[i & 1], 0);
+        if (e != cudaSuccess) break;
+        // samples past s1 are not on the device yet, and no frame before `end` reads them
+        if (v->d.basis_t) vad_encode16_kernel<<<cdiv(end - f, VE_F), VE_THREADS, VE_SMEM, v->copy>>>(v->d, b.audio, (long long)s1, f, end, xz);
+        else vad_encode_kernel<<<end - f, 256, v->smem, v->copy>>>(v->d, b.audio, (long long)s1, f, xz);
+        e = cudaEventRecord(v->encoded, v->copy);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(v->stream, v->encoded, 0);
+        if (e != cudaSuccess) break;
+        vad_lstm_kernel<<<VL_CTAS, VL_THREADS, 0, v->stream>>>(v->d, xz, f, end, b.hist, v->c_state, v->status);
+        note_launch(2);
+        e = cudaEventRecord(v->walked[i & 1], v->stream);
+        f = end;
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
+    int st = 0;
+    if (e == cudaSuccess) {
+        vad_head_kernel<<<cdiv(frames, 8), 256, 0, v->stream>>>(v->d, b.hist, frames, b.probs);
+        note_launch();
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(probs.data(), b.probs, (size_t)frames * sizeof(float), cudaMemcpyDeviceToHost, v->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&st, v->status, sizeof(int), cudaMemcpyDeviceToHost, v->stream);
+    const cudaError_t es = cudaStreamSynchronize(v->stream);
+    cudaStreamSynchronize(v->copy);
+    if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) { set_error("vad: %s", cudaGetErrorString(e)); return -1; }
+    if (st) { set_error("vad: a bounded wait inside the recurrence ran out (code %d)", st); return -1; }
     return frames;
 }
 
@@ -242,19 +624,17 @@ std::vector<Span> spans_from_probs(const mynah_b200_vad_config &c, const std::ve
 }
 
 // find_split_point (src/mynah_asr.c:1178-1192) on the resident signal: -1 on a device error
-long long split_point_dev(const float *audio_dev, long long lo, long long hi, int sr, cudaStream_t st, std::vector<double> &host) {
+long long split_point_dev(VadBuffers &b, long long lo, long long hi, int sr, cudaStream_t st, std::vector<double> &host) {
     const int win = sr / 50, hop = win / 2;
     if (hop <= 0 || lo + win > hi) return hi;
     const int nw = (int)((hi - win - lo) / hop) + 1;
-    double *e = nullptr;
-    if (cudaMallocAsync((void **)&e, (size_t)nw * sizeof(double), st) != cudaSuccess) { cudaGetLastError(); set_error("plan_segments: allocation failed"); return -1; }
-    window_energy_kernel<<<cdiv(nw, 128), 128, 0, st>>>(audio_dev, lo, win, hop, nw, e);
+    if (!VadBuffers::grow(b.energy, b.energy_cap, (size_t)nw, 1)) return -1;
+    window_energy_kernel<<<cdiv(nw, 128), 128, 0, st>>>(b.audio, lo, win, hop, nw, b.energy);
     note_launch();
     host.resize((size_t)nw);
     cudaError_t err = cudaGetLastError();
-    if (err == cudaSuccess) err = cudaMemcpyAsync(host.data(), e, (size_t)nw * sizeof(double), cudaMemcpyDeviceToHost, st);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(host.data(), b.energy, (size_t)nw * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (err == cudaSuccess) err = cudaStreamSynchronize(st);
-    cudaFreeAsync(e, st);
     if (err != cudaSuccess) { set_error("plan_segments: %s", cudaGetErrorString(err)); return -1; }
     double best = 1e300;
     long long pos = hi;
@@ -308,8 +688,28 @@ mynah_b200_vad *mynah_b200_vad_new(const mynah_b200_vad_config *c, const float *
     d.act_max = act_max;
     v->smem = ((size_t)d.context + d.frame + d.pad + 2 * (size_t)d.n_bins * d.stft_frames + 2 * (size_t)act_max) * sizeof(float);
     if (ok && v->smem > 200 * 1024) ok = false;
-    if (ok && cudaStreamCreateWithFlags(&v->stream, cudaStreamNonBlocking) != cudaSuccess) ok = false;
-    if (ok && cudaFuncSetAttribute(vad_lstm_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 512 * (int)sizeof(float)) != cudaSuccess) ok = false;
+    if (ok && vad_published_geometry(d)) {
+        std::vector<float> bt((size_t)256 * 256), ny(512);
+        for (int k = 0; k < 256; k++) {
+            for (int r = 0; r < 128; r++) { bt[(size_t)k * 256 + r] = basis[(size_t)r * 256 + k]; bt[(size_t)k * 256 + 128 + r] = basis[(size_t)(129 + r) * 256 + k]; }
+            ny[k] = basis[(size_t)128 * 256 + k]; ny[256 + k] = basis[(size_t)257 * 256 + k];
+        }
+        d.basis_ny = vad_upload(v, ny.data(), ny.size());
+        for (int i = 0; i < 4 && ok; i++) ok = (d.enc_t[i] = vad_upload_t(v, enc_w[i], d.cout[i], d.cin[i] * 3)) != nullptr;
+        d.w_ih_t = vad_upload_t(v, w_ih, 512, 128);
+        d.basis_t = vad_upload(v, bt.data(), bt.size());
+        ok = ok && d.basis_ny && d.w_ih_t && d.basis_t;
+        if (ok && cudaFuncSetAttribute(vad_encode16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VE_SMEM) != cudaSuccess) ok = false;
+    }
+    if (ok && (cudaStreamCreateWithFlags(&v->stream, cudaStreamNonBlocking) != cudaSuccess || cudaStreamCreateWithFlags(&v->copy, cudaStreamNonBlocking) != cudaSuccess ||
+               cudaEventCreateWithFlags(&v->encoded, cudaEventDisableTiming) != cudaSuccess)) ok = false;
+    for (int i = 0; i < 2 && ok; i++) ok = cudaEventCreateWithFlags(&v->walked[i], cudaEventDisableTiming) == cudaSuccess;
+    if (ok) {
+        std::vector<float> zero(VL_H + 1, 0.f);
+        v->c_state = vad_upload(v, zero.data(), VL_H);
+        v->status = reinterpret_cast<int *>(vad_upload(v, zero.data(), 1));
+        ok = v->c_state && v->status;
+    }
     if (ok && v->smem > 48 * 1024 && cudaFuncSetAttribute(vad_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v->smem) != cudaSuccess) ok = false;
     cudaDeviceSynchronize();
     if (!ok) { set_error("vad_new: the tensors contradict the geometry, or a device call failed"); mynah_b200_vad_free(v); return nullptr; }
@@ -319,29 +719,21 @@ mynah_b200_vad *mynah_b200_vad_new(const mynah_b200_vad_config *c, const float *
 void mynah_b200_vad_free(mynah_b200_vad *v) {
     if (!v) return;
     for (void *p : v->owned) cudaFree(p);
+    if (v->encoded) cudaEventDestroy(v->encoded);
+    for (cudaEvent_t e : v->walked) if (e) cudaEventDestroy(e);
+    if (v->copy) cudaStreamDestroy(v->copy);
     if (v->stream) cudaStreamDestroy(v->stream);
     delete v;
 }
 
 int mynah_b200_vad_frame_samples(const mynah_b200_vad *v) { return v ? v->d.frame : 0; }
 
-// uploads the signal; the caller frees with cudaFree
-static float *upload_signal(const float *samples, size_t n, cudaStream_t st) {
-    float *a = nullptr;
-    if (cudaMalloc((void **)&a, (n ? n : 1) * sizeof(float)) != cudaSuccess) { cudaGetLastError(); set_error("device allocation failed"); return nullptr; }
-    if (n && (cudaMemcpyAsync(a, samples, n * sizeof(float), cudaMemcpyHostToDevice, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)) {
-        set_error("H2D copy failed"); cudaFree(a); return nullptr;
-    }
-    return a;
-}
-
 int mynah_b200_vad_probs(mynah_b200_vad *v, const float *samples, size_t n, float *probs, int cap) {
     if (!v || (!samples && n) || !probs) { set_error("vad_probs: bad argument"); return -1; }
-    float *a = upload_signal(samples, n, v->stream);
-    if (!a) return -1;
+    std::lock_guard<std::mutex> lk(v->mu);
     std::vector<float> p;
-    const int frames = vad_probs_dev(v, a, n, p);
-    cudaFree(a);
+    const int frames = vad_run(v, samples, n, p);
+    v->buf.end_call();
     if (frames < 0) return -1;
     if (frames > cap) { set_error("vad_probs: %d frames, room for %d", frames, cap); return -1; }
     memcpy(probs, p.data(), (size_t)frames * sizeof(float));
@@ -350,11 +742,10 @@ int mynah_b200_vad_probs(mynah_b200_vad *v, const float *samples, size_t n, floa
 
 int mynah_b200_vad_speech_spans(mynah_b200_vad *v, const float *samples, size_t n, long long *spans, int cap) {
     if (!v || (!samples && n) || !spans || cap < 0) { set_error("vad_speech_spans: bad argument"); return -1; }
-    float *a = upload_signal(samples, n, v->stream);
-    if (!a) return -1;
+    std::lock_guard<std::mutex> lk(v->mu);
     std::vector<float> p;
-    const int frames = vad_probs_dev(v, a, n, p);
-    cudaFree(a);
+    const int frames = vad_run(v, samples, n, p);
+    v->buf.end_call();
     if (frames < 0) return -1;
     const std::vector<Span> sp = spans_from_probs(v->cfg, p, (long long)n);
     if ((int)sp.size() > cap) { set_error("vad_speech_spans: more than %d spans", cap); return -1; }
@@ -367,14 +758,16 @@ int mynah_b200_plan_segments(mynah_b200_vad *v, const float *samples, size_t n_s
     if ((!samples && n_samples) || !segs || cap < 1 || sample_rate <= 0 || seg_sec <= 0) { set_error("plan_segments: bad argument"); return -1; }
     if (!mynah_b200_available()) { set_error("plan_segments: no sm_100 device"); return -1; }
     cudaStream_t st = v ? v->stream : nullptr;
-    float *a = upload_signal(samples, n_samples, st);
-    if (!a) return -1;
+    VadBuffers own;                                 // of a call without a network
+    VadBuffers &buf = v ? v->buf : own;
+    std::unique_lock<std::mutex> lk;
+    if (v) lk = std::unique_lock<std::mutex>(v->mu);
     const long long n = (long long)n_samples, sr = sample_rate, seg_max = (long long)(seg_sec * (double)sample_rate);
     std::vector<Span> ranges;                       // what gets cut: the whole signal, or the widened and merged speech spans
     bool vad_plan = false;
     if (v && n > 0) {
         std::vector<float> p;
-        if (vad_probs_dev(v, a, n_samples, p) >= 0) {
+        if (vad_run(v, samples, n_samples, p) >= 0) {
             std::vector<Span> sp = spans_from_probs(v->cfg, p, n);
             const long long ctx = (long long)(0.6 * (double)sample_rate);      // MYNAH_ASR_VAD_CONTEXT_SEC (src/mynah_asr.c:67-68)
             for (Span &s : sp) { s.t0 = s.t0 > ctx ? s.t0 - ctx : 0; s.t1 = s.t1 + ctx < n ? s.t1 + ctx : n; }
@@ -385,7 +778,13 @@ int mynah_b200_plan_segments(mynah_b200_vad *v, const float *samples, size_t n_s
             vad_plan = true;
         }
     }
-    if (!vad_plan) ranges.assign(1, Span{0, n});
+    if (!vad_plan) {
+        ranges.assign(1, Span{0, n});
+        if (!VadBuffers::grow(buf.audio, buf.audio_cap, n_samples ? n_samples : 1, 1)) return -1;
+        if (n && (cudaMemcpyAsync(buf.audio, samples, n_samples * sizeof(float), cudaMemcpyHostToDevice, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)) {
+            cudaGetLastError(); set_error("H2D copy failed"); buf.end_call(); return -1;
+        }
+    }
     std::vector<long long> out;
     std::vector<double> scratch;
     int rc = 0;
@@ -397,7 +796,7 @@ int mynah_b200_plan_segments(mynah_b200_vad *v, const float *samples, size_t n_s
                 const long long hi = cur + seg_max;
                 long long lo = seg_max > 20 * sr ? hi - 20 * sr : cur + sr;    // the last 20 s of the window, at least 1 s in
                 if (lo <= cur) lo = cur + 1;
-                end = split_point_dev(a, lo, hi, sample_rate, st, scratch);
+                end = split_point_dev(buf, lo, hi, sample_rate, st, scratch);
                 if (end < 0) { rc = -1; break; }
                 if (vad_plan && (end <= cur || end > r.t1)) end = hi;
             }
@@ -406,7 +805,7 @@ int mynah_b200_plan_segments(mynah_b200_vad *v, const float *samples, size_t n_s
             cur = end;
         }
     }
-    cudaFree(a);
+    buf.end_call();
     if (rc) return -1;
     if (out.empty()) { out.push_back(0); out.push_back(0); }                  // nothing to decode: one empty segment
     const int k = (int)(out.size() / 2);
