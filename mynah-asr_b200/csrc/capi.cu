@@ -111,6 +111,12 @@ struct mynah_b200_qmat {
     mutable uint8_t *host = nullptr;     // from the pinned pool, taken by the first call
     mutable uint8_t *ws = nullptr;
     mutable size_t ws_cap = 0;
+    // A small call repeated with the same rows and flags is one graph (copy in, kernels, copy out): issuing its four or five
+    // pieces one by one took longer than running them. Recorded on the second such call, kept for the last few.
+    struct Graph { int T = 0, flags = 0, uses = 0, launches = 0; cudaGraphExec_t exec = nullptr; };
+    mutable Graph graphs[4];
+    mutable int graph_next = 0;
+    void drop_graphs() const { for (Graph &g : graphs) { if (g.exec) cudaGraphExecDestroy(g.exec); g = Graph(); } }
 };
 static constexpr size_t QMAT_HEAD = 256, QMAT_SMALL = 128 << 10, QMAT_BLOCK = QMAT_HEAD + 2 * QMAT_SMALL;
 static constexpr size_t QMAT_KEEP = 64 << 20;
@@ -179,6 +185,7 @@ public:
             p_ = (uint8_t *)own_;
             return;
         }
+        q->drop_graphs();                                        // they hold the old address
         if (q->ws) cudaFree(q->ws);                              // waits for the products that use it
         q->ws = nullptr; q->ws_cap = 0;
         size_t cap = 1 << 20;
@@ -1215,6 +1222,7 @@ mynah_b200_qmat *mynah_b200_qmat_create(int fmt, const void *data, const float *
 
 void mynah_b200_qmat_free(mynah_b200_qmat *q) {
     if (!q) return;
+    q->drop_graphs();
     for (void *p : q->owned) cudaFree(p);                       // waits for the handle's products
     if (q->ws) cudaFree(q->ws);
     if (q->stream) cudaStreamDestroy(q->stream);
@@ -1324,15 +1332,51 @@ int mynah_b200_qmat_mul(const mynah_b200_qmat *q, const float *x, float *out, in
     float *od = (float *)(small_out ? block + QMAT_HEAD : s.get() + nt + nxw);
     const void *src = x;
     if (small_x) src = memcpy(q->host + QMAT_HEAD + QMAT_SMALL, x, nx);
-    if (cudaMemcpyAsync(xd, src, nx, cudaMemcpyHostToDevice, q->stream) != cudaSuccess) { cudaGetLastError(); set_error("qmat_mul: H2D copy failed"); return -1; }
-    const int rc = qmat_mul_locked(q, xd, od, T, flags, s.get());
-    bool copied = true;
-    if (rc == 0 && !small_out) copied = cudaMemcpyAsync(out, od, no, cudaMemcpyDeviceToHost, q->stream) == cudaSuccess;
-    copied = cudaMemcpyAsync(q->host, block, QMAT_HEAD + (small_out ? no : 0), cudaMemcpyDeviceToHost, q->stream) == cudaSuccess && copied;
-    if (cudaStreamSynchronize(q->stream) != cudaSuccess || !copied) { cudaGetLastError(); set_error("qmat_mul: D2H copy failed"); return -1; }
+    auto issue = [&]() -> int {
+        if (cudaMemcpyAsync(xd, src, nx, cudaMemcpyHostToDevice, q->stream) != cudaSuccess) { cudaGetLastError(); set_error("qmat_mul: H2D copy failed"); return -1; }
+        if (qmat_mul_locked(q, xd, od, T, flags, s.get())) return -1;
+        bool ok = small_out || cudaMemcpyAsync(out, od, no, cudaMemcpyDeviceToHost, q->stream) == cudaSuccess;
+        ok = cudaMemcpyAsync(q->host, block, QMAT_HEAD + (small_out ? no : 0), cudaMemcpyDeviceToHost, q->stream) == cudaSuccess && ok;
+        if (!ok) { cudaGetLastError(); set_error("qmat_mul: D2H copy failed"); return -1; }
+        return 0;
+    };
+    mynah_b200_qmat::Graph *g = nullptr;
+    if (small_x && small_out && !(flags & MYNAH_B200_A8)) {      // (the int8-row path allocates for itself)
+        for (auto &e : q->graphs) if (e.uses && e.T == T && e.flags == flags) g = &e;
+        if (!g) {
+            g = &q->graphs[q->graph_next];
+            q->graph_next = (q->graph_next + 1) & 3;
+            if (g->exec) cudaGraphExecDestroy(g->exec);
+            *g = mynah_b200_qmat::Graph();
+            g->T = T; g->flags = flags;
+        }
+        if (++g->uses == 2) {
+            const long long before = launch_count(false);
+            cudaGraph_t rec = nullptr;
+            if (cudaStreamBeginCapture(q->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+                const int rc = issue();
+                const cudaError_t e = cudaStreamEndCapture(q->stream, &rec);
+                g->launches = (int)(launch_count(false) - before);
+                note_launch(-g->launches);                       // recorded, not launched
+                if (rc || e != cudaSuccess || !rec || cudaGraphInstantiate(&g->exec, rec, 0) != cudaSuccess) g->exec = nullptr;
+                if (rec) cudaGraphDestroy(rec);
+            }
+            cudaGetLastError();
+        }
+    }
+    int rc;
+    if (g && g->exec) {
+        rc = cudaGraphLaunch(g->exec, q->stream) == cudaSuccess ? 0 : -1;
+        if (rc) { cudaGetLastError(); set_error("qmat_mul: graph launch failed"); }
+        else note_launch(g->launches);
+    } else {
+        rc = issue();
+    }
+    if (cudaStreamSynchronize(q->stream) != cudaSuccess) { cudaGetLastError(); set_error("qmat_mul: a copy or kernel failed"); return -1; }
+    if (rc) return rc;
     if (qmat_status(q, *(const int *)q->host)) return -1;
-    if (rc == 0 && small_out) memcpy(out, q->host + QMAT_HEAD, no);
-    return rc;
+    if (small_out) memcpy(out, q->host + QMAT_HEAD, no);
+    return 0;
 }
 
 int mynah_b200_qmat_block_dots(const mynah_b200_qmat *q, const float *x, int T, int32_t *dots, float *sx, float *out) {
