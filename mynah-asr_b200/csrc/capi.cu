@@ -506,6 +506,18 @@ int mynah_b200_model_finalize(mynah_b200_model *h) {
             return -1;
     }
     m.ffn_dim = m.layers[0].ff1_w1.n;
+    // tiles for the persistent few-row kernel: cache-aware streaming needs causal convs and the LayerNorm conv norm
+    m.fr_stream = m.causal && !bn && m.d_model <= 1024 && m.d_model % 64 == 0 && fr_attn_fits(m.d_head);
+    for (const EncLayer &L : m.layers)
+        for (const QWeight *w : {&L.ff1_w1, &L.ff1_w2, &L.ff2_w1, &L.ff2_w2, &L.q_w, &L.k_w, &L.v_w, &L.o_w, &L.pw1_w, &L.pw2_w})
+            m.fr_stream = m.fr_stream && fr_can_tile(*w) && w->n % 8 == 0;
+    if (m.fr_stream)
+        for (EncLayer &L : m.layers) {
+            L.t_ff1a = m.fr_tiles({&L.ff1_w1}); L.t_ff1b = m.fr_tiles({&L.ff1_w2}); L.t_qkv = m.fr_tiles({&L.q_w, &L.k_w, &L.v_w});
+            L.t_o = m.fr_tiles({&L.o_w}); L.t_pw1 = m.fr_tiles({&L.pw1_w}, true); L.t_pw2 = m.fr_tiles({&L.pw2_w});
+            L.t_ff2a = m.fr_tiles({&L.ff2_w1}); L.t_ff2b = m.fr_tiles({&L.ff2_w2});
+            if (!L.t_ff1a || !L.t_ff1b || !L.t_qkv || !L.t_o || !L.t_pw1 || !L.t_pw2 || !L.t_ff2a || !L.t_ff2b) return -1;
+        }
     m.d_out = m.d_model;
     if (m.cfg.a8) {
         for (int li = 0; li < nl; li++) {
@@ -635,6 +647,18 @@ int mynah_b200_model_finalize(mynah_b200_model *h) {
             }
         }
         m.aed_ffn = m.aed_layers[0].ff1.n;
+        m.fr_aed = m.aed_d <= 1024 && fr_attn_fits(m.aed_d / m.aed_heads) && fr_can_tile(m.aed_head);
+        for (const AedLayer &A : m.aed_layers)
+            for (const QWeight *w : {&A.sqkv, &A.so, &A.cq, &A.co, &A.ff1, &A.ff2}) m.fr_aed = m.fr_aed && fr_can_tile(*w);
+        if (m.fr_aed) {
+            for (AedLayer &A : m.aed_layers) {
+                A.t_sqkv = m.fr_tiles({&A.sqkv}); A.t_so = m.fr_tiles({&A.so}); A.t_cq = m.fr_tiles({&A.cq});
+                A.t_co = m.fr_tiles({&A.co}); A.t_ff1 = m.fr_tiles({&A.ff1}); A.t_ff2 = m.fr_tiles({&A.ff2});
+                if (!A.t_sqkv || !A.t_so || !A.t_cq || !A.t_co || !A.t_ff1 || !A.t_ff2) return -1;
+            }
+            m.t_aed_head = m.fr_tiles({&m.aed_head});
+            if (!m.t_aed_head) return -1;
+        }
         m.has_aed = true;
     }
     m.host.clear();

@@ -328,7 +328,7 @@ static GemmEpilogue aed_epi(int mode, int act, float alpha, const float *bias, f
 size_t Model::aed_bytes(int total_T, int B, int max_len) const {
     const size_t D = aed_d, F = aed_ffn, L = aed_layers.size();
     return (size_t)total_T * (d_out * 4 + D * 4 + (L + 1) * 2 * D * 4) + L * 2 * (size_t)B * max_len * D * 4 +
-           (size_t)B * (D * 24 + 3 * D * 4 + F * 4 + (size_t)aed_vocab * 4) + (size_t)B * (max_len + 64) * 8 + (1 << 20);
+           (size_t)B * (D * 24 + 3 * D * 4 + F * 4 + (size_t)aed_vocab * 4) + (size_t)B * (max_len + 64 + 148) * 8 + fr_table_bytes(11 * L + 3) + (1 << 20);
 }
 
 int Model::decode_aed(const float *enc_dev, const std::vector<int> &lens, const std::vector<std::vector<int>> &prompts, int eos,
@@ -444,6 +444,70 @@ int Model::decode_aed(const float *enc_dev, const std::vector<int> &lens, const 
         return 0;
     };
     const int *pos_b = st + 6 * B + 4;
+    // all positions as one persistent launch (fewrow.cu) where the decoder has tiles for it; its bits per utterance do not
+    // depend on the batch
+    int mtiles = 0, ngroups = 0;
+    if (fr_aed && B <= FR_MAX_ROWS && fr_grid(B, 16, &mtiles, &ngroups) == 0) {
+        FrArgs a;
+        memset(&a, 0, sizeof(a));
+        uint8_t *table_dev = ws.get<uint8_t>(fr_table_bytes((size_t)11 * L + 3));
+        a.cand_v = ws.get<float>((size_t)B * ngroups); a.cand_i = ws.get<int>((size_t)B * ngroups);
+        a.bar = ws.get<unsigned>(2);
+        if (!table_dev || !a.cand_v || !a.cand_i || !a.bar) return -1;
+        const bool fuse = B <= FR_FUSE_ROWS;
+        std::vector<FrOp> ops;
+        auto blank = [](int type) { FrOp o; memset(&o, 0, sizeof(o)); o.type = type; o.alpha = 1.f; return o; };
+        // a contraction over LayerNorm rows of x: fused, or behind an operation of its own that makes their planes
+        auto from_x = [&](FrOp o, int epi, const uint8_t *w, const float *bias, int N, const float *lw, const float *lb) {
+            const bool turn = ops.empty();                   // position's first: selection and embedding
+            FrOp n = blank(FR_LN);
+            n.rows = turn ? FR_ROWS_AED_NEXT : FR_ROWS_LN; n.x = x; n.ln_w = lw; n.ln_b = lb; n.K = D; n.o_hi = xn.hi; n.o_lo = xn.lo;
+            if (turn) { n.ln0_w = aed_embln_w; n.ln0_b = aed_embln_b; n.x_copy = x; }
+            if (fuse) { o.rows = n.rows; o.x = x; o.ln_w = lw; o.ln_b = lb; o.ln0_w = n.ln0_w; o.ln0_b = n.ln0_b; o.x_copy = n.x_copy; }
+            else { ops.push_back(n); o.rows = FR_ROWS_PLANES; o.a_hi = xn.hi; o.a_lo = xn.lo; }
+            o.epi = epi; o.w = w; o.bias = bias; o.N = N; o.K = D; o.ldo = N;
+            ops.push_back(o);
+        };
+        auto into_x = [&](const H16 &h, const uint8_t *w, const float *bias, int K) {
+            FrOp o = blank(FR_GEMM);
+            o.rows = FR_ROWS_PLANES; o.epi = FR_EPI_RESID; o.w = w; o.bias = bias; o.N = D; o.K = K; o.ldo = D;
+            o.a_hi = h.hi; o.a_lo = h.lo; o.out = x; o.res = x;
+            ops.push_back(o);
+        };
+        for (int l = 0; l < L; l++) {
+            const AedLayer &A = aed_layers[l];
+            FrOp o = blank(FR_GEMM);
+            o.out = qkv;
+            from_x(o, FR_EPI_F32, A.t_sqkv, A.sqkv_b, 3 * D, A.ln_self_w, A.ln_self_b);
+            o = blank(FR_AED_SELF);
+            o.q = qkv; o.ldq = 3 * D; o.ck = sk + (size_t)(2 * l) * B * max_len * D; o.cv = o.ck + (size_t)B * max_len * D; o.o_hi = att.hi; o.o_lo = att.lo;
+            ops.push_back(o);
+            into_x(att, A.t_so, A.so_b, D);
+            o = blank(FR_GEMM);
+            o.out = q;
+            from_x(o, FR_EPI_F32, A.t_cq, A.cq_b, D, A.ln_cross_w, A.ln_cross_b);
+            o = blank(FR_AED_CROSS);
+            o.q = q; o.ldq = D; o.a_hi = ckv[l].hi; o.a_lo = ckv[l].lo; o.o_hi = att.hi; o.o_lo = att.lo;
+            ops.push_back(o);
+            into_x(att, A.t_co, A.co_b, D);
+            o = blank(FR_GEMM);
+            o.act = ACT_RELU; o.o_hi = ff.hi; o.o_lo = ff.lo;
+            from_x(o, FR_EPI_PLANES, A.t_ff1, A.ff1_b, F, A.ln_ffn_w, A.ln_ffn_b);
+            into_x(ff, A.t_ff2, A.ff2_b, F);
+        }
+        from_x(blank(FR_GEMM), FR_EPI_ARGMAX, t_aed_head, aed_head_b, V, aed_fin_w, aed_fin_b);
+        if (ops.size() % 2) ops.push_back(blank(FR_NOP));
+        const std::vector<uint8_t> table = fr_table(ops);
+        MB_CUDA(cudaMemcpyAsync(table_dev, table.data(), table.size(), cudaMemcpyHostToDevice, stream));
+        a.M = B; a.tile_rows = 16; a.mtiles = mtiles; a.ngroups = ngroups;
+        a.terms = cfg.strict ? 3 : 1; a.d = D; a.H = H; a.dk = dk; a.status = status; a.positions = max_len;
+        a.V = V; a.B = B; a.eos = eos; a.cap_stride = capn; a.max_prompt = max_prompt; a.max_seq = aed_max_seq; a.max_len = max_len;
+        a.st = st; a.prompts = d_prompts; a.tokens = d_tokens; a.emb = aed_emb; a.pos = aed_pos; a.enc_off = d_off; a.enc_len = d_off + B; a.v_off = v_off;
+        if (fr_launch(a, ops, table_dev, stream)) return -1;
+        prof_end_span(sp);
+        if (sp >= 0) prof_launches[PROF_DECODE]++;
+        return aed_fetch(st, d_tokens, B, capn, mark, tokens);
+    }
     auto position = [&]() -> int {
         // every launch of a position is chained: blocks of the next kernel are placed while the one before drains
         if (!ln_tail) {
@@ -522,6 +586,10 @@ int Model::decode_aed(const float *enc_dev, const std::vector<int> &lens, const 
     if (rc) return -1;
     prof_end_span(sp);
     if (sp >= 0) prof_launches[PROF_DECODE]++;
+    return aed_fetch(st, d_tokens, B, capn, mark, tokens);
+}
+
+int Model::aed_fetch(const int *st, const int *d_tokens, int B, int capn, size_t mark, std::vector<std::vector<int>> &tokens) {
     std::vector<int> hn(B), ht((size_t)B * capn);
     MB_CUDA(cudaMemcpyAsync(hn.data(), st + B, B * sizeof(int), cudaMemcpyDeviceToHost, stream));
     MB_CUDA(cudaMemcpyAsync(ht.data(), d_tokens, ht.size() * sizeof(int), cudaMemcpyDeviceToHost, stream));

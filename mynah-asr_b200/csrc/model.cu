@@ -573,6 +573,28 @@ int Model::encoder_layers(float *x, const std::vector<int> &lens, int left, int 
     return 0;
 }
 
+const uint8_t *Model::fr_tiles(const std::vector<const QWeight *> &parts, bool glu) {
+    size_t bytes = 0, off = 0;
+    for (const QWeight *w : parts) bytes += fr_tile_bytes(w->n, w->k);
+    uint8_t *dst = (uint8_t *)dev_alloc(bytes);
+    for (const QWeight *w : parts) {
+        if (!dst || fr_retile(*w, dst + off, glu, stream)) return nullptr;
+        off += fr_tile_bytes(w->n, w->k);
+    }
+    return dst;
+}
+
+// The table of a chain on the device, copied only when it changed: in steady state the step that gets captured into a graph
+// copies nothing. The kernels of earlier calls have finished by then (a call ends with its stream).
+int Model::fr_upload(std::vector<uint8_t> &have, uint8_t *dev, const std::vector<uint8_t> &want) {
+    if (have == want) return 0;
+    if (!copy) MB_CUDA(cudaStreamCreateWithFlags(&copy, cudaStreamNonBlocking));
+    have = want;
+    MB_CUDA(cudaMemcpyAsync(dev, have.data(), have.size(), cudaMemcpyHostToDevice, copy));
+    MB_CUDA(cudaStreamSynchronize(copy));
+    return 0;
+}
+
 int Model::rk_layers(int rk_rows, int n_run) const {
     static constexpr size_t RK_BYTES = 512u << 20;
     const size_t per = (size_t)rk_rows * d_model * 2;

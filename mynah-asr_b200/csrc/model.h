@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "../../include/mynah_b200.h"
+#include "fewrow.h"
 #include "kernels.h"
 #include "qweight.h"
 
@@ -56,6 +57,8 @@ struct FrontItem {
 struct EncLayer {
     const float *ln_ff1_w, *ln_ff1_b, *ln_att_w, *ln_att_b, *ln_conv_w, *ln_conv_b, *ln_ff2_w, *ln_ff2_b, *ln_out_w, *ln_out_b;
     QWeight ff1_w1, ff1_w2, ff2_w1, ff2_w2, q_w, k_w, v_w, o_w, pw1_w, pw2_w, relk;
+    // tiles of the persistent few-row kernel (fewrow.cu), where the model has them
+    const uint8_t *t_ff1a = nullptr, *t_ff1b = nullptr, *t_qkv = nullptr, *t_o = nullptr, *t_pw1 = nullptr, *t_pw2 = nullptr, *t_ff2a = nullptr, *t_ff2b = nullptr;
     QWeight qkv;                 // q_w, k_w, v_w one below the other ([3 d, d]): their operands sit in one block
     const float *bias_u, *bias_v, *dw_w, *dw_b, *cnorm_w, *cnorm_b, *cnorm_scale, *cnorm_shift;
 };
@@ -66,6 +69,7 @@ struct AedLayer {
     const float *ln_self_w, *ln_self_b, *ln_cross_w, *ln_cross_b, *ln_ffn_w, *ln_ffn_b;
     QWeight sqkv, so, cq, ckv, co, ff1, ff2;
     const float *sqkv_b, *so_b, *cq_b, *ckv_b, *co_b, *ff1_b, *ff2_b;
+    const uint8_t *t_sqkv = nullptr, *t_so = nullptr, *t_cq = nullptr, *t_co = nullptr, *t_ff1 = nullptr, *t_ff2 = nullptr;   // fewrow.cu
 };
 
 // Cache-aware streaming state of S streams that advance in lock step (the device counterpart of S
@@ -77,6 +81,11 @@ struct StreamState {
     // a group of at most 128 rows per regular step (S q <= 128) runs the linears of its layers on the few-row kernel
     // (gemm_skinny.cu), a larger one on the many-row kernel: fixed when the group opens, for its whole life
     bool few_rows = false;
+    // ... and, where the layers have tiles for it (Model::fr_stream), the whole layer stack as the one persistent kernel
+    bool persistent = false;
+    std::vector<uint8_t> fr_table_host;                 // what fr_table_dev holds
+    uint8_t *fr_table_dev = nullptr;
+    unsigned *fr_bar = nullptr;
     // rel-pos key projections rk = pos_emb(K) relk^T of every layer for the steady key count K = left + q: they depend on
     // nothing but the weights, so they are computed on the first full step with full caches and reused afterwards
     __half *rk_cache = nullptr;                         // [L][2 (left + q) - 1][d] fp16
@@ -165,6 +174,12 @@ struct Model {
                 *aed_fin_b = nullptr, *aed_head_b = nullptr, *aed_proj_b = nullptr;
     QWeight aed_head, aed_proj;
     std::vector<AedLayer> aed_layers;
+    const uint8_t *t_aed_head = nullptr;
+    // every linear of the encoder layers / of the AED decoder has tiles for the persistent few-row kernel (fewrow.cu)
+    bool fr_stream = false, fr_aed = false;
+    const uint8_t *fr_tiles(const std::vector<const QWeight *> &parts, bool glu = false);   // one below the other; null on failure
+    int fr_upload(std::vector<uint8_t> &have, uint8_t *dev, const std::vector<uint8_t> &want);
+    int stream_layers(StreamState &st, float *x, int Q, const __half *rk, int ldrk);
 
     // mel
     std::vector<float> mel_fb_host, window_host;
@@ -234,6 +249,7 @@ struct Model {
     // packed encoder output [sum T, d_out] -> generated tokens per utterance (prompt and EOS excluded); caps[b] bounds utterance b
     int decode_aed(const float *enc_dev, const std::vector<int> &lens, const std::vector<std::vector<int>> &prompts, int eos,
                    const std::vector<int> &caps, std::vector<std::vector<int>> &tokens);
+    int aed_fetch(const int *st, const int *d_tokens, int B, int capn, size_t mark, std::vector<std::vector<int>> &tokens);
     size_t aed_bytes(int total_T, int B, int max_len) const;
     // one chunk of every stream: mel_dev [S, n_mel, n_mels] -> out_dev [S, q, d_out]; returns q or -1
     int stream_open(StreamState &st, int S, int left, int right);

@@ -263,6 +263,14 @@ int Model::stream_open(StreamState &st, int S, int left, int right) {
         if (!st.ln_count) return -1;
         MB_CUDA(cudaMemsetAsync(st.ln_count, 0, rows * sizeof(int), stream));
     }
+    int mt = 0, ng = 0;
+    st.persistent = st.few_rows && fr_stream && n_layers <= FR_MAX_LAYERS && left > 0 && st.q + 2 <= 16 &&
+                    fr_grid(S * (st.q + 2), 16 / (st.q + 2) * (st.q + 2), &mt, &ng) == 0;
+    if (st.persistent) {
+        st.fr_table_dev = (uint8_t *)stream_alloc(st, fr_table_bytes((size_t)n_layers * 14));
+        st.fr_bar = (unsigned *)stream_alloc(st, 2 * sizeof(unsigned));
+        if (!st.fr_table_dev || !st.fr_bar) return -1;
+    }
     const int C = channels;
     int F = cfg.n_mels;
     for (int s = 0; s < 3; s++) {
@@ -301,7 +309,7 @@ void Model::stream_close(StreamState &st) {
 size_t Model::stream_bytes(const StreamState &st, int n_mel) const {
     const size_t S = st.S, C = channels, d = d_model, Q = st.q + 2, M = S * Q, P = 2 * ((size_t)st.left + Q) - 1;
     const size_t T1 = n_mel / 2 + 2, F1 = cfg.n_mels / 2 + 2;
-    return S * T1 * F1 * C * 4 * 4 + M * (d * 44 + (size_t)ffn_dim * 4) + P * d * 8 + (4 << 20);
+    return S * T1 * F1 * C * 4 * 4 + M * (d * 72 + (size_t)ffn_dim * 8) + P * d * (8 + (st.persistent ? 2 * (size_t)n_layers : 0)) + (4 << 20);
 }
 
 // In steady state (caches full, full-size chunk, same input / output / workspace addresses as last time, no
@@ -338,6 +346,73 @@ int Model::stream_step(StreamState &st, const float *mel, int n_mel, int is_last
     if (cudaGraphLaunch(st.exec, stream) != cudaSuccess) { set_error("stream_step: graph launch failed"); return -1; }
     note_launch(recorded);
     return q;
+}
+
+// The layer stack of one chunk as one persistent launch (fewrow.cu). x [S Q, d] in place.
+int Model::stream_layers(StreamState &st, float *x, int Q, const __half *rk, int ldrk) {
+    const int S = st.S, d = d_model, F = ffn_dim, M = S * Q;
+    FrArgs a;
+    memset(&a, 0, sizeof(a));
+    a.tile_rows = 16 / Q * Q;
+    if (fr_grid(M, a.tile_rows, &a.mtiles, &a.ngroups)) { set_error("stream_step: too many rows for the persistent kernel"); return -1; }
+    const bool fuse = M <= FR_FUSE_ROWS;
+    H16 hA = ws.planes((size_t)M * d), hC = ws.planes((size_t)M * d), hF = ws.planes((size_t)M * F), kvn = ws.planes((size_t)M * d);
+    float *x2 = ws.get<float>((size_t)M * d), *q = ws.get<float>((size_t)M * d), *cbuf = ws.get<float>((size_t)M * d);
+    if (!hA.lo || !hC.lo || !hF.lo || !kvn.lo || !x2 || !q || !cbuf) return -1;
+    std::vector<FrOp> ops;
+    auto blank = [](int type) { FrOp o; memset(&o, 0, sizeof(o)); o.type = type; o.alpha = 1.f; return o; };
+    float *cur = x, *other = x2;
+    // a contraction over LayerNorm rows: fused, or behind an operation of its own that makes their planes
+    auto ln = [&](FrOp o, int rows, const float *src, const float *w, const float *b, const EncLayer *closing, int epi, const uint8_t *tiles, const float *bias, int N) {
+        FrOp n = blank(FR_LN);
+        n.rows = rows; n.x = src; n.ln_w = w; n.ln_b = b; n.K = d; n.o_hi = hA.hi; n.o_lo = hA.lo;
+        if (closing) {                                       // the layer before closes here: its output becomes the residual base
+            n.ln0_w = closing->ln_out_w; n.ln0_b = closing->ln_out_b; n.x_copy = other;
+            float *t = cur; cur = other; other = t;
+        }
+        if (fuse) { o.rows = n.rows; o.x = n.x; o.ln_w = w; o.ln_b = b; o.ln0_w = n.ln0_w; o.ln0_b = n.ln0_b; o.x_copy = n.x_copy; }
+        else { ops.push_back(n); o.rows = FR_ROWS_PLANES; o.a_hi = hA.hi; o.a_lo = hA.lo; }
+        o.epi = epi; o.w = tiles; o.bias = bias; o.N = N; o.K = d;
+        if (!o.ldo) o.ldo = N;
+        if (epi == FR_EPI_RESID) { o.out = cur; o.res = cur; }
+        ops.push_back(o);
+    };
+    auto resid = [&](const H16 &h, const uint8_t *w, const float *bias, int K, float alpha) {
+        FrOp o = blank(FR_GEMM);
+        o.rows = FR_ROWS_PLANES; o.epi = FR_EPI_RESID; o.w = w; o.bias = bias; o.N = d; o.K = K; o.ldo = d; o.alpha = alpha;
+        o.a_hi = h.hi; o.a_lo = h.lo; o.out = cur; o.res = cur;
+        ops.push_back(o);
+    };
+    FrOp up = blank(FR_GEMM);                                // rows -> SiLU planes of the FFN width
+    up.act = ACT_SILU; up.o_hi = hF.hi; up.o_lo = hF.lo;
+    for (int li = 0; li < n_layers; li++) {
+        const EncLayer &L = layers[li];
+        ln(up, li ? FR_ROWS_LN2 : FR_ROWS_LN, cur, L.ln_ff1_w, L.ln_ff1_b, li ? &layers[li - 1] : nullptr, FR_EPI_PLANES, L.t_ff1a, L.ff1_w1.bias, F);
+        resid(hF, L.t_ff1b, L.ff1_w2.bias, F, 0.5f);
+        FrOp o = blank(FR_GEMM);
+        o.n_split = d; o.out = q; o.ldo = d; o.o_hi = kvn.hi; o.o_lo = kvn.lo;
+        ln(o, FR_ROWS_LN, cur, L.ln_att_w, L.ln_att_b, nullptr, FR_EPI_QKV, L.t_qkv, L.qkv.bias, 3 * d);
+        o = blank(FR_STREAM_ATTN);
+        o.q = q; o.ldq = d; o.kn = kvn.hi; o.vn = kvn.lo; o.rk = rk + (size_t)li * d; o.ldrk = ldrk;
+        o.kc = st.k_cache + (size_t)li * S * st.left * d; o.vc = st.v_cache + (size_t)li * S * st.left * d;
+        o.bias_u = L.bias_u; o.bias_v = L.bias_v; o.o_hi = hC.hi; o.o_lo = hC.lo;
+        ops.push_back(o);
+        resid(hC, L.t_o, L.o_w.bias, d, 1.f);
+        o = blank(FR_GEMM);
+        o.out = cbuf; o.dw_w = L.dw_w; o.conv_k = conv_k; o.conv_cache = st.conv_cache + (size_t)li * S * (conv_k - 1) * d;
+        ln(o, FR_ROWS_LN, cur, L.ln_conv_w, L.ln_conv_b, nullptr, FR_EPI_GLU_CONV, L.t_pw1, L.pw1_w.bias, 2 * d);
+        ln(blank(FR_GEMM), FR_ROWS_LN_SILU, cbuf, L.cnorm_w, L.cnorm_b, nullptr, FR_EPI_RESID, L.t_pw2, L.pw2_w.bias, d);
+        ln(up, FR_ROWS_LN, cur, L.ln_ff2_w, L.ln_ff2_b, nullptr, FR_EPI_PLANES, L.t_ff2a, L.ff2_w1.bias, F);
+        resid(hF, L.t_ff2b, L.ff2_w2.bias, F, 0.5f);
+    }
+    if (fr_upload(st.fr_table_host, st.fr_table_dev, fr_table(ops))) return -1;
+    a.M = M; a.terms = cfg.strict ? 3 : 1; a.d = d; a.H = n_heads; a.dk = d_head;
+    a.bar = st.fr_bar; a.status = status; a.S = S; a.Q = Q; a.left = st.left; a.valid = st.valid; a.d_start = st.d_start;
+    if (fr_launch(a, ops, st.fr_table_dev, stream)) return -1;
+    const EncLayer &Z = layers[n_layers - 1];
+    if (layer_norm(cur, Z.ln_out_w, Z.ln_out_b, x, H16{nullptr, nullptr}, M, d, ACT_NONE, stream)) return -1;
+    note_launch();
+    return 0;
 }
 
 int Model::stream_step_eager(StreamState &st, const float *mel, int n_mel, int is_last, float *out) {
@@ -400,6 +475,18 @@ int Model::stream_step_eager(StreamState &st, const float *mel, int n_mel, int i
     }
     const H16 none{nullptr, nullptr};
     const int leftn = st.left > 0 ? st.left : 1;
+    if (st.persistent) {
+        // the position keys of all layers from one contraction, side by side: [P][layers d]
+        const int ldrk = n_layers * d;
+        __half *rk_all = rk_keep ? st.rk_cache : ws.planes((size_t)P * ldrk, false).hi;
+        if (!rk_all) return -1;
+        if (!rk_have) {
+            QWeight w = layers[0].relk;
+            w.n = ldrk;
+            if (gemm(pe, d, w, st_epi(OUT_H16, ACT_NONE, 1.f, nullptr, nullptr, 0, H16{rk_all, nullptr}, ldrk), P)) return -1;
+        }
+        if (stream_layers(st, x, Q, rk_all, ldrk)) return -1;
+    }
     // In a few-row group the LayerNorm that follows a residual update runs inside the contraction that makes it
     const bool tail = st.few_rows && st.ln_count && gemm_skinny_ln_width(d);
     auto resid = [&](float alpha, const float *bias, const float *nw, const float *nb) {
@@ -407,7 +494,7 @@ int Model::stream_step_eager(StreamState &st, const float *mel, int n_mel, int i
         if (tail) { e.ln_w = nw; e.ln_b = nb; e.ln_hi = hA.hi; e.ln_lo = hA.lo; e.ln_count = st.ln_count; }
         return e;
     };
-    for (int li = 0; li < n_layers; li++) {
+    for (int li = 0; li < n_layers && !st.persistent; li++) {
         const EncLayer &L = layers[li];
         __half *kc = st.k_cache + (size_t)li * S * leftn * d, *vc = st.v_cache + (size_t)li * S * leftn * d;
         float *cc = st.conv_cache + (size_t)li * S * (conv_k - 1) * d;

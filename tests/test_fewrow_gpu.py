@@ -1,0 +1,53 @@
+"""The persistent few-row kernel (csrc/fewrow.cu) where its tiles end: one row, the largest rows with fused LayerNorms,
+a tile and one row more, several tiles; slabs of K (one partial, one whole, two); a depthwise width without a register
+path. Streams against the numpy oracle, attention-decoder batches against each utterance alone and the oracle."""
+from contextlib import closing
+
+import numpy as np
+import pytest
+
+import cases
+from oracle import mynah_oracle as O, model_io
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {
+    "partial_slab": dict(d_model=192, n_heads=6, ffn_dim=448, wtype="q8_0", use_bias=True),
+    "two_slabs": dict(d_model=128, n_heads=1, ffn_dim=2048, wtype="q4_0", conv_k=5),
+    "whole_slab": dict(d_model=1024, n_heads=8, ffn_dim=1024, wtype="q8_0"),
+}
+
+
+@pytest.mark.parametrize("shape,streams,right", [
+    ("partial_slab", 1, 0), ("partial_slab", 4, 0), ("partial_slab", 5, 0), ("partial_slab", 17, 0), ("partial_slab", 64, 1),
+    ("two_slabs", 1, 2), ("two_slabs", 3, 1), ("two_slabs", 33, 0), ("whole_slab", 2, 0), ("whole_slab", 9, 0)])
+def test_streams(gpu_pkg, synth, shape, streams, right):
+    cfg = synth.config(shape, n_layers=2, n_mels=80, decoder="rnnt", vocab=33, pred_hidden=32, pred_layers=1, causal=True,
+                       normalize=False, **SHAPES[shape])
+    tensors = synth.make_model(cfg, seed=3)
+    with closing(cases.device_model(gpu_pkg, synth, cfg, tensors)) as dm:
+        mels = np.random.default_rng(streams).standard_normal((streams, 96, 80), dtype=np.float32) - 5.0
+        g, outs, pos = dm.stream_open(streams, 5, right), [], 0
+        while pos < 96:
+            n = min(g.need(), 96 - pos)
+            outs.append(g.step(mels[:, pos:pos + n], pos + n >= 96))
+            pos += n
+        g.close()
+        out = np.concatenate(outs, axis=1)
+    M = model_io.oracle_model(cfg, tensors)
+    for s in {0, streams // 2, streams - 1}:
+        ref = O.stream_encode(M, mels[s], 5, right)
+        assert out[s].shape == ref.shape and np.linalg.norm(out[s] - ref) < 1e-3 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("batch", [1, 2, 4, 5, 16, 17])
+def test_attention_decoder(gpu_pkg, synth, batch):
+    cfg, tensors = cases.build(synth, "aed_proj")
+    A = model_io.oracle_model(cfg, tensors)["aed"]
+    rng = np.random.default_rng(batch)
+    encs = [rng.standard_normal((3 + 5 * i, cfg.d_model), dtype=np.float32) for i in range(batch)]
+    with closing(cases.device_model(gpu_pkg, synth, cfg, tensors, aed_heads=cfg.aed_heads)) as dm:
+        got = dm.aed_decode_batch(encs, [cases.AED_PROMPT[:1 + i % 3] for i in range(batch)], -1, [12] * batch)
+        for i in {0, batch // 2, batch - 1}:
+            p = cases.AED_PROMPT[:1 + i % 3]
+            assert list(got[i]) == dm.aed_decode(encs[i], p, -1, 12).tolist() == O.aed_decode(A, encs[i], p, -1, 12).tolist()
