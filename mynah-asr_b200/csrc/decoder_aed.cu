@@ -328,7 +328,7 @@ static GemmEpilogue aed_epi(int mode, int act, float alpha, const float *bias, f
 size_t Model::aed_bytes(int total_T, int B, int max_len) const {
     const size_t D = aed_d, F = aed_ffn, L = aed_layers.size();
     return (size_t)total_T * (d_out * 4 + D * 4 + (L + 1) * 2 * D * 4) + L * 2 * (size_t)B * max_len * D * 4 +
-           (size_t)B * (D * 24 + 3 * D * 4 + F * 4 + (size_t)aed_vocab * 4) + (size_t)B * (max_len + 64 + 148) * 8 + fr_table_bytes(11 * L + 3) + (1 << 20);
+           (size_t)B * (D * 24 + 3 * D * 4 + F * 4 + (size_t)aed_vocab * 4) + (size_t)B * (max_len + 64 + 148) * 8 + fr_table_bytes(8 * L + 1) + FR_BAR_WORDS * 4 + (1 << 20);
 }
 
 int Model::decode_aed(const float *enc_dev, const std::vector<int> &lens, const std::vector<std::vector<int>> &prompts, int eos,
@@ -450,21 +450,16 @@ int Model::decode_aed(const float *enc_dev, const std::vector<int> &lens, const 
     if (fr_aed && B <= FR_MAX_ROWS && fr_grid(B, 16, &mtiles, &ngroups) == 0) {
         FrArgs a;
         memset(&a, 0, sizeof(a));
-        uint8_t *table_dev = ws.get<uint8_t>(fr_table_bytes((size_t)11 * L + 3));
+        uint8_t *table_dev = ws.get<uint8_t>(fr_table_bytes((size_t)8 * L + 1));
         a.cand_v = ws.get<float>((size_t)B * ngroups); a.cand_i = ws.get<int>((size_t)B * ngroups);
-        a.bar = ws.get<unsigned>(2);
+        a.bar = ws.get<unsigned>(FR_BAR_WORDS);
         if (!table_dev || !a.cand_v || !a.cand_i || !a.bar) return -1;
-        const bool fuse = B <= FR_FUSE_ROWS;
         std::vector<FrOp> ops;
         auto blank = [](int type) { FrOp o; memset(&o, 0, sizeof(o)); o.type = type; o.alpha = 1.f; return o; };
-        // a contraction over LayerNorm rows of x: fused, or behind an operation of its own that makes their planes
+        // a contraction over LayerNorm rows of x; the position's first over its selection and embedding
         auto from_x = [&](FrOp o, int epi, const uint8_t *w, const float *bias, int N, const float *lw, const float *lb) {
-            const bool turn = ops.empty();                   // position's first: selection and embedding
-            FrOp n = blank(FR_LN);
-            n.rows = turn ? FR_ROWS_AED_NEXT : FR_ROWS_LN; n.x = x; n.ln_w = lw; n.ln_b = lb; n.K = D; n.o_hi = xn.hi; n.o_lo = xn.lo;
-            if (turn) { n.ln0_w = aed_embln_w; n.ln0_b = aed_embln_b; n.x_copy = x; }
-            if (fuse) { o.rows = n.rows; o.x = x; o.ln_w = lw; o.ln_b = lb; o.ln0_w = n.ln0_w; o.ln0_b = n.ln0_b; o.x_copy = n.x_copy; }
-            else { ops.push_back(n); o.rows = FR_ROWS_PLANES; o.a_hi = xn.hi; o.a_lo = xn.lo; }
+            o.rows = FR_ROWS_LN; o.x = x; o.ln_w = lw; o.ln_b = lb;
+            if (ops.empty()) { o.rows = FR_ROWS_AED_NEXT; o.ln0_w = aed_embln_w; o.ln0_b = aed_embln_b; o.x_copy = x; }
             o.epi = epi; o.w = w; o.bias = bias; o.N = N; o.K = D; o.ldo = N;
             ops.push_back(o);
         };
@@ -496,7 +491,6 @@ int Model::decode_aed(const float *enc_dev, const std::vector<int> &lens, const 
             into_x(ff, A.t_ff2, A.ff2_b, F);
         }
         from_x(blank(FR_GEMM), FR_EPI_ARGMAX, t_aed_head, aed_head_b, V, aed_fin_w, aed_fin_b);
-        if (ops.size() % 2) ops.push_back(blank(FR_NOP));
         const std::vector<uint8_t> table = fr_table(ops);
         MB_CUDA(cudaMemcpyAsync(table_dev, table.data(), table.size(), cudaMemcpyHostToDevice, stream));
         a.M = B; a.tile_rows = 16; a.mtiles = mtiles; a.ngroups = ngroups;

@@ -3,24 +3,22 @@
 // A streaming step or an AED position is a few hundred dependent operations of at most 128 rows. As launches, chained and
 // replayed from a graph, each of them costs 9-11 us (set-up, tensor-memory allocation, slice sums over a cluster, LayerNorm
 // by the last warp to arrive) where its bytes would need one. Here one cooperative launch walks the whole chain; what
-// separates two operations is a grid barrier (about 1 us):
+// separates two operations is a barrier over the CTAs of a row tile (about 1.3 us):
 //   * a CTA keeps its place: a row tile of at most sixteen rows and every ngroups-th unit of eight weight rows. It sums a
-//     unit over all of K itself (eight warps take alternate 64-wide pieces of K, added in warp order), so nothing is
-//     exchanged between CTAs inside an operation, and a row's bits do not depend on how many other rows there are;
-//   * weights are the stored 8-bit blocks (1.06 bytes per parameter instead of 4 as operand planes) in fragment order; a
-//     producer warp streams them into a ring of shared memory with bulk copies and runs ahead through the barriers, so
-//     that HBM works while the chain waits for its latencies;
+//     unit over all of K itself (sixteen warps take 64-wide pieces of K, added in warp order), so nothing is exchanged
+//     between CTAs inside an operation, and a row's bits do not depend on how many other rows there are;
+//   * weights are the stored 8-bit blocks (1.06 bytes per parameter instead of 4 as operand planes) in fragment order; every
+//     warp copies its pieces ahead into a ring of its own, through the barriers, so that HBM works while the chain waits;
 //   * the products are mma.sync m16n8k16 on the integers themselves (exact in fp16) against the activations' (hi, lo)
 //     planes, summed per 32-element block, then one f32 multiply-add per block with its scale: the quantised weight is
 //     never rounded. (tcgen05 wants 128 rows on one side: a unit of eight weight rows per SM is what keeps all SMs busy
 //     with N = 1024 and no exchange of partial sums.)
-//   * with few rows the LayerNorms are computed where their result is staged, by every CTA; with more, as an operation that
-//     spreads the rows over the CTAs. The conv module's middle sits in the epilogue of the contraction before it.
-// Measured: a step of 24 layers of d = 1024 takes 1.34 ms for one stream (2.74 as launches), 2.25 for 22, 4.1 for 64 with
-// decoding (4.8), 5.3 for 120 (5.9); AED with 32 + 8 layers takes 31 ms for one sentence (48.7), 61 for eight (78).
+//   * the LayerNorms are computed where their result is staged, by every CTA. The conv module's middle sits in the epilogue
+//     of the contraction before it.
+// Measured: a step of 24 layers of d = 1024 takes 1.16 ms for one stream (2.74 as launches), 2.25 for 22, 3.7 for 64 with
+// decoding (4.8), 4.9 for 120 (5.9); AED with 32 + 8 layers takes 27.5 ms for one sentence (48.7), 53 for eight (78).
 // Values that other CTAs write are read past the L1 (ld.cg, cp.async.cg). All waits are bounded: one that runs out sets the
-// status word and the abort flag, and every CTA leaves. Nothing may spill: beside 220 KB of shared memory the L1 holds less
-// than the stacks of 256 threads, and every spilled value then goes to the L2.
+// status word and the abort flag, and every CTA leaves.
 #include "fewrow.h"
 
 #include <string.h>
@@ -30,23 +28,19 @@
 
 namespace mb {
 
-static constexpr int FR_WARPS = 8, FR_THREADS = FR_WARPS * 32, FR_LAUNCH = FR_THREADS + 128;
-static constexpr int FR_SLAB = 1024;                     // K per staged slab and per ring piece
+static constexpr int FR_WARPS = 16, FR_THREADS = FR_WARPS * 32;
+static constexpr int FR_SLAB = 1024;                     // K per staged slab and per piece of a unit: 64 for each warp
 static constexpr int FR_PAIR_BYTES = 544;                // 64 k x 8 rows: 512 bytes of quants, 32 of scales
-static constexpr int FR_PAIRS = FR_SLAB / 64;
-static constexpr int FR_PIECE = FR_PAIRS * FR_PAIR_BYTES;
-static constexpr int FR_STAGES = 8;
-static constexpr int FR_GU = 4;                          // units whose sums a CTA holds at a time
+static constexpr int FR_AHEAD = 6;                       // pieces of weights a warp has asked for
+static constexpr int FR_CT = 160;                        // floats of a warp's sums of two units and eight rows (fr_red)
 static constexpr int FR_CONV_K = 9;                      // depthwise width with a register path
-static constexpr int FR_MAX_GEMMS = FR_MAX_LAYERS * 8;   // contractions of a chain (their weights' places sit in shared memory)
+static constexpr int FR_LISTS = 16;                      // lists of keys of an attention
 static constexpr int FR_XS = FR_SLAB + 32;               // halves per staged row: rows four 16-byte columns apart, no bank conflicts
 static constexpr int FR_XPLANE = 32 * FR_XS * 2;         // bytes of one plane of 32 rows
-static constexpr int FR_RED_FLOATS = FR_WARPS * FR_GU * 128;      // (also four LayerNorm vectors)
-static constexpr int FR_VALS = FR_GU * 128;
-static constexpr int FR_SMEM = FR_STAGES * FR_PIECE + 2 * FR_XPLANE + FR_RED_FLOATS * 4 + FR_VALS * 4 + FR_MAX_GEMMS * 16 + 256;
-static_assert(FR_SMEM <= 230000, "shared memory");
-static_assert(FR_RED_FLOATS >= 4 * FR_SLAB, "LayerNorm vectors");
-static_assert(FR_GU * 128 == 2 * FR_THREADS, "two outputs per thread and group");
+static constexpr int FR_RED_FLOATS = FR_WARPS * 4 * FR_CT;
+static_assert(16 * FR_XS * 2 >= 4 * FR_SLAB * 4, "LayerNorm vectors behind the rows of a tile");
+static_assert(2 * FR_XPLANE >= FR_WARPS * FR_LISTS * 128 * 4, "lists of an attention per warp");
+static_assert(FR_RED_FLOATS >= 8 * 8 * 32 * 4, "exchange of the LayerNorms' sums");
 
 // ------------------------------------------------------------------------------------------------ weight tiles
 bool fr_can_tile(const QWeight &w) {
@@ -72,7 +66,7 @@ __global__ void fr_retile_kernel(const uint8_t *__restrict__ raw, uint8_t *__res
             int v;
             if (FMT == FMT_GGML_Q8_0) v = (int8_t)blk[2 + e];
             else v = (e < 16 ? blk[2 + e] & 15 : blk[2 + e - 16] >> 4) - 8;
-            q[8 * b + j] = row < n ? (uint8_t)(int8_t)v : 0;
+            q[8 * b + j] = (uint8_t)((row < n ? v : 0) + 128);
         }
         sc[b] = __ushort_as_half(row < n ? (unsigned short)(blk[0] | (blk[1] << 8)) : (unsigned short)0);
     }
@@ -93,23 +87,18 @@ int fr_retile(const QWeight &w, uint8_t *dst, bool glu, cudaStream_t st) {
 }
 
 // ----------------------------------------------------------------------------------------------------- helpers
-__device__ __forceinline__ void fr_sync() { asm volatile("bar.sync 1, %0;" ::"n"(FR_THREADS) : "memory"); }   // the computing warps
+__device__ __forceinline__ void fr_sync() { __syncthreads(); }
 
-__device__ __forceinline__ void fr_bulk(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
 // not volatile: the products of the four blocks of a piece are independent and may interleave
 __device__ __forceinline__ void fr_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// four int8 -> two half2, exact: the byte q + 128 under the exponent of 1024, minus 1152
+// four bytes q + 128 -> two half2 of q, exact: the byte under the exponent of 1024, minus 1152
 __device__ __forceinline__ void fr_widen(uint32_t q, uint32_t &h0, uint32_t &h1) {
-    const uint32_t u = q ^ 0x80808080u;
     const __half2 k = __halves2half2(__ushort_as_half(0xE480), __ushort_as_half(0xE480));       // -1152
-    const uint32_t a = __byte_perm(u, 0x64646464u, 0x4140), b = __byte_perm(u, 0x64646464u, 0x4342);
+    const uint32_t a = __byte_perm(q, 0x64646464u, 0x4140), b = __byte_perm(q, 0x64646464u, 0x4342);
     const __half2 x = __hadd2(*reinterpret_cast<const __half2 *>(&a), k), y = __hadd2(*reinterpret_cast<const __half2 *>(&b), k);
     h0 = *reinterpret_cast<const uint32_t *>(&x);
     h1 = *reinterpret_cast<const uint32_t *>(&y);
@@ -119,91 +108,158 @@ __device__ __forceinline__ void fr_cp16(uint32_t dst, const void *src) {
 }
 __device__ __forceinline__ void fr_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void fr_cp_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void fr_cp_wait_but() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-struct alignas(16) FrWeights { const uint8_t *w; int N, K; };
-
+// Shared memory by fixed offsets: nothing of it takes a register.
+extern __shared__ __align__(128) uint8_t fr_smem[];
 struct FrShared {
-    uint8_t *ring;                        // FR_STAGES pieces
-    uint8_t *xs;                          // [plane][32 rows]: two slabs of 16 rows, or all slabs of few rows one behind the other
-    float *red, *vals;                    // partial sums per warp; finished sums of a group
-    uint64_t *full, *empty;
-    volatile int *stop;                   // the computing warps have left, or a wait ran out
-    const FrWeights *tab;                 // the chain's contractions in order
-    float *best_v;                        // running maximum per row of the tile (FR_EPI_ARGMAX)
-    int *best_i;
-    __device__ __forceinline__ __half *x(int row, int plane) const { return reinterpret_cast<__half *>(xs + plane * FR_XPLANE) + row * FR_XS; }
+    static constexpr int RING = 0, XS = FR_AHEAD * FR_WARPS * FR_PAIR_BYTES, RED = XS + 2 * FR_XPLANE, VALS = RED + FR_RED_FLOATS * 4, OPS = VALS + FR_THREADS * 4,
+                         BEST = OPS + 2 * (int)sizeof(FrOp), STOP = BEST + 128, END = STOP + 16;
+    template <typename T> static __device__ __forceinline__ T *at(int o) { return reinterpret_cast<T *>(fr_smem + o); }
+    static __device__ __forceinline__ uint8_t *ring(int warp, int slot) { return fr_smem + RING + (warp * FR_AHEAD + slot) * FR_PAIR_BYTES; }
+    // [plane][32 rows]: two slabs of 16 rows, or all slabs of few rows one behind the other
+    static __device__ __forceinline__ __half *x(int row, int plane) { return at<__half>(XS + plane * FR_XPLANE) + row * FR_XS; }
+    static __device__ __forceinline__ float *red() { return at<float>(RED); }                   // partial sums per warp
+    static __device__ __forceinline__ float *vals() { return at<float>(VALS); }                 // finished sums of a group
+    static __device__ __forceinline__ FrOp &op(unsigned i) { return at<FrOp>(OPS)[i & 1]; }     // this operation and the next one
+    static __device__ __forceinline__ float *best_v() { return at<float>(BEST); }               // running maximum per row (FR_EPI_ARGMAX)
+    static __device__ __forceinline__ int *best_i() { return at<int>(BEST + 64); }
+    static __device__ __forceinline__ volatile int *stop() { return at<int>(STOP); }            // a wait ran out
 };
+static_assert(FrShared::END <= 232448, "shared memory");
+static constexpr int FR_SMEM = FrShared::END;
 
 struct FrPlace {                          // the CTA's place
-    int ng, row0, rows;                   // unit group, first row and rows of the tile
+    int ng, mt, row0, rows;               // unit group, row tile, its first row and rows
     int tid, warp, lane;
 };
 
-// Every CTA has arrived `target / gridDim.x` times. False: a wait ran out here or elsewhere.
-__device__ __forceinline__ bool fr_grid_sync(const FrArgs &a, const FrShared &s, const FrPlace &c, unsigned target) {
-    fr_sync();
-    if (c.tid == 0) {
-        // the block barrier before and the release make the CTA's writes visible with the arrival, the acquire and the block
-        // barrier behind it those of the others to all warps
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
-        const long long t0 = clock64();
-        unsigned v;
-        for (int tries = 1;; tries++) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
-            if (v >= target) break;
-            if (tries & 63) continue;
-            if (*reinterpret_cast<volatile unsigned *>(a.bar + 1) || clock64() - t0 > (1ll << 31)) {
-                atomicExch(a.bar + 1, 1u);
-                atomicCAS(a.status, ST_OK, ST_TIMEOUT_EPILOGUE);
-                *s.stop = 1;
-                break;
-            }
+// The LayerNorm vectors of a contraction, asked for ahead of it: behind the rows of its tile, where nothing else is then.
+__device__ __forceinline__ float *fr_vectors() { return reinterpret_cast<float *>(FrShared::x(16, 0)); }
+__device__ __forceinline__ void fr_ask_vectors(const FrOp &op, int tid, int n) {
+    if (op.type != FR_GEMM || op.rows == FR_ROWS_PLANES) return;
+    const bool two = op.rows == FR_ROWS_LN2 || op.rows == FR_ROWS_AED_NEXT;
+    const uint32_t v = smem_u32(fr_vectors());
+    for (int i = tid; i < op.K >> 2; i += n) {
+        fr_cp16(v + 16 * i, op.ln_w + 4 * i);
+        fr_cp16(v + 4 * FR_SLAB + 16 * i, op.ln_b + 4 * i);
+        if (two) { fr_cp16(v + 8 * FR_SLAB + 16 * i, op.ln0_w + 4 * i); fr_cp16(v + 12 * FR_SLAB + 16 * i, op.ln0_b + 4 * i); }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------------ weights
+// NB: eight-row halves of a row tile. Units whose sums a CTA holds at a time:
+__host__ __device__ constexpr int fr_gu(int NB) { return 8 / NB; }
+
+// A warp's way through the weights of a contraction: its 64 wide parts of this CTA's units, in groups of fr_gu units, in a group
+// slab by slab, unit by unit. The next FR_AHEAD of them are on their way into a ring of the warp's own, the first ones since
+// before the grid barrier: what comes from HBM travels while the chain waits for its latencies. One commit group per piece,
+// empty ones behind the last. (A producer warp with bulk copies costs every warp a wait and an arrival per unit, 350 of 800
+// cycles; in registers the pieces leave the LayerNorms too few.)
+struct FrFeed {
+    const uint8_t *base;                  // of slab 0 of the CTA's first unit, at the warp's part
+    uint32_t ustep, sstep;                // bytes to the CTA's next unit, to the next slab
+    int mine, slabs, first, sl, u;        // units and slabs; the next piece to ask for
+    int slot;                             // where it goes: the place of the piece that is used next
+};
+template <int NB>
+__device__ __forceinline__ void fr_ask(FrFeed &f, const FrPlace &c) {
+    if (f.first < f.mine) {
+        const uint8_t *p = f.base + (size_t)(f.first + f.u) * f.ustep + f.sl * f.sstep + c.lane * 16;
+        const uint32_t to = smem_u32(FrShared::ring(c.warp, f.slot)) + c.lane * 16;
+        fr_cp16(to, p);
+        if (c.lane < 2) fr_cp16(to + 512, p + 512);
+        if (++f.u >= fr_gu(NB) || f.first + f.u >= f.mine) {
+            f.u = 0;
+            if (++f.sl >= f.slabs) { f.sl = 0; f.first += fr_gu(NB); }
         }
     }
+    fr_cp_commit();
+    f.slot = f.slot + 1 == FR_AHEAD ? 0 : f.slot + 1;
+}
+template <int NB>
+__device__ __forceinline__ void fr_open(const FrArgs &a, const FrOp &op, const FrPlace &c, FrFeed &f) {
+    f.mine = f.first = f.sl = f.u = f.slot = 0;
+    if (op.type != FR_GEMM) return;
+    const int units = (op.N + 7) >> 3, ks = op.K < FR_SLAB ? op.K : FR_SLAB;
+    f.slabs = op.K <= FR_SLAB ? 1 : op.K / FR_SLAB;
+    f.sstep = (ks >> 6) * FR_PAIR_BYTES;
+    f.ustep = a.ngroups * f.slabs * f.sstep;
+    f.base = op.w + (size_t)c.ng * f.slabs * f.sstep + c.warp * FR_PAIR_BYTES;
+    if (c.warp < (ks >> 6) && units > c.ng) f.mine = (units - c.ng + a.ngroups - 1) / a.ngroups;
+#pragma unroll 1
+    for (int i = 0; i < FR_AHEAD; i++) fr_ask<NB>(f, c);
+}
+
+// All CTAs of this row tile have come `target / ngroups` times (a row tile's chain never looks at another tile's rows).
+// Meanwhile the next operation's LayerNorm vectors and first weights are asked for. False: a wait ran out here or elsewhere.
+// (A word per CTA that one warp of every CTA watches, instead of one counter: 2.5 k cycles become 6 k, all read the same lines.)
+template <int NB>
+__device__ __forceinline__ bool fr_tile_sync(const FrArgs &a, const FrPlace &c, const FrOp &next, FrFeed &f, unsigned target) {
     fr_sync();
-    return *s.stop == 0;
+    unsigned *count = a.bar + 32 * (1 + c.mt);
+    // the block barrier before and the release make the CTA's writes visible with the arrival, the acquire and the block
+    // barrier behind it those of the others to all warps
+    if (c.tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    fr_open<NB>(a, next, c, f);
+    if (c.warp == 0) {
+        if (c.lane == 0) {
+            const long long t0 = clock64();
+            unsigned v;
+            for (int tries = 1;; tries++) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+                if (v >= target) break;
+                if (tries & 63) continue;
+                if (*reinterpret_cast<volatile unsigned *>(a.bar) || clock64() - t0 > (1ll << 31)) {
+                    atomicExch(a.bar, 1u);
+                    atomicCAS(a.status, ST_OK, ST_TIMEOUT_EPILOGUE);
+                    *FrShared::stop() = 1;
+                    break;
+                }
+            }
+        }
+    } else {
+        fr_ask_vectors(next, c.tid - 32, FR_THREADS - 32);
+        fr_cp_commit();
+    }
+    fr_sync();
+    return *FrShared::stop() == 0;
 }
 
 // --------------------------------------------------------------------------------------------------- LayerNorms
-// LayerNorm of rows that are spread over 8 / NC warps each: a warp holds the NC 128-wide chunks sub, sub + 8 / NC, .. of its row,
-// a lane four columns of each. The statistics are ln_stats' (ln_row.cuh), formed chunk by chunk in chunk order whatever NC is, so
-// that a row's bits do not depend on how many rows share the CTA. slot: the exchange buffer of this use. All warps call it.
+// LayerNorm of a row of at most 1024 by 8 / NC warps: warp `sub` of them holds the 128-wide chunks sub, sub + 8 / NC, .., a lane
+// four columns of each. Sums in double, each lane over the chunks in order (the row's warps exchange them), then a butterfly: a
+// row's bits do not depend on how many rows share the CTA. All warps call it.
 template <int NC>
-__device__ __forceinline__ void fr_ln(const FrShared &s, float4 (&v)[NC], const float *w, const float *b, int K, float first, int row, int sub, int lane, int slot) {
-    constexpr int WPR = FR_WARPS / NC;
-    const int n4 = K >> 2;
-    const double x0 = (double)first, rk = 1.0 / (double)K;
-    double2 *part = reinterpret_cast<double2 *>(s.vals) + slot * 64 + row * 8;
-    double t[NC], q[NC];
+__device__ __forceinline__ void fr_ln(float4 (&v)[NC], const float4 *w, const float4 *b, int n4, double rk, int row, int sub, int lane) {
+    constexpr int WPR = 8 / NC;
+    double t = 0.0, q = 0.0;
+    double2 *part = reinterpret_cast<double2 *>(FrShared::red()) + row * 8 * 32 + lane;
 #pragma unroll
     for (int i = 0; i < NC; i++) {
-        t[i] = q[i] = 0.0;
-        if (lane + 32 * (sub + WPR * i) < n4) {
-            const double d0 = (double)v[i].x - x0, d1 = (double)v[i].y - x0, d2 = (double)v[i].z - x0, d3 = (double)v[i].w - x0;
-            t[i] = (d0 + d1) + (d2 + d3);
-            q[i] = fma(d0, d0, d1 * d1) + fma(d2, d2, d3 * d3);
-        }
+        const double x = v[i].x, y = v[i].y, z = v[i].z, u = v[i].w;             // zeros beyond the row
+        const double ct = (x + y) + (z + u), cq = fma(x, x, y * y) + fma(z, z, u * u);
+        if (WPR > 1) part[(sub + WPR * i) * 32] = make_double2(ct, cq);
+        else { t += ct; q += cq; }
+    }
+    if (WPR > 1) {
+        fr_sync();
+#pragma unroll
+        for (int j = 0; j < 8; j++) { const double2 e = part[j * 32]; t += e.x; q += e.y; }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int i = 0; i < NC; i++) { t[i] += __shfl_xor_sync(0xffffffffu, t[i], o); q[i] += __shfl_xor_sync(0xffffffffu, q[i], o); }
-#pragma unroll
-    for (int i = 0; i < NC; i++) if (lane == 0) part[sub + WPR * i] = make_double2(t[i], q[i]);
-    fr_sync();
-    double sum = 0.0, sq = 0.0;
-#pragma unroll
-    for (int j = 0; j < FR_WARPS; j++) { const double2 p = part[j]; sum += p.x; sq += p.y; }
-    const double m = sum * rk, ve = fma(-sum, m, sq) * rk + 1e-5;
-    const float muf = (float)(x0 + m), inv = (float)rsqrt(ve);
+    for (int o = 16; o > 0; o >>= 1) { t += __shfl_xor_sync(0xffffffffu, t, o); q += __shfl_xor_sync(0xffffffffu, q, o); }
+    // 1 / sqrt: the single precision value and one Newton step in double
+    const double m = t * rk, ve = fma(-t, m, q) * rk + 1e-5, y = (double)rsqrtf((float)ve);
+    const float mu = (float)m, inv = (float)(y * fma(-0.5 * ve * y, y, 1.5));
 #pragma unroll
     for (int i = 0; i < NC; i++) {
         const int at = lane + 32 * (sub + WPR * i);
-        if (at < n4) {
-            const float4 ww = reinterpret_cast<const float4 *>(w)[at], bb = reinterpret_cast<const float4 *>(b)[at];
-            v[i] = make_float4(((v[i].x - muf) * inv) * ww.x + bb.x, ((v[i].y - muf) * inv) * ww.y + bb.y,
-                               ((v[i].z - muf) * inv) * ww.z + bb.z, ((v[i].w - muf) * inv) * ww.w + bb.w);
-        }
+        if (at >= n4) continue;
+        const float4 ww = w[at], bb = b[at];
+        v[i] = make_float4(((v[i].x - mu) * inv) * ww.x + bb.x, ((v[i].y - mu) * inv) * ww.y + bb.y,
+                           ((v[i].z - mu) * inv) * ww.z + bb.z, ((v[i].w - mu) * inv) * ww.w + bb.w);
     }
 }
 
@@ -235,160 +291,141 @@ __device__ __forceinline__ int fr_aed_turn(const FrArgs &a, int lane, int b, int
             else { a.tokens[(size_t)b * a.cap_stride + n] = bi; st[B + b] = n + 1; }
         }
         if (p >= st[4 * B + b]) fin = true;
-        if (fin) { st[2 * B + b] = 1; atomicAdd(st + 6 * B, 1); }
+        if (fin) st[2 * B + b] = 1;
     }
     return cur;
 }
 
-// Rows row0, row0 + 1, .. (n of them, NC at a time) through the operation's LayerNorms. FUSED: into the X tile of a contraction,
-// every unit group for itself; else into the planes o_hi, o_lo. first_group: this CTA keeps LN2's rows and an AED row's books.
-template <int NC, bool FUSED, bool AED>
-__device__ __forceinline__ void fr_rows(const FrArgs &a, const FrOp &op, const FrShared &s, const FrPlace &c, int row0, int n, bool first_group, int p) {
-    constexpr int WPR = FR_WARPS / NC;                           // warps per row
-    bool fits = true;
-    const int K = op.K, n4 = K >> 2, sub = c.warp % WPR, slot = c.warp / WPR;
-    // the LayerNorms' vectors, by all threads, into the (idle) sums' place while the rows are on their way
-    const bool two = op.rows == FR_ROWS_LN2 || (AED && op.rows == FR_ROWS_AED_NEXT);
-    float *lw = s.red, *lb = lw + FR_SLAB, *lw0 = lb + FR_SLAB, *lb0 = lw0 + FR_SLAB;
-    for (int i = c.tid; i < n4; i += FR_THREADS) {
-        fr_cp16(smem_u32(lw + 4 * i), op.ln_w + 4 * i);
-        fr_cp16(smem_u32(lb + 4 * i), op.ln_b + 4 * i);
-        if (two) { fr_cp16(smem_u32(lw0 + 4 * i), op.ln0_w + 4 * i); fr_cp16(smem_u32(lb0 + 4 * i), op.ln0_b + 4 * i); }
-    }
-    fr_cp_commit();
-    float *firsts = s.best_v;                                    // the second LayerNorm's first value of every row
-    for (int r0 = 0; r0 < n; r0 += NC) {
-        const int r = r0 + slot, m = row0 + (r < n ? r : 0);
-        const bool on = r < n;
-        float4 v[NC];
-        float first;
+// The rows of the tile through the contraction's LayerNorms into X, 8 / NC warps to a row; every unit group for itself. Group 0 keeps
+// LN2's rows and an AED row's books.
+template <bool AED, int NC>
+__device__ __forceinline__ void fr_rows(const FrArgs &a, const FrOp &op, const FrPlace &c, int p) {
+    const int K = op.K, n4 = K >> 2, r = c.warp / (8 / NC), sub = c.warp % (8 / NC), m = c.row0 + r;
+    const bool on = r < c.rows;
+    const float4 *vec = reinterpret_cast<const float4 *>(fr_vectors());
+    float4 v[NC];
+    if (on) {
+        const float *x = op.x + (size_t)m * K, *pe = nullptr;
         if (AED && op.rows == FR_ROWS_AED_NEXT) {
-            const int cur = fr_aed_turn(a, c.lane, m, p, on && first_group && sub == 0), at = p < a.max_seq ? p : a.max_seq - 1;
-            const float *e = a.emb + (size_t)cur * K, *pe = a.pos + (size_t)at * K;
-#pragma unroll
-            for (int i = 0; i < NC; i++) {
-                const int col = c.lane + 32 * (sub + WPR * i);
-                v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (col < n4) {
-                    const float4 x = __ldg(reinterpret_cast<const float4 *>(e) + col), y = __ldg(reinterpret_cast<const float4 *>(pe) + col);
-                    v[i] = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
-                }
-            }
-            first = __ldg(e) + __ldg(pe);
-        } else {
-            const float *x = op.x + (size_t)m * K;
-#pragma unroll
-            for (int i = 0; i < NC; i++) {
-                const int col = c.lane + 32 * (sub + WPR * i);
-                v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (col < n4) v[i] = __ldcg(reinterpret_cast<const float4 *>(x) + col);
-            }
-            first = __ldcg(x);
-        }
-        fr_cp_wait();
-        fr_sync();
-        if (two) {
-            fr_ln<NC>(s, v, lw0, lb0, K, first, slot, sub, c.lane, 0);
-            if (first_group && on) {
-#pragma unroll
-                for (int i = 0; i < NC; i++) {
-                    const int col = c.lane + 32 * (sub + WPR * i);
-                    if (col < n4) reinterpret_cast<float4 *>(op.x_copy + (size_t)m * K)[col] = v[i];
-                }
-            }
-            if (sub == 0 && c.lane == 0) firsts[slot] = v[0].x;
-            fr_sync();
-            first = firsts[slot];
-        }
-        fr_ln<NC>(s, v, lw, lb, K, first, slot, sub, c.lane, 1);
-        if (op.rows == FR_ROWS_LN_SILU) {
-#pragma unroll
-            for (int i = 0; i < NC; i++) v[i] = make_float4(silu_f(v[i].x), silu_f(v[i].y), silu_f(v[i].z), silu_f(v[i].w));
+            x = a.emb + (size_t)fr_aed_turn(a, c.lane, m, p, c.ng == 0 && sub == 0) * K;
+            pe = a.pos + (size_t)(p < a.max_seq ? p : a.max_seq - 1) * K;
         }
 #pragma unroll
         for (int i = 0; i < NC; i++) {
-            const int col = c.lane + 32 * (sub + WPR * i);
-            if (col >= n4 || !on) continue;
-            __align__(8) __half h[4], l[4];
-            fits &= split_h16(v[i].x, h[0], l[0]); fits &= split_h16(v[i].y, h[1], l[1]);
-            fits &= split_h16(v[i].z, h[2], l[2]); fits &= split_h16(v[i].w, h[3], l[3]);
-            __half *ph = FUSED ? s.x(r, 0) : op.o_hi + (size_t)m * K, *pl = FUSED ? s.x(r, 1) : op.o_lo + (size_t)m * K;
-            *reinterpret_cast<uint2 *>(ph + 4 * col) = *reinterpret_cast<const uint2 *>(h);
-            *reinterpret_cast<uint2 *>(pl + 4 * col) = *reinterpret_cast<const uint2 *>(l);
+            const int at = c.lane + 32 * (sub + 8 / NC * i);
+            v[i] = at < n4 ? __ldcg(reinterpret_cast<const float4 *>(x) + at) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        // (the exchange buffers of the next rows: its first barrier comes after everybody's reads of this round)
+        if (AED && pe) {
+#pragma unroll
+            for (int i = 0; i < NC; i++) {
+                const int at = c.lane + 32 * (sub + 8 / NC * i);
+                if (at >= n4) continue;
+                const float4 y = __ldg(reinterpret_cast<const float4 *>(pe) + at);
+                v[i] = make_float4(v[i].x + y.x, v[i].y + y.y, v[i].z + y.z, v[i].w + y.w);
+            }
+        }
+    }
+    fr_cp_wait();
+    fr_sync();                                                   // the vectors are everybody's
+    if (!on) { for (int i = 0; i < NC; i++) v[i] = make_float4(0.f, 0.f, 0.f, 0.f); }
+    if (op.rows == FR_ROWS_LN2 || (AED && op.rows == FR_ROWS_AED_NEXT)) {
+        fr_ln(v, vec + 2 * (FR_SLAB / 4), vec + 3 * (FR_SLAB / 4), n4, a.inv_d, r, sub, c.lane);
+        if (NC < 8) fr_sync();                                   // the sums have been read
+        if (c.ng == 0 && on) {
+#pragma unroll
+            for (int i = 0; i < NC; i++)
+                if (c.lane + 32 * (sub + 8 / NC * i) < n4) reinterpret_cast<float4 *>(op.x_copy + (size_t)m * K)[c.lane + 32 * (sub + 8 / NC * i)] = v[i];
+        }
+    }
+    fr_ln(v, vec, vec + FR_SLAB / 4, n4, a.inv_d, r, sub, c.lane);
+    if (!on) return;
+    bool fits = true;
+#pragma unroll
+    for (int i = 0; i < NC; i++) {
+        const int at = c.lane + 32 * (sub + 8 / NC * i);
+        if (at >= n4) continue;
+        if (!AED && op.rows == FR_ROWS_LN_SILU) v[i] = make_float4(silu_f(v[i].x), silu_f(v[i].y), silu_f(v[i].z), silu_f(v[i].w));
+        __align__(8) __half h[4], l[4];
+        fits &= split_h16(v[i].x, h[0], l[0]); fits &= split_h16(v[i].y, h[1], l[1]);
+        fits &= split_h16(v[i].z, h[2], l[2]); fits &= split_h16(v[i].w, h[3], l[3]);
+        *reinterpret_cast<uint2 *>(FrShared::x(r, 0) + 4 * at) = *reinterpret_cast<const uint2 *>(h);
+        *reinterpret_cast<uint2 *>(FrShared::x(r, 1) + 4 * at) = *reinterpret_cast<const uint2 *>(l);
     }
     if (!fits) atomicCAS(a.status, ST_OK, ST_RANGE);
 }
 
 // --------------------------------------------------------------------------------------------------- contraction
-// slab `sl` of the tile's planes to rows `at` on (asynchronous)
-__device__ __forceinline__ void fr_stage_planes(const FrOp &op, const FrShared &s, const FrPlace &c, int sl, int ks, int at, bool lo) {
-    const int per = ks >> 3, n = c.rows * per;
-    for (int i = c.tid; i < n; i += FR_THREADS) {
-        const int r = i / per, col = (i - r * per) * 8;
-        const size_t o = (size_t)(c.row0 + r) * op.K + (size_t)sl * FR_SLAB + col;
-        fr_cp16(smem_u32(s.x(at + r, 0) + col), op.a_hi + o);
-        if (lo) fr_cp16(smem_u32(s.x(at + r, 1) + col), op.a_lo + o);
+// slabs `sl`, .. `sl + n - 1` of the tile's planes to rows `at` on, one behind the other (asynchronous). A warp takes a row.
+__device__ __forceinline__ void fr_stage_planes(const FrOp &op, const FrPlace &c, int sl, int n, int ks, int at, int planes) {
+    for (int i = c.warp; i < n * c.rows * planes; i += FR_WARPS) {
+        const int j = planes == 2 ? i >> 1 : i, k = n == 1 ? 0 : j / c.rows, r = j - k * c.rows;
+        const __half *src = (planes == 2 && (i & 1) ? op.a_lo : op.a_hi) + (size_t)(c.row0 + r) * op.K + (size_t)(sl + k) * FR_SLAB;
+        const uint32_t dst = smem_u32(FrShared::x(at + j, planes == 2 ? i & 1 : 0));
+#pragma unroll
+        for (int col = c.lane * 8; col < FR_SLAB; col += 256) if (col < ks) fr_cp16(dst + col * 2, src + col);
     }
     fr_cp_commit();
 }
 
-// the finished sum of (row, column) of unit u of the group: the warps' parts in warp order
-__device__ __forceinline__ float fr_sum(const FrShared &s, int u, int row, int col) {
-    const int at = (((row & 7) * 4 + (col >> 1)) << 2) + ((row >> 3) << 1) + (col & 1);
+// A thread's output of a group of units: unit slot, row of the tile, column of the unit (columns side by side).
+struct FrOut {
+    int u, row, col, n;                   // n: column of the contraction
+    bool on;
+    float bias, res;                      // asked for under the products
+};
+template <int NB>
+__device__ __forceinline__ FrOut fr_out(const FrArgs &a, const FrOp &op, const FrPlace &c, int first, int nu, bool glu) {
+    FrOut o;
+    o.u = c.tid / (64 * NB); o.row = (c.tid >> 3) & (8 * NB - 1); o.col = c.tid & 7;
+    const int unit = c.ng + (first + o.u) * a.ngroups;
+    o.n = !glu ? unit * 8 + o.col : o.col < 4 ? unit * 4 + o.col : op.N / 2 + unit * 4 + o.col - 4;
+    o.on = o.u < nu && o.row < c.rows && o.n < op.N;
+    o.bias = o.on && op.bias ? __ldg(op.bias + o.n) : 0.f;
+    o.res = o.on && op.epi == FR_EPI_RESID ? __ldcg(op.res + (size_t)(c.row0 + o.row) * op.ldo + o.n) : 0.f;
+    return o;
+}
+// A warp's sums: per two units and eight rows a block of FR_CT floats, in it (column g of both units, rows 2 t and 2 t + 1) at
+// 20 g + 4 t: [unit][row]. Steps of 20 keep the columns of a row in different banks.
+__device__ __forceinline__ float *fr_red(int warp, int block) { return FrShared::red() + (warp * 4 + block) * FR_CT; }
+
+// np: warps that have a part of the sums; they are added in warp order
+template <bool AED, int NB>
+__device__ __forceinline__ void fr_epilogue(const FrArgs &a, const FrOp &op, const FrPlace &c, int first, int nu, int mine, int np, const FrOut &o) {
     float v = 0.f;
+    if (o.on) {
+        const float *red = fr_red(0, (o.u >> 1) * NB + (o.row >> 3)) + 20 * o.col + ((o.row & 7) >> 1) * 4 + (o.u & 1) * 2 + (o.row & 1);
+        if (np == FR_WARPS) {
 #pragma unroll
-    for (int w = 0; w < FR_WARPS; w++) v += s.red[(w * FR_GU + u) * 128 + at];
-    return v;
-}
-
-// bias and residual of the (up to two) outputs a thread will store, asked for under the products
-struct FrPre { float b[2], r[2]; };
-__device__ __forceinline__ void fr_prefetch(const FrArgs &a, const FrOp &op, const FrPlace &c, int first, int nu, FrPre &pre) {
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-        const int i = c.tid + q * FR_THREADS, u = i >> 7, row = (i >> 3) & 15, n = (c.ng + (first + u) * a.ngroups) * 8 + (i & 7);
-        const bool on = u < nu && row < c.rows && n < op.N && op.epi <= FR_EPI_F32;
-        pre.b[q] = on && op.bias ? __ldg(op.bias + n) : 0.f;
-        pre.r[q] = on && op.epi == FR_EPI_RESID ? __ldcg(op.res + (size_t)(c.row0 + row) * op.ldo + n) : 0.f;
-    }
-}
-
-template <bool AED>
-__device__ __forceinline__ void fr_epilogue(const FrArgs &a, const FrOp &op, const FrShared &s, const FrPlace &c, int first, int nu, int mine, const FrPre &pre) {
-    bool fits = true;                                            // unit of slot u: ng + (first + u) ngroups
-    if (op.epi >= FR_EPI_GLU_CONV) {
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            const int i = c.tid + q * FR_THREADS, u = i >> 7, row = (i >> 3) & 15, col = i & 7, unit = c.ng + (first + u) * a.ngroups;
-            if (u >= nu) continue;
-            float v = fr_sum(s, u, row, col);
-            const int n = AED ? unit * 8 + col : (col < 4 ? unit * 4 + col : op.N / 2 + unit * 4 + col - 4);
-            if (op.bias && n < op.N) v += op.bias[n];
-            s.vals[i] = v;
+            for (int w = 0; w < FR_WARPS; w++) v += red[w * 4 * FR_CT];
+        } else {
+            for (int w = 0; w < np; w++) v += red[w * 4 * FR_CT];
         }
+        v += o.bias;
+    }
+    if (op.epi >= FR_EPI_GLU_CONV) {
+        FrShared::vals()[c.tid] = v;                             // [unit][row][column]
         fr_sync();
         if (AED) {
-            const int row = c.tid >> 4, j = c.tid & 15;             // sixteen threads per row
+            const int row = c.warp;                              // a warp per row
+            if (row >= 8 * NB) return;
             float bv = -3.0e38f;
             int bi = 0x7fffffff;
-            for (int i = j; i < nu * 8; i += 16) {
+            for (int i = c.lane; i < nu * 8; i += 32) {
                 const int n = (c.ng + (first + (i >> 3)) * a.ngroups) * 8 + (i & 7);
-                const float v = s.vals[(i >> 3) * 128 + row * 8 + (i & 7)];
-                if (n < op.N && (v > bv || (v == bv && n < bi))) { bv = v; bi = n; }
+                const float x = FrShared::vals()[((i >> 3) * 8 * NB + row) * 8 + (i & 7)];
+                if (n < op.N && (x > bv || (x == bv && n < bi))) { bv = x; bi = n; }
             }
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) {
-                const float v = __shfl_xor_sync(0xffffffffu, bv, o);
-                const int k = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (v > bv || (v == bv && k < bi)) { bv = v; bi = k; }
+            for (int q = 16; q > 0; q >>= 1) {
+                const float x = __shfl_xor_sync(0xffffffffu, bv, q);
+                const int k = __shfl_xor_sync(0xffffffffu, bi, q);
+                if (x > bv || (x == bv && k < bi)) { bv = x; bi = k; }
             }
-            if (j == 0) {
-                if (first == 0 || bv > s.best_v[row] || (bv == s.best_v[row] && bi < s.best_i[row])) { s.best_v[row] = bv; s.best_i[row] = bi; }
+            if (c.lane == 0) {
+                if (first == 0 || bv > FrShared::best_v()[row] || (bv == FrShared::best_v()[row] && bi < FrShared::best_i()[row])) { FrShared::best_v()[row] = bv; FrShared::best_i()[row] = bi; }
                 if (first + nu >= mine && row < c.rows) {
-                    a.cand_v[(size_t)(c.row0 + row) * a.ngroups + c.ng] = s.best_v[row];
-                    a.cand_i[(size_t)(c.row0 + row) * a.ngroups + c.ng] = s.best_i[row];
+                    a.cand_v[(size_t)(c.row0 + row) * a.ngroups + c.ng] = FrShared::best_v()[row];
+                    a.cand_i[(size_t)(c.row0 + row) * a.ngroups + c.ng] = FrShared::best_i()[row];
                 }
             }
             return;
@@ -398,7 +435,7 @@ __device__ __forceinline__ void fr_epilogue(const FrArgs &a, const FrOp &op, con
         for (int i = c.tid; i < nu * ns * 4; i += FR_THREADS) {
             const int j = i & 3, sl = (i >> 2) % ns, u = (i >> 2) / ns, ch = (c.ng + (first + u) * a.ngroups) * 4 + j, stream = c.row0 / Q + sl;
             float *cc = op.conv_cache + (size_t)stream * (k - 1) * d + ch;
-            const float *val = s.vals + u * 128 + sl * Q * 8 + j, *w = op.dw_w + (size_t)ch * k;
+            const float *val = FrShared::vals() + (u * NB * 8 + sl * Q) * 8 + j, *w = op.dw_w + (size_t)ch * k;
             auto glu = [&](int t) { return val[t * 8] * sigmoid_fast(val[t * 8 + 4]); };
             if (k == FR_CONV_K) {                                // the usual width: taps and cached rows in registers
                 float wk[FR_CONV_K], row[FR_CONV_K];
@@ -427,207 +464,201 @@ __device__ __forceinline__ void fr_epilogue(const FrArgs &a, const FrOp &op, con
         }
         return;
     }
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-        const int i = c.tid + q * FR_THREADS, u = i >> 7, row = (i >> 3) & 15, col = i & 7, n = (c.ng + (first + u) * a.ngroups) * 8 + col, m = c.row0 + row;
-        if (u >= nu || row >= c.rows || n >= op.N) continue;
-        float v = fr_sum(s, u, row, col) + pre.b[q];
-        if (op.act == ACT_SILU) v = v * __frcp_rn(1.0f + __expf(-v));
-        else if (op.act == ACT_RELU) v = fmaxf(v, 0.0f);
-        if (op.epi == FR_EPI_PLANES) {
-            __half h, l;
-            fits &= split_h16(v, h, l);
-            op.o_hi[(size_t)m * op.N + n] = h;
-            op.o_lo[(size_t)m * op.N + n] = l;
-        } else if (op.epi == FR_EPI_RESID) {
-            op.out[(size_t)m * op.ldo + n] = pre.r[q] + op.alpha * v;
-        } else if (op.epi == FR_EPI_QKV && n >= op.n_split) {
-            const int e = n - op.n_split, half_n = (op.N - op.n_split) / 2;
-            __half h, l;
-            fits &= split_h16(v, h, l);
-            (e < half_n ? op.o_hi : op.o_lo)[(size_t)m * half_n + (e < half_n ? e : e - half_n)] = h;
-        } else {
-            op.out[(size_t)m * op.ldo + n] = v;
-        }
+    if (!o.on) return;
+    const int m = c.row0 + o.row;
+    bool fits = true;
+    if (op.act == ACT_SILU) v = v * __frcp_rn(1.0f + __expf(-v));
+    else if (op.act == ACT_RELU) v = fmaxf(v, 0.0f);
+    if (op.epi == FR_EPI_PLANES) {
+        __half h, l;
+        fits = split_h16(v, h, l);
+        op.o_hi[(size_t)m * op.N + o.n] = h;
+        op.o_lo[(size_t)m * op.N + o.n] = l;
+    } else if (op.epi == FR_EPI_RESID) {
+        op.out[(size_t)m * op.ldo + o.n] = o.res + op.alpha * v;
+    } else if (op.epi == FR_EPI_QKV && o.n >= op.n_split) {
+        const int e = o.n - op.n_split, half_n = (op.N - op.n_split) / 2;
+        __half h, l;
+        fits = split_h16(v, h, l);
+        (e < half_n ? op.o_hi : op.o_lo)[(size_t)m * half_n + (e < half_n ? e : e - half_n)] = h;
+    } else {
+        op.out[(size_t)m * op.ldo + o.n] = v;
     }
     if (!fits) atomicCAS(a.status, ST_OK, ST_RANGE);
 }
 
-// The products of one piece (unit, slab): acc += this warp's 64-wide parts of K. FULL: a slab of 1024, two parts per warp; else
-// parts beyond np do not exist.
-template <int TERMS>
-__device__ __forceinline__ void fr_pair(const uint8_t *pair, const FrPlace &c, const uint4 (&xh)[2][2], const uint4 (&xl)[2][2], float (&acc)[4]) {
-    const uint4 wq = *reinterpret_cast<const uint4 *>(pair + c.lane * 16);
-    const uint2 sc = *reinterpret_cast<const uint2 *>(pair + 512 + (c.lane & 3) * 8);
-    float ch[2][4], cl[2][4];
-    uint32_t w[2][4];
+// A warp's 64-wide parts of two units (BOTH; else one) and NB times eight rows: acc += ... The weights are the 16-row operand of
+// m16n8k16 (unit 0 above unit 1), X the 8-column one, so that up to eight rows cost half of what sixteen do.
+template <int TERMS, int NB, bool BOTH>
+__device__ __forceinline__ void fr_pair(const uint8_t *p0, const uint8_t *p1, int lane, const uint4 (&xh)[2][NB], const uint4 (&xl)[2][NB], float (&acc)[NB][4]) {
+    const uint4 q0 = *reinterpret_cast<const uint4 *>(p0 + lane * 16), q1 = BOTH ? *reinterpret_cast<const uint4 *>(p1 + lane * 16) : make_uint4(0, 0, 0, 0);
+    const __half *s0 = reinterpret_cast<const __half *>(p0 + 512) + (lane >> 3) * 4 + ((lane >> 2) & 1), *s1 = reinterpret_cast<const __half *>(p1 + 512) + (lane >> 3) * 4 + ((lane >> 2) & 1);
 #pragma unroll
     for (int b = 0; b < 2; b++) {
-        fr_widen(b ? wq.z : wq.x, w[b][0], w[b][1]);
-        fr_widen(b ? wq.w : wq.y, w[b][2], w[b][3]);
+        uint32_t w[4], v[4] = {0, 0, 0, 0};
+        fr_widen(b ? q0.z : q0.x, w[0], w[1]);
+        fr_widen(b ? q0.w : q0.y, w[2], w[3]);
+        if (BOTH) { fr_widen(b ? q1.z : q1.x, v[0], v[1]); fr_widen(b ? q1.w : q1.y, v[2], v[3]); }
+        float ch[NB][4], cl[NB][4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) ch[b][i] = cl[b][i] = 0.f;
-    }
+        for (int n = 0; n < NB; n++) {
 #pragma unroll
-    for (int b = 0; b < 2; b++) {
-        fr_mma(ch[b], xh[b][0].x, xh[b][1].x, xh[b][0].y, xh[b][1].y, w[b][0], w[b][1]);
-        if (TERMS > 1) fr_mma(cl[b], xl[b][0].x, xl[b][1].x, xl[b][0].y, xl[b][1].y, w[b][0], w[b][1]);
-    }
+            for (int i = 0; i < 4; i++) ch[n][i] = cl[n][i] = 0.f;
+            fr_mma(ch[n], w[0], v[0], w[1], v[1], xh[b][n].x, xh[b][n].y);
+            if (TERMS > 1) fr_mma(cl[n], w[0], v[0], w[1], v[1], xl[b][n].x, xl[b][n].y);
+        }
 #pragma unroll
-    for (int b = 0; b < 2; b++) {
-        fr_mma(ch[b], xh[b][0].z, xh[b][1].z, xh[b][0].w, xh[b][1].w, w[b][2], w[b][3]);
-        if (TERMS > 1) fr_mma(cl[b], xl[b][0].z, xl[b][1].z, xl[b][0].w, xl[b][1].w, w[b][2], w[b][3]);
-    }
+        for (int n = 0; n < NB; n++) {
+            fr_mma(ch[n], w[2], v[2], w[3], v[3], xh[b][n].z, xh[b][n].w);
+            if (TERMS > 1) fr_mma(cl[n], w[2], v[2], w[3], v[3], xl[b][n].z, xl[b][n].w);
+        }
+        const float d0 = __half2float(s0[b * 2]), d1 = BOTH ? __half2float(s1[b * 2]) : 0.f;
 #pragma unroll
-    for (int b = 0; b < 2; b++) {
-        const float2 d = __half22float2(*reinterpret_cast<const __half2 *>(b ? &sc.y : &sc.x));
+        for (int n = 0; n < NB; n++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) acc[i] = fmaf((i & 1) ? d.y : d.x, TERMS > 1 ? fmaf(cl[b][i], H16_LO_INV, ch[b][i]) : ch[b][i], acc[i]);
+            for (int i = 0; i < (BOTH ? 4 : 2); i++) acc[n][i] = fmaf(i < 2 ? d0 : d1, TERMS > 1 ? fmaf(cl[n][i], H16_LO_INV, ch[n][i]) : ch[n][i], acc[n][i]);
     }
 }
 
-// One slab of a group of nu units: the rows' fragments stay in registers for all of them.
-template <int TERMS, bool FULL>
-__device__ __forceinline__ bool fr_slab(const FrArgs &a, const FrShared &s, const FrPlace &c, int xrow, int np, int nu, unsigned &it, bool ok, float (&acc)[FR_GU][4]) {
+// One slab of a group of nu units, two at a time: the rows' fragments stay in registers for all of them; the sums of units wait
+// in shared memory for their next slab. The loop is not unrolled: sixteen warps hide the latencies, and what bounds it is the
+// instructions issued.
+template <int TERMS, int NB>
+__device__ __forceinline__ void fr_slab(const FrPlace &c, FrFeed &f, int xrow, int nu, bool more) {
     const int g = c.lane >> 2, t = c.lane & 3;
-    uint4 xh[2][2][2], xl[2][2][2];                              // [part][block][row g / g + 8]
-    // a row that the tile does not have is the first one again; its sums are never stored
-    const int r0 = xrow + (g < c.rows ? g : 0), r1 = xrow + (g + 8 < c.rows ? g + 8 : 0);
+    uint4 xh[2][NB], xl[2][NB];                                  // [block][rows g, g + 8]
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
-        const int pr = c.warp + q * FR_WARPS;
-        if (!FULL && pr >= np) continue;
+    for (int n = 0; n < NB; n++) {
+        const int r = xrow + (g + 8 * n < c.rows ? g + 8 * n : 0);       // a row that the tile does not have is the first one again; its sums are never stored
 #pragma unroll
         for (int b = 0; b < 2; b++) {
-            const int at = pr * 64 + b * 32 + 8 * t;
-            xh[q][b][0] = *reinterpret_cast<const uint4 *>(s.x(r0, 0) + at);
-            xh[q][b][1] = *reinterpret_cast<const uint4 *>(s.x(r1, 0) + at);
-            if (TERMS > 1) {
-                xl[q][b][0] = *reinterpret_cast<const uint4 *>(s.x(r0, 1) + at);
-                xl[q][b][1] = *reinterpret_cast<const uint4 *>(s.x(r1, 1) + at);
-            }
+            const int at = c.warp * 64 + b * 32 + 8 * t;
+            xh[b][n] = *reinterpret_cast<const uint4 *>(FrShared::x(r, 0) + at);
+            if (TERMS > 1) xl[b][n] = *reinterpret_cast<const uint4 *>(FrShared::x(r, 1) + at);
         }
     }
+    float *sums = fr_red(c.warp, 0) + 20 * g + 4 * t;
+#pragma unroll 1
+    for (int u = 0; u < nu; u += 2, sums += NB * FR_CT) {
+        float acc[NB][4];
 #pragma unroll
-    for (int u = 0; u < FR_GU; u++) {
-        if (u >= nu) break;
-        const unsigned stg = it % FR_STAGES;
-        if (ok && !__all_sync(0xffffffffu, mbar_wait(&s.full[stg], (it / FR_STAGES) & 1))) {
-            ok = false;
-            if (c.lane == 0) { *s.stop = 1; atomicExch(a.bar + 1, 1u); atomicCAS(a.status, ST_OK, ST_TIMEOUT_MMA); }
+        for (int n = 0; n < NB; n++) {
+            acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+            if (more) { const float4 v = *reinterpret_cast<const float4 *>(sums + n * FR_CT); acc[n][0] = v.x; acc[n][1] = v.y; acc[n][2] = v.z; acc[n][3] = v.w; }
         }
-        it++;
-        if (!ok) continue;
-        const uint8_t *piece = s.ring + stg * FR_PIECE + c.warp * FR_PAIR_BYTES;
-#pragma unroll
-        for (int q = 0; q < 2; q++)
-            if (FULL || c.warp + q * FR_WARPS < np) fr_pair<TERMS>(piece + q * FR_WARPS * FR_PAIR_BYTES, c, xh[q], xl[q], acc[u]);
+        fr_cp_wait_but<FR_AHEAD - 2>();
         __syncwarp();
-        if (c.lane == 0) mbar_arrive(&s.empty[stg]);
+        const uint8_t *p0 = FrShared::ring(c.warp, f.slot), *p1 = FrShared::ring(c.warp, f.slot + 1 == FR_AHEAD ? 0 : f.slot + 1);
+        const bool both = u + 1 < nu;
+        if (both) fr_pair<TERMS, NB, true>(p0, p1, c.lane, xh, xl, acc);
+        else fr_pair<TERMS, NB, false>(p0, p0, c.lane, xh, xl, acc);
+#pragma unroll
+        for (int n = 0; n < NB; n++) *reinterpret_cast<float4 *>(sums + n * FR_CT) = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
+        __syncwarp();                                            // all lanes have read the pieces
+        fr_ask<NB>(f, c);
+        if (both) fr_ask<NB>(f, c);
     }
-    return ok;
 }
 
-// One contraction over this CTA's rows and units. it: ring pieces consumed so far. A wait that runs out sets the stop flag;
-// the warp then goes through the rest without waiting or computing, and the grid barrier behind the operation ends it all.
-template <bool AED, int TERMS>
-__device__ __forceinline__ void fr_gemm(const FrArgs &a, const FrOp &op, const FrShared &s, const FrPlace &c, int p, unsigned &it) {
+// What the attention behind this contraction will read of the caches and the position keys, on its way to the L2 meanwhile.
+__device__ __forceinline__ void fr_stream_prefetch(const FrArgs &a, const FrOp &op, const FrPlace &c) {
+    const int tasks = c.rows / a.Q * a.H, K = a.valid + a.Q;
+    for (int task = c.ng + c.warp * a.ngroups; task < tasks; task += FR_WARPS * a.ngroups) {
+        const size_t base = ((size_t)(c.row0 / a.Q) * a.H + task) * a.left * a.dk;
+        const int h = task % a.H, bytes = a.left * a.dk * 2;
+        for (int i = c.lane * 128; i < bytes; i += 32 * 128) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(op.kc + base) + i));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(op.vc + base) + i));
+        }
+        if (c.row0 == 0 && task < a.H)                           // once for all streams
+            for (int j = c.lane; j < K; j += 32) {
+                const uint8_t *p = reinterpret_cast<const uint8_t *>(op.rk + (size_t)j * op.ldrk + h * a.dk);
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p + a.dk * 2 - 2));
+            }
+    }
+}
+
+// One contraction over this CTA's rows and units.
+template <bool AED, int TERMS, int NB>
+__device__ __forceinline__ void fr_gemm(const FrArgs &a, const FrOp &op, const FrPlace &c, int p, FrFeed &f) {
     const int units = (op.N + 7) >> 3, mine = units > c.ng ? (units - c.ng + a.ngroups - 1) / a.ngroups : 0;
-    const int ks = op.K < FR_SLAB ? op.K : FR_SLAB, slabs = op.K <= FR_SLAB ? 1 : op.K / FR_SLAB, np = ks >> 6;
+    const int ks = op.K < FR_SLAB ? op.K : FR_SLAB, slabs = op.K <= FR_SLAB ? 1 : op.K / FR_SLAB, np = ks >> 6, planes = TERMS > 1 ? 2 : 1;
     if (AED && op.epi == FR_EPI_ARGMAX && mine == 0 && c.tid < c.rows) {
         a.cand_v[(size_t)(c.row0 + c.tid) * a.ngroups + c.ng] = -3.0e38f;
         a.cand_i[(size_t)(c.row0 + c.tid) * a.ngroups + c.ng] = 0x7fffffff;
     }
-    const bool planes = op.rows == FR_ROWS_PLANES, all = c.rows * slabs <= 32;
-    if (!planes) {
-        // group 0 leaves LN2's rows behind and keeps the AED books even where no unit is its own
-        if (mine > 0 || c.ng == 0) {
-            if (c.rows == 1) fr_rows<1, true, AED>(a, op, s, c, c.row0, c.rows, c.ng == 0, p);
-            else if (c.rows == 2) fr_rows<2, true, AED>(a, op, s, c, c.row0, c.rows, c.ng == 0, p);
-            else fr_rows<4, true, AED>(a, op, s, c, c.row0, c.rows, c.ng == 0, p);
-        }
-        fr_sync();
+    // few rows: all slabs are asked for at once, and once; else two slabs in turn, again for every group of units
+    const bool from_planes = op.rows == FR_ROWS_PLANES, all = !from_planes || c.rows * slabs <= 32;
+    if (mine == 0 && (from_planes || c.ng != 0)) return;         // (group 0 keeps rows and books even where no unit is its own)
+    if (!from_planes) {                                          // (8 / NC warps to a row)
+        if (NB > 1) fr_rows<AED, 8>(a, op, c, p);
+        else if (c.rows <= 2) fr_rows<AED, 1>(a, op, c, p);
+        else if (c.rows <= 4) fr_rows<AED, 2>(a, op, c, p);
+        else fr_rows<AED, 4>(a, op, c, p);
     }
-    if (mine == 0) return;
-    bool ok = true;
-    for (int first = 0; first < mine; first += FR_GU) {
-        const int nu = mine - first < FR_GU ? mine - first : FR_GU;
-        float acc[FR_GU][4];
-#pragma unroll
-        for (int u = 0; u < FR_GU; u++) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.f;
-        // few rows: all slabs are asked for at once, and once; else two slabs in turn, again for every group of units
-        if (planes && first == 0 && all) {
-            for (int sl = 0; sl < slabs; sl++) fr_stage_planes(op, s, c, sl, ks, sl * c.rows, TERMS > 1);
-        } else if (planes && !all) {
+    if (from_planes && all) fr_stage_planes(op, c, 0, slabs, ks, 0, planes);
+    if (!AED && op.epi == FR_EPI_QKV) fr_stream_prefetch(a, op, c);
+    constexpr int GU = fr_gu(NB);
+    for (int first = 0; first < mine; first += GU) {
+        const int nu = mine - first < GU ? mine - first : GU;
+        if (!all) {
             if (first) fr_sync();
-            fr_stage_planes(op, s, c, 0, ks, 0, TERMS > 1);
+            fr_stage_planes(op, c, 0, 1, ks, 0, planes);
         }
-        FrPre pre;
-        fr_prefetch(a, op, c, first, nu, pre);
+        const FrOut o = fr_out<NB>(a, op, c, first, nu, !AED && op.epi == FR_EPI_GLU_CONV);
+        if (all && first == 0) { fr_cp_wait(); fr_sync(); }
         for (int sl = 0; sl < slabs; sl++) {
-            if (planes && (!all || (first == 0 && sl == 0))) {
-                fr_cp_wait();
+            if (!all) {
+                // (a slab's rows were asked for before the pieces of the slab before it were used: nu groups ago)
+                if (sl == 0) fr_cp_wait();
+                else if (nu == GU) fr_cp_wait_but<GU>();
+                else fr_cp_wait_but<1>();
                 fr_sync();
-                if (!all && sl + 1 < slabs) fr_stage_planes(op, s, c, sl + 1, ks, ((sl + 1) & 1) * 16, TERMS > 1);
+                if (sl + 1 < slabs) fr_stage_planes(op, c, sl + 1, 1, ks, ((sl + 1) & 1) * 16, planes);
             }
-            const int xrow = !planes ? 0 : all ? sl * c.rows : (sl & 1) * 16;
-            if (np == FR_PAIRS) ok = fr_slab<TERMS, true>(a, s, c, xrow, np, nu, it, ok, acc);
-            else ok = fr_slab<TERMS, false>(a, s, c, xrow, np, nu, it, ok, acc);
+            if (c.warp < np) fr_slab<TERMS, NB>(c, f, from_planes ? (all ? sl * c.rows : (sl & 1) * 16) : 0, nu, sl > 0);
         }
-#pragma unroll
-        for (int u = 0; u < FR_GU; u++)
-            if (u < nu) *reinterpret_cast<float4 *>(s.red + (c.warp * FR_GU + u) * 128 + c.lane * 4) = make_float4(acc[u][0], acc[u][1], acc[u][2], acc[u][3]);
         fr_sync();
-        fr_epilogue<AED>(a, op, s, c, first, nu, mine, pre);
-        if (first + FR_GU < mine) fr_sync();                     // the sums are read before the next group writes its own
+        fr_epilogue<AED, NB>(a, op, c, first, nu, mine, np, o);
+        if (first + GU < mine) fr_sync();                     // the sums are read before the next group writes its own
     }
-}
-
-// The producer warp asks for every piece of every contraction in the order the warps use them: groups of FR_GU units, in a
-// group slab by slab, unit by unit.
-__device__ __forceinline__ void fr_produce(const FrArgs &a, const FrShared &s, const FrPlace &c) {
-    unsigned it = 0;
-    bool ok = true;
-    for (int p = 0; p <= a.positions && ok; p++)
-        for (int i = 0; i < a.n_gemms && ok; i++) {
-            const int units = (s.tab[i].N + 7) >> 3, K = s.tab[i].K, ks = K < FR_SLAB ? K : FR_SLAB, slabs = K <= FR_SLAB ? 1 : K / FR_SLAB;
-            const uint32_t bytes = (uint32_t)(ks >> 6) * FR_PAIR_BYTES;
-            const size_t step = (size_t)a.ngroups * slabs * bytes;
-            const uint8_t *w = s.tab[i].w + (size_t)c.ng * slabs * bytes;
-            for (int left = units > c.ng ? (units - c.ng + a.ngroups - 1) / a.ngroups : 0; left > 0 && ok; left -= FR_GU, w += FR_GU * step)
-                for (int sl = 0; sl < slabs && ok; sl++)
-                    for (int u = 0; u < FR_GU && u < left; u++) {
-                        const unsigned stg = it % FR_STAGES;
-                        const long long t0 = clock64();
-                        while (!mbar_try_wait(&s.empty[stg], ((it / FR_STAGES) & 1) ^ 1))
-                            // other CTAs may hold the chain up at a barrier: give up when the computing warps have (their waits are shorter)
-                            if (*s.stop || clock64() - t0 > (1ll << 33)) { ok = false; break; }
-                        if (!ok) break;
-                        mbar_expect_tx(&s.full[stg], bytes);
-                        fr_bulk(smem_u32(s.ring + stg * FR_PIECE), w + u * step + (size_t)sl * bytes, bytes, &s.full[stg]);
-                        it++;
-                    }
-        }
-    // copies still in flight must land before the CTA's shared memory goes away
-    for (unsigned j = it > FR_STAGES ? it - FR_STAGES : 0; j < it; j++) mbar_wait(&s.full[j % FR_STAGES], (j / FR_STAGES) & 1);
 }
 
 // ---------------------------------------------------------------------------------------------------- attentions
-// One query over n keys, in eight lists: list w holds the keys w, w + 8, ... A warp walks a list in rounds of KB keys: all key
-// and value rows of a round are asked for at once (one round covers a list of the usual 71 streaming keys), the scores stay in
-// its lanes, the softmax is a running maximum per list. A lane owns four columns; dk is a multiple of 4 up to 128. The lists
-// meet in fr_context, in list order: the bits are the same whether eight warps take one list each or one warp takes all.
+// One query over n keys, in FR_LISTS lists: list w holds the keys w, w + FR_LISTS, ... A warp walks a list in rounds of KB
+// keys: all key and value rows of a round are asked for at once (one round covers a list of the usual 71 streaming keys), the
+// scores stay in its lanes, the softmax is a running maximum per list. A lane owns four columns; dk is a multiple of 4 up to
+// 128. The lists meet in fr_context in a fixed order: the bits are the same whether sixteen warps take one list each or one
+// warp takes all.
 bool fr_attn_fits(int dk) { return dk % 4 == 0 && dk <= 128; }
+
+struct FrTask {                           // a warp's share of a round of (query group, head) tasks
+    int wpt;                              // warps per task
+    int slot, sub;                        // task of the round, warp in it
+    float *part;                          // [FR_LISTS][128] sums of the task
+    float2 *ml;                           // [FR_LISTS] running maximum and sum of weights
+};
+// as many warps per task as leaves the CTA's tasks one round where they fit into one
+__device__ __forceinline__ FrTask fr_task(const FrArgs &a, const FrPlace &c, int tasks) {
+    FrTask t;
+    const int mine = (tasks + a.ngroups - 1) / a.ngroups;
+    t.wpt = mine <= 1 ? 16 : mine <= 2 ? 8 : mine <= 4 ? 4 : mine <= 8 ? 2 : 1;
+    t.slot = c.warp / t.wpt; t.sub = c.warp - t.slot * t.wpt;
+    t.part = reinterpret_cast<float *>(FrShared::x(0, 0)) + t.slot * FR_LISTS * 128;
+    t.ml = reinterpret_cast<float2 *>(FrShared::red()) + t.slot * FR_LISTS;
+    return t;
+}
 
 // load(j, u) fetches key and value of key j into slot u, score(u) is the lane's part of the dot product, value(u) its columns
 template <int KB, typename FL, typename FS, typename FV>
-__device__ __forceinline__ void fr_list(float *part, float2 *ml, int list, int n, int dk, int lane, FL load, FS score, FV value) {
+__device__ __forceinline__ void fr_list(const FrTask &k, int list, int n, int dk, int lane, FL load, FS score, FV value) {
     const bool on = lane * 4 < dk;
     float m = -INFINITY, l = 0.f;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int j0 = list; j0 < n; j0 += KB * FR_WARPS) {
+    for (int j0 = list; j0 < n; j0 += KB * FR_LISTS) {
 #pragma unroll
-        for (int u = 0; u < KB; u++) load(j0 + FR_WARPS * u < n ? j0 + FR_WARPS * u : j0, u);
+        for (int u = 0; u < KB; u++) load(j0 + FR_LISTS * u < n ? j0 + FR_LISTS * u : j0, u);
         float sc[KB], mx = m;
 #pragma unroll
         for (int u = 0; u < KB; u++) sc[u] = on ? score(u) : 0.f;
@@ -636,7 +667,7 @@ __device__ __forceinline__ void fr_list(float *part, float2 *ml, int list, int n
 #pragma unroll
             for (int u = 0; u < KB; u++) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o2);
 #pragma unroll
-        for (int u = 0; u < KB; u++) { if (j0 + FR_WARPS * u >= n) sc[u] = -INFINITY; mx = fmaxf(mx, sc[u]); }
+        for (int u = 0; u < KB; u++) { if (j0 + FR_LISTS * u >= n) sc[u] = -INFINITY; mx = fmaxf(mx, sc[u]); }
         const float f = expf(m - mx);
         m = mx; l *= f;
         o.x *= f; o.y *= f; o.z *= f; o.w *= f;
@@ -648,23 +679,30 @@ __device__ __forceinline__ void fr_list(float *part, float2 *ml, int list, int n
             o.x = fmaf(w, v.x, o.x); o.y = fmaf(w, v.y, o.y); o.z = fmaf(w, v.z, o.z); o.w = fmaf(w, v.w, o.w);
         }
     }
-    if (on) *reinterpret_cast<float4 *>(part + list * 128 + lane * 4) = o;
-    if (lane == 0) ml[list] = make_float2(m, l);
+    if (on) *reinterpret_cast<float4 *>(k.part + list * 128 + lane * 4) = o;
+    if (lane == 0) k.ml[list] = make_float2(m, l);
 }
-__device__ __forceinline__ void fr_context(const FrOp &op, const float *part, const float2 *ml, size_t out, int i) {
-    float mx = ml[0].x, sum = 0.f, v = 0.f;
+// the task's lists into its context row
+__device__ __forceinline__ void fr_context(const FrOp &op, const FrTask &k, size_t out, int dk, int lane) {
+    const float2 e = k.ml[lane % FR_LISTS];
+    float mx = e.x;
 #pragma unroll
-    for (int w = 1; w < FR_WARPS; w++) mx = fmaxf(mx, ml[w].x);
+    for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float f = expf(e.x - mx);                              // an empty list: exp(-inf) = 0
+    float sum = f * e.y;
 #pragma unroll
-    for (int w = 0; w < FR_WARPS; w++) {
-        const float f = expf(ml[w].x - mx);                      // an empty list: exp(-inf) = 0
-        sum = fmaf(f, ml[w].y, sum);
-        v = fmaf(f, part[w * 128 + i], v);
+    for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    for (int i0 = k.sub * 32; i0 < dk; i0 += 32 * k.wpt) {
+        const int i = i0 + lane;
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < FR_LISTS; w++) v = fmaf(__shfl_sync(0xffffffffu, f, w), k.part[w * 128 + i], v);
+        if (i >= dk) continue;
+        __half hi, lo;
+        split_h16(v / sum, hi, lo);
+        op.o_hi[out + i] = hi;
+        op.o_lo[out + i] = lo;
     }
-    __half hi, lo;
-    split_h16(v / sum, hi, lo);
-    op.o_hi[out + i] = hi;
-    op.o_lo[out + i] = lo;
 }
 __device__ __forceinline__ float4 fr_unpack(uint2 a) {
     const float2 x = __half22float2(*reinterpret_cast<const __half2 *>(&a.x)), y = __half22float2(*reinterpret_cast<const __half2 *>(&a.y));
@@ -675,184 +713,164 @@ __device__ __forceinline__ float fr_dot(float4 a, float4 b) { return fmaf(a.x, b
 
 // score(t, j) = ((q_t + u) . k_j + (q_t + v) . rk[K - 1 - valid - t + j]) / sqrt(dk) over [cached frames ; chunk]; afterwards the
 // chunk's k / v rows go to their ring slots (update_kv_cache, src/encoder.c:763-776): a (stream, head) is read by its own task alone.
-__device__ __forceinline__ void fr_stream_attn(const FrArgs &a, const FrOp &op, const FrShared &s, const FrPlace &c, int start) {
-    constexpr int KB = 9;
-    const int H = a.H, dk = a.dk, d = a.d, Q = a.Q, left = a.left, valid = a.valid, K = valid + Q, tasks = a.S * H;
-    // one task per warp when there are enough of them to fill the chip (no block barriers, loads of eight tasks in flight per
-    // SM), else one per CTA (64 streams x 8 heads: 39 k -> 15 k cycles)
-    const bool warps = tasks >= 3 * (int)gridDim.x;
-    float *part = reinterpret_cast<float *>(s.xs) + (warps ? c.warp * FR_WARPS * 128 : 0);
-    float2 *ml = reinterpret_cast<float2 *>(s.red) + (warps ? c.warp * FR_WARPS : 0);
+__device__ __forceinline__ void fr_stream_attn(const FrArgs &a, const FrOp &op, const FrPlace &c, int start) {
+    constexpr int KB = 5;
+    const int H = a.H, dk = a.dk, d = a.d, Q = a.Q, left = a.left, valid = a.valid, K = valid + Q, tasks = c.rows / Q * H;
+    const FrTask k = fr_task(a, c, tasks);
     const float scale = 1.0f / sqrtf((float)dk);
     const int i0 = c.lane * 4 < dk ? c.lane * 4 : 0;
-    for (int task = warps ? c.warp * gridDim.x + blockIdx.x : blockIdx.x; task < tasks; task += warps ? FR_WARPS * gridDim.x : gridDim.x) {
-        const int st = task / H, h = task - st * H;
+    for (int base = c.ng; base < tasks; base += FR_WARPS / k.wpt * a.ngroups) {
+        const int task = base + k.slot * a.ngroups, st = c.row0 / Q + task / H, h = task % H;
+        const bool on = task < tasks;
         const size_t cbase = ((size_t)st * H + h) * left * dk, nbase = (size_t)st * Q * d + h * dk;
         for (int t = 0; t < Q; t++) {
             const size_t row = (size_t)st * Q + t;
-            const __half *rk = op.rk + (size_t)(K - 1 - valid - t) * op.ldrk + h * dk + i0;
-            const float4 q4 = __ldcg(reinterpret_cast<const float4 *>(op.q + row * op.ldq + h * dk + i0));
-            const float4 bu = __ldg(reinterpret_cast<const float4 *>(op.bias_u + h * dk + i0)), bv = __ldg(reinterpret_cast<const float4 *>(op.bias_v + h * dk + i0));
-            const float4 qu = make_float4(q4.x + bu.x, q4.y + bu.y, q4.z + bu.z, q4.w + bu.w), qv = make_float4(q4.x + bv.x, q4.y + bv.y, q4.z + bv.z, q4.w + bv.w);
-            uint2 kk[KB], rr[KB], vv[KB];
-            auto load = [&](int j, int u) {
-                int x = start + j;
-                if (x >= left) x -= left;
-                const size_t o = j < valid ? cbase + (size_t)x * dk + i0 : nbase + (size_t)(j - valid) * d + i0;
-                kk[u] = fr_ld8((j < valid ? op.kc : op.kn) + o);
-                rr[u] = fr_ld8(rk + (size_t)j * op.ldrk);
-                vv[u] = fr_ld8((j < valid ? op.vc : op.vn) + o);
-            };
-            auto score = [&](int u) { return (fr_dot(qu, fr_unpack(kk[u])) + fr_dot(qv, fr_unpack(rr[u]))) * scale; };
-            auto value = [&](int u) { return fr_unpack(vv[u]); };
-            for (int list = warps ? 0 : c.warp; list < (warps ? FR_WARPS : c.warp + 1); list++) fr_list<KB>(part, ml, list, K, dk, c.lane, load, score, value);
-            if (warps) {
-                __syncwarp();
-                for (int i = c.lane; i < dk; i += 32) fr_context(op, part, ml, row * d + h * dk, i);
-                __syncwarp();
-            } else {
-                fr_sync();
-                if (c.tid < dk) fr_context(op, part, ml, row * d + h * dk, c.tid);
-                fr_sync();
+            if (on) {
+                const __half *rk = op.rk + (size_t)(K - 1 - valid - t) * op.ldrk + h * dk + i0;
+                const float4 q4 = __ldcg(reinterpret_cast<const float4 *>(op.q + row * op.ldq + h * dk + i0));
+                const float4 bu = __ldg(reinterpret_cast<const float4 *>(op.bias_u + h * dk + i0)), bv = __ldg(reinterpret_cast<const float4 *>(op.bias_v + h * dk + i0));
+                const float4 qu = make_float4(q4.x + bu.x, q4.y + bu.y, q4.z + bu.z, q4.w + bu.w), qv = make_float4(q4.x + bv.x, q4.y + bv.y, q4.z + bv.z, q4.w + bv.w);
+                uint2 kk[KB], rr[KB], vv[KB];
+                for (int list = k.sub; list < FR_LISTS; list += k.wpt)
+                    fr_list<KB>(k, list, K, dk, c.lane,
+                                [&](int j, int u) {
+                                    int x = start + j;
+                                    if (x >= left) x -= left;
+                                    const size_t o = j < valid ? cbase + (size_t)x * dk + i0 : nbase + (size_t)(j - valid) * d + i0;
+                                    kk[u] = fr_ld8((j < valid ? op.kc : op.kn) + o);
+                                    rr[u] = fr_ld8(rk + (size_t)j * op.ldrk);
+                                    vv[u] = fr_ld8((j < valid ? op.vc : op.vn) + o);
+                                },
+                                [&](int u) { return (fr_dot(qu, fr_unpack(kk[u])) + fr_dot(qv, fr_unpack(rr[u]))) * scale; },
+                                [&](int u) { return fr_unpack(vv[u]); });
             }
+            fr_sync();
+            if (on) fr_context(op, k, row * d + h * dk, dk, c.lane);
+            if (t + 1 < Q || base + FR_WARPS / k.wpt * a.ngroups < tasks) fr_sync();
         }
-        const int i1 = warps ? c.lane : c.tid, step = warps ? 32 : FR_THREADS;
-        for (int i = i1; i < Q * dk; i += step) {
-            const int t = i / dk, e = i - t * dk;
-            int x = start + valid + t;
-            while (x >= left) x -= left;
-            op.kc[cbase + (size_t)x * dk + e] = __ldcg(op.kn + nbase + (size_t)t * d + e);
-            op.vc[cbase + (size_t)x * dk + e] = __ldcg(op.vn + nbase + (size_t)t * d + e);
-        }
+        if (on)
+            for (int i = k.sub * 32 + c.lane; i < Q * dk; i += 32 * k.wpt) {
+                const int t = i / dk, e = i - t * dk;
+                int x = start + valid + t;
+                while (x >= left) x -= left;
+                op.kc[cbase + (size_t)x * dk + e] = __ldcg(op.kn + nbase + (size_t)t * d + e);
+                op.vc[cbase + (size_t)x * dk + e] = __ldcg(op.vn + nbase + (size_t)t * d + e);
+            }
     }
 }
 
 // One query per utterance over its own past (src/decoder_aed.c:186-197), f32 cache [B][max_len][d].
-__device__ __forceinline__ void fr_aed_self(const FrArgs &a, const FrOp &op, const FrShared &s, const FrPlace &c, int p) {
-    constexpr int KB = 10;
-    const int H = a.H, dk = a.dk, d = a.d;
-    float *part = reinterpret_cast<float *>(s.xs);
-    float2 *ml = reinterpret_cast<float2 *>(s.red);
+__device__ __forceinline__ void fr_aed_self(const FrArgs &a, const FrOp &op, const FrPlace &c, int p) {
+    constexpr int KB = 4;
+    const int H = a.H, dk = a.dk, d = a.d, tasks = c.rows * H;
+    const FrTask k = fr_task(a, c, tasks);
     const float scale = 1.0f / sqrtf((float)dk);
     const int i0 = c.lane * 4 < dk ? c.lane * 4 : 0;
-    for (int task = blockIdx.x; task < a.B * H; task += gridDim.x) {
-        const int b = task / H, h = task - b * H;
+    for (int base = c.ng; base < tasks; base += FR_WARPS / k.wpt * a.ngroups) {
+        const int task = base + k.slot * a.ngroups, b = c.row0 + task / H, h = task % H;
+        const bool on = task < tasks;
         const float *row = op.q + (size_t)b * op.ldq + h * dk;
         float *Kc = op.ck + (size_t)b * a.max_len * d + h * dk, *Vc = op.cv + (size_t)b * a.max_len * d + h * dk;
-        const float4 q4 = __ldcg(reinterpret_cast<const float4 *>(row + i0));
-        float4 kk[KB], vv[KB];
-        fr_list<KB>(part, ml, c.warp, p + 1, dk, c.lane,
-                    [&](int j, int u) {                          // this position's row straight from the projection
-                        kk[u] = __ldcg(reinterpret_cast<const float4 *>(j < p ? Kc + (size_t)j * d + i0 : row + d + i0));
-                        vv[u] = __ldcg(reinterpret_cast<const float4 *>(j < p ? Vc + (size_t)j * d + i0 : row + 2 * d + i0));
-                    },
-                    [&](int u) { return fr_dot(q4, kk[u]) * scale; }, [&](int u) { return vv[u]; });
-        fr_sync();
-        if (c.tid < dk) {
-            Kc[(size_t)p * d + c.tid] = __ldcg(row + d + c.tid);
-            Vc[(size_t)p * d + c.tid] = __ldcg(row + 2 * d + c.tid);
-            fr_context(op, part, ml, (size_t)b * d + h * dk, c.tid);
+        if (on) {
+            const float4 q4 = __ldcg(reinterpret_cast<const float4 *>(row + i0));
+            float4 kk[KB], vv[KB];
+            for (int list = k.sub; list < FR_LISTS; list += k.wpt)
+                fr_list<KB>(k, list, p + 1, dk, c.lane,
+                            [&](int j, int u) {                  // this position's row straight from the projection
+                                kk[u] = __ldcg(reinterpret_cast<const float4 *>(j < p ? Kc + (size_t)j * d + i0 : row + d + i0));
+                                vv[u] = __ldcg(reinterpret_cast<const float4 *>(j < p ? Vc + (size_t)j * d + i0 : row + 2 * d + i0));
+                            },
+                            [&](int u) { return fr_dot(q4, kk[u]) * scale; }, [&](int u) { return vv[u]; });
         }
         fr_sync();
+        if (on) {
+            for (int i = k.sub * 32 + c.lane; i < dk; i += 32 * k.wpt) {
+                Kc[(size_t)p * d + i] = __ldcg(row + d + i);
+                Vc[(size_t)p * d + i] = __ldcg(row + 2 * d + i);
+            }
+            fr_context(op, k, (size_t)b * d + h * dk, dk, c.lane);
+        }
+        if (base + FR_WARPS / k.wpt * a.ngroups < tasks) fr_sync();
     }
 }
 
 // One query per utterance over its projected encoder frames (src/decoder_aed.c:199-202), (hi, lo) planes by (utterance, head).
-__device__ __forceinline__ void fr_aed_cross(const FrArgs &a, const FrOp &op, const FrShared &s, const FrPlace &c) {
-    constexpr int KB = 11;
-    const int H = a.H, dk = a.dk, d = a.d;
-    float *part = reinterpret_cast<float *>(s.xs);
-    float2 *ml = reinterpret_cast<float2 *>(s.red);
+__device__ __forceinline__ void fr_aed_cross(const FrArgs &a, const FrOp &op, const FrPlace &c) {
+    constexpr int KB = 4;
+    const int H = a.H, dk = a.dk, d = a.d, tasks = c.rows * H;
+    const FrTask k = fr_task(a, c, tasks);
     const float scale = 1.0f / sqrtf((float)dk);
     const int i0 = c.lane * 4 < dk ? c.lane * 4 : 0;
-    for (int task = blockIdx.x; task < a.B * H; task += gridDim.x) {
-        const int b = task / H, h = task - b * H, T = a.enc_len[b];
-        const size_t kb = ((size_t)a.enc_off[b] * H + (size_t)h * T) * dk + i0;
-        const __half *khp = op.a_hi + kb, *klp = op.a_lo + kb, *vhp = khp + a.v_off, *vlp = klp + a.v_off;
-        const float4 q4 = __ldcg(reinterpret_cast<const float4 *>(op.q + (size_t)b * op.ldq + h * dk + i0));
-        uint2 kh[KB], kl[KB], vh[KB], vl[KB];
-        auto join = [&](uint2 x, uint2 y) {
-            const float4 h4 = fr_unpack(x), l4 = fr_unpack(y);
-            return make_float4(fmaf(l4.x, H16_LO_INV, h4.x), fmaf(l4.y, H16_LO_INV, h4.y), fmaf(l4.z, H16_LO_INV, h4.z), fmaf(l4.w, H16_LO_INV, h4.w));
-        };
-        fr_list<KB>(part, ml, c.warp, T, dk, c.lane,
-                    [&](int j, int u) {
-                        const int o = j * dk;
-                        kh[u] = __ldg(reinterpret_cast<const uint2 *>(khp + o)); kl[u] = __ldg(reinterpret_cast<const uint2 *>(klp + o));
-                        vh[u] = __ldg(reinterpret_cast<const uint2 *>(vhp + o)); vl[u] = __ldg(reinterpret_cast<const uint2 *>(vlp + o));
-                    },
-                    [&](int u) { return fr_dot(q4, join(kh[u], kl[u])) * scale; }, [&](int u) { return join(vh[u], vl[u]); });
+    for (int base = c.ng; base < tasks; base += FR_WARPS / k.wpt * a.ngroups) {
+        const int task = base + k.slot * a.ngroups, b = c.row0 + task / H, h = task % H;
+        const bool on = task < tasks;
+        if (on) {
+            const int T = a.enc_len[b];
+            const size_t kb = ((size_t)a.enc_off[b] * H + (size_t)h * T) * dk + i0;
+            const __half *khp = op.a_hi + kb, *klp = op.a_lo + kb, *vhp = khp + a.v_off, *vlp = klp + a.v_off;
+            const float4 q4 = __ldcg(reinterpret_cast<const float4 *>(op.q + (size_t)b * op.ldq + h * dk + i0));
+            uint2 kh[KB], kl[KB], vh[KB], vl[KB];
+            auto join = [&](uint2 x, uint2 y) {
+                const float4 h4 = fr_unpack(x), l4 = fr_unpack(y);
+                return make_float4(fmaf(l4.x, H16_LO_INV, h4.x), fmaf(l4.y, H16_LO_INV, h4.y), fmaf(l4.z, H16_LO_INV, h4.z), fmaf(l4.w, H16_LO_INV, h4.w));
+            };
+            for (int list = k.sub; list < FR_LISTS; list += k.wpt)
+                fr_list<KB>(k, list, T, dk, c.lane,
+                            [&](int j, int u) {
+                                const int o = j * dk;
+                                kh[u] = __ldg(reinterpret_cast<const uint2 *>(khp + o)); kl[u] = __ldg(reinterpret_cast<const uint2 *>(klp + o));
+                                vh[u] = __ldg(reinterpret_cast<const uint2 *>(vhp + o)); vl[u] = __ldg(reinterpret_cast<const uint2 *>(vlp + o));
+                            },
+                            [&](int u) { return fr_dot(q4, join(kh[u], kl[u])) * scale; }, [&](int u) { return join(vh[u], vl[u]); });
+        }
         fr_sync();
-        if (c.tid < dk) fr_context(op, part, ml, (size_t)b * d + h * dk, c.tid);
-        fr_sync();
+        if (on) fr_context(op, k, (size_t)b * d + h * dk, dk, c.lane);
+        if (base + FR_WARPS / k.wpt * a.ngroups < tasks) fr_sync();
     }
 }
 
-template <bool AED, int TERMS>
-__global__ void __launch_bounds__(FR_LAUNCH, 1)
+template <bool AED, int TERMS, int NB>
+__global__ void __launch_bounds__(FR_THREADS, 1)
 fr_kernel(const __grid_constant__ FrArgs a) {
-    extern __shared__ __align__(128) uint8_t fr_smem[];
-    __shared__ uint64_t bars[2 * FR_STAGES];
-    __shared__ int stop_flag;
-    __shared__ float best_v[16];
-    __shared__ int best_i[16];
-    __shared__ FrOp ops[2];                                      // this operation and the next one
-    FrShared s;
-    s.ring = fr_smem;
-    s.xs = s.ring + FR_STAGES * FR_PIECE;
-    s.red = reinterpret_cast<float *>(s.xs + 2 * FR_XPLANE);
-    s.vals = s.red + FR_RED_FLOATS;
-    s.tab = reinterpret_cast<const FrWeights *>(s.vals + FR_VALS);
-    s.full = bars; s.empty = bars + FR_STAGES; s.stop = &stop_flag; s.best_v = best_v; s.best_i = best_i;
     FrPlace c;
     c.tid = threadIdx.x; c.warp = threadIdx.x >> 5; c.lane = threadIdx.x & 31;
-    c.ng = blockIdx.x / a.mtiles;
-    c.row0 = (blockIdx.x % a.mtiles) * a.tile_rows;
+    c.ng = blockIdx.x / a.mtiles; c.mt = blockIdx.x % a.mtiles;
+    c.row0 = c.mt * a.tile_rows;
     c.rows = a.M - c.row0 < a.tile_rows ? a.M - c.row0 : a.tile_rows;
-    if (threadIdx.x == 0) {
-        stop_flag = 0;
-        for (int i = 0; i < FR_STAGES; i++) { mbar_init(&s.full[i], 1); mbar_init(&s.empty[i], FR_WARPS); }
-        mbar_fence_init();
-    }
-    for (int i = threadIdx.x; i < a.n_gemms; i += FR_LAUNCH) const_cast<FrWeights *>(s.tab)[i] = static_cast<const FrWeights *>(a.weights)[i];
-    for (int i = threadIdx.x; i < (int)(sizeof(FrOp) / 4); i += FR_LAUNCH) reinterpret_cast<int *>(&ops[0])[i] = reinterpret_cast<const int *>(a.ops)[i];
+    if (threadIdx.x == 0) *FrShared::stop() = 0;
+    for (int i = threadIdx.x; i < (int)(sizeof(FrOp) / 4); i += FR_THREADS) reinterpret_cast<int *>(&FrShared::op(0))[i] = reinterpret_cast<const int *>(a.ops)[i];
     __syncthreads();
-    // registers move from the producer's warpgroup to the two that compute: 256 x 232 + 128 x 24 of the 384 x 168 launched
-    if (c.warp >= FR_WARPS) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
-        if (c.warp == FR_WARPS && c.lane == 0) fr_produce(a, s, c);
-        return;
-    }
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
-    unsigned it = 0, target = 0;
+    FrFeed f;
+    fr_open<NB>(a, FrShared::op(0), c, f);
+    fr_ask_vectors(FrShared::op(0), c.tid, FR_THREADS);
+    fr_cp_commit();
+    unsigned turn = 0;
     const int rounds = AED ? a.positions + 1 : 1, start = AED ? 0 : *a.d_start;
     bool go = true;
     for (int p = 0; p < rounds && go; p++)
         for (int i = 0; i < a.n_ops && go; i++) {
-            const FrOp &op = ops[i & 1];
-            // the turn that opened this position counted the utterances that are done (all CTAs read it behind its barrier)
-            if (AED && i == 1 && *reinterpret_cast<volatile int *>(a.st + 6 * a.B) >= a.B) { go = false; break; }
+            const FrOp &op = FrShared::op(turn), &next = FrShared::op(turn + 1);
+            // the turn that opened this position marked the rows that are done (all CTAs of the tile read it behind the barrier)
+            if (AED && i == 1) {
+                bool done = true;
+                for (int r = 0; r < c.rows; r++) done &= __ldcg(a.st + 2 * a.B + c.row0 + r) != 0;
+                if (done) { go = false; break; }
+            }
             {   // the next operation's description arrives meanwhile
                 const int nx = i + 1 < a.n_ops ? i + 1 : 0;
-                if (c.tid < (int)(sizeof(FrOp) / 16)) fr_cp16(smem_u32(&ops[(i + 1) & 1]) + c.tid * 16, reinterpret_cast<const uint8_t *>(a.ops + nx) + c.tid * 16);
+                if (c.tid < (int)(sizeof(FrOp) / 16)) fr_cp16(smem_u32(&next) + c.tid * 16, reinterpret_cast<const uint8_t *>(a.ops + nx) + c.tid * 16);
                 fr_cp_commit();
             }
-            if (op.type == FR_GEMM) fr_gemm<AED, TERMS>(a, op, s, c, p, it);
-            else if (op.type == FR_LN) {
-                for (int m = blockIdx.x; m < a.M; m += gridDim.x) {
-                    if (m != (int)blockIdx.x) fr_sync();
-                    fr_rows<1, false, AED>(a, op, s, c, m, 1, true, p);
-                }
-            } else if (!AED && op.type == FR_STREAM_ATTN) fr_stream_attn(a, op, s, c, start);
-            else if (AED && op.type == FR_AED_SELF) fr_aed_self(a, op, s, c, p);
-            else if (AED && op.type == FR_AED_CROSS) fr_aed_cross(a, op, s, c);
+            if (op.type == FR_GEMM) fr_gemm<AED, TERMS, NB>(a, op, c, p, f);
+            else if (!AED) fr_stream_attn(a, op, c, start);
+            else if (op.type == FR_AED_SELF) fr_aed_self(a, op, c, p);
+            else fr_aed_cross(a, op, c);
             if (p + 1 == rounds && i + 1 == a.n_ops) break;
-            fr_cp_wait();                                        // (the grid barrier begins with a block barrier)
-            target += gridDim.x;
-            go = fr_grid_sync(a, s, c, target);
+            fr_cp_wait();                                        // (the barrier begins with a block barrier)
+            turn++;
+            go = fr_tile_sync<NB>(a, c, next, f, turn * a.ngroups);
         }
-    fr_sync();
-    if (c.tid == 0) *s.stop = 1;                                 // the producer may be waiting for room that nobody will make
+    fr_cp_wait();
 }
 
 // ------------------------------------------------------------------------------------------------------ host side
@@ -862,40 +880,34 @@ int fr_grid(int M, int tile_rows, int *mtiles, int *ngroups) {
     return *ngroups >= 1 ? 0 : -1;
 }
 
-// The device table of a chain: the operations, then the weights of its contractions in order.
-size_t fr_table_bytes(size_t n_ops) { return n_ops * (sizeof(FrOp) + sizeof(FrWeights)); }
+// The device table of a chain
+size_t fr_table_bytes(size_t n_ops) { return n_ops * sizeof(FrOp); }
 std::vector<uint8_t> fr_table(const std::vector<FrOp> &ops) {
-    std::vector<uint8_t> t(fr_table_bytes(ops.size()), 0);
-    memcpy(t.data(), ops.data(), ops.size() * sizeof(FrOp));
-    FrWeights *w = reinterpret_cast<FrWeights *>(t.data() + ops.size() * sizeof(FrOp));
-    for (const FrOp &o : ops) if (o.type == FR_GEMM) { w->w = o.w; w->N = o.N; w->K = o.K; w++; }
-    return t;
+    const uint8_t *p = reinterpret_cast<const uint8_t *>(ops.data());
+    return std::vector<uint8_t>(p, p + fr_table_bytes(ops.size()));
 }
 
 int fr_launch(FrArgs a, const std::vector<FrOp> &ops, const void *table, cudaStream_t st) {
     a.ops = static_cast<const FrOp *>(table);
-    a.weights = a.ops + ops.size();
     a.n_ops = (int)ops.size();
-    a.n_gemms = 0;
-    for (const FrOp &o : ops) a.n_gemms += o.type == FR_GEMM;
-    if (a.n_gemms > FR_MAX_GEMMS) { set_error("fr_launch: %d contractions in one chain", a.n_gemms); return -1; }
-    if (a.positions > 0 && a.n_ops % 2) { set_error("fr_launch: an odd chain repeats out of step with its description slots"); return -1; }
-    void (*kernel)(FrArgs) = a.positions > 0 ? (a.terms > 1 ? fr_kernel<true, 3> : fr_kernel<true, 1>) : (a.terms > 1 ? fr_kernel<false, 3> : fr_kernel<false, 1>);
+    a.inv_d = 1.0 / a.d;
+    const int pick = (a.positions > 0) * 4 + (a.terms > 1) * 2 + (a.tile_rows > 8 && a.M > 8);    // eight rows or fewer: one half
+    void (*const kernels[8])(FrArgs) = {fr_kernel<false, 1, 1>, fr_kernel<false, 1, 2>, fr_kernel<false, 3, 1>, fr_kernel<false, 3, 2>,
+                                        fr_kernel<true, 1, 1>, fr_kernel<true, 1, 2>, fr_kernel<true, 3, 1>, fr_kernel<true, 3, 2>};
     static PerDevice configured = {};
     int dev = 0;
     if (configured.below((size_t)FR_SMEM, &dev)) {
-        for (void (*k)(FrArgs) : {fr_kernel<true, 3>, fr_kernel<true, 1>, fr_kernel<false, 3>, fr_kernel<false, 1>})
-            MB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, FR_SMEM));
+        for (void (*k)(FrArgs) : kernels) MB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, FR_SMEM));
         configured.record(dev, (size_t)FR_SMEM);
     }
-    MB_CUDA(cudaMemsetAsync(a.bar, 0, 2 * sizeof(unsigned), st));
+    MB_CUDA(cudaMemsetAsync(a.bar, 0, FR_BAR_WORDS * sizeof(unsigned), st));
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(a.mtiles * a.ngroups); lc.blockDim = dim3(FR_LAUNCH); lc.dynamicSmemBytes = FR_SMEM; lc.stream = st;
+    lc.gridDim = dim3(a.mtiles * a.ngroups); lc.blockDim = dim3(FR_THREADS); lc.dynamicSmemBytes = FR_SMEM; lc.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;                   // the barriers need every CTA on an SM
     at[0].val.cooperative = 1;
     lc.attrs = at; lc.numAttrs = 1;
-    MB_CUDA(cudaLaunchKernelEx(&lc, kernel, a));
+    MB_CUDA(cudaLaunchKernelEx(&lc, kernels[pick], a));
     note_launch();
     return 0;
 }

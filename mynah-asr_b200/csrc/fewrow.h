@@ -9,9 +9,9 @@
 
 namespace mb {
 
-enum { FR_GEMM = 0, FR_LN = 1, FR_STREAM_ATTN = 2, FR_AED_SELF = 3, FR_AED_CROSS = 4, FR_NOP = 5 };
-// rows that a FR_LN operation makes, or a contraction stages for itself (`rows` of FrOp)
-enum { FR_ROWS_PLANES = 0,   // contraction: fp16 (hi, lo) planes [M, K] as they are
+enum { FR_GEMM = 0, FR_STREAM_ATTN = 1, FR_AED_SELF = 2, FR_AED_CROSS = 3 };
+// the rows of a contraction (`rows` of FrOp)
+enum { FR_ROWS_PLANES = 0,   // fp16 (hi, lo) planes [M, K] as they are
        FR_ROWS_LN = 1,       // LayerNorm(x; ln), x [M, K] f32
        FR_ROWS_LN2 = 2,      // y = LayerNorm(x; ln0), kept in x_copy; then LayerNorm(y; ln)
        FR_ROWS_LN_SILU = 3,  // SiLU(LayerNorm(x; ln))
@@ -49,15 +49,15 @@ struct alignas(16) FrOp {
 };
 
 struct FrArgs {
-    const FrOp *ops;                      // device; these four are fr_launch's
-    const void *weights;
-    int n_ops, n_gemms;
+    const FrOp *ops;                      // device; these three are fr_launch's
+    int n_ops;
+    double inv_d;
     int M;                                // rows
     int tile_rows;                        // rows of a row tile (at most 16, whole streams)
     int mtiles, ngroups;                  // grid = mtiles x ngroups CTAs
     int terms;                            // 3: hi and lo planes of the activations; 1: hi only
     int d, H, dk;
-    unsigned *bar;                        // grid barrier and abort flag
+    unsigned *bar;                        // [FR_BAR_WORDS]
     int *status;
     // streaming
     int S, Q, left, valid;
@@ -84,7 +84,7 @@ int fr_retile(const QWeight &w, uint8_t *dst, bool glu, cudaStream_t st);
 
 static constexpr int FR_MAX_ROWS = 128;   // rows of an AED batch
 static constexpr int FR_MAX_LAYERS = 48;  // encoder layers a chain has room for
-static constexpr int FR_FUSE_ROWS = 4;    // row tiles of at most this many rows make their LayerNorms where they stage them
+static constexpr int FR_BAR_WORDS = 32 * (1 + FR_MAX_ROWS);   // the abort flag, then a counter per row tile, in a line each
 bool fr_attn_fits(int dk);
 int fr_grid(int M, int tile_rows, int *mtiles, int *ngroups);
 size_t fr_table_bytes(size_t n_ops);

@@ -267,8 +267,8 @@ int Model::stream_open(StreamState &st, int S, int left, int right) {
     st.persistent = st.few_rows && fr_stream && n_layers <= FR_MAX_LAYERS && left > 0 && st.q + 2 <= 16 &&
                     fr_grid(S * (st.q + 2), 16 / (st.q + 2) * (st.q + 2), &mt, &ng) == 0;
     if (st.persistent) {
-        st.fr_table_dev = (uint8_t *)stream_alloc(st, fr_table_bytes((size_t)n_layers * 14));
-        st.fr_bar = (unsigned *)stream_alloc(st, 2 * sizeof(unsigned));
+        st.fr_table_dev = (uint8_t *)stream_alloc(st, fr_table_bytes((size_t)n_layers * 9));
+        st.fr_bar = (unsigned *)stream_alloc(st, FR_BAR_WORDS * sizeof(unsigned));
         if (!st.fr_table_dev || !st.fr_bar) return -1;
     }
     const int C = channels;
@@ -355,24 +355,19 @@ int Model::stream_layers(StreamState &st, float *x, int Q, const __half *rk, int
     memset(&a, 0, sizeof(a));
     a.tile_rows = 16 / Q * Q;
     if (fr_grid(M, a.tile_rows, &a.mtiles, &a.ngroups)) { set_error("stream_step: too many rows for the persistent kernel"); return -1; }
-    const bool fuse = M <= FR_FUSE_ROWS;
-    H16 hA = ws.planes((size_t)M * d), hC = ws.planes((size_t)M * d), hF = ws.planes((size_t)M * F), kvn = ws.planes((size_t)M * d);
+    H16 hC = ws.planes((size_t)M * d), hF = ws.planes((size_t)M * F), kvn = ws.planes((size_t)M * d);
     float *x2 = ws.get<float>((size_t)M * d), *q = ws.get<float>((size_t)M * d), *cbuf = ws.get<float>((size_t)M * d);
-    if (!hA.lo || !hC.lo || !hF.lo || !kvn.lo || !x2 || !q || !cbuf) return -1;
+    if (!hC.lo || !hF.lo || !kvn.lo || !x2 || !q || !cbuf) return -1;
     std::vector<FrOp> ops;
     auto blank = [](int type) { FrOp o; memset(&o, 0, sizeof(o)); o.type = type; o.alpha = 1.f; return o; };
     float *cur = x, *other = x2;
-    // a contraction over LayerNorm rows: fused, or behind an operation of its own that makes their planes
+    // a contraction over LayerNorm rows
     auto ln = [&](FrOp o, int rows, const float *src, const float *w, const float *b, const EncLayer *closing, int epi, const uint8_t *tiles, const float *bias, int N) {
-        FrOp n = blank(FR_LN);
-        n.rows = rows; n.x = src; n.ln_w = w; n.ln_b = b; n.K = d; n.o_hi = hA.hi; n.o_lo = hA.lo;
+        o.rows = rows; o.x = src; o.ln_w = w; o.ln_b = b; o.epi = epi; o.w = tiles; o.bias = bias; o.N = N; o.K = d;
         if (closing) {                                       // the layer before closes here: its output becomes the residual base
-            n.ln0_w = closing->ln_out_w; n.ln0_b = closing->ln_out_b; n.x_copy = other;
+            o.ln0_w = closing->ln_out_w; o.ln0_b = closing->ln_out_b; o.x_copy = other;
             float *t = cur; cur = other; other = t;
         }
-        if (fuse) { o.rows = n.rows; o.x = n.x; o.ln_w = w; o.ln_b = b; o.ln0_w = n.ln0_w; o.ln0_b = n.ln0_b; o.x_copy = n.x_copy; }
-        else { ops.push_back(n); o.rows = FR_ROWS_PLANES; o.a_hi = hA.hi; o.a_lo = hA.lo; }
-        o.epi = epi; o.w = tiles; o.bias = bias; o.N = N; o.K = d;
         if (!o.ldo) o.ldo = N;
         if (epi == FR_EPI_RESID) { o.out = cur; o.res = cur; }
         ops.push_back(o);
@@ -391,6 +386,7 @@ int Model::stream_layers(StreamState &st, float *x, int Q, const __half *rk, int
         resid(hF, L.t_ff1b, L.ff1_w2.bias, F, 0.5f);
         FrOp o = blank(FR_GEMM);
         o.n_split = d; o.out = q; o.ldo = d; o.o_hi = kvn.hi; o.o_lo = kvn.lo;
+        o.kc = st.k_cache + (size_t)li * S * st.left * d; o.vc = st.v_cache + (size_t)li * S * st.left * d; o.rk = rk + (size_t)li * d; o.ldrk = ldrk;
         ln(o, FR_ROWS_LN, cur, L.ln_att_w, L.ln_att_b, nullptr, FR_EPI_QKV, L.t_qkv, L.qkv.bias, 3 * d);
         o = blank(FR_STREAM_ATTN);
         o.q = q; o.ldq = d; o.kn = kvn.hi; o.vn = kvn.lo; o.rk = rk + (size_t)li * d; o.ldrk = ldrk;
