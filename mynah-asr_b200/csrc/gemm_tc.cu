@@ -145,7 +145,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, lt++) {
             int m0, n0, width;
             units.at(tile, BN, m0, n0, width);
-            const uint32_t idesc = umma_idesc_f16(BM, width);
+            const uint32_t idesc = umma_idesc_f16(BM, width), idesc_both = umma_idesc_f16(BM, NTERMS > 1 ? 2 * BN : BN);
             const int buf = lt & 1;
             const uint32_t acc = tmem_base + buf * Cfg::ACC_COLS;
             // the epilogue must have drained this accumulator (two tiles ago)
@@ -163,12 +163,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
 #pragma unroll
                 for (int kk = 0; kk < BK / 16; kk++) {
                     const uint32_t off = kk * 32;   // 16 fp16 = 32 bytes inside the swizzle atom
-                    tc_mma_f16(acc, umma_desc_sw128(a_hi + off), umma_desc_sw128(b_hi + off), idesc, (kb | kk) != 0);
-                    if (NTERMS > 1) {
-                        tc_mma_f16(acc + BN, umma_desc_sw128(a_lo + off), umma_desc_sw128(b_hi + off), idesc,
-                                   (kb | kk) != 0);
-                        tc_mma_f16(acc + BN, umma_desc_sw128(a_hi + off), umma_desc_sw128(b_lo + off), idesc, 1);
+                    const uint64_t da = umma_desc_sw128(a_hi + off), db = umma_desc_sw128(b_hi + off);
+                    if (NTERMS == 1) {
+                        tc_mma_f16(acc, da, db, idesc, (kb | kk) != 0);
+                        continue;
                     }
+                    // The hi and the lo rows of B lie one below the other, as the two accumulators lie side by side: hi*hi and
+                    // hi*lo can be one MMA of twice the width. With narrow tiles the MMA's fixed time is what counts (3.7 s of
+                    // audio through 17 layers of 512: 2.24 -> 2.14 ms); from 64 columns on every MMA then waits for both
+                    // accumulators of the one before it, which costs more than the second read of A (a minute through 24
+                    // layers of 1024: 14.4 -> 15.1 ms). The first step has to clear both accumulators, and a strip's hi and lo
+                    // rows do not touch.
+                    const bool both = BN == 32 && width == BN && (kb | kk) != 0;
+                    if (!both) tc_mma_f16(acc, da, db, idesc, (kb | kk) != 0);
+                    tc_mma_f16(acc + BN, umma_desc_sw128(a_lo + off), db, idesc, (kb | kk) != 0);
+                    if (both) tc_mma_f16(acc, da, db, idesc_both, 1);
+                    else tc_mma_f16(acc + BN, da, umma_desc_sw128(b_lo + off), idesc, 1);
                 }
                 tc_commit(&empty_bar[s]);           // frees the stage once these MMAs have read it
             }
