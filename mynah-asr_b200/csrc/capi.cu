@@ -866,7 +866,7 @@ int mynah_b200_greedy_decode(mynah_b200_model *h, const float *enc, int T, int *
     MB_CUDA(cudaMemcpyAsync(e, enc, (size_t)T * m.d_out * 4, cudaMemcpyHostToDevice, m.stream));
     std::vector<int> lens{T};
     std::vector<std::vector<int>> tk, fr;
-    if (m.decode_greedy(e, lens, tk, fr)) return -1;
+    if (m.decode_greedy(e, lens, tk, fr) || m.check_status("greedy_decode")) return -1;
     int n = 0;
     for (size_t i = 0; i < tk[0].size() && n < cap; i++, n++) { tokens[n] = tk[0][i]; if (frames) frames[n] = fr[0][i]; }
     return n;

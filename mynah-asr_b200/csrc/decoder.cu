@@ -11,8 +11,8 @@
 // per step. Every step is a few grid-wide phases separated by grid syncs:
 //   head    logits[b] = head . relu(enc[b][t_b] + g[b]); a warp owns 16 rows of the
 //           V (+durations) rows for all utterances and emits first-argmax candidates
-//   select  one CTA per utterance merges the candidates and applies the emission
-//           rule: non-blank -> emit, advance by the predicted duration (RNNT: 0),
+//   select  the candidates meet in one 64-bit maximum per utterance; every CTA applies the
+//           emission rule to its own copy of the utterances' state, no barrier behind it: non-blank -> emit, advance by the predicted duration (RNNT: 0),
 //           blank with duration 0 -> 1, max_symbols guard (src/decoder.c:161-176)
 //   lstm    (only if some utterance emitted) a row block is 4 hidden units x 4 gates of
 //           [W_ih | W_hh] against [input ; previous h] of all utterances, then the cell
@@ -22,12 +22,8 @@
 // dimension: weights as fp16 (hi, lo) planes (a decoded Q4_0/Q8_0 weight is exact in
 // that form), activations split the same way, three MMAs per k-step, f32 accumulate —
 // f32-grade like the reference's sgemv/sgemm path.
-#include <cooperative_groups.h>
-
 #include "kernels.h"
 #include "model.h"
-
-namespace cg = cooperative_groups;
 
 namespace mb {
 
@@ -175,6 +171,48 @@ __device__ __forceinline__ void stage_planes(__half *xhi, __half *xlo, int xs, i
     }
 }
 
+// What every CTA knows of the utterances, kept in step by applying the same rule to the same maxima
+struct GreedyShared {
+    int t[DEC_MAX_B], len[DEC_MAX_B], off[DEC_MAX_B];            // frame, frames, first row in enc
+    int eh[DEC_MAX_B], no[DEC_MAX_B], tok[DEC_MAX_B], emit[DEC_MAX_B];
+    unsigned long long best[DEC_MAX_B][2];                       // this CTA's candidates: token, duration
+    int stop;
+};
+
+// All CTAs have come `target / gridDim.x` times. One counter; 2.2 k cycles against 2.9 k of the cooperative groups' barrier.
+// Bounded: a wait that runs out sets the status and the abort flag, and every CTA leaves (false).
+__device__ __forceinline__ bool greedy_sync(const GreedyDev &p, GreedyShared &sh, unsigned &target) {
+    target += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        // the block barrier before and the release make the CTA's writes visible with the arrival, the acquire and the block
+        // barrier behind it those of the others to all threads
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.scratch) : "memory");
+        const long long t0 = clock64();
+        unsigned v;
+        for (int tries = 1;; tries++) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.scratch) : "memory");
+            if (v >= target) break;
+            if (tries & 63) continue;
+            if (*reinterpret_cast<volatile int *>(p.scratch + 1) || clock64() - t0 > (1ll << 31)) {
+                atomicExch(p.scratch + 1, 1);
+                atomicCAS(p.status, ST_OK, ST_TIMEOUT_EPILOGUE);
+                sh.stop = 1;
+                break;
+            }
+        }
+    }
+    __syncthreads();
+    return sh.stop == 0;
+}
+
+// (value, index) in one word: the larger word is the larger value, among equals the smaller index. 0 stands for none.
+__device__ __forceinline__ unsigned long long cand_word(float v, int i) {
+    const unsigned u = __float_as_uint(v + 0.0f);                // -0 counts as 0
+    return ((unsigned long long)(u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u)) << 32) | (0xffffffffu - (unsigned)i);
+}
+__device__ __forceinline__ int cand_index(unsigned long long w) { return w ? (int)(0xffffffffu - (unsigned)w) : 0x7fffffff; }
+
 struct Cand { float v; int i; };
 __device__ __forceinline__ void cand_take(Cand &a, float v, int i) {
     if (v > a.v || (v == a.v && i < a.i)) { a.v = v; a.i = i; }
@@ -184,7 +222,7 @@ __device__ __forceinline__ void cand_take(Cand &a, float v, int i) {
 // block is 4 units x 4 gates (i, f, g, o); k = [input ; previous h] is split over
 // NSL warps and reduced through shared memory. Reads h[par], writes h[par^1]; c in
 // place. Utterances that did not emit copy their state through.
-__device__ void lstm_phase(const GreedyDev &p, int l, int par, __half *xhi, __half *xlo, float *red, int lane, int wib) {
+__device__ void lstm_phase(const GreedyDev &p, const GreedyShared &sh, int l, int par, __half *xhi, __half *xlo, float *red, int lane, int wib) {
     const int H = p.H, B = p.B, K = 2 * H, xs = K + XPAD;
     // hidden states live as fp16 (hi, lo) planes: h[parity] = [hi: L][B][H] then [lo: L][B][H] halves
     const size_t nstate = (size_t)p.L * B * H;
@@ -197,8 +235,8 @@ __device__ void lstm_phase(const GreedyDev &p, int l, int par, __half *xhi, __ha
     const int nrb = H / 4, chunks = K / 32, per = (chunks + NSL - 1) / NSL;
     if (blockIdx.x * 8 < nrb * NSL) {        // a CTA without a row block to work on does not pull the activations either
         if (l == 0)
-            stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return p.emb_hi + (size_t)p.last_tok[b] * H; },
-                         [&](int b) { return p.emb_lo + (size_t)p.last_tok[b] * H; });
+            stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return p.emb_hi + (size_t)sh.tok[b] * H; },
+                         [&](int b) { return p.emb_lo + (size_t)sh.tok[b] * H; });
         else
             stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return xin_hi + (size_t)b * H; }, [&](int b) { return xin_lo + (size_t)b * H; });
         stage_planes(xhi, xlo, xs, H, H, B, [&](int b) { return hold_hi + (size_t)b * H; }, [&](int b) { return hold_lo + (size_t)b * H; });
@@ -223,7 +261,7 @@ __device__ void lstm_phase(const GreedyDev &p, int l, int par, __half *xhi, __ha
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
                     const int b = nb * 8 + 2 * t + e;
-                    if (b < B) { em[nb][e] = p.emit[b]; cprev[nb][e] = cc[(size_t)b * H + unit]; }
+                    if (b < B) { em[nb][e] = sh.emit[b]; cprev[nb][e] = cc[(size_t)b * H + unit]; }
                 }
         }
         if (on) {
@@ -280,7 +318,7 @@ __device__ void lstm_phase(const GreedyDev &p, int l, int par, __half *xhi, __ha
 }
 
 // g[b] = proj_b + proj_w . h_last[b] for the utterances that emitted.
-__device__ void proj_phase(const GreedyDev &p, int par, bool all, __half *xhi, __half *xlo, float *red, int lane, int wib) {
+__device__ void proj_phase(const GreedyDev &p, const GreedyShared &sh, int par, bool all, __half *xhi, __half *xlo, float *red, int lane, int wib) {
     const int H = p.H, B = p.B, xs = 2 * H + XPAD;
     const size_t nstate = (size_t)p.L * B * H;
     const __half *hl_hi = reinterpret_cast<const __half *>(p.h[par]) + (size_t)(p.L - 1) * B * H, *hl_lo = hl_hi + nstate;
@@ -307,10 +345,9 @@ __device__ void proj_phase(const GreedyDev &p, int par, bool all, __half *xhi, _
                 const int r = rb * 16 + g + (i >> 1) * 8, b = nb * 8 + 2 * t + (i & 1);
                 ev[nb][i] = -1.f; addv[nb][i] = 0.f; fresh[nb][i] = false;
                 if (on && sl == 0 && r < H && b < B) {
-                    fresh[nb][i] = all || p.emit[b] != 0;
+                    fresh[nb][i] = all || sh.emit[b] != 0;
                     addv[nb][i] = fresh[nb][i] ? p.proj_b[r] : p.g[(size_t)b * H + r];
-                    const int tb = p.t[b];
-                    if (tb < p.enc_len[b]) ev[nb][i] = p.enc[(size_t)(p.enc_off[b] + tb) * H + r];
+                    if (sh.t[b] < sh.len[b]) ev[nb][i] = p.enc[(size_t)(sh.off[b] + sh.t[b]) * H + r];
                 }
             }
         bool past[2][4];
@@ -319,7 +356,7 @@ __device__ void proj_phase(const GreedyDev &p, int par, bool all, __half *xhi, _
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int b = nb * 8 + 2 * t + (i & 1);
-                past[nb][i] = !(on && sl == 0 && b < B && p.t[b] < p.enc_len[b]);
+                past[nb][i] = !(on && sl == 0 && b < B && sh.t[b] < sh.len[b]);
             }
         if (on) {
             const int rA = rb * 16 + g, rB = rA + 8;
@@ -358,7 +395,6 @@ __device__ void proj_phase(const GreedyDev &p, int par, bool all, __half *xhi, _
 
 __global__ void __launch_bounds__(256, 1)
 greedy_kernel(GreedyDev p) {
-    cg::grid_group grid = cg::this_grid();
     extern __shared__ __align__(16) uint8_t dsm[];
     const int H = p.H, B = p.B, V = p.V, VL = p.V + p.ND;
     const int xs = 2 * H + XPAD;
@@ -367,47 +403,49 @@ greedy_kernel(GreedyDev p) {
     float *red = reinterpret_cast<float *>(xlo + 16 * xs);          // [8 warps][32 lanes][8]
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
+    __shared__ GreedyShared sh;
+    unsigned target = 0;
+    unsigned long long *cand = reinterpret_cast<unsigned long long *>(p.scratch + 16);
+    if (threadIdx.x < DEC_MAX_B) {
+        const int b = threadIdx.x;
+        const bool on = b < B;
+        sh.t[b] = on ? p.t[b] : 0; sh.len[b] = on ? p.enc_len[b] : 0; sh.off[b] = on ? p.enc_off[b] : 0;
+        sh.eh[b] = on ? p.emitted_here[b] : 0; sh.no[b] = on ? p.n_out[b] : 0;
+        sh.tok[b] = !on || p.init_state ? p.blank : p.last_tok[b]; sh.emit[b] = on && p.init_state;
+        if (b == 0) sh.stop = 0;
+    }
     int par = (!p.init_state && p.par_state) ? *p.par_state : 0;   // read before the first grid sync; written after the last
     for (int i = threadIdx.x; i < 16 * xs; i += blockDim.x) { xhi[i] = __float2half_rn(0.f); xlo[i] = __float2half_rn(0.f); }
     __syncthreads();                                               // rows of absent utterances stay zero for every plane copy
 
     if (p.init_state) {
         // SOS = blank on a zero state (src/decoder.c:151): run the prediction net once
-        if (blockIdx.x == 0 && threadIdx.x < B) { p.emit[threadIdx.x] = 1; p.last_tok[threadIdx.x] = p.blank; }
-        grid.sync();
-        for (int l = 0; l < p.L; l++) { lstm_phase(p, l, par, xhi, xlo, red, lane, wib); grid.sync(); }
+        for (int l = 0; l < p.L; l++) { lstm_phase(p, sh, l, par, xhi, xlo, red, lane, wib); if (!greedy_sync(p, sh, target)) return; }
         par ^= 1;
-        proj_phase(p, par, true, xhi, xlo, red, lane, wib);
-        grid.sync();
+        proj_phase(p, sh, par, true, xhi, xlo, red, lane, wib);
+        if (!greedy_sync(p, sh, target)) return;
     }
     bool jx_valid = p.init_state != 0;     // the planes of relu(enc[t] + g) left by the last projector phase are current
 
     constexpr int NSL = 2;
     const int nrb = (VL + 15) / 16, chunks = H / 32, per = (chunks + NSL - 1) / NSL;
-    __shared__ int srow[16];
     // optional phase timers (clock64 of CTA 0): head, sync, select+sync, lstm+syncs, proj+sync, steps, emit steps
     const bool timing = p.dbg != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
     long long tq = timing ? clock64() : 0;
 #define PHASE_MARK(slot) do { if (timing) { const long long n_ = clock64(); p.dbg[slot] += n_ - tq; tq = n_; } } while (0)
     for (int step = 0; step < p.max_steps; step++) {
         // ---- head: joint = relu(enc[t] + g) -> logits -> first-argmax candidates per row block
-        // frame of every utterance first (one round trip), so that the row loads below depend on nothing
-        // they have to wait for: an utterance past its end reads its last frame and is zeroed afterwards
-        if (threadIdx.x < 16) {
-            int row = -1;
-            if (threadIdx.x < B) {
-                const int tb = p.t[threadIdx.x], len = p.enc_len[threadIdx.x];
-                if (tb < len) row = p.enc_off[threadIdx.x] + tb;
-            }
-            srow[threadIdx.x] = row;
+        // (an utterance past its end gets zeros)
+        if (threadIdx.x < 2 * DEC_MAX_B) {
+            (&sh.best[0][0])[threadIdx.x] = 0;
+            if (blockIdx.x == 0) cand[(step + 1) % 3 * 2 * DEC_MAX_B + threadIdx.x] = 0;    // last read two steps ago
         }
-        __syncthreads();
         if (blockIdx.x * 8 < nrb * NSL && jx_valid) {
             stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return p.jx_hi + (size_t)b * H; }, [&](int b) { return p.jx_lo + (size_t)b * H; });
             cp_wait_all();
         } else if (blockIdx.x * 8 < nrb * NSL)
         stage_x(xhi, xlo, xs, 0, H, B, [&](int b, int k) {
-            const int row = srow[b];
+            const int row = sh.t[b] < sh.len[b] ? sh.off[b] + sh.t[b] : -1;
             const float4 e = ld4(p.enc + (size_t)(row < 0 ? 0 : row) * H + k), gg = ld4(p.g + (size_t)b * H + k);
             const float z = row < 0 ? 0.f : 1.f;
             return make_float4(z * fmaxf(e.x + gg.x, 0.f), z * fmaxf(e.y + gg.y, 0.f), z * fmaxf(e.z + gg.z, 0.f), z * fmaxf(e.w + gg.w, 0.f));
@@ -447,93 +485,71 @@ greedy_kernel(GreedyDev p) {
                         }
                         const int b = nb * 8 + 2 * t + e;
                         if (g == 0 && b < B) {
-                            p.cand_v[((size_t)b * 2 + 0) * nrb + rb] = tk.v; p.cand_i[((size_t)b * 2 + 0) * nrb + rb] = tk.i;
-                            p.cand_v[((size_t)b * 2 + 1) * nrb + rb] = du.v; p.cand_i[((size_t)b * 2 + 1) * nrb + rb] = du.i;
+                            if (tk.i != 0x7fffffff) atomicMax(&sh.best[b][0], cand_word(tk.v, tk.i));
+                            if (du.i != 0x7fffffff) atomicMax(&sh.best[b][1], cand_word(du.v, du.i));
                         }
                     }
             }
             __syncthreads();
         }
-        // flags are double-buffered by step parity: a CTA that runs ahead into the next
-        // step must not overwrite what a slower CTA is still reading
-        int *fl = p.flags + (step & 1) * 2;
-        if (blockIdx.x == 0 && threadIdx.x == 0) { fl[0] = 0; fl[1] = 1; }
-        PHASE_MARK(0);
-        grid.sync();
-        PHASE_MARK(1);
-        // ---- select: CTA b merges candidates and applies the emission rule
-        if (blockIdx.x < B) {
-            const int b = blockIdx.x;
-            __shared__ float sv[2][8];
-            __shared__ int si[2][8];
-            // the utterance's state is fetched while the candidates are merged
-            int tb = 0, st_len = 0, st_no = 0, st_eh = 0;
-            if (threadIdx.x == 0) { tb = p.t[b]; st_len = p.enc_len[b]; st_no = p.n_out[b]; st_eh = p.emitted_here[b]; }
-            Cand best[2];
-            for (int kind = 0; kind < 2; kind++) {
-                Cand c{-3.0e38f, 0x7fffffff};
-                for (int w = threadIdx.x; w < nrb; w += blockDim.x)
-                    cand_take(c, p.cand_v[((size_t)b * 2 + kind) * nrb + w], p.cand_i[((size_t)b * 2 + kind) * nrb + w]);
-                best[kind] = c;
-            }
-#pragma unroll
-            for (int kind = 0; kind < 2; kind++) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-                    cand_take(best[kind], __shfl_xor_sync(0xffffffffu, best[kind].v, o), __shfl_xor_sync(0xffffffffu, best[kind].i, o));
-                if (lane == 0) { sv[kind][wib] = best[kind].v; si[kind][wib] = best[kind].i; }
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-#pragma unroll
-                for (int kind = 0; kind < 2; kind++) {
-                    Cand c{sv[kind][0], si[kind][0]};
-#pragma unroll
-                    for (int w = 1; w < 8; w++) cand_take(c, sv[kind][w], si[kind][w]);
-                    best[kind] = c;
-                }
-                int em = 0;
-                if (tb < st_len) {
-                    const int k = best[0].i;
-                    int dur = p.ND > 0 ? p.durations[best[1].i - V] : (k == p.blank ? 1 : 0);
-                    if (k != p.blank) {
-                        const int no = st_no;
-                        if (no < p.cap) { p.tokens[(size_t)b * p.cap + no] = k; p.frames[(size_t)b * p.cap + no] = tb; p.n_out[b] = no + 1; }
-                        em = 1;
-                        p.last_tok[b] = k;
-                        const int eh = st_eh + 1;
-                        p.emitted_here[b] = eh;
-                        if (dur == 0 && eh >= p.max_symbols) dur = 1;
-                    } else if (dur == 0) {
-                        dur = 1;
-                    }
-                    if (dur > 0) p.emitted_here[b] = 0;
-                    tb += dur;
-                    p.t[b] = tb;
-                }
-                p.emit[b] = em;
-                if (em) atomicExch(&fl[0], 1);
-                if (tb < st_len) atomicExch(&fl[1], 0);
-            }
+        unsigned long long *best = cand + step % 3 * 2 * DEC_MAX_B;
+        if (threadIdx.x < 2 * B) {
+            const unsigned long long w = (&sh.best[0][0])[threadIdx.x];
+            if (w) atomicMax(best + threadIdx.x, w);
         }
-        grid.sync();
+        PHASE_MARK(0);
+        if (!greedy_sync(p, sh, target)) return;
+        PHASE_MARK(1);
+        // ---- select: the emission rule, by every CTA for itself
+        int em = 0;
+        bool over = true;
+        if (threadIdx.x < B) {
+            const int b = threadIdx.x;
+            int tb = sh.t[b];
+            const unsigned long long bt = __ldcg(best + 2 * b), bd = __ldcg(best + 2 * b + 1);
+            if (tb < sh.len[b]) {
+                const int k = cand_index(bt);
+                int dur = p.ND > 0 ? (bd ? p.durations[cand_index(bd) - V] : 0) : (k == p.blank ? 1 : 0);
+                if (k != p.blank) {
+                    const int no = sh.no[b], eh = sh.eh[b] + 1;
+                    if (no < p.cap) {
+                        if (blockIdx.x == 0) { p.tokens[(size_t)b * p.cap + no] = k; p.frames[(size_t)b * p.cap + no] = tb; }
+                        sh.no[b] = no + 1;
+                    }
+                    em = 1;
+                    sh.tok[b] = k < V ? k : 0;
+                    sh.eh[b] = eh;
+                    if (dur == 0 && eh >= p.max_symbols) dur = 1;
+                } else if (dur == 0) {
+                    dur = 1;
+                }
+                if (dur > 0) sh.eh[b] = 0;
+                tb += dur;
+                sh.t[b] = tb;
+            }
+            sh.emit[b] = em;
+            over = tb >= sh.len[b];
+        }
+        const int any_emit = __syncthreads_or(em), all_done = __syncthreads_and(over);
         PHASE_MARK(2);
-        const int any_emit = *reinterpret_cast<volatile int *>(&fl[0]);
-        const int all_done = *reinterpret_cast<volatile int *>(&fl[1]);
-        if (timing) { p.dbg[5] += 1; p.dbg[6] += any_emit; }
+        if (timing) { p.dbg[5] += 1; p.dbg[6] += any_emit != 0; }
         if (any_emit) {
-            for (int l = 0; l < p.L; l++) { lstm_phase(p, l, par, xhi, xlo, red, lane, wib); grid.sync(); }
+            for (int l = 0; l < p.L; l++) { lstm_phase(p, sh, l, par, xhi, xlo, red, lane, wib); if (!greedy_sync(p, sh, target)) return; }
             PHASE_MARK(3);
             par ^= 1;
-            proj_phase(p, par, false, xhi, xlo, red, lane, wib);
-            grid.sync();
+            proj_phase(p, sh, par, false, xhi, xlo, red, lane, wib);
+            if (!greedy_sync(p, sh, target)) return;
             PHASE_MARK(4);
         }
         jx_valid = any_emit != 0;
         if (all_done) break;
     }
 #undef PHASE_MARK
-    if (blockIdx.x == 0 && threadIdx.x == 0) { p.flags[4] = par; if (p.par_state) *p.par_state = par; }
+    if (blockIdx.x == 0 && threadIdx.x < B) {
+        const int b = threadIdx.x;
+        p.t[b] = sh.t[b]; p.emitted_here[b] = sh.eh[b]; p.n_out[b] = sh.no[b]; p.last_tok[b] = sh.tok[b]; p.emit[b] = sh.emit[b];
+        if (b == 0 && p.par_state) *p.par_state = par;
+    }
 }
 
 int greedy_launch(const GreedyDev &p, cudaStream_t st, int want_blocks) {

@@ -692,7 +692,6 @@ int Model::decode_greedy(const float *enc_dev, const std::vector<int> &lens, std
     if (!has_dec) { set_error("model has no transducer decoder"); return -1; }
     std::vector<int> offs(Ball);
     for (int b = 0, o = 0; b < Ball; o += lens[b], b++) offs[b] = o;
-    const int nw = (vocab + cfg.n_durations + 15) / 16;     // candidate slots: one per 16-row block of the head
     // lock-step groups of DEC_MAX_B utterances; with several groups they run side by side on the decode lanes
     struct Group { int g0, B, cap; int *n_out, *tokens, *frames; long long *dbg; };
     std::vector<Group> groups;
@@ -718,11 +717,11 @@ int Model::decode_greedy(const float *enc_dev, const std::vector<int> &lens, std
         const int B = G.B, cap = G.cap;
         cudaStream_t ls = lane_stream(lanes, (int)gi);
         const size_t nstate = (size_t)L * B * H;
-        float *fz = ws.get<float>(3 * nstate + (size_t)B * H + 2 * (size_t)B * nw + (size_t)DEC_MAX_B * H);
-        int *iz = ws.get<int>(8 * (size_t)B + 2 * (size_t)B * nw + 2 * (size_t)B * cap + 16);
+        float *fz = ws.get<float>(3 * nstate + (size_t)B * H + (size_t)DEC_MAX_B * H);
+        int *iz = ws.get<int>(DEC_SCRATCH + 8 * (size_t)B + 2 * (size_t)B * cap);
         if (!fz || !iz) return -1;
         MB_CUDA(cudaMemsetAsync(fz, 0, (3 * nstate + (size_t)B * H) * sizeof(float), ls));
-        MB_CUDA(cudaMemsetAsync(iz, 0, (8 * (size_t)B + 16) * sizeof(int), ls));
+        MB_CUDA(cudaMemsetAsync(iz, 0, (DEC_SCRATCH + 8 * (size_t)B) * sizeof(int), ls));
         GreedyDev p;
         memset(&p, 0, sizeof(p));
         p.emb = emb; p.head_b = head_b; p.proj_b = proj_b;
@@ -735,12 +734,11 @@ int Model::decode_greedy(const float *enc_dev, const std::vector<int> &lens, std
         p.h[0] = fz; p.h[1] = fz + nstate; p.c = fz + 2 * nstate; p.g = fz + 3 * nstate;
         // the planes first: they are copied in 16-byte pieces and B * H floats keep that alignment
         p.jx_hi = reinterpret_cast<__half *>(p.g + (size_t)B * H); p.jx_lo = p.jx_hi + (size_t)DEC_MAX_B * H;
-        p.cand_v = p.g + (size_t)B * H + (size_t)DEC_MAX_B * H;
         int *q = iz;
-        p.flags = q; q += 16;
+        p.scratch = q; q += DEC_SCRATCH;
+        p.status = status;
         p.t = q; q += B; p.emitted_here = q; q += B; p.n_out = q; q += B; p.last_tok = q; q += B; p.emit = q; q += B;
         q += 3 * B;
-        p.cand_i = q; q += 2 * (size_t)B * nw;
         p.tokens = q; q += (size_t)B * cap; p.frames = q;
         p.cap = cap; p.enc_off = hm_dev + G.g0; p.enc_len = hm_dev + Ball + G.g0;
         int max_len = cap / cfg.max_symbols;

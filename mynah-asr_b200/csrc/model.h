@@ -271,6 +271,7 @@ struct Model {
 };
 
 // Everything the lock-step greedy kernel needs (decoder.cu).
+static constexpr int DEC_SCRATCH = 16 + 3 * 2 * DEC_MAX_B * 2;
 struct GreedyDev {
     // model
     const float *emb, *head_b, *proj_b;
@@ -290,10 +291,10 @@ struct GreedyDev {
     __half *jx_hi, *jx_lo;       // [16][H] each: relu(enc[t] + g) of the coming step as operand planes (written with g)
     int *t, *emitted_here, *n_out, *last_tok, *emit;
     int *tokens, *frames, cap;
-    // scratch
-    float *cand_v;               // [B][2][row blocks]  (token / duration candidates)
-    int *cand_i;
-    int *flags;                  // [2][2] {any_emit, all_done} by step parity, [4] final h parity
+    // scratch of DEC_SCRATCH ints, zero at launch: grid barrier, abort flag, then from word 16 on the best token and duration of
+    // every utterance as ordered 64-bit words, by step modulo three
+    int *scratch;
+    int *status;
     int max_steps, init_state;
     int *par_state;              // optional: parity of h carried between launches on the same state
     long long *dbg;              // optional [8] phase timers (clock64 ticks of CTA 0), null = off

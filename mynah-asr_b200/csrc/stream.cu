@@ -612,7 +612,7 @@ int Model::stream_decode(StreamState &st, const float *enc_dev, int q, std::vect
         MB_CUDA(cudaMemsetAsync(st.dec_f, 0, ngroups * fblock * sizeof(float), stream));
         MB_CUDA(cudaMemsetAsync(st.dec_i, 0, ngroups * iblock * sizeof(int), stream));
     }
-    const int nw = (vocab + cfg.n_durations + 15) / 16, cap = q * cfg.max_symbols;
+    const int cap = q * cfg.max_symbols;
     const size_t mark = ws.off;
     struct Out { int *n_out, *tokens, *frames; int B; };
     std::vector<Out> outs(ngroups);
@@ -622,9 +622,9 @@ int Model::stream_decode(StreamState &st, const float *enc_dev, int q, std::vect
         for (int b = 0; b < B; b++) { hm[o + b] = (g0 + b) * q; hm[o + B + b] = q; }
         o += 2 * B;
     }
-    // every group's integer block (flags, per-utterance state, candidates, emitted tokens and frames) sits in one
+    // every group's integer block (scratch, per-utterance state, emitted tokens and frames) sits in one
     // region so that a single copy brings all results back
-    const size_t ipg = 8 * (size_t)DEC_MAX_B + 2 * (size_t)DEC_MAX_B * nw + 2 * (size_t)DEC_MAX_B * cap + 16;
+    const size_t ipg = DEC_SCRATCH + 8 * (size_t)DEC_MAX_B + 2 * (size_t)DEC_MAX_B * cap;      // (even: the scratch holds 64-bit words)
     int *iz_all = ws.get<int>(ipg * ngroups);
     if (!iz_all) return -1;
     MB_CUDA(cudaMemsetAsync(iz_all, 0, ipg * ngroups * sizeof(int), stream));
@@ -640,7 +640,7 @@ int Model::stream_decode(StreamState &st, const float *enc_dev, int q, std::vect
         const size_t nstate = (size_t)L * B * H;
         float *fs = st.dec_f + gi * fblock;
         int *is = st.dec_i + gi * iblock;
-        float *cand = ws.get<float>(2 * (size_t)B * nw + (size_t)DEC_MAX_B * H);
+        float *cand = ws.get<float>((size_t)DEC_MAX_B * H);
         int *iz = iz_all + gi * ipg;
         if (!cand) return -1;
         GreedyDev p;
@@ -654,12 +654,11 @@ int Model::stream_decode(StreamState &st, const float *enc_dev, int q, std::vect
         p.B = B; p.enc = enc_dev;
         p.h[0] = fs; p.h[1] = fs + nstate; p.c = fs + 2 * nstate; p.g = fs + 3 * nstate;
         p.jx_hi = reinterpret_cast<__half *>(cand); p.jx_lo = p.jx_hi + (size_t)DEC_MAX_B * H;
-        p.cand_v = cand + (size_t)DEC_MAX_B * H;
         int *qi = iz;
-        p.flags = qi; qi += 16;
+        p.scratch = qi; qi += DEC_SCRATCH;
+        p.status = status;
         p.t = qi; qi += B; p.emitted_here = qi; qi += B; p.n_out = qi; qi += B; p.emit = qi; qi += B;
         qi += 4 * B;
-        p.cand_i = qi; qi += 2 * (size_t)B * nw;
         p.tokens = qi; qi += (size_t)B * cap; p.frames = qi;
         p.last_tok = is; p.par_state = is + DEC_MAX_B;
         p.cap = cap; p.enc_off = hm_dev + 2 * (size_t)g0; p.enc_len = hm_dev + 2 * (size_t)g0 + B;
