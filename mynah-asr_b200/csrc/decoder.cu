@@ -80,48 +80,89 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Accumulates chunks [c0, c1) of 32 k for rows rowA (fragment rows g) and rowB (g + 8).
-// acc[nb][0..3]: rows g (0,1) and g+8 (2,3) x utterances nb*8 + 2t, +1.
-__device__ __forceinline__ void rowblock_mma(const __half *__restrict__ whi, const __half *__restrict__ wlo, int ldw,
-                                             int rowA, int rowB, int c0, int c1, const __half *xhi,
-                                             const __half *xlo, int xs, int lane, float (&acc)[2][4]) {
-    const int g = lane >> 2, t = lane & 3;
-    float d0[2][4], d1[2][4];
+__device__ __forceinline__ uint4 ld_weight(const __half *p) {
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+// A warp's 16 weight rows (fragment rows g and g + 8) and its sums. Weights do not depend on the state: ask() sends for the
+// first AHEAD chunks of 32 k, which a phase does before it waits at the grid barrier in front of it (the loads are volatile,
+// they stay there), so that the L2 delivers them meanwhile. NB: blocks of eight utterances.
+template <int NB>
+struct RowTask {
+    static constexpr int AHEAD = 5;
+    const __half *hi, *lo;
+    int oA, oB;                                       // the lane's columns of its two rows
+    uint4 ah[AHEAD], bh[AHEAD], al[AHEAD], bl[AHEAD];
+    float d0[NB][4], d1[NB][4];                       // hi x hi; the terms with a low plane
+    __device__ __forceinline__ void at(const __half *whi, const __half *wlo, int ld, int rowA, int rowB, int lane) {
+        hi = whi; lo = wlo;
+        oA = rowA * ld + 8 * (lane & 3); oB = rowB * ld + 8 * (lane & 3);
 #pragma unroll
-    for (int nb = 0; nb < 2; nb++)
+        for (int n = 0; n < NB; n++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) { d0[nb][i] = 0.f; d1[nb][i] = 0.f; }
-    const uint4 *pAh = reinterpret_cast<const uint4 *>(whi + (size_t)rowA * ldw + 8 * t);
-    const uint4 *pBh = reinterpret_cast<const uint4 *>(whi + (size_t)rowB * ldw + 8 * t);
-    const uint4 *pAl = reinterpret_cast<const uint4 *>(wlo + (size_t)rowA * ldw + 8 * t);
-    const uint4 *pBl = reinterpret_cast<const uint4 *>(wlo + (size_t)rowB * ldw + 8 * t);
-    const uint4 *x0h = reinterpret_cast<const uint4 *>(xhi + (size_t)g * xs + 8 * t);
-    const uint4 *x1h = reinterpret_cast<const uint4 *>(xhi + (size_t)(g + 8) * xs + 8 * t);
-    const uint4 *x0l = reinterpret_cast<const uint4 *>(xlo + (size_t)g * xs + 8 * t);
-    const uint4 *x1l = reinterpret_cast<const uint4 *>(xlo + (size_t)(g + 8) * xs + 8 * t);
-#pragma unroll 5
-    for (int c = c0; c < c1; c++) {
-        const uint4 ah = __ldg(pAh + c * 4), bh = __ldg(pBh + c * 4);      // 32 halves = 4 uint4 per chunk
-        const uint4 al = __ldg(pAl + c * 4), bl = __ldg(pBl + c * 4);
-        const uint4 u0h = x0h[c * 4], u1h = x1h[c * 4], u0l = x0l[c * 4], u1l = x1l[c * 4];
-        // k-step 0: elements 0..3, k-step 1: elements 4..7
-        mma_f16(d0[0], ah.x, bh.x, ah.y, bh.y, u0h.x, u0h.y);
-        mma_f16(d0[1], ah.x, bh.x, ah.y, bh.y, u1h.x, u1h.y);
-        mma_f16(d1[0], al.x, bl.x, al.y, bl.y, u0h.x, u0h.y);
-        mma_f16(d1[1], al.x, bl.x, al.y, bl.y, u1h.x, u1h.y);
-        mma_f16(d1[0], ah.x, bh.x, ah.y, bh.y, u0l.x, u0l.y);
-        mma_f16(d1[1], ah.x, bh.x, ah.y, bh.y, u1l.x, u1l.y);
-        mma_f16(d0[0], ah.z, bh.z, ah.w, bh.w, u0h.z, u0h.w);
-        mma_f16(d0[1], ah.z, bh.z, ah.w, bh.w, u1h.z, u1h.w);
-        mma_f16(d1[0], al.z, bl.z, al.w, bl.w, u0h.z, u0h.w);
-        mma_f16(d1[1], al.z, bl.z, al.w, bl.w, u1h.z, u1h.w);
-        mma_f16(d1[0], ah.z, bh.z, ah.w, bh.w, u0l.z, u0l.w);
-        mma_f16(d1[1], ah.z, bh.z, ah.w, bh.w, u1l.z, u1l.w);
+            for (int i = 0; i < 4; i++) d0[n][i] = d1[n][i] = 0.f;
     }
+    __device__ __forceinline__ void ask(int c0, int c1) {
 #pragma unroll
-    for (int nb = 0; nb < 2; nb++)
+        for (int i = 0; i < AHEAD; i++)
+            if (c0 + i < c1) {
+                const int o = (c0 + i) * 32;
+                ah[i] = ld_weight(hi + oA + o); bh[i] = ld_weight(hi + oB + o); al[i] = ld_weight(lo + oA + o); bl[i] = ld_weight(lo + oB + o);
+            }
+    }
+    __device__ __forceinline__ void chunk(uint4 a, uint4 b, uint4 c, uint4 d, const __half *xhi, const __half *xlo, int xs) {
+        uint4 xh[NB], xl[NB];
 #pragma unroll
-        for (int i = 0; i < 4; i++) acc[nb][i] = fmaf(d1[nb][i], H16_LO_INV, d0[nb][i]);
+        for (int n = 0; n < NB; n++) {
+            xh[n] = *reinterpret_cast<const uint4 *>(xhi + n * 8 * xs);
+            xl[n] = *reinterpret_cast<const uint4 *>(xlo + n * 8 * xs);
+        }
+        // k-step 0: elements 0..3, k-step 1: elements 4..7
+#pragma unroll
+        for (int n = 0; n < NB; n++) {
+            mma_f16(d0[n], a.x, b.x, a.y, b.y, xh[n].x, xh[n].y);
+            mma_f16(d1[n], c.x, d.x, c.y, d.y, xh[n].x, xh[n].y);
+            mma_f16(d1[n], a.x, b.x, a.y, b.y, xl[n].x, xl[n].y);
+        }
+#pragma unroll
+        for (int n = 0; n < NB; n++) {
+            mma_f16(d0[n], a.z, b.z, a.w, b.w, xh[n].z, xh[n].w);
+            mma_f16(d1[n], c.z, d.z, c.w, d.w, xh[n].z, xh[n].w);
+            mma_f16(d1[n], a.z, b.z, a.w, b.w, xl[n].z, xl[n].w);
+        }
+    }
+    // adds chunks [c0, c1), the first of them asked for before
+    __device__ __forceinline__ void add(int c0, int c1, const __half *xhi, const __half *xlo, int xs, int lane) {
+        xhi += (size_t)(lane >> 2) * xs + 8 * (lane & 3);
+        xlo += (size_t)(lane >> 2) * xs + 8 * (lane & 3);
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++)
+            if (c0 + i < c1) chunk(ah[i], bh[i], al[i], bl[i], xhi + (c0 + i) * 32, xlo + (c0 + i) * 32, xs);
+        for (int c = c0 + AHEAD; c < c1; c += AHEAD) {
+            ask(c, c1);
+#pragma unroll
+            for (int i = 0; i < AHEAD; i++)
+                if (c + i < c1) chunk(ah[i], bh[i], al[i], bl[i], xhi + (c + i) * 32, xlo + (c + i) * 32, xs);
+        }
+    }
+    // to red[warp][4 n + i][lane]: rows g (i = 0, 1) and g + 8 (2, 3) x utterances 8 n + 2 t, + 1
+    __device__ __forceinline__ void put(float *red, int lane, int wib) const {
+#pragma unroll
+        for (int n = 0; n < NB; n++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) red[(wib * 8 + n * 4 + i) * 32 + lane] = fmaf(d1[n][i], H16_LO_INV, d0[n][i]);
+    }
+};
+// The matvecs' tasks: a row block of 16 rows in NSL slices of K, a warp each.
+static constexpr int LSTM_NSL = 4, HEAD_NSL = 2;
+struct Task { int rb, sl, c0, c1; bool on; };
+__device__ __forceinline__ Task task_of(int base, int wib, int nsl, int nrb, int chunks) {
+    Task k;
+    k.rb = (base + wib) / nsl; k.sl = (base + wib) % nsl; k.on = k.rb < nrb;
+    const int per = (chunks + nsl - 1) / nsl;
+    k.c0 = k.sl * per; k.c1 = k.c0 + per < chunks ? k.c0 + per : chunks;
+    return k;
 }
 
 // Writes f32 rows [16][K] (rows >= B zero) as (hi, lo) planes into shared memory.
@@ -181,13 +222,15 @@ struct GreedyShared {
 
 // All CTAs have come `target / gridDim.x` times. One counter; 2.2 k cycles against 2.9 k of the cooperative groups' barrier.
 // Bounded: a wait that runs out sets the status and the abort flag, and every CTA leaves (false).
-__device__ __forceinline__ bool greedy_sync(const GreedyDev &p, GreedyShared &sh, unsigned &target) {
+__device__ __forceinline__ void greedy_arrive(const GreedyDev &p, unsigned &target) {
     target += gridDim.x;
     __syncthreads();
+    // the block barrier before and the release make the CTA's writes visible with the arrival, the acquire and the block
+    // barrier behind it those of the others to all threads
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.scratch) : "memory");
+}
+__device__ __forceinline__ bool greedy_wait(const GreedyDev &p, GreedyShared &sh, unsigned target) {
     if (threadIdx.x == 0) {
-        // the block barrier before and the release make the CTA's writes visible with the arrival, the acquire and the block
-        // barrier behind it those of the others to all threads
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.scratch) : "memory");
         const long long t0 = clock64();
         unsigned v;
         for (int tries = 1;; tries++) {
@@ -218,12 +261,34 @@ __device__ __forceinline__ void cand_take(Cand &a, float v, int i) {
     if (v > a.v || (v == a.v && i < a.i)) { a.v = v; a.i = i; }
 }
 
-// One stacked-LSTM layer (pred_step, src/decoder.c:73-99) for all utterances. A row
-// block is 4 units x 4 gates (i, f, g, o); k = [input ; previous h] is split over
-// NSL warps and reduced through shared memory. Reads h[par], writes h[par^1]; c in
-// place. Utterances that did not emit copy their state through.
-__device__ void lstm_phase(const GreedyDev &p, const GreedyShared &sh, int l, int par, __half *xhi, __half *xlo, float *red, int lane, int wib) {
-    const int H = p.H, B = p.B, K = 2 * H, xs = K + XPAD;
+// One stacked-LSTM layer (pred_step, src/decoder.c:73-99) for all utterances. A row block is 4 units x 4 gates (i, f, g, o); a
+// slice of K is a piece of the previous h and the same piece of the input. Reads h[par], writes h[par^1]; c in place. Utterances
+// that did not emit copy their state through.
+// lstm_open, between arrival and wait of the barrier in front of the phase: the CTA's first tasks over the previous h, which is
+// known by then, and the first weights over the input.
+template <int NB>
+__device__ __forceinline__ void lstm_rows(const GreedyDev &p, int l, const Task &k, int lane, RowTask<NB> &w) {
+    // fragment row lr -> gate lr/4, unit rb*4 + lr%4
+    const int g = lane >> 2, rowA = (g >> 2) * p.H + k.rb * 4 + (g & 3);
+    w.at(p.wcat_hi[l], p.wcat_lo[l], 2 * p.H, rowA, rowA + 2 * p.H, lane);
+    w.ask(p.H / 32 + k.c0, p.H / 32 + k.c1);
+}
+template <int NB>
+__device__ __forceinline__ void lstm_open(const GreedyDev &p, int l, int par, __half *xhi, __half *xlo, int lane, int wib, RowTask<NB> &w) {
+    const int H = p.H, B = p.B, xs = 2 * H + XPAD, hc = H / 32;
+    const Task k = task_of(blockIdx.x * 8, wib, LSTM_NSL, H / 4, hc);
+    if (k.on) lstm_rows<NB>(p, l, k, lane, w);
+    if (blockIdx.x * 8 < H / 4 * LSTM_NSL) {          // a CTA without a row block to work on does not pull the activations either
+        const __half *hold_hi = reinterpret_cast<const __half *>(p.h[par]) + (size_t)l * B * H, *hold_lo = hold_hi + (size_t)p.L * B * H;
+        stage_planes(xhi, xlo, xs, H, H, B, [&](int b) { return hold_hi + (size_t)b * H; }, [&](int b) { return hold_lo + (size_t)b * H; });
+        cp_wait_all();
+    }
+    __syncthreads();
+    if (k.on) { w.add(hc + k.c0, hc + k.c1, xhi, xlo, xs, lane); w.ask(k.c0, k.c1); }
+}
+template <int NB>
+__device__ __forceinline__ void lstm_phase(const GreedyDev &p, const GreedyShared &sh, int l, int par, __half *xhi, __half *xlo, float *red, int lane, int wib, RowTask<NB> &w) {
+    const int H = p.H, B = p.B, xs = 2 * H + XPAD, hc = H / 32;
     // hidden states live as fp16 (hi, lo) planes: h[parity] = [hi: L][B][H] then [lo: L][B][H] halves
     const size_t nstate = (size_t)p.L * B * H;
     const __half *hold_hi = reinterpret_cast<const __half *>(p.h[par]) + (size_t)l * B * H, *hold_lo = hold_hi + nstate;
@@ -231,63 +296,64 @@ __device__ void lstm_phase(const GreedyDev &p, const GreedyShared &sh, int l, in
     float *cc = p.c + (size_t)l * B * H;
     const __half *xin_hi = l == 0 ? nullptr : reinterpret_cast<const __half *>(p.h[par ^ 1]) + (size_t)(l - 1) * B * H;
     const __half *xin_lo = l == 0 ? nullptr : xin_hi + nstate;
-    constexpr int NSL = 4;
-    const int nrb = H / 4, chunks = K / 32, per = (chunks + NSL - 1) / NSL;
-    if (blockIdx.x * 8 < nrb * NSL) {        // a CTA without a row block to work on does not pull the activations either
-        if (l == 0)
-            stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return p.emb_hi + (size_t)sh.tok[b] * H; },
-                         [&](int b) { return p.emb_lo + (size_t)sh.tok[b] * H; });
-        else
-            stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return xin_hi + (size_t)b * H; }, [&](int b) { return xin_lo + (size_t)b * H; });
-        stage_planes(xhi, xlo, xs, H, H, B, [&](int b) { return hold_hi + (size_t)b * H; }, [&](int b) { return hold_lo + (size_t)b * H; });
-        cp_wait_all();
-    }
-    __syncthreads();
+    constexpr int NSL = LSTM_NSL;
+    const int nrb = H / 4;
     const int g = lane >> 2, t = lane & 3;
     for (int base = blockIdx.x * 8; base < nrb * NSL; base += gridDim.x * 8) {
-        const int task = base + wib, rb = task / NSL, sl = task % NSL;
-        const bool on = task < nrb * NSL;
-        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        const bool again = base != (int)blockIdx.x * 8;
+        const Task k = task_of(base, wib, NSL, nrb, hc);
+        const int rb = k.rb, sl = k.sl;
+        const bool on = k.on;
         // what the cell update needs besides the sums — biases, previous cell state, emission flags — is
         // fetched now, under the contraction
-        float bih[4] = {0.f, 0.f, 0.f, 0.f}, bhh[4] = {0.f, 0.f, 0.f, 0.f}, cprev[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-        int em[2][2] = {{0, 0}, {0, 0}};
+        float bih[4] = {0.f, 0.f, 0.f, 0.f}, bhh[4] = {0.f, 0.f, 0.f, 0.f}, cprev[NB][2];
+        int em[NB][2];
+#pragma unroll
+        for (int nb = 0; nb < NB; nb++) { cprev[nb][0] = cprev[nb][1] = 0.f; em[nb][0] = em[nb][1] = 0; }
         if (on && sl == 0 && g < 4) {
             const int unit = rb * 4 + g;
 #pragma unroll
             for (int q = 0; q < 4; q++) { bih[q] = p.b_ih[l][q * H + unit]; bhh[q] = p.b_hh[l][q * H + unit]; }
 #pragma unroll
-            for (int nb = 0; nb < 2; nb++)
+            for (int nb = 0; nb < NB; nb++)
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
                     const int b = nb * 8 + 2 * t + e;
                     if (b < B) { em[nb][e] = sh.emit[b]; cprev[nb][e] = cc[(size_t)b * H + unit]; }
                 }
         }
-        if (on) {
-            // fragment row lr -> gate lr/4, unit rb*4 + lr%4
-            const int rowA = (g >> 2) * H + rb * 4 + (g & 3), rowB = (2 + (g >> 2)) * H + rb * 4 + (g & 3);
-            const int c0 = sl * per, c1 = (sl + 1) * per < chunks ? (sl + 1) * per : chunks;
-            rowblock_mma(p.wcat_hi[l], p.wcat_lo[l], K, rowA, rowB, c0, c1, xhi, xlo, xs, lane, acc);
+        if (!again) {
+            if (l == 0)
+                stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return p.emb_hi + (size_t)sh.tok[b] * H; },
+                             [&](int b) { return p.emb_lo + (size_t)sh.tok[b] * H; });
+            else
+                stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return xin_hi + (size_t)b * H; }, [&](int b) { return xin_lo + (size_t)b * H; });
+            cp_wait_all();
+            __syncthreads();
+        } else if (on) {
+            lstm_rows<NB>(p, l, k, lane, w);
+            w.add(hc + k.c0, hc + k.c1, xhi, xlo, xs, lane);
+            w.ask(k.c0, k.c1);
         }
-#pragma unroll
-        for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-            for (int i = 0; i < 4; i++) red[(wib * 32 + lane) * 8 + nb * 4 + i] = acc[nb][i];
+        if (on) {
+            w.add(k.c0, k.c1, xhi, xlo, xs, lane);
+            w.put(red, lane, wib);
+        }
         __syncthreads();
         if (on && sl == 0) {
-            float z[2][4];
+            float z[NB][4];
 #pragma unroll
-            for (int nb = 0; nb < 2; nb++)
+            for (int nb = 0; nb < NB; nb++)
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    float s = 0.f;
-                    for (int q = 0; q < NSL; q++) s += red[((wib + q) * 32 + lane) * 8 + nb * 4 + i];
-                    z[nb][i] = s;
+                    float v = 0.f;
+#pragma unroll
+                    for (int q = 0; q < NSL; q++) v += red[((wib + q) * 8 + nb * 4 + i) * 32 + lane];
+                    z[nb][i] = v;
                 }
             // lane g<4 holds gates i (rows g) and g (rows g+8) of unit g; lane g+4 holds f and o
 #pragma unroll
-            for (int nb = 0; nb < 2; nb++)
+            for (int nb = 0; nb < NB; nb++)
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
                     const float za = z[nb][e], zb = z[nb][2 + e];
@@ -317,29 +383,34 @@ __device__ void lstm_phase(const GreedyDev &p, const GreedyShared &sh, int l, in
     }
 }
 
-// g[b] = proj_b + proj_w . h_last[b] for the utterances that emitted.
-__device__ void proj_phase(const GreedyDev &p, const GreedyShared &sh, int par, bool all, __half *xhi, __half *xlo, float *red, int lane, int wib) {
+// g[b] = proj_b + proj_w . h_last[b] for the utterances that emitted. proj_open: the first weights, in front of the barrier's wait.
+template <int NB>
+__device__ __forceinline__ void proj_open(const GreedyDev &p, const Task &k, int lane, RowTask<NB> &w) {
+    const int H = p.H, rA = k.rb * 16 + (lane >> 2), rB = rA + 8;
+    if (!k.on) return;
+    w.at(p.proj_hi, p.proj_lo, H, rA < H ? rA : H - 1, rB < H ? rB : H - 1, lane);
+    w.ask(k.c0, k.c1);
+}
+template <int NB>
+__device__ __forceinline__ void proj_phase(const GreedyDev &p, const GreedyShared &sh, int par, bool all, __half *xhi, __half *xlo, float *red, int lane, int wib, RowTask<NB> &w) {
     const int H = p.H, B = p.B, xs = 2 * H + XPAD;
     const size_t nstate = (size_t)p.L * B * H;
     const __half *hl_hi = reinterpret_cast<const __half *>(p.h[par]) + (size_t)(p.L - 1) * B * H, *hl_lo = hl_hi + nstate;
-    constexpr int NSL = 4;
-    const int nrb = (H + 15) / 16, chunks = H / 32, per = (chunks + NSL - 1) / NSL;
-    if (blockIdx.x * 8 < nrb * NSL) {
-        stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return hl_hi + (size_t)b * H; }, [&](int b) { return hl_lo + (size_t)b * H; });
-        cp_wait_all();
-    }
-    __syncthreads();
+    constexpr int NSL = LSTM_NSL;
+    const int nrb = (H + 15) / 16;
     const int g = lane >> 2, t = lane & 3;
     for (int base = blockIdx.x * 8; base < nrb * NSL; base += gridDim.x * 8) {
-        const int task = base + wib, rb = task / NSL, sl = task % NSL;
-        const bool on = task < nrb * NSL;
-        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        const bool again = base != (int)blockIdx.x * 8;
+        const Task k = task_of(base, wib, NSL, nrb, H / 32);
+        const int rb = k.rb, sl = k.sl;
+        const bool on = k.on;
+        if (again) proj_open<NB>(p, k, lane, w);
         // the encoder values the epilogue adds to g are fetched now, under the contraction (-1: past the end)
         // likewise the projector bias of an utterance that emitted, or the g an utterance that did not keeps
-        float ev[2][4], addv[2][4];
-        bool fresh[2][4];
+        float ev[NB][4], addv[NB][4];
+        bool fresh[NB][4];
 #pragma unroll
-        for (int nb = 0; nb < 2; nb++)
+        for (int nb = 0; nb < NB; nb++)
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int r = rb * 16 + g + (i >> 1) * 8, b = nb * 8 + 2 * t + (i & 1);
@@ -350,31 +421,32 @@ __device__ void proj_phase(const GreedyDev &p, const GreedyShared &sh, int par, 
                     if (sh.t[b] < sh.len[b]) ev[nb][i] = p.enc[(size_t)(sh.off[b] + sh.t[b]) * H + r];
                 }
             }
-        bool past[2][4];
+        bool past[NB][4];
 #pragma unroll
-        for (int nb = 0; nb < 2; nb++)
+        for (int nb = 0; nb < NB; nb++)
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int b = nb * 8 + 2 * t + (i & 1);
                 past[nb][i] = !(on && sl == 0 && b < B && sh.t[b] < sh.len[b]);
             }
-        if (on) {
-            const int rA = rb * 16 + g, rB = rA + 8;
-            const int c0 = sl * per, c1 = (sl + 1) * per < chunks ? (sl + 1) * per : chunks;
-            rowblock_mma(p.proj_hi, p.proj_lo, H, rA < H ? rA : H - 1, rB < H ? rB : H - 1, c0, c1, xhi, xlo, xs, lane, acc);
+        if (!again) {
+            stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return hl_hi + (size_t)b * H; }, [&](int b) { return hl_lo + (size_t)b * H; });
+            cp_wait_all();
+            __syncthreads();
         }
-#pragma unroll
-        for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-            for (int i = 0; i < 4; i++) red[(wib * 32 + lane) * 8 + nb * 4 + i] = acc[nb][i];
+        if (on) {
+            w.add(k.c0, k.c1, xhi, xlo, xs, lane);
+            w.put(red, lane, wib);
+        }
         __syncthreads();
         if (on && sl == 0) {
 #pragma unroll
-            for (int nb = 0; nb < 2; nb++)
+            for (int nb = 0; nb < NB; nb++)
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     float s = 0.f;
-                    for (int q = 0; q < NSL; q++) s += red[((wib + q) * 32 + lane) * 8 + nb * 4 + i];
+#pragma unroll
+                    for (int q = 0; q < NSL; q++) s += red[((wib + q) * 8 + nb * 4 + i) * 32 + lane];
                     const int r = rb * 16 + g + (i >> 1) * 8, b = nb * 8 + 2 * t + (i & 1);
                     if (r < H && b < B) {
                         // g, and with it the joint input of the coming step for this utterance's current frame
@@ -393,6 +465,16 @@ __device__ void proj_phase(const GreedyDev &p, const GreedyShared &sh, int par, 
     }
 }
 
+// A head block's first weights
+template <int NB>
+__device__ __forceinline__ void head_open(const GreedyDev &p, const Task &k, int lane, RowTask<NB> &w) {
+    const int VL = p.V + p.ND, rA = k.rb * 16 + (lane >> 2), rB = rA + 8;
+    if (!k.on) return;
+    w.at(p.head_hi, p.head_lo, p.H, rA < VL ? rA : VL - 1, rB < VL ? rB : VL - 1, lane);
+    w.ask(k.c0, k.c1);
+}
+
+template <int NB>
 __global__ void __launch_bounds__(256, 1)
 greedy_kernel(GreedyDev p) {
     extern __shared__ __align__(16) uint8_t dsm[];
@@ -400,7 +482,8 @@ greedy_kernel(GreedyDev p) {
     const int xs = 2 * H + XPAD;
     __half *xhi = reinterpret_cast<__half *>(dsm);
     __half *xlo = xhi + 16 * xs;
-    float *red = reinterpret_cast<float *>(xlo + 16 * xs);          // [8 warps][32 lanes][8]
+    float *red = reinterpret_cast<float *>(xlo + 16 * xs);          // [8 warps][8][32 lanes]
+    RowTask<NB> w;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     __shared__ GreedyShared sh;
@@ -418,18 +501,32 @@ greedy_kernel(GreedyDev p) {
     for (int i = threadIdx.x; i < 16 * xs; i += blockDim.x) { xhi[i] = __float2half_rn(0.f); xlo[i] = __float2half_rn(0.f); }
     __syncthreads();                                               // rows of absent utterances stay zero for every plane copy
 
+    constexpr int NSL = HEAD_NSL;
+    const int nrb = (VL + 15) / 16;
+    const Task first_head = task_of(blockIdx.x * 8, wib, NSL, nrb, H / 32), first_proj = task_of(blockIdx.x * 8, wib, LSTM_NSL, (H + 15) / 16, H / 32);
+    // the prediction net on the tokens just emitted, from lstm_open of layer 0 to the head's first weights
+    auto predict = [&](bool all) -> bool {
+        for (int l = 0; l < p.L; l++) {
+            lstm_phase<NB>(p, sh, l, par, xhi, xlo, red, lane, wib, w);
+            greedy_arrive(p, target);
+            if (l + 1 < p.L) lstm_open<NB>(p, l + 1, par, xhi, xlo, lane, wib, w);
+            else proj_open<NB>(p, first_proj, lane, w);
+            if (!greedy_wait(p, sh, target)) return false;
+        }
+        par ^= 1;
+        proj_phase<NB>(p, sh, par, all, xhi, xlo, red, lane, wib, w);
+        greedy_arrive(p, target);
+        head_open<NB>(p, first_head, lane, w);
+        return greedy_wait(p, sh, target);
+    };
     if (p.init_state) {
         // SOS = blank on a zero state (src/decoder.c:151): run the prediction net once
-        for (int l = 0; l < p.L; l++) { lstm_phase(p, sh, l, par, xhi, xlo, red, lane, wib); if (!greedy_sync(p, sh, target)) return; }
-        par ^= 1;
-        proj_phase(p, sh, par, true, xhi, xlo, red, lane, wib);
-        if (!greedy_sync(p, sh, target)) return;
-    }
+        lstm_open<NB>(p, 0, par, xhi, xlo, lane, wib, w);
+        if (!predict(true)) return;
+    } else head_open<NB>(p, first_head, lane, w);
     bool jx_valid = p.init_state != 0;     // the planes of relu(enc[t] + g) left by the last projector phase are current
 
-    constexpr int NSL = 2;
-    const int nrb = (VL + 15) / 16, chunks = H / 32, per = (chunks + NSL - 1) / NSL;
-    // optional phase timers (clock64 of CTA 0): head, sync, select+sync, lstm+syncs, proj+sync, steps, emit steps
+    // optional phase timers (clock64 of CTA 0): head, sync with the first layer opened, select, prediction net with its syncs, -, steps, emit steps, staging
     const bool timing = p.dbg != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
     long long tq = timing ? clock64() : 0;
 #define PHASE_MARK(slot) do { if (timing) { const long long n_ = clock64(); p.dbg[slot] += n_ - tq; tq = n_; } } while (0)
@@ -453,27 +550,24 @@ greedy_kernel(GreedyDev p) {
         __syncthreads();
         PHASE_MARK(7);
         for (int base = blockIdx.x * 8; base < nrb * NSL; base += gridDim.x * 8) {
-            const int task = base + wib, rb = task / NSL, sl = task % NSL;
-            const bool on = task < nrb * NSL;
-            float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+            const Task k = task_of(base, wib, NSL, nrb, H / 32);
+            const int rb = k.rb, sl = k.sl;
+            const bool on = k.on;
+            if (base != (int)blockIdx.x * 8) head_open<NB>(p, k, lane, w);
             const int rA = rb * 16 + g, rB = rA + 8;
             const float biasA = on && sl == 0 && rA < VL ? p.head_b[rA] : 0.f, biasB = on && sl == 0 && rB < VL ? p.head_b[rB] : 0.f;
             if (on) {
-                const int c0 = sl * per, c1 = (sl + 1) * per < chunks ? (sl + 1) * per : chunks;
-                rowblock_mma(p.head_hi, p.head_lo, H, rA < VL ? rA : VL - 1, rB < VL ? rB : VL - 1, c0, c1, xhi, xlo, xs, lane, acc);
+                w.add(k.c0, k.c1, xhi, xlo, xs, lane);
+                w.put(red, lane, wib);
             }
-#pragma unroll
-            for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-                for (int i = 0; i < 4; i++) red[(wib * 32 + lane) * 8 + nb * 4 + i] = acc[nb][i];
             __syncthreads();
             if (on && sl == 0) {
 #pragma unroll
-                for (int nb = 0; nb < 2; nb++)
+                for (int nb = 0; nb < NB; nb++)
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
-                        const float va = red[(wib * 32 + lane) * 8 + nb * 4 + e] + red[((wib + 1) * 32 + lane) * 8 + nb * 4 + e] + biasA;
-                        const float vb = red[(wib * 32 + lane) * 8 + nb * 4 + 2 + e] + red[((wib + 1) * 32 + lane) * 8 + nb * 4 + 2 + e] + biasB;
+                        const float va = red[(wib * 8 + nb * 4 + e) * 32 + lane] + red[((wib + 1) * 8 + nb * 4 + e) * 32 + lane] + biasA;
+                        const float vb = red[(wib * 8 + nb * 4 + 2 + e) * 32 + lane] + red[((wib + 1) * 8 + nb * 4 + 2 + e) * 32 + lane] + biasB;
                         Cand tk{-3.0e38f, 0x7fffffff}, du{-3.0e38f, 0x7fffffff};
                         if (rA < V) cand_take(tk, va, rA); else if (rA < VL) cand_take(du, va, rA);
                         if (rB < V) cand_take(tk, vb, rB); else if (rB < VL) cand_take(du, vb, rB);
@@ -498,7 +592,9 @@ greedy_kernel(GreedyDev p) {
             if (w) atomicMax(best + threadIdx.x, w);
         }
         PHASE_MARK(0);
-        if (!greedy_sync(p, sh, target)) return;
+        greedy_arrive(p, target);
+        lstm_open<NB>(p, 0, par, xhi, xlo, lane, wib, w);       // most steps emit
+        if (!greedy_wait(p, sh, target)) return;
         PHASE_MARK(1);
         // ---- select: the emission rule, by every CTA for itself
         int em = 0;
@@ -534,13 +630,9 @@ greedy_kernel(GreedyDev p) {
         PHASE_MARK(2);
         if (timing) { p.dbg[5] += 1; p.dbg[6] += any_emit != 0; }
         if (any_emit) {
-            for (int l = 0; l < p.L; l++) { lstm_phase(p, sh, l, par, xhi, xlo, red, lane, wib); if (!greedy_sync(p, sh, target)) return; }
+            if (!predict(false)) return;
             PHASE_MARK(3);
-            par ^= 1;
-            proj_phase(p, sh, par, false, xhi, xlo, red, lane, wib);
-            if (!greedy_sync(p, sh, target)) return;
-            PHASE_MARK(4);
-        }
+        } else head_open<NB>(p, first_head, lane, w);
         jx_valid = any_emit != 0;
         if (all_done) break;
     }
@@ -558,17 +650,18 @@ int greedy_launch(const GreedyDev &p, cudaStream_t st, int want_blocks) {
     MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     MB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop) { set_error("greedy decode: device lacks cooperative launch"); return -1; }
+    void (*const kernel)(GreedyDev) = p.B <= 8 ? greedy_kernel<1> : greedy_kernel<2>;
     const size_t smem = 2 * 16 * (size_t)(2 * p.H + XPAD) * sizeof(__half) + 8 * 32 * 8 * sizeof(float);
     if (smem > 48 * 1024)
-        MB_CUDA(cudaFuncSetAttribute(greedy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        MB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, greedy_kernel, 256, smem));
+    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem));
     if (per_sm < 1) { set_error("greedy decode: kernel does not fit an SM"); return -1; }
     int blocks = want_blocks > 0 && want_blocks < sms ? want_blocks : sms;
     if (blocks < p.B) { set_error("greedy decode: batch %d exceeds SM count", p.B); return -1; }
     GreedyDev pc = p;
     void *args[] = {&pc};
-    MB_CUDA(cudaLaunchCooperativeKernel((void *)greedy_kernel, dim3(blocks), dim3(256), args, smem, st));
+    MB_CUDA(cudaLaunchCooperativeKernel((void *)kernel, dim3(blocks), dim3(256), args, smem, st));
     return 0;
 }
 
