@@ -298,29 +298,20 @@ __device__ __forceinline__ void lstm_phase(const GreedyDev &p, const GreedyShare
     const __half *xin_lo = l == 0 ? nullptr : xin_hi + nstate;
     constexpr int NSL = LSTM_NSL;
     const int nrb = H / 4;
-    const int g = lane >> 2, t = lane & 3;
     for (int base = blockIdx.x * 8; base < nrb * NSL; base += gridDim.x * 8) {
         const bool again = base != (int)blockIdx.x * 8;
         const Task k = task_of(base, wib, NSL, nrb, hc);
-        const int rb = k.rb, sl = k.sl;
+        const int rb = k.rb;
         const bool on = k.on;
-        // what the cell update needs besides the sums — biases, previous cell state, emission flags — is
-        // fetched now, under the contraction
-        float bih[4] = {0.f, 0.f, 0.f, 0.f}, bhh[4] = {0.f, 0.f, 0.f, 0.f}, cprev[NB][2];
-        int em[NB][2];
-#pragma unroll
-        for (int nb = 0; nb < NB; nb++) { cprev[nb][0] = cprev[nb][1] = 0.f; em[nb][0] = em[nb][1] = 0; }
-        if (on && sl == 0 && g < 4) {
-            const int unit = rb * 4 + g;
+        // The four warps of a row block share its cells, (utterance, unit) by thread: one warp for all of them took 6.6 k cycles
+        // with sixteen utterances. What a cell needs besides the sums — biases, previous state, emission flag — is fetched now.
+        const int j = (wib & 3) * 32 + lane, b = j >> 2, unit = rb * 4 + (j & 3);
+        const bool cell = on && b < B;                           // (B <= 16: the first two warps)
+        float bih[4] = {0.f, 0.f, 0.f, 0.f}, bhh[4] = {0.f, 0.f, 0.f, 0.f}, cprev = 0.f;
+        if (cell) {
 #pragma unroll
             for (int q = 0; q < 4; q++) { bih[q] = p.b_ih[l][q * H + unit]; bhh[q] = p.b_hh[l][q * H + unit]; }
-#pragma unroll
-            for (int nb = 0; nb < NB; nb++)
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int b = nb * 8 + 2 * t + e;
-                    if (b < B) { em[nb][e] = sh.emit[b]; cprev[nb][e] = cc[(size_t)b * H + unit]; }
-                }
+            cprev = cc[(size_t)b * H + unit];
         }
         if (!again) {
             if (l == 0)
@@ -340,44 +331,27 @@ __device__ __forceinline__ void lstm_phase(const GreedyDev &p, const GreedyShare
             w.put(red, lane, wib);
         }
         __syncthreads();
-        if (on && sl == 0) {
-            float z[NB][4];
+        if (cell) {
+            // gate q of unit u is fragment row 4 q + u: lane group 4 (q & 1) + u, upper or lower half by q >> 1
+            float z[4];
 #pragma unroll
-            for (int nb = 0; nb < NB; nb++)
+            for (int q = 0; q < 4; q++) {
+                const int at = (wib & 4) * 8 + (b >> 3) * 4 + (q >> 1) * 2 + (b & 1), from = (4 * (q & 1) + (j & 3)) * 4 + ((b & 7) >> 1);
+                float v = 0.f;
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    float v = 0.f;
-#pragma unroll
-                    for (int q = 0; q < NSL; q++) v += red[((wib + q) * 8 + nb * 4 + i) * 32 + lane];
-                    z[nb][i] = v;
-                }
-            // lane g<4 holds gates i (rows g) and g (rows g+8) of unit g; lane g+4 holds f and o
-#pragma unroll
-            for (int nb = 0; nb < NB; nb++)
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const float za = z[nb][e], zb = z[nb][2 + e];
-                    const float oa = __shfl_xor_sync(0xffffffffu, za, 16), ob = __shfl_xor_sync(0xffffffffu, zb, 16);
-                    if (g < 4) {
-                        const int unit = rb * 4 + g, b = nb * 8 + 2 * t + e;
-                        if (b < B) {
-                            const size_t o = (size_t)b * H + unit;
-                            if (em[nb][e]) {
-                                const float zi = za + bih[0] + bhh[0];
-                                const float zf = oa + bih[1] + bhh[1];
-                                const float zg = zb + bih[2] + bhh[2];
-                                const float zo = ob + bih[3] + bhh[3];
-                                const float cn = sigmoid_stable(zf) * cprev[nb][e] + sigmoid_stable(zi) * tanhf(zg);
-                                cc[o] = cn;
-                                __half hh, hl;
-                                split_h16(sigmoid_stable(zo) * tanhf(cn), hh, hl);
-                                hnew_hi[o] = hh; hnew_lo[o] = hl;
-                            } else {
-                                hnew_hi[o] = hold_hi[o]; hnew_lo[o] = hold_lo[o];
-                            }
-                        }
-                    }
-                }
+                for (int e = 0; e < NSL; e++) v += red[(at + e * 8) * 32 + from];
+                z[q] = v + bih[q] + bhh[q];
+            }
+            const size_t o = (size_t)b * H + unit;
+            if (sh.emit[b]) {
+                const float cn = sigmoid_stable(z[1]) * cprev + sigmoid_stable(z[0]) * tanhf(z[2]);
+                cc[o] = cn;
+                __half hh, hl;
+                split_h16(sigmoid_stable(z[3]) * tanhf(cn), hh, hl);
+                hnew_hi[o] = hh; hnew_lo[o] = hl;
+            } else {
+                hnew_hi[o] = hold_hi[o]; hnew_lo[o] = hold_lo[o];
+            }
         }
         __syncthreads();
     }
@@ -398,37 +372,29 @@ __device__ __forceinline__ void proj_phase(const GreedyDev &p, const GreedyShare
     const __half *hl_hi = reinterpret_cast<const __half *>(p.h[par]) + (size_t)(p.L - 1) * B * H, *hl_lo = hl_hi + nstate;
     constexpr int NSL = LSTM_NSL;
     const int nrb = (H + 15) / 16;
-    const int g = lane >> 2, t = lane & 3;
     for (int base = blockIdx.x * 8; base < nrb * NSL; base += gridDim.x * 8) {
         const bool again = base != (int)blockIdx.x * 8;
         const Task k = task_of(base, wib, NSL, nrb, H / 32);
-        const int rb = k.rb, sl = k.sl;
+        const int rb = k.rb;
         const bool on = k.on;
         if (again) proj_open<NB>(p, k, lane, w);
-        // the encoder values the epilogue adds to g are fetched now, under the contraction (-1: past the end)
-        // likewise the projector bias of an utterance that emitted, or the g an utterance that did not keeps
-        float ev[NB][4], addv[NB][4];
-        bool fresh[NB][4];
+        // (utterance, row) by thread of the row block's four warps. The encoder value that the epilogue adds to g is fetched now,
+        // under the contraction, and the projector bias of an utterance that emitted or the g that the others keep
+        const int r = rb * 16 + (lane & 15);
+        float ev[NB], addv[NB];
+        bool fresh[NB], past[NB];
 #pragma unroll
-        for (int nb = 0; nb < NB; nb++)
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int r = rb * 16 + g + (i >> 1) * 8, b = nb * 8 + 2 * t + (i & 1);
-                ev[nb][i] = -1.f; addv[nb][i] = 0.f; fresh[nb][i] = false;
-                if (on && sl == 0 && r < H && b < B) {
-                    fresh[nb][i] = all || sh.emit[b] != 0;
-                    addv[nb][i] = fresh[nb][i] ? p.proj_b[r] : p.g[(size_t)b * H + r];
-                    if (sh.t[b] < sh.len[b]) ev[nb][i] = p.enc[(size_t)(sh.off[b] + sh.t[b]) * H + r];
-                }
+        for (int n = 0; n < NB; n++) {
+            const int b = n * 8 + (wib & 3) * 2 + (lane >> 4);
+            ev[n] = addv[n] = 0.f;
+            fresh[n] = false; past[n] = true;
+            if (on && r < H && b < B) {
+                fresh[n] = all || sh.emit[b] != 0;
+                addv[n] = fresh[n] ? p.proj_b[r] : p.g[(size_t)b * H + r];
+                past[n] = sh.t[b] >= sh.len[b];
+                if (!past[n]) ev[n] = p.enc[(size_t)(sh.off[b] + sh.t[b]) * H + r];
             }
-        bool past[NB][4];
-#pragma unroll
-        for (int nb = 0; nb < NB; nb++)
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int b = nb * 8 + 2 * t + (i & 1);
-                past[nb][i] = !(on && sl == 0 && b < B && sh.t[b] < sh.len[b]);
-            }
+        }
         if (!again) {
             stage_planes(xhi, xlo, xs, 0, H, B, [&](int b) { return hl_hi + (size_t)b * H; }, [&](int b) { return hl_lo + (size_t)b * H; });
             cp_wait_all();
@@ -439,27 +405,25 @@ __device__ __forceinline__ void proj_phase(const GreedyDev &p, const GreedyShare
             w.put(red, lane, wib);
         }
         __syncthreads();
-        if (on && sl == 0) {
 #pragma unroll
-            for (int nb = 0; nb < NB; nb++)
+        for (int n = 0; n < NB; n++) {
+            const int b = n * 8 + (wib & 3) * 2 + (lane >> 4), lr = lane & 15;
+            if (!on || r >= H || b >= B) continue;
+            // g, and with it the joint input of the coming step for this utterance's current frame
+            // (an utterance that did not emit keeps its g but may have moved to another frame)
+            const size_t o = (size_t)b * H + r;
+            float gv = addv[n];
+            if (fresh[n]) {
+                float v = 0.f;
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    float s = 0.f;
-#pragma unroll
-                    for (int q = 0; q < NSL; q++) s += red[((wib + q) * 8 + nb * 4 + i) * 32 + lane];
-                    const int r = rb * 16 + g + (i >> 1) * 8, b = nb * 8 + 2 * t + (i & 1);
-                    if (r < H && b < B) {
-                        // g, and with it the joint input of the coming step for this utterance's current frame
-                        // (an utterance that did not emit keeps its g but may have moved to another frame)
-                        const size_t o = (size_t)b * H + r;
-                        float gv = addv[nb][i];
-                        if (fresh[nb][i]) { gv = s + addv[nb][i]; p.g[o] = gv; }
-                        const float jv = past[nb][i] ? 0.f : fmaxf(ev[nb][i] + gv, 0.f);
-                        __half jh, jl;
-                        split_h16(jv, jh, jl);
-                        p.jx_hi[o] = jh; p.jx_lo[o] = jl;
-                    }
-                }
+                for (int e = 0; e < NSL; e++) v += red[(((wib & 4) + e) * 8 + n * 4 + (lr >> 3) * 2 + (b & 1)) * 32 + (lr & 7) * 4 + ((b & 7) >> 1)];
+                gv = v + addv[n];
+                p.g[o] = gv;
+            }
+            const float jv = past[n] ? 0.f : fmaxf(ev[n] + gv, 0.f);
+            __half jh, jl;
+            split_h16(jv, jh, jl);
+            p.jx_hi[o] = jh; p.jx_lo[o] = jl;
         }
         __syncthreads();
     }
@@ -555,33 +519,32 @@ greedy_kernel(GreedyDev p) {
             const bool on = k.on;
             if (base != (int)blockIdx.x * 8) head_open<NB>(p, k, lane, w);
             const int rA = rb * 16 + g, rB = rA + 8;
-            const float biasA = on && sl == 0 && rA < VL ? p.head_b[rA] : 0.f, biasB = on && sl == 0 && rB < VL ? p.head_b[rB] : 0.f;
+            const float biasA = on && rA < VL ? p.head_b[rA] : 0.f, biasB = on && rB < VL ? p.head_b[rB] : 0.f;
             if (on) {
                 w.add(k.c0, k.c1, xhi, xlo, xs, lane);
                 w.put(red, lane, wib);
             }
             __syncthreads();
-            if (on && sl == 0) {
+            if (on) {                                            // the block's two warps share the utterances
 #pragma unroll
-                for (int nb = 0; nb < NB; nb++)
+                for (int q = 0; q < NB; q++) {
+                    const int nb = NB == 1 ? 0 : sl, e = NB == 1 ? sl : q, w0 = (wib & ~1) * 8 + nb * 4 + e;
+                    const float va = red[w0 * 32 + lane] + red[(w0 + 8) * 32 + lane] + biasA;
+                    const float vb = red[(w0 + 2) * 32 + lane] + red[(w0 + 10) * 32 + lane] + biasB;
+                    Cand tk{-3.0e38f, 0x7fffffff}, du{-3.0e38f, 0x7fffffff};
+                    if (rA < V) cand_take(tk, va, rA); else if (rA < VL) cand_take(du, va, rA);
+                    if (rB < V) cand_take(tk, vb, rB); else if (rB < VL) cand_take(du, vb, rB);
+                    // reduce over the eight lanes that hold the other rows of this utterance
 #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const float va = red[(wib * 8 + nb * 4 + e) * 32 + lane] + red[((wib + 1) * 8 + nb * 4 + e) * 32 + lane] + biasA;
-                        const float vb = red[(wib * 8 + nb * 4 + 2 + e) * 32 + lane] + red[((wib + 1) * 8 + nb * 4 + 2 + e) * 32 + lane] + biasB;
-                        Cand tk{-3.0e38f, 0x7fffffff}, du{-3.0e38f, 0x7fffffff};
-                        if (rA < V) cand_take(tk, va, rA); else if (rA < VL) cand_take(du, va, rA);
-                        if (rB < V) cand_take(tk, vb, rB); else if (rB < VL) cand_take(du, vb, rB);
-                        // reduce over the eight lanes that hold the other rows of this utterance
-#pragma unroll
-                        for (int o = 4; o < 32; o <<= 1) {
-                            cand_take(tk, __shfl_xor_sync(0xffffffffu, tk.v, o), __shfl_xor_sync(0xffffffffu, tk.i, o));
-                            cand_take(du, __shfl_xor_sync(0xffffffffu, du.v, o), __shfl_xor_sync(0xffffffffu, du.i, o));
-                        }
-                        const int b = nb * 8 + 2 * t + e;
-                        if (g == 0 && b < B) {
-                            if (tk.i != 0x7fffffff) atomicMax(&sh.best[b][0], cand_word(tk.v, tk.i));
-                            if (du.i != 0x7fffffff) atomicMax(&sh.best[b][1], cand_word(du.v, du.i));
-                        }
+                    for (int o = 4; o < 32; o <<= 1) {
+                        cand_take(tk, __shfl_xor_sync(0xffffffffu, tk.v, o), __shfl_xor_sync(0xffffffffu, tk.i, o));
+                        if (rb * 16 + 16 > V) cand_take(du, __shfl_xor_sync(0xffffffffu, du.v, o), __shfl_xor_sync(0xffffffffu, du.i, o));
+                    }
+                    const int b = nb * 8 + 2 * t + e;
+                    if (g == 0 && b < B) {
+                        if (tk.i != 0x7fffffff) atomicMax(&sh.best[b][0], cand_word(tk.v, tk.i));
+                        if (du.i != 0x7fffffff) atomicMax(&sh.best[b][1], cand_word(du.v, du.i));
+                    }
                     }
             }
             __syncthreads();
