@@ -340,12 +340,15 @@ int gemm_tc(const GemmOperand &A, const GemmOperand &B, const GemmEpilogue &ep, 
     // positions, streaming chunks): more CTAs pull the operands. An output element sees the same k order
     // and the same instruction sequence whatever the tile width, so its bits do not change with it.
     const int sms = device_sm_count();
-    // waves of CTAs x time of one tile (the MMAs scale with the tile width, prologue and epilogue do not)
-    const int tm = cdiv(M, BM);
+    // waves of CTAs x time of one tile (the MMAs scale with the tile width and K, prologue and epilogue do not: as much as 48
+    // columns of K = 1024); what a last partial wave is cut into counts with its strips' width (GemmUnits)
+    const int tm = cdiv(M, BM), fixed = K >= 49152 ? 1 : 49152 / K;
     int bn = 128;
     long best = -1;
     for (int cand = 128; cand >= 32; cand >>= 1) {
-        const long cost = (long)cdiv(tm * cdiv(N, cand), sms) * (cand + 48);
+        const int tiles = tm * cdiv(N, cand), rem = tiles % sms;
+        const int split = tiles < sms ? 1 : rem * 4 <= sms && cand % 128 == 0 ? 4 : rem * 2 <= sms && cand % 64 == 0 ? 2 : 1;
+        const long cost = (long)(tiles / sms) * (cand + fixed) + (rem ? cand / split + fixed : 0);
         if (best < 0 || cost < best) { best = cost; bn = cand; }
     }
     const bool low = M <= 64;                        // one half-height row tile
