@@ -124,8 +124,16 @@ glu_dw_kernel(const float *__restrict__ h2, const float *__restrict__ dw_w, cons
               const float *__restrict__ scale, const float *__restrict__ shift, float *__restrict__ out,
               __half *__restrict__ hi, __half *__restrict__ lo, const int *__restrict__ seg_off,
               const int *__restrict__ seg_len, int d, int k, int pad_left) {
-    __shared__ float4 g[(DW_TT + DW_KMAX - 1) * (DW_CH / 4)];
+    constexpr int KU = KW > 0 ? KW : DW_KMAX;
+    __shared__ float4 g[(DW_TT + KU - 1) * (DW_CH / 4)];
+    // The taps of the block's channels, tap by tap: read from memory as they lie (a channel's taps side by side) a warp's load of
+    // one tap touches 32 lines, 1152 of them per warp, which set the time (16 x 750 rows of 1024: 70 us, 57 so).
+    __shared__ float4 ws[KW > 0 ? KW * (DW_CH / 4) : 1];
     chain_trigger();
+    if (KW > 0) {
+        const int c0 = blockIdx.x * DW_CH, n = (d - c0 < DW_CH ? d - c0 : DW_CH) * KW;
+        for (int i = threadIdx.y * 32 + threadIdx.x; i < n; i += 32 * DW_TY) reinterpret_cast<float *>(ws)[i % KU * DW_CH + i / KU] = dw_w[(size_t)c0 * KW + i];
+    }
     chain_wait();
     const int b = blockIdx.z;
     const int len = seg_len[b], off = seg_off[b];
@@ -154,7 +162,6 @@ glu_dw_kernel(const float *__restrict__ h2, const float *__restrict__ dw_w, cons
 #pragma unroll
     for (int i = 0; i < DW_RPT; i++) acc[i] = bias;
     // row tt0 + i uses staged rows tt0 + i + j, j < k: walk the staged rows once, each feeds up to DW_RPT outputs
-    constexpr int KU = KW > 0 ? KW : DW_KMAX;
     const float *w0 = dw_w + (size_t)c * k, *w1 = w0 + k, *w2 = w1 + k, *w3 = w2 + k;
 #pragma unroll
     for (int rr = 0; rr < KU + DW_RPT - 1; rr++) {
@@ -164,8 +171,9 @@ glu_dw_kernel(const float *__restrict__ h2, const float *__restrict__ dw_w, cons
         for (int i = 0; i < DW_RPT; i++) {
             const int j = rr - i;                                 // tap of output i fed by this row
             if (j >= 0 && j < KU && (KW > 0 || j < k)) {
-                acc[i].x = fmaf(w0[j], v.x, acc[i].x); acc[i].y = fmaf(w1[j], v.y, acc[i].y);
-                acc[i].z = fmaf(w2[j], v.z, acc[i].z); acc[i].w = fmaf(w3[j], v.w, acc[i].w);
+                const float4 w = KW > 0 ? ws[j * (DW_CH / 4) + threadIdx.x] : make_float4(w0[j], w1[j], w2[j], w3[j]);
+                acc[i].x = fmaf(w.x, v.x, acc[i].x); acc[i].y = fmaf(w.y, v.y, acc[i].y);
+                acc[i].z = fmaf(w.z, v.z, acc[i].z); acc[i].w = fmaf(w.w, v.w, acc[i].w);
             }
         }
     }
