@@ -469,23 +469,32 @@ __global__ void window_energy_kernel(const float *__restrict__ s, long long lo, 
 }  // namespace
 
 namespace {
+// A device buffer with its own capacity: one that could not be grown has none, whatever became of the others.
+template <typename T>
+struct KeptBuffer {
+    T *p = nullptr;
+    size_t cap = 0;                                                             // in elements
+    bool grow(size_t need) {
+        if (need <= cap) return true;
+        drop();
+        if (cudaMalloc((void **)&p, need * sizeof(T)) != cudaSuccess) { cudaGetLastError(); p = nullptr; set_error("device allocation failed"); return false; }
+        cap = need;
+        return true;
+    }
+    void drop() { if (p) cudaFree(p); p = nullptr; cap = 0; }
+    KeptBuffer() = default;
+    KeptBuffer(const KeptBuffer &) = delete;
+    KeptBuffer &operator=(const KeptBuffer &) = delete;
+    ~KeptBuffer() { drop(); }
+};
+
 // Device buffers of one handle (or one call without a handle), kept from call to call and grown when needed. An audio
 // buffer above KEEP bytes is given back when its call ends.
 struct VadBuffers {
     static constexpr size_t KEEP = 256u << 20;
-    float *audio = nullptr, *xz = nullptr, *hist = nullptr, *probs = nullptr;   // hist [frames][128]; xz: two chunks
-    double *energy = nullptr;
-    size_t audio_cap = 0, frame_cap = 0, energy_cap = 0;                        // in elements
-    template <typename T> static bool grow(T *&p, size_t &cap, size_t need, size_t per) {
-        if (need <= cap) return true;
-        if (p) cudaFree(p);
-        p = nullptr; cap = 0;
-        if (cudaMalloc((void **)&p, need * per * sizeof(T)) != cudaSuccess) { cudaGetLastError(); set_error("device allocation failed"); return false; }
-        cap = need;
-        return true;
-    }
-    void end_call() { if (audio_cap * sizeof(float) > KEEP) { cudaFree(audio); audio = nullptr; audio_cap = 0; } }
-    ~VadBuffers() { cudaFree(audio); cudaFree(xz); cudaFree(hist); cudaFree(probs); cudaFree(energy); }
+    KeptBuffer<float> audio, xz, hist, probs;                                   // xz: two pieces; hist [frames][128]
+    KeptBuffer<double> energy;
+    void end_call() { if (audio.cap * sizeof(float) > KEEP) audio.drop(); }
 };
 }  // namespace
 
@@ -533,27 +542,25 @@ int vad_run(mynah_b200_vad *v, const float *samples, size_t n, std::vector<float
     const int F = v->d.frame, frames = (int)((n + F - 1) / F);
     VadBuffers &b = v->buf;
     probs.assign((size_t)frames, 0.f);
-    size_t hist_cap = b.frame_cap;
-    if (!VadBuffers::grow(b.audio, b.audio_cap, n ? n : 1, 1)) return -1;
+    if (!b.audio.grow(n ? n : 1)) return -1;
     if (frames == 0) return 0;
-    if (!VadBuffers::grow(b.hist, hist_cap, (size_t)frames, VL_H) || !VadBuffers::grow(b.probs, b.frame_cap, (size_t)frames, 1)) return -1;
     const size_t nxz = (size_t)VAD_CHUNK * 4 * VL_H;
-    if (!b.xz && cudaMalloc((void **)&b.xz, 2 * nxz * sizeof(float)) != cudaSuccess) { cudaGetLastError(); b.xz = nullptr; set_error("vad: allocation failed"); return -1; }
+    if (!b.hist.grow((size_t)frames * VL_H) || !b.probs.grow((size_t)frames) || !b.xz.grow(2 * nxz)) return -1;
     cudaError_t e = cudaMemsetAsync(v->status, 0, sizeof(int), v->stream);
     for (int f = 0, i = 0; f < frames && e == cudaSuccess; i++) {
         const int end = f == 0 ? (frames < VAD_CHUNK / 4 ? frames : VAD_CHUNK / 4) : (frames - f < VAD_CHUNK ? frames : f + VAD_CHUNK);
         const size_t s0 = (size_t)f * F, s1 = (size_t)end * F < n ? (size_t)end * F : n;
-        float *xz = b.xz + (i & 1) * nxz;
-        e = cudaMemcpyAsync(b.audio + s0, samples + s0, (s1 - s0) * sizeof(float), cudaMemcpyHostToDevice, v->copy);
+        float *xz = b.xz.p + (i & 1) * nxz;
+        e = cudaMemcpyAsync(b.audio.p + s0, samples + s0, (s1 - s0) * sizeof(float), cudaMemcpyHostToDevice, v->copy);
         if (e == cudaSuccess && i >= 2) e = cudaStreamWaitEvent(v->copy, v->walked[i & 1], 0);
         if (e != cudaSuccess) break;
         // samples past s1 are not on the device yet, and no frame before `end` reads them
-        if (v->d.basis_t) vad_encode16_kernel<<<cdiv(end - f, VE_F), VE_THREADS, VE_SMEM, v->copy>>>(v->d, b.audio, (long long)s1, f, end, xz);
-        else vad_encode_kernel<<<end - f, 256, v->smem, v->copy>>>(v->d, b.audio, (long long)s1, f, xz);
+        if (v->d.basis_t) vad_encode16_kernel<<<cdiv(end - f, VE_F), VE_THREADS, VE_SMEM, v->copy>>>(v->d, b.audio.p, (long long)s1, f, end, xz);
+        else vad_encode_kernel<<<end - f, 256, v->smem, v->copy>>>(v->d, b.audio.p, (long long)s1, f, xz);
         e = cudaEventRecord(v->encoded, v->copy);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(v->stream, v->encoded, 0);
         if (e != cudaSuccess) break;
-        vad_lstm_kernel<<<VL_CTAS, VL_THREADS, 0, v->stream>>>(v->d, xz, f, end, b.hist, v->c_state, v->status);
+        vad_lstm_kernel<<<VL_CTAS, VL_THREADS, 0, v->stream>>>(v->d, xz, f, end, b.hist.p, v->c_state, v->status);
         note_launch(2);
         e = cudaEventRecord(v->walked[i & 1], v->stream);
         f = end;
@@ -561,11 +568,11 @@ int vad_run(mynah_b200_vad *v, const float *samples, size_t n, std::vector<float
     if (e == cudaSuccess) e = cudaGetLastError();
     int st = 0;
     if (e == cudaSuccess) {
-        vad_head_kernel<<<cdiv(frames, 8), 256, 0, v->stream>>>(v->d, b.hist, frames, b.probs);
+        vad_head_kernel<<<cdiv(frames, 8), 256, 0, v->stream>>>(v->d, b.hist.p, frames, b.probs.p);
         note_launch();
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(probs.data(), b.probs, (size_t)frames * sizeof(float), cudaMemcpyDeviceToHost, v->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(probs.data(), b.probs.p, (size_t)frames * sizeof(float), cudaMemcpyDeviceToHost, v->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&st, v->status, sizeof(int), cudaMemcpyDeviceToHost, v->stream);
     const cudaError_t es = cudaStreamSynchronize(v->stream);
     cudaStreamSynchronize(v->copy);
@@ -628,12 +635,12 @@ long long split_point_dev(VadBuffers &b, long long lo, long long hi, int sr, cud
     const int win = sr / 50, hop = win / 2;
     if (hop <= 0 || lo + win > hi) return hi;
     const int nw = (int)((hi - win - lo) / hop) + 1;
-    if (!VadBuffers::grow(b.energy, b.energy_cap, (size_t)nw, 1)) return -1;
-    window_energy_kernel<<<cdiv(nw, 128), 128, 0, st>>>(b.audio, lo, win, hop, nw, b.energy);
+    if (!b.energy.grow((size_t)nw)) return -1;
+    window_energy_kernel<<<cdiv(nw, 128), 128, 0, st>>>(b.audio.p, lo, win, hop, nw, b.energy.p);
     note_launch();
     host.resize((size_t)nw);
     cudaError_t err = cudaGetLastError();
-    if (err == cudaSuccess) err = cudaMemcpyAsync(host.data(), b.energy, (size_t)nw * sizeof(double), cudaMemcpyDeviceToHost, st);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(host.data(), b.energy.p, (size_t)nw * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (err == cudaSuccess) err = cudaStreamSynchronize(st);
     if (err != cudaSuccess) { set_error("plan_segments: %s", cudaGetErrorString(err)); return -1; }
     double best = 1e300;
@@ -780,8 +787,8 @@ int mynah_b200_plan_segments(mynah_b200_vad *v, const float *samples, size_t n_s
     }
     if (!vad_plan) {
         ranges.assign(1, Span{0, n});
-        if (!VadBuffers::grow(buf.audio, buf.audio_cap, n_samples ? n_samples : 1, 1)) return -1;
-        if (n && (cudaMemcpyAsync(buf.audio, samples, n_samples * sizeof(float), cudaMemcpyHostToDevice, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)) {
+        if (!buf.audio.grow(n_samples ? n_samples : 1)) return -1;
+        if (n && (cudaMemcpyAsync(buf.audio.p, samples, n_samples * sizeof(float), cudaMemcpyHostToDevice, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)) {
             cudaGetLastError(); set_error("H2D copy failed"); buf.end_call(); return -1;
         }
     }

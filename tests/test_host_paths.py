@@ -1,0 +1,102 @@
+"""Host paths that a GPU shows only when a device call fails or threads meet: the built library on a CUDA runtime of host
+memory (fake_cudart.cpp), where any call can be made to fail and every launch and its arguments can be looked at. A
+scenario runs in a process of its own, whose loader finds that runtime instead of the real one."""
+import ctypes as C
+import os
+import subprocess
+import sys
+from contextlib import closing
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SCENARIOS = {}
+
+
+def scenario(f):
+    SCENARIOS[f.__name__] = f
+    return f
+
+
+@pytest.fixture(scope="session")
+def fake_runtime(tmp_path_factory, pkg):
+    if not os.path.exists(pkg.LIB_PATH):
+        import mynah_asr_b200.build as b
+        b.build()
+    out = tmp_path_factory.mktemp("fake_cudart")
+    (out / "versions").write_text("libcudart.so.12 { global: *; };\n")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-I", os.path.join(cuda, "include"), os.path.join(HERE, "fake_cudart.cpp"),
+                    "-o", str(out / "libcudart.so.12"), "-Wl,-soname,libcudart.so.12", "-Wl,--version-script," + str(out / "versions")], check=True)
+    return str(out)
+
+
+@pytest.mark.parametrize("name", [
+    "vad_allocation_fails",
+])
+def test_host_path(fake_runtime, name):
+    env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), name], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+# ------------------------------------------------------------------------------------------- in the child process
+def _fake():
+    L = C.CDLL("libcudart.so.12")
+    for f in ("fake_device_bytes", "fake_device_peak", "fake_room"):
+        getattr(L, f).restype = C.c_size_t
+    L.fake_calls.restype = C.c_longlong
+    L.fake_calls.argtypes = [C.c_char_p]
+    L.fake_fail.argtypes = [C.c_char_p, C.c_longlong]
+    L.fake_room.argtypes = [C.c_void_p]
+    return L
+
+
+LAUNCH = C.CFUNCTYPE(None, C.c_char_p, C.POINTER(C.c_void_p), C.c_void_p)
+HOOK = C.CFUNCTYPE(None)
+
+
+def _arg(args, i, kind):
+    return C.cast(args[i], C.POINTER(kind)).contents.value
+
+
+@scenario
+def vad_allocation_fails(pkg, synth, fake):
+    """Whatever allocation of a longer signal fails, the calls after it run on buffers of their own size."""
+    cfg, tensors = synth.make_vad()
+    frame = cfg["vad"]["frame_samples"]
+    seen = []
+
+    def look(name, args, stream):
+        if b"vad_lstm_kernel" in name:                   # (v, xz, f0, f1, hist, c_state, status)
+            seen.append((_arg(args, 3, C.c_int), fake.fake_room(_arg(args, 4, C.c_void_p))))
+        if b"vad_head_kernel" in name:                   # (v, hist, frames, probs)
+            seen.append((_arg(args, 2, C.c_int), fake.fake_room(_arg(args, 1, C.c_void_p))))
+            assert fake.fake_room(_arg(args, 3, C.c_void_p)) >= 4 * _arg(args, 2, C.c_int)
+
+    cb = LAUNCH(look)
+    fake.fake_on_launch(cb)
+    for nth in (1, 2, 3):                                # audio, states, probabilities
+        with closing(pkg.Vad(cfg["vad"], tensors)) as v:
+            v.probs(np.zeros(100 * frame, np.float32))
+            fake.fake_fail(b"cudaMalloc", nth)
+            try:
+                v.probs(np.zeros(200 * frame, np.float32))
+                raise AssertionError("the allocation did not fail")
+            except pkg.BackendError:
+                assert fake.fake_failed()
+            seen.clear()
+            for frames in (50, 100, 150, 200):
+                assert len(v.probs(np.zeros(frames * frame, np.float32))) == frames
+            assert seen and all(room >= 512 * frames for frames, room in seen), seen
+
+
+if __name__ == "__main__":
+    sys.path.insert(0, HERE)
+    import conftest
+    package = conftest.load_package()
+    import mynah_asr_b200.synth as synth_module
+    runtime = _fake()
+    assert package.available()
+    SCENARIOS[sys.argv[1]](package, synth_module, runtime)
