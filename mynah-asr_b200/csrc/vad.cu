@@ -488,13 +488,17 @@ struct KeptBuffer {
     ~KeptBuffer() { drop(); }
 };
 
-// Device buffers of one handle (or one call without a handle), kept from call to call and grown when needed. An audio
-// buffer above KEEP bytes is given back when its call ends.
+// Device buffers of one handle (or one call without a handle), kept from call to call and grown when needed. When a call
+// ends, audio above KEEP bytes is given back, and so are the LSTM states above a quarter of that (512 bytes per frame of 512
+// samples: both lines lie at a signal of 70 minutes) with the probabilities. xz and energy (20 s) have a size of their own.
 struct VadBuffers {
     static constexpr size_t KEEP = 256u << 20;
     KeptBuffer<float> audio, xz, hist, probs;                                   // xz: two pieces; hist [frames][128]
     KeptBuffer<double> energy;
-    void end_call() { if (audio.cap * sizeof(float) > KEEP) audio.drop(); }
+    void end_call() {
+        if (audio.cap * sizeof(float) > KEEP) audio.drop();
+        if (hist.cap * sizeof(float) > KEEP / 4) { hist.drop(); probs.drop(); }
+    }
 };
 }  // namespace
 

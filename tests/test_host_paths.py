@@ -33,7 +33,7 @@ def fake_runtime(tmp_path_factory, pkg):
 
 
 @pytest.mark.parametrize("name", [
-    "vad_allocation_fails",
+    "vad_allocation_fails", "vad_gives_back",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -90,6 +90,32 @@ def vad_allocation_fails(pkg, synth, fake):
             for frames in (50, 100, 150, 200):
                 assert len(v.probs(np.zeros(frames * frame, np.float32))) == frames
             assert seen and all(room >= 512 * frames for frames, room in seen), seen
+
+
+@scenario
+def vad_gives_back(pkg, synth, fake):
+    """What a handle keeps is bounded by the lines of its buffers, not by the longest signal it ever saw."""
+    cfg, tensors = synth.make_vad()
+    frame, keep = cfg["vad"]["frame_samples"], 256 << 20
+    with closing(pkg.Vad(cfg["vad"], tensors)) as v:
+        v.probs(np.zeros(frame, np.float32))
+        small = fake.fake_device_bytes()
+        line = np.zeros(keep // 4, np.float32)                   # the longest signal whose buffers stay
+        v.probs(line)
+        kept = fake.fake_device_bytes()
+        assert kept - small > line.size * 4
+        v.probs(line)
+        assert fake.fake_device_bytes() == kept
+        v.probs(np.zeros(keep // 4 + 64 * frame, np.float32))
+        assert fake.fake_device_bytes() <= small
+        assert fake.fake_device_peak() > kept
+        v.probs(np.zeros(3 * frame, np.float32))
+        # frames of few samples: the states have their own line
+    with closing(pkg.Vad(dict(cfg["vad"], frame_samples=64, context_samples=512), tensors)) as v:
+        before = fake.fake_device_bytes()
+        v.probs(np.zeros(64 * 140000, np.float32))
+        assert fake.fake_device_bytes() - before < (48 << 20)
+    assert fake.fake_device_bytes() == 0
 
 
 if __name__ == "__main__":
