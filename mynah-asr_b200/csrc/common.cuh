@@ -12,10 +12,12 @@ namespace mb {
 void set_error(const char *fmt, ...);
 const char *last_error();
 
+// (the error also comes off the thread: the next call's cudaGetLastError would report it as its own)
 #define MB_CUDA(call)                                                                    \
     do {                                                                                 \
         cudaError_t e_ = (call);                                                         \
         if (e_ != cudaSuccess) {                                                         \
+            cudaGetLastError();                                                          \
             mb::set_error("%s:%d %s -> %s", __FILE__, __LINE__, #call, cudaGetErrorString(e_)); \
             return -1;                                                                   \
         }                                                                                \
@@ -25,6 +27,7 @@ const char *last_error();
     do {                                                                                 \
         cudaError_t e_ = (call);                                                         \
         if (e_ != cudaSuccess) {                                                         \
+            cudaGetLastError();                                                          \
             mb::set_error("%s:%d %s -> %s", __FILE__, __LINE__, #call, cudaGetErrorString(e_)); \
             return nullptr;                                                              \
         }                                                                                \

@@ -9,7 +9,6 @@
 #include <functional>
 #include <map>
 #include <mutex>
-#include <set>
 #include <string>
 #include <vector>
 
@@ -19,7 +18,18 @@ using Lock = std::lock_guard<std::recursive_mutex>;
 std::map<void *, size_t> dev_mem;                        // live device allocations
 size_t dev_bytes = 0, dev_peak = 0;
 std::map<const void *, std::string> kernel_names;
-std::set<cudaStream_t> pending;                          // streams with work nobody has waited for
+// work issued to a stream and how much of it the host has waited for; what an event or a stream stands behind, by stream
+struct Stream { long long issued = 0, done = 0; };
+std::map<cudaStream_t, Stream> streams;
+typedef std::map<cudaStream_t, long long> Behind;
+std::map<cudaStream_t, Behind> stream_behind;
+std::map<cudaEvent_t, Behind> event_behind;
+void merge(Behind &a, const Behind &b) { for (auto &e : b) if (a[e.first] < e.second) a[e.first] = e.second; }
+void wait_all() { for (auto &s : streams) s.second.done = s.second.issued; }
+void wait_stream(cudaStream_t s) {
+    streams[s].done = streams[s].issued;
+    for (auto &e : stream_behind[s]) if (streams[e.first].done < e.second) streams[e.first].done = e.second;
+}
 std::map<cudaStream_t, std::vector<std::function<void()>>> capturing;
 std::map<std::string, long long> calls;
 std::string fail_name;                                   // the fail_at-th call of this function from now on fails
@@ -28,6 +38,7 @@ typedef void (*launch_cb)(const char *kernel, void **args, cudaStream_t st);
 typedef void (*hook_cb)();
 launch_cb on_launch = nullptr;
 hook_cb on_capture = nullptr;
+thread_local cudaError_t last_error = cudaSuccess;
 thread_local dim3 cfg_grid, cfg_block;
 thread_local size_t cfg_smem;
 thread_local cudaStream_t cfg_stream;
@@ -37,6 +48,7 @@ bool fails(const char *name) {
     calls[name]++;
     if (fail_name != name || --fail_at != 0) return false;
     fail_name.clear();
+    last_error = cudaErrorUnknown;
     return true;
 }
 template <typename T> T handle() { next_handle += 16; return reinterpret_cast<T>(next_handle); }
@@ -44,7 +56,7 @@ template <typename T> T handle() { next_handle += 16; return reinterpret_cast<T>
 template <typename F> cudaError_t work(cudaStream_t st, F f) {
     auto c = capturing.find(st);
     if (c != capturing.end()) { c->second.push_back(f); return cudaSuccess; }
-    pending.insert(st);
+    streams[st].issued++;
     f();
     return cudaSuccess;
 }
@@ -56,7 +68,7 @@ cudaError_t launch(const void *func, void **args, cudaStream_t st) {
         if (fails("cudaLaunchKernel")) return cudaErrorLaunchFailure;
         if (capturing.count(st)) capturing[st].push_back([] {});
         else {
-            pending.insert(st);
+            streams[st].issued++;
             if (on_launch) on_launch(kernel_names[func].c_str(), args, st);
         }
         if (capturing.count(st)) { hook = on_capture; on_capture = nullptr; }
@@ -75,7 +87,12 @@ void fake_reset() { Lock l(mu); calls.clear(); fail_name.clear(); fail_at = 0; d
 void fake_fail(const char *name, long long nth) { Lock l(mu); fail_name = name; fail_at = nth; }
 int fake_failed() { Lock l(mu); return fail_name.empty(); }
 long long fake_calls(const char *name) { Lock l(mu); return calls[name]; }
-int fake_pending() { Lock l(mu); return (int)pending.size(); }
+int fake_pending() {                                     // streams with work nobody has waited for
+    Lock l(mu);
+    int n = 0;
+    for (auto &s : streams) n += s.second.done < s.second.issued;
+    return n;
+}
 size_t fake_device_bytes() { Lock l(mu); return dev_bytes; }
 size_t fake_device_peak() { Lock l(mu); return dev_peak; }
 size_t fake_room(const void *p) {                        // bytes from p to the end of its allocation, 0 outside of all
@@ -100,11 +117,11 @@ cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
-    *v = a == cudaDevAttrComputeCapabilityMajor ? 10 : a == cudaDevAttrMultiProcessorCount ? 148 : 0;
+    *v = a == cudaDevAttrComputeCapabilityMajor ? 10 : a == cudaDevAttrMultiProcessorCount ? 148 : a == cudaDevAttrCooperativeLaunch ? 1 : 0;
     return cudaSuccess;
 }
-cudaError_t cudaDeviceSynchronize() { Lock l(mu); pending.clear(); return cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { Lock l(mu); wait_all(); return cudaSuccess; }
+cudaError_t cudaGetLastError() { const cudaError_t e = last_error; last_error = cudaSuccess; return e; }
 const char *cudaGetErrorString(cudaError_t) { return "an error of the fake runtime"; }
 cudaError_t cudaGetSymbolAddress(void **p, const void *) { *p = nullptr; return cudaErrorInvalidSymbol; }
 cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
@@ -130,7 +147,7 @@ cudaError_t cudaFree(void *p) {                          // waits for the device
     calls["cudaFree"]++;
     if (!p) return cudaSuccess;
     if (!dev_mem.count(p)) return cudaErrorInvalidValue;
-    pending.clear();
+    wait_all();
     dev_bytes -= dev_mem[p];
     dev_mem.erase(p);
     free(p);
@@ -160,16 +177,30 @@ cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t st) {
 
 // ---- streams and events
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { Lock l(mu); if (fails("cudaStreamCreate")) return cudaErrorMemoryAllocation; *s = handle<cudaStream_t>(); return cudaSuccess; }
-cudaError_t cudaStreamDestroy(cudaStream_t s) { Lock l(mu); pending.erase(s); return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { Lock l(mu); calls["cudaStreamSynchronize"]++; pending.erase(s); return cudaSuccess; }
-cudaError_t cudaStreamQuery(cudaStream_t s) { Lock l(mu); return pending.count(s) ? cudaErrorNotReady : cudaSuccess; }
-cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t, unsigned) { Lock l(mu); calls["cudaStreamWaitEvent"]++; return work(s, [] {}); }
+cudaError_t cudaStreamDestroy(cudaStream_t s) { Lock l(mu); streams.erase(s); stream_behind.erase(s); return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { Lock l(mu); calls["cudaStreamSynchronize"]++; wait_stream(s); return cudaSuccess; }
+cudaError_t cudaStreamQuery(cudaStream_t s) { Lock l(mu); return streams[s].done < streams[s].issued ? cudaErrorNotReady : cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) { Lock l(mu); calls["cudaStreamWaitEvent"]++; merge(stream_behind[s], event_behind[e]); return work(s, [] {}); }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { Lock l(mu); if (fails("cudaEventCreate")) return cudaErrorMemoryAllocation; *e = handle<cudaEvent_t>(); return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t s) { Lock l(mu); if (fails("cudaEventRecord")) return cudaErrorInvalidValue; return work(s, [] {}); }
-cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    Lock l(mu);
+    if (fails("cudaEventRecord")) return cudaErrorInvalidValue;
+    event_behind[e] = stream_behind[s];
+    event_behind[e][s] = streams[s].issued;
+    return cudaSuccess;
+}
+cudaError_t cudaEventQuery(cudaEvent_t e) {
+    Lock l(mu);
+    for (auto &b : event_behind[e]) if (streams.count(b.first) && streams[b.first].done < b.second) return cudaErrorNotReady;
+    return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    Lock l(mu);
+    for (auto &b : event_behind[e]) if (streams.count(b.first) && streams[b.first].done < b.second) streams[b.first].done = b.second;
+    return cudaSuccess;
+}
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { *ms = 1.f; return cudaSuccess; }
 
 // ---- launches and graphs
@@ -190,7 +221,7 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) { Lock l(mu); calls["cudaGra
 cudaError_t cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t s) {
     Lock l(mu);
     if (fails("cudaGraphLaunch")) return cudaErrorInvalidValue;
-    pending.insert(s);
+    streams[s].issued++;
     for (auto &f : execs[x]) f();
     return cudaSuccess;
 }

@@ -33,7 +33,7 @@ def fake_runtime(tmp_path_factory, pkg):
 
 
 @pytest.mark.parametrize("name", [
-    "vad_allocation_fails", "vad_gives_back",
+    "vad_allocation_fails", "vad_gives_back", "error_is_reported_once",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -116,6 +116,68 @@ def vad_gives_back(pkg, synth, fake):
         v.probs(np.zeros(64 * 140000, np.float32))
         assert fake.fake_device_bytes() - before < (48 << 20)
     assert fake.fake_device_bytes() == 0
+
+
+def _small_calls(pkg, synth):
+    """Calls that between them reach the front end's groups, the decoder's lanes, the attention decoder and the streams."""
+    import cases
+    rng = np.random.default_rng(0)
+    audio = [rng.standard_normal(16000 * s).astype(np.float32) for s in (2, 61, 1)]      # two groups of the front end
+    feats = [rng.standard_normal((t, 80), dtype=np.float32) for t in (200, 6100, 90)]
+    models = {}
+    for name in ("tdt_q4", "ctc_q8", "aed_same", "rnnt_kq"):
+        cfg, tensors = cases.build(synth, name)
+        models[name] = cases.device_model(pkg, synth, cfg, tensors, **({"aed_heads": cfg.aed_heads} if name == "aed_same" else {}))
+
+    def stream():
+        with closing(models["rnnt_kq"].stream_open(2, 5, 1)) as g:
+            for i in range(8):
+                g.step_decode(np.zeros((2, g.need(), 128), np.float32))
+
+    return {
+        "transcribe": lambda: models["tdt_q4"].transcribe_batch(audio * 6),              # two decoder groups
+        "encoder": lambda: models["ctc_q8"].encoder_forward_batch(feats),
+        "aed": lambda: models["aed_same"].transcribe_batch_aed(audio[:1], cases.AED_PROMPT, -1, 5),
+        "stream": stream,
+    }
+
+
+def _each_failure(pkg, synth, fake, functions, after):
+    """Every call with the first, some and the last of its calls of each device function failing; after(what) follows."""
+    for what, call in _small_calls(pkg, synth).items():
+        call()                                                                           # streams, events, attributes
+        for f in functions:
+            fake.fake_reset()
+            call()
+            n = fake.fake_calls(f)
+            for nth in sorted({1, 2, 3, 5, 8, n // 2, n - 1, n} & set(range(1, n + 1))):
+                fake.fake_fail(f, nth)
+                try:
+                    call()
+                    raise AssertionError((what, f, nth, "did not fail"))
+                except pkg.BackendError:
+                    assert fake.fake_failed()
+                after((what, f, nth), call)
+
+
+ASYNC = (b"cudaMemcpyAsync", b"cudaMemsetAsync", b"cudaEventRecord", b"cudaLaunchKernel")
+
+
+@scenario
+def error_is_reported_once(pkg, synth, fake):
+    """The error of a failed device call is that call's: the next call on the thread does not find it again."""
+    _each_failure(pkg, synth, fake, ASYNC, lambda what, call: call())
+    import cases
+    cfg, tensors = cases.build(synth, "ctc_q8")
+    with closing(cases.device_model(pkg, synth, cfg, tensors)) as m:
+        for f in (b"cudaMalloc", b"cudaMallocHost", b"cudaStreamCreate"):                # workspace, tables, copy stream
+            fake.fake_fail(f, 1)
+            try:
+                m.transcribe_batch([np.zeros(16000, np.float32)], decoder=1)
+                raise AssertionError((f, "did not fail"))
+            except pkg.BackendError:
+                assert fake.fake_failed()
+        m.transcribe_batch([np.zeros(16000, np.float32)], decoder=1)
 
 
 if __name__ == "__main__":
