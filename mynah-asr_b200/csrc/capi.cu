@@ -60,6 +60,7 @@ public:
         h->busy[(size_t)idx_] = 1;
     }
     ~Lease() {
+        model().settle();
         { std::lock_guard<std::mutex> lk(h_->pool_mu); h_->busy[(size_t)idx_] = 0; }
         h_->pool_cv.notify_all();
     }

@@ -86,6 +86,18 @@ int Model::lanes_join(int lanes) {
     }
     return 0;
 }
+void Model::settle() {
+    bool left = false;
+    auto wait = [&](cudaStream_t s) { if (s && cudaStreamQuery(s) != cudaSuccess) { cudaStreamSynchronize(s); left = true; } };
+    wait(copy);
+    for (cudaStream_t s : lane) wait(s);
+    wait(stream);
+    if (!left) return;
+    // what the abandoned kernels reported is not the next call's
+    cudaMemsetAsync(status, 0, sizeof(int), stream);
+    cudaStreamSynchronize(stream);
+    cudaGetLastError();
+}
 void Model::release_load_buffers() {
     for (int i = 0; i < 2; i++) {
         if (stage_ev[i]) { cudaEventSynchronize(stage_ev[i]); cudaEventDestroy(stage_ev[i]); stage_ev[i] = nullptr; }

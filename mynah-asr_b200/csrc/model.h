@@ -215,6 +215,9 @@ struct Model {
     int lanes_begin(int n_groups);                   // lanes in use (1 = everything stays on `stream`); forks them off `stream`
     cudaStream_t lane_stream(int lanes, int gi) const { return lanes > 1 ? lane[gi % lanes] : stream; }
     int lanes_join(int lanes);                       // `stream` waits for every lane
+    // Waits for what a call left on the context's streams. One that succeeded leaves nothing; one that failed on the way may
+    // leave copies out of its caller's memory and kernels on the arena that the next call lays out anew.
+    void settle();
 
     ~Model();
     void *dev_alloc(size_t bytes);

@@ -33,7 +33,7 @@ def fake_runtime(tmp_path_factory, pkg):
 
 
 @pytest.mark.parametrize("name", [
-    "vad_allocation_fails", "vad_gives_back", "error_is_reported_once",
+    "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -178,6 +178,16 @@ def error_is_reported_once(pkg, synth, fake):
             except pkg.BackendError:
                 assert fake.fake_failed()
         m.transcribe_batch([np.zeros(16000, np.float32)], decoder=1)
+
+
+@scenario
+def failed_call_waits(pkg, synth, fake):
+    """A call that fails anywhere returns with nothing in flight: neither copies out of the caller's memory nor kernels on
+    the workspace that the next call lays out anew."""
+    def idle(what, call):
+        assert fake.fake_pending() == 0, what
+
+    _each_failure(pkg, synth, fake, ASYNC, idle)
 
 
 if __name__ == "__main__":
