@@ -1376,13 +1376,12 @@ int mynah_b200_qmat_mul(const mynah_b200_qmat *q, const float *x, float *out, in
             g->T = T; g->flags = flags;
         }
         if (++g->uses == 2) {
-            const long long before = launch_count(false);
+            LaunchRecord record;
             cudaGraph_t rec = nullptr;
             if (cudaStreamBeginCapture(q->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
                 const int rc = issue();
                 const cudaError_t e = cudaStreamEndCapture(q->stream, &rec);
-                g->launches = (int)(launch_count(false) - before);
-                note_launch(-g->launches);                       // recorded, not launched
+                g->launches = record.launches;
                 if (rc || e != cudaSuccess || !rec || cudaGraphInstantiate(&g->exec, rec, 0) != cudaSuccess) g->exec = nullptr;
                 if (rec) cudaGraphDestroy(rec);
             }

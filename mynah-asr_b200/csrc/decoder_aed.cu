@@ -553,8 +553,8 @@ int Model::decode_aed(const float *enc_dev, const std::vector<int> &lens, const 
                 const bool was_on = prof_on;
                 prof_on = false;                             // no event records inside the capture
                 if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-                    const int prc = position();
-                    note_launch(-gemms_per_position);        // recorded, not launched
+                    int prc;
+                    { LaunchRecord record; prc = position(); }
                     cudaGraph_t g = nullptr;
                     const cudaError_t e = cudaStreamEndCapture(stream, &g);
                     if (prc == 0 && e == cudaSuccess && g && cudaGraphInstantiate(&exec, g, 0) == cudaSuccess) graph = g;

@@ -120,6 +120,14 @@ int align_ctc_device(const float *scores_dev, int T, int V, const int *tokens, i
 // ---- launch accounting (model.cu): every kernel launch of the library is counted
 void note_launch(int n = 1);
 long long launch_count(bool reset);
+// While one lives, what its thread notes is recorded into a graph: counted here, and by the process at every launch of the graph.
+struct LaunchRecord {
+    int launches = 0;
+    LaunchRecord();
+    ~LaunchRecord();
+    LaunchRecord(const LaunchRecord &) = delete;
+    LaunchRecord &operator=(const LaunchRecord &) = delete;
+};
 
 // ---- decoder.cu
 int argmax_rows(const float *logits, int ld, const float *bias, int T, int V, int *best, cudaStream_t st, bool chain = false);

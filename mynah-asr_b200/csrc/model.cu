@@ -13,7 +13,13 @@
 namespace mb {
 
 static std::atomic<long long> g_launches{0};
-void note_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+static thread_local LaunchRecord *t_record = nullptr;
+void note_launch(int n) {
+    if (t_record) t_record->launches += n;
+    else g_launches.fetch_add(n, std::memory_order_relaxed);
+}
+LaunchRecord::LaunchRecord() { t_record = this; }
+LaunchRecord::~LaunchRecord() { t_record = nullptr; }
 long long launch_count(bool reset) { return reset ? g_launches.exchange(0) : g_launches.load(); }
 
 // -------------------------------------------------------------------- arena

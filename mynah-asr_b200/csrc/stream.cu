@@ -328,14 +328,16 @@ int Model::stream_step(StreamState &st, const float *mel, int n_mel, int is_last
         if (st.exec) { cudaGraphExecDestroy(st.exec); cudaGraphDestroy(st.graph); st.exec = nullptr; st.graph = nullptr; }
         return stream_step_eager(st, mel, n_mel, is_last, out);
     }
-    const long long before = launch_count(false);
     if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); return stream_step_eager(st, mel, n_mel, is_last, out); }
     const size_t mark = ws.off;
-    const int q = stream_step_eager(st, mel, n_mel, is_last, out);
+    int q, recorded;
+    {
+        LaunchRecord record;
+        q = stream_step_eager(st, mel, n_mel, is_last, out);
+        recorded = record.launches;
+    }
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(stream, &g);
-    const int recorded = (int)(launch_count(false) - before);
-    note_launch(-recorded);                                  // recorded, not launched
     if (q < 0 || e != cudaSuccess || !g || cudaGraphInstantiate(&st.exec, g, 0) != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         st.exec = nullptr;

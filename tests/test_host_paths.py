@@ -33,7 +33,7 @@ def fake_runtime(tmp_path_factory, pkg):
 
 
 @pytest.mark.parametrize("name", [
-    "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits",
+    "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -188,6 +188,51 @@ def failed_call_waits(pkg, synth, fake):
         assert fake.fake_pending() == 0, what
 
     _each_failure(pkg, synth, fake, ASYNC, idle)
+
+
+@scenario
+def launches_of_other_threads(pkg, synth, fake):
+    """A thread that records a graph takes its own launches out of the count, not those of the threads beside it."""
+    import threading
+    import cases
+    w = np.ones((64, 128), np.float32)
+    x = np.ones((3, 128), np.float32)
+    beside = pkg.QMat(pkg.F32, w, 64, 128)
+    beside.mul(x)
+
+    def count(call, during=0):
+        hits = []
+
+        def hook():
+            t = threading.Thread(target=lambda: [beside.mul(np.ones((100, 128), np.float32)) for _ in range(during)])
+            t.start()
+            t.join()
+            hits.append(1)
+
+        cb = HOOK(hook)
+        fake.fake_on_capture(cb)
+        before = pkg.launch_count()
+        call()
+        fake.fake_on_capture(HOOK(0))
+        assert hits, "nothing was recorded"
+        return pkg.launch_count() - before
+
+    before = pkg.launch_count()
+    beside.mul(np.ones((100, 128), np.float32))
+    one = pkg.launch_count() - before
+    assert one > 0
+
+    def products():
+        with closing(pkg.QMat(pkg.F32, w, 64, 128)) as q:
+            for _ in range(4):
+                q.mul(x)
+
+    calls = _small_calls(pkg, synth)
+    cfg = synth.config("aed_f32", **dict(cases.AED["aed_same"], wtype="f32"))            # no tiles: a graph per position
+    aed = cases.device_model(pkg, synth, cfg, synth.make_model(cfg, seed=1), aed_heads=cfg.aed_heads)
+    for call in (products, calls["stream"], lambda: aed.aed_decode(np.ones((9, 128), np.float32), (1, 2), -1, 9)):
+        call()                                                                           # buffers
+        assert count(call, 3) == count(call) + 3 * one
 
 
 if __name__ == "__main__":
