@@ -4,6 +4,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
 #include <chrono>
 #include <condition_variable>
 #include <memory>
@@ -97,29 +98,32 @@ void with_all_contexts_idle(mynah_b200_model *h, F fn) {
     for (int i = 0; i < h->n_ctx(); i++) fn(h->ctx(i));
 }
 }  // namespace
-// A resident weight and the buffers of its products. Allocating them per call cost 0.48 ms of a 16 us product: the
-// stream-ordered pool gives its memory back at every synchronisation and maps it anew at the next allocation.
-//   block  device [status, 256 B | QMAT_SMALL out | QMAT_SMALL x], pinned twin `host`: small calls move the rows in with
-//          one copy and the result with the status word out with one copy
-//   ws     device workspace of larger calls, kept up to QMAT_KEEP bytes (a larger one is freed when its call ends)
-// One lock per handle: products of one weight share these and run one after the other on the handle's stream.
+// A resident weight and what its products need.
+//   block  device [status, 256 B | QMAT_SMALL out | QMAT_SMALL x | temporaries of that x]: a small call moves its rows in with
+//          one copy and the result with the status word out with one copy, through a pinned twin
+// Anything larger comes from the workspaces that all handles of a device share (WorkspacePool). Allocating it per call
+// cost 0.48 ms of a 16 us product: the stream-ordered pool gives its memory back at every synchronisation and maps it anew at
+// the next allocation; a workspace per handle moves that cost into the first product of each of a model's linears (187 rows
+// of [1024 x 4096]: 680 us instead of 309).
+// One lock per handle: products of one weight share the block and run one after the other on the handle's stream.
 struct mynah_b200_qmat {
     QWeight w;
     std::vector<void *> owned;
     cudaStream_t stream = nullptr;
     int *status = nullptr;               // = the first word of the block
+    int device = 0;
+    uint64_t id = 0;                     // never used again, unlike an address or a stream
     mutable std::mutex mu;
-    mutable uint8_t *host = nullptr;     // from the pinned pool, taken by the first call
-    mutable uint8_t *ws = nullptr;
-    mutable size_t ws_cap = 0;
+    mutable uint8_t *host = nullptr;     // the block's pinned twin, once a graph names it; until then a call borrows one
     // A small call repeated with the same rows and flags is one graph (copy in, kernels, copy out): issuing its four or five
     // pieces one by one took longer than running them. Recorded on the second such call, kept for the last few.
     struct Graph { int T = 0, flags = 0, uses = 0, launches = 0; cudaGraphExec_t exec = nullptr; };
     mutable Graph graphs[4];
     mutable int graph_next = 0;
-    void drop_graphs() const { for (Graph &g : graphs) { if (g.exec) cudaGraphExecDestroy(g.exec); g = Graph(); } }
 };
-static constexpr size_t QMAT_HEAD = 256, QMAT_SMALL = 128 << 10, QMAT_BLOCK = QMAT_HEAD + 2 * QMAT_SMALL;
+static constexpr size_t QMAT_HEAD = 256, QMAT_SMALL = 128 << 10;
+static constexpr size_t QMAT_TEMP_AT = QMAT_HEAD + 2 * QMAT_SMALL, QMAT_TEMP = QMAT_SMALL + 512;   // two fp16 planes of x, aligned
+static constexpr size_t QMAT_PINNED = QMAT_TEMP_AT, QMAT_BLOCK = QMAT_TEMP_AT + QMAT_TEMP;
 static constexpr size_t QMAT_KEEP = 64 << 20;
 struct mynah_b200_batch {
     int batch = 0;
@@ -146,8 +150,8 @@ QmatView qmat_view(const void *handle) {
 }  // namespace mb
 
 namespace {
-// Pinned twins of the handles' blocks. Pinning costs more than a product, so up to POOL_MAX blocks outlive their handle
-// and serve the next one.
+// Pinned twins of the handles' blocks. Pinning costs more than a product, so up to POOL_MAX free ones (8 MB) stay, for the
+// next call that borrows one and beyond the handles.
 class PinnedPool {
 public:
     uint8_t *take() {
@@ -156,7 +160,7 @@ public:
             if (!free_.empty()) { uint8_t *p = free_.back(); free_.pop_back(); return p; }
         }
         void *p = nullptr;
-        if (cudaHostAlloc(&p, QMAT_BLOCK, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        if (cudaHostAlloc(&p, QMAT_PINNED, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
         return (uint8_t *)p;
     }
     void give(uint8_t *p) {
@@ -175,34 +179,120 @@ private:
 };
 PinnedPool &pinned_pool() { static PinnedPool *p = new PinnedPool(); return *p; }   // alive until the process ends
 
-// `bytes` of device workspace on a handle whose lock is held: the kept one, or (above QMAT_KEEP) a stream-ordered
-// allocation that ends with the call.
+// The pinned twin for one call: the handle's own, or one that goes back when the call ends (it has waited for its stream by
+// then) unless a graph has come to name it.
+class PinnedTwin {
+public:
+    explicit PinnedTwin(const mynah_b200_qmat *q) : q_(q), p_(q->host ? q->host : pinned_pool().take()) {}
+    ~PinnedTwin() { if (p_ != q_->host) pinned_pool().give(p_); }
+    uint8_t *get() const { return p_; }
+    void keep() { q_->host = p_; }
+    PinnedTwin(const PinnedTwin &) = delete;
+    PinnedTwin &operator=(const PinnedTwin &) = delete;
+
+private:
+    const mynah_b200_qmat *q_;
+    uint8_t *p_;
+};
+
+// Device workspaces of the products, shared by the handles of a device. A call takes a block for as long as it issues work
+// and gives it back with an event behind that work; whoever takes it next waits for the event on its own stream (the same
+// handle need not: its products share a stream). A block whose work has finished goes first, then a fresh one while fewer than
+// KEEP_BLOCKS are free, so that products of several handles still overlap. Free blocks are at most KEEP_BLOCKS per device, of
+// at most QMAT_KEEP bytes each, and all go when the device's last handle does.
+struct Workspace { uint8_t *p = nullptr; size_t cap = 0; int device = 0; uint64_t user = 0; cudaEvent_t done = nullptr; };
+class WorkspacePool {
+public:
+    int handle_made() { const int dev = current(); std::lock_guard<std::mutex> lk(mu_); handles_[dev]++; return dev; }
+    void handle_gone(int dev) {
+        std::vector<Workspace> drop;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (--handles_[dev] > 0) return;
+            for (size_t i = 0; i < free_.size();)
+                if (free_[i].device == dev) { drop.push_back(free_[i]); free_.erase(free_.begin() + i); } else i++;
+        }
+        for (Workspace &w : drop) destroy(w);
+    }
+    // Workspace::p is null on failure
+    Workspace take(size_t bytes, uint64_t user, cudaStream_t st) {
+        Workspace w;
+        w.device = current();
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            int best = -1, waits = -1, here = 0;
+            for (int i = 0; i < (int)free_.size(); i++) {
+                const Workspace &f = free_[(size_t)i];
+                if (f.device != w.device) continue;
+                here++;
+                if (f.cap < bytes) continue;
+                int &pick = f.user == user || cudaEventQuery(f.done) == cudaSuccess ? best : waits;
+                if (pick < 0 || f.cap < free_[(size_t)pick].cap) pick = i;
+            }
+            cudaGetLastError();                                  // "not ready" is noted as an error
+            if (best < 0 && here >= KEEP_BLOCKS) best = waits;
+            if (best >= 0) { w = free_[(size_t)best]; free_.erase(free_.begin() + best); }
+        }
+        if (w.p) {
+            if (w.user != user && cudaStreamWaitEvent(st, w.done, 0) != cudaSuccess) { cudaGetLastError(); cudaEventSynchronize(w.done); }
+            return w;
+        }
+        w.cap = 1 << 20;
+        while (w.cap < bytes) w.cap <<= 1;
+        if (cudaEventCreateWithFlags(&w.done, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); return Workspace(); }
+        if (cudaMalloc((void **)&w.p, w.cap) != cudaSuccess) { cudaGetLastError(); cudaEventDestroy(w.done); return Workspace(); }
+        return w;
+    }
+    void give(Workspace w, uint64_t user, cudaStream_t st) {
+        w.user = user;
+        if (cudaEventRecord(w.done, st) != cudaSuccess) { cudaGetLastError(); cudaStreamSynchronize(st); destroy(w); return; }
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            free_.push_back(w);
+            int here = 0;
+            size_t least = free_.size() - 1;
+            for (size_t i = 0; i < free_.size(); i++)
+                if (free_[i].device == w.device) { here++; if (free_[i].cap < free_[least].cap) least = i; }
+            if (here <= KEEP_BLOCKS) return;
+            w = free_[least];
+            free_.erase(free_.begin() + (long)least);
+        }
+        destroy(w);
+    }
+
+private:
+    static constexpr int KEEP_BLOCKS = 4;
+    static int current() { int d = 0; if (cudaGetDevice(&d) != cudaSuccess) cudaGetLastError(); return d; }
+    static void destroy(Workspace &w) { cudaEventSynchronize(w.done); cudaEventDestroy(w.done); cudaFree(w.p); cudaGetLastError(); }
+    std::mutex mu_;
+    std::vector<Workspace> free_;
+    std::map<int, int> handles_;
+};
+WorkspacePool &workspace_pool() { static WorkspacePool *p = new WorkspacePool(); return *p; }   // alive until the process ends
+
+// `bytes` of device workspace for what a call issues on a handle whose lock is held: a shared block, or (above QMAT_KEEP) a
+// stream-ordered allocation that ends with the call.
 class QmatScratch {
 public:
     QmatScratch(const mynah_b200_qmat *q, size_t bytes) : q_(q) {
-        if (bytes <= q->ws_cap) { p_ = q->ws; return; }
+        if (bytes == 0) return;
         if (bytes > QMAT_KEEP) {
             if (cudaMallocAsync(&own_, bytes, q->stream) != cudaSuccess) { cudaGetLastError(); own_ = nullptr; }
-            p_ = (uint8_t *)own_;
-            return;
+        } else {
+            ws_ = workspace_pool().take(bytes, q->id, q->stream);
         }
-        q->drop_graphs();                                        // they hold the old address
-        if (q->ws) cudaFree(q->ws);                              // waits for the products that use it
-        q->ws = nullptr; q->ws_cap = 0;
-        size_t cap = 1 << 20;
-        while (cap < bytes) cap <<= 1;
-        if (cudaMalloc((void **)&q->ws, cap) != cudaSuccess) { cudaGetLastError(); q->ws = nullptr; return; }
-        q->ws_cap = cap;
-        p_ = q->ws;
     }
-    ~QmatScratch() { if (own_) cudaFreeAsync(own_, q_->stream); }
-    uint8_t *get() const { return p_; }
+    ~QmatScratch() {
+        if (own_) cudaFreeAsync(own_, q_->stream);
+        if (ws_.p) workspace_pool().give(ws_, q_->id, q_->stream);
+    }
+    uint8_t *get() const { return own_ ? (uint8_t *)own_ : ws_.p; }
     QmatScratch(const QmatScratch &) = delete;
     QmatScratch &operator=(const QmatScratch &) = delete;
 
 private:
     const mynah_b200_qmat *q_;
-    uint8_t *p_ = nullptr;
+    Workspace ws_;
     void *own_ = nullptr;
 };
 }  // namespace
@@ -1242,17 +1332,21 @@ mynah_b200_qmat *mynah_b200_qmat_create(int fmt, const void *data, const float *
     q->owned.swap(tmp.owned);
     q->stream = tmp.stream;
     tmp.stream = nullptr;
+    static std::atomic<uint64_t> last_id{0};
+    q->id = ++last_id;
+    q->device = workspace_pool().handle_made();
     return q;
 }
 
 void mynah_b200_qmat_free(mynah_b200_qmat *q) {
     if (!q) return;
-    q->drop_graphs();
+    const int device = q->device;
+    for (mynah_b200_qmat::Graph &g : q->graphs) if (g.exec) cudaGraphExecDestroy(g.exec);
     for (void *p : q->owned) cudaFree(p);                       // waits for the handle's products
-    if (q->ws) cudaFree(q->ws);
     if (q->stream) cudaStreamDestroy(q->stream);
     pinned_pool().give(q->host);
     delete q;
+    workspace_pool().handle_gone(device);
 }
 
 // device bytes of temporaries that a product of T rows needs beside its input and output
@@ -1270,9 +1364,10 @@ int mynah_b200_qmat_mul_device(const mynah_b200_qmat *q, const float *x, float *
     if (T == 0) return 0;
     std::lock_guard<std::mutex> lk(q->mu);
     const size_t bytes = qmat_temp_bytes(q->w, T, flags);
-    QmatScratch s(q, bytes);
-    if (bytes && !s.get()) { set_error("qmat_mul: device allocation failed"); return -1; }
-    return qmat_mul_locked(q, x, out, T, flags, s.get());
+    const bool in_block = bytes <= QMAT_TEMP;
+    QmatScratch s(q, in_block ? 0 : bytes);
+    if (!in_block && !s.get()) { set_error("qmat_mul: device allocation failed"); return -1; }
+    return qmat_mul_locked(q, x, out, T, flags, in_block ? (uint8_t *)q->status + QMAT_TEMP_AT : s.get());
 }
 
 static int qmat_mul_locked(const mynah_b200_qmat *q, const float *x, float *out, int T, int flags, uint8_t *temp) {
@@ -1346,22 +1441,27 @@ int mynah_b200_qmat_mul(const mynah_b200_qmat *q, const float *x, float *out, in
     if (!q || !x || !out || T < 0) { set_error("qmat_mul: bad argument"); return -1; }
     if (T == 0) return 0;
     std::lock_guard<std::mutex> lk(q->mu);
-    if (!q->host && !(q->host = pinned_pool().take())) { set_error("qmat_mul: host allocation failed"); return -1; }
+    PinnedTwin twin(q);
+    uint8_t *host = twin.get();
+    if (!host) { set_error("qmat_mul: host allocation failed"); return -1; }
     const size_t nx = (size_t)T * q->w.k * 4, no = (size_t)T * q->w.n * 4;
     uint8_t *block = (uint8_t *)q->status;
     const bool small_x = nx <= QMAT_SMALL, small_out = no <= QMAT_SMALL;
-    const size_t nt = align_up(qmat_temp_bytes(q->w, T, flags), 256), nxw = small_x ? 0 : align_up(nx, 256);
-    QmatScratch s(q, nt + nxw + (small_out ? 0 : no));
-    if (nt + nxw + (small_out ? 0 : no) && !s.get()) { set_error("qmat_mul: device allocation failed"); return -1; }
+    // small rows and their temporaries (their planes take as much as they do) have a place in the handle's block
+    const size_t nt = small_x ? 0 : align_up(qmat_temp_bytes(q->w, T, flags), 256), nxw = small_x ? 0 : align_up(nx, 256);
+    const size_t shared = nt + nxw + (small_out ? 0 : no);
+    QmatScratch s(q, shared);
+    if (shared && !s.get()) { set_error("qmat_mul: device allocation failed"); return -1; }
     float *xd = (float *)(small_x ? block + QMAT_HEAD + QMAT_SMALL : s.get() + nt);
     float *od = (float *)(small_out ? block + QMAT_HEAD : s.get() + nt + nxw);
+    uint8_t *temp = small_x ? block + QMAT_TEMP_AT : s.get();
     const void *src = x;
-    if (small_x) src = memcpy(q->host + QMAT_HEAD + QMAT_SMALL, x, nx);
+    if (small_x) src = memcpy(host + QMAT_HEAD + QMAT_SMALL, x, nx);
     auto issue = [&]() -> int {
         if (cudaMemcpyAsync(xd, src, nx, cudaMemcpyHostToDevice, q->stream) != cudaSuccess) { cudaGetLastError(); set_error("qmat_mul: H2D copy failed"); return -1; }
-        if (qmat_mul_locked(q, xd, od, T, flags, s.get())) return -1;
+        if (qmat_mul_locked(q, xd, od, T, flags, temp)) return -1;
         bool ok = small_out || cudaMemcpyAsync(out, od, no, cudaMemcpyDeviceToHost, q->stream) == cudaSuccess;
-        ok = cudaMemcpyAsync(q->host, block, QMAT_HEAD + (small_out ? no : 0), cudaMemcpyDeviceToHost, q->stream) == cudaSuccess && ok;
+        ok = cudaMemcpyAsync(host, block, QMAT_HEAD + (small_out ? no : 0), cudaMemcpyDeviceToHost, q->stream) == cudaSuccess && ok;
         if (!ok) { cudaGetLastError(); set_error("qmat_mul: D2H copy failed"); return -1; }
         return 0;
     };
@@ -1383,6 +1483,7 @@ int mynah_b200_qmat_mul(const mynah_b200_qmat *q, const float *x, float *out, in
                 const cudaError_t e = cudaStreamEndCapture(q->stream, &rec);
                 g->launches = record.launches;
                 if (rc || e != cudaSuccess || !rec || cudaGraphInstantiate(&g->exec, rec, 0) != cudaSuccess) g->exec = nullptr;
+                if (g->exec) twin.keep();
                 if (rec) cudaGraphDestroy(rec);
             }
             cudaGetLastError();
@@ -1398,8 +1499,8 @@ int mynah_b200_qmat_mul(const mynah_b200_qmat *q, const float *x, float *out, in
     }
     if (cudaStreamSynchronize(q->stream) != cudaSuccess) { cudaGetLastError(); set_error("qmat_mul: a copy or kernel failed"); return -1; }
     if (rc) return rc;
-    if (qmat_status(q, *(const int *)q->host)) return -1;
-    if (small_out) memcpy(out, q->host + QMAT_HEAD, no);
+    if (qmat_status(q, *(const int *)host)) return -1;
+    if (small_out) memcpy(out, host + QMAT_HEAD, no);
     return 0;
 }
 

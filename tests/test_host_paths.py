@@ -33,7 +33,7 @@ def fake_runtime(tmp_path_factory, pkg):
 
 
 @pytest.mark.parametrize("name", [
-    "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads",
+    "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads", "qmat_workspace_is_shared",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -233,6 +233,57 @@ def launches_of_other_threads(pkg, synth, fake):
     for call in (products, calls["stream"], lambda: aed.aed_decode(np.ones((9, 128), np.float32), (1, 2), -1, 9)):
         call()                                                                           # buffers
         assert count(call, 3) == count(call) + 3 * one
+
+
+@scenario
+def qmat_workspace_is_shared(pkg, synth, fake):
+    """Handles share the workspace of their products: the first product of a handle allocates nothing that another handle
+    has allocated, memory does not grow with the handles that were used, and the last handle gives it back. Products that
+    may overlap on the device have blocks of their own, or wait for one another there."""
+    n, k, rows = 128, 512, 600                               # 2.7 MB of rows, planes and results
+    w = np.ones((n, k), np.float32)
+    x = np.ones((rows, k), np.float32)
+    handles = [pkg.QMat(pkg.F32, w, n, k) for _ in range(12)]
+    created = fake.fake_device_bytes()
+    handles[0].mul(x)
+    handles[0].mul(x[:2])
+    used = fake.fake_device_bytes() - created
+    fake.fake_reset()
+    for q in handles[1:]:
+        q.mul(x)
+        q.mul(x[:2])                                         # (a small call, the first with these rows: not a graph yet)
+    assert fake.fake_device_bytes() - created == used <= 4 << 20
+    for f in (b"cudaMalloc", b"cudaFree", b"cudaHostAlloc"):
+        assert fake.fake_calls(f) == 0, f
+
+    planes = []
+    cb = LAUNCH(lambda name, args, stream: planes.append(_arg(args, 1, C.c_void_p)) if b"split" in name else None)
+    fake.fake_on_launch(cb)
+    L = pkg.lib()
+    L.mynah_b200_qmat_mul_device.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int]
+    xd, od = np.ones((rows, k), np.float32), np.ones((rows, n), np.float32)
+
+    def device(q):
+        fake.fake_reset()
+        assert L.mynah_b200_qmat_mul_device(q.h, xd.ctypes.data, od.ctypes.data, rows, 0) == 0
+        return planes[-1], fake.fake_calls(b"cudaStreamWaitEvent")
+
+    busy = set()
+    for q in handles[:8]:                                    # nothing waits for them on the host
+        block, waits = device(q)
+        assert block not in busy or waits, "a block in use was handed to another stream without a wait"
+        busy.add(block)
+    assert 1 < len(busy) <= 4
+    block, waits = device(handles[7])                        # its own work is in order on its stream
+    assert block in busy and not waits
+    assert fake.fake_device_bytes() - created <= 4 * (4 << 20)
+    for q in handles[:8]:
+        assert L.mynah_b200_qmat_sync(q.h) == 0
+    for q in handles:
+        q.mul(x)
+    for i, q in enumerate(handles):
+        q.close()
+    assert fake.fake_device_bytes() == 0
 
 
 if __name__ == "__main__":
