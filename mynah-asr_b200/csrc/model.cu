@@ -607,9 +607,10 @@ const uint8_t *Model::fr_tiles(const std::vector<const QWeight *> &parts, bool g
 int Model::fr_upload(std::vector<uint8_t> &have, uint8_t *dev, const std::vector<uint8_t> &want) {
     if (have == want) return 0;
     if (!copy) MB_CUDA(cudaStreamCreateWithFlags(&copy, cudaStreamNonBlocking));
-    have = want;
-    MB_CUDA(cudaMemcpyAsync(dev, have.data(), have.size(), cudaMemcpyHostToDevice, copy));
+    have.clear();                                            // until the device has it
+    MB_CUDA(cudaMemcpyAsync(dev, want.data(), want.size(), cudaMemcpyHostToDevice, copy));
     MB_CUDA(cudaStreamSynchronize(copy));
+    have = want;
     return 0;
 }
 

@@ -34,7 +34,7 @@ std::map<cudaStream_t, std::vector<std::function<void()>>> capturing;
 std::map<std::string, long long> calls;
 std::string fail_name;                                   // the fail_at-th call of this function from now on fails
 long long fail_at = 0;
-typedef void (*launch_cb)(const char *kernel, void **args, cudaStream_t st);
+typedef void (*launch_cb)(const char *kernel, void **args, int recorded);   // kernel "": a graph is launched
 typedef void (*hook_cb)();
 launch_cb on_launch = nullptr;
 hook_cb on_capture = nullptr;
@@ -60,18 +60,17 @@ template <typename F> cudaError_t work(cudaStream_t st, F f) {
     f();
     return cudaSuccess;
 }
-// kernel arguments live on the caller's stack: a recorded launch is not shown again
+// kernel arguments live on the caller's stack: a recorded launch is shown when it is recorded
 cudaError_t launch(const void *func, void **args, cudaStream_t st) {
     hook_cb hook = nullptr;
     {
         Lock l(mu);
         if (fails("cudaLaunchKernel")) return cudaErrorLaunchFailure;
-        if (capturing.count(st)) capturing[st].push_back([] {});
-        else {
-            streams[st].issued++;
-            if (on_launch) on_launch(kernel_names[func].c_str(), args, st);
-        }
-        if (capturing.count(st)) { hook = on_capture; on_capture = nullptr; }
+        const bool recorded = capturing.count(st) != 0;
+        if (recorded) capturing[st].push_back([] {});
+        else streams[st].issued++;
+        if (on_launch) on_launch(kernel_names[func].c_str(), args, recorded);
+        if (recorded) { hook = on_capture; on_capture = nullptr; }
     }
     if (hook) hook();                                    // once, in the middle of a capture, outside the lock
     return cudaSuccess;
@@ -222,6 +221,7 @@ cudaError_t cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t s) {
     Lock l(mu);
     if (fails("cudaGraphLaunch")) return cudaErrorInvalidValue;
     streams[s].issued++;
+    if (on_launch) on_launch("", nullptr, 0);
     for (auto &f : execs[x]) f();
     return cudaSuccess;
 }

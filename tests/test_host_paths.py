@@ -34,6 +34,7 @@ def fake_runtime(tmp_path_factory, pkg):
 
 @pytest.mark.parametrize("name", [
     "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads", "qmat_workspace_is_shared",
+    "chain_table_copy_fails",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -53,7 +54,7 @@ def _fake():
     return L
 
 
-LAUNCH = C.CFUNCTYPE(None, C.c_char_p, C.POINTER(C.c_void_p), C.c_void_p)
+LAUNCH = C.CFUNCTYPE(None, C.c_char_p, C.POINTER(C.c_void_p), C.c_int)
 HOOK = C.CFUNCTYPE(None)
 
 
@@ -68,7 +69,7 @@ def vad_allocation_fails(pkg, synth, fake):
     frame = cfg["vad"]["frame_samples"]
     seen = []
 
-    def look(name, args, stream):
+    def look(name, args, recorded):
         if b"vad_lstm_kernel" in name:                   # (v, xz, f0, f1, hist, c_state, status)
             seen.append((_arg(args, 3, C.c_int), fake.fake_room(_arg(args, 4, C.c_void_p))))
         if b"vad_head_kernel" in name:                   # (v, hist, frames, probs)
@@ -257,7 +258,7 @@ def qmat_workspace_is_shared(pkg, synth, fake):
         assert fake.fake_calls(f) == 0, f
 
     planes = []
-    cb = LAUNCH(lambda name, args, stream: planes.append(_arg(args, 1, C.c_void_p)) if b"split" in name else None)
+    cb = LAUNCH(lambda name, args, recorded: planes.append(_arg(args, 1, C.c_void_p)) if b"split" in name else None)
     fake.fake_on_launch(cb)
     L = pkg.lib()
     L.mynah_b200_qmat_mul_device.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int]
@@ -284,6 +285,52 @@ def qmat_workspace_is_shared(pkg, synth, fake):
     for i, q in enumerate(handles):
         q.close()
     assert fake.fake_device_bytes() == 0
+
+
+def _chain_model(pkg, synth):
+    """A streaming model whose layers run as the persistent few-row chain."""
+    import cases
+    cfg = synth.config("chain", d_model=128, n_layers=2, n_heads=1, ffn_dim=256, n_mels=80, decoder="rnnt", vocab=33, pred_hidden=32, pred_layers=1,
+                       causal=True, normalize=False, wtype="q8_0")
+    return cases.device_model(pkg, synth, cfg, synth.make_model(cfg, seed=3))
+
+
+class ChainArgs(C.Structure):                                # the head of FrArgs and of FrOp (fewrow.h)
+    _fields_ = [("ops", C.c_void_p), ("n_ops", C.c_int)]
+
+
+OP_BYTES = 256
+
+
+def _table(args):
+    a = C.cast(args[0], C.POINTER(ChainArgs)).contents
+    return a.ops, C.string_at(a.ops, a.n_ops * OP_BYTES)
+
+
+@scenario
+def chain_table_copy_fails(pkg, synth, fake):
+    """If the table of a chain did not reach the device, the next step copies it again: its kernel never reads a table that
+    was not written."""
+    m = _chain_model(pkg, synth)
+    seen = []
+
+    def look(name, args, recorded):
+        if b"fr_kernel" in name:
+            table = np.frombuffer(_table(args)[1], np.int32).reshape(-1, OP_BYTES // 4)
+            seen.append(bool((table[:, 0] <= 3).all() and (table.any(axis=1)).all() and (table[0, 4:6] > 0).all()))
+
+    cb = LAUNCH(look)
+    fake.fake_on_launch(cb)
+    for nth in range(1, 9):
+        with closing(m.stream_open(2, 5, 0)) as g:
+            fake.fake_reset()
+            fake.fake_fail(b"cudaMemcpyAsync", nth)
+            for i in range(4):
+                try:
+                    g.step(np.zeros((2, g.need(), 80), np.float32))
+                except pkg.BackendError:
+                    pass
+    assert len(seen) > 16 and all(seen), seen
 
 
 if __name__ == "__main__":
