@@ -98,6 +98,11 @@ struct StreamState {
     const void *g_mel = nullptr, *g_out = nullptr, *g_base = nullptr;
     size_t g_mark = 0;
     int g_launches = 0, g_q = 0, steady_runs = 0;
+    void drop_graph() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+        exec = nullptr; graph = nullptr; steady_runs = 0;
+    }
     // transducer state carried from chunk to chunk (mynah_asr_dec_state, src/decoder.h:31-38), one block per
     // DEC_MAX_B streams: h[2][L][B][H], c[L][B][H], g[B][H] floats; last_tok[B] and the h parity as ints
     float *dec_f = nullptr;

@@ -300,8 +300,7 @@ int Model::stream_open(StreamState &st, int S, int left, int right) {
 }
 
 void Model::stream_close(StreamState &st) {
-    if (st.exec) cudaGraphExecDestroy(st.exec);
-    if (st.graph) cudaGraphDestroy(st.graph);
+    st.drop_graph();
     for (void *p : st.owned) cudaFree(p);
     st = StreamState();
 }
@@ -324,12 +323,12 @@ int Model::stream_step(StreamState &st, const float *mel, int n_mel, int is_last
         note_launch(st.g_launches);
         return st.g_q;
     }
-    if (st.steady_runs++ == 0 || (st.exec && !same)) {       // first steady step eagerly (launch attributes), or other buffers: re-capture next time
-        if (st.exec) { cudaGraphExecDestroy(st.exec); cudaGraphDestroy(st.graph); st.exec = nullptr; st.graph = nullptr; }
+    if (!same || st.steady_runs++ == 0) {                    // first step on these buffers eagerly (launch attributes, table of the chain)
+        st.drop_graph();
+        st.g_mel = mel; st.g_out = out; st.g_base = ws.base; st.g_mark = ws.off; st.steady_runs = 1;
         return stream_step_eager(st, mel, n_mel, is_last, out);
     }
     if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); return stream_step_eager(st, mel, n_mel, is_last, out); }
-    const size_t mark = ws.off;
     int q, recorded;
     {
         LaunchRecord record;
@@ -344,7 +343,7 @@ int Model::stream_step(StreamState &st, const float *mel, int n_mel, int is_last
         cudaGetLastError();
         return q < 0 ? -1 : stream_step_eager(st, mel, n_mel, is_last, out);
     }
-    st.graph = g; st.g_mel = mel; st.g_out = out; st.g_base = ws.base; st.g_mark = mark; st.g_launches = recorded; st.g_q = q;
+    st.graph = g; st.g_launches = recorded; st.g_q = q;
     if (cudaGraphLaunch(st.exec, stream) != cudaSuccess) { set_error("stream_step: graph launch failed"); return -1; }
     note_launch(recorded);
     return q;
@@ -403,7 +402,11 @@ int Model::stream_layers(StreamState &st, float *x, int Q, const __half *rk, int
         ln(up, FR_ROWS_LN, cur, L.ln_ff2_w, L.ln_ff2_b, nullptr, FR_EPI_PLANES, L.t_ff2a, L.ff2_w1.bias, F);
         resid(hF, L.t_ff2b, L.ff2_w2.bias, F, 0.5f);
     }
-    if (fr_upload(st.fr_table_host, st.fr_table_dev, fr_table(ops))) return -1;
+    // a graph of the steady step replays over the table that it was recorded with: where this step lays the buffers out
+    // differently (a short last chunk, after which the streams may go on), it is recorded anew, after a step that copies the table
+    const std::vector<uint8_t> table = fr_table(ops);
+    if (st.exec && st.fr_table_host != table) st.drop_graph();
+    if (fr_upload(st.fr_table_host, st.fr_table_dev, table)) return -1;
     a.M = M; a.terms = cfg.strict ? 3 : 1; a.d = d; a.H = n_heads; a.dk = d_head;
     a.bar = st.fr_bar; a.status = status; a.S = S; a.Q = Q; a.left = st.left; a.valid = st.valid; a.d_start = st.d_start;
     if (fr_launch(a, ops, st.fr_table_dev, stream)) return -1;

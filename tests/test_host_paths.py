@@ -34,7 +34,7 @@ def fake_runtime(tmp_path_factory, pkg):
 
 @pytest.mark.parametrize("name", [
     "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads", "qmat_workspace_is_shared",
-    "chain_table_copy_fails",
+    "chain_table_copy_fails", "chain_graph_reads_its_own_table",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -331,6 +331,29 @@ def chain_table_copy_fails(pkg, synth, fake):
                 except pkg.BackendError:
                     pass
     assert len(seen) > 16 and all(seen), seen
+
+
+@scenario
+def chain_graph_reads_its_own_table(pkg, synth, fake):
+    """A step of another size lays the buffers of the chain out anew. A graph recorded before it must not be replayed over the
+    other table: its buffers would overlap."""
+    m = _chain_model(pkg, synth)
+    recorded_table, replays = {}, []
+
+    def look(name, args, recorded):
+        if b"fr_kernel" in name and recorded:
+            recorded_table["now"] = _table(args)
+        if name == b"" and recorded_table:
+            at, table = recorded_table["now"]
+            replays.append(C.string_at(at, len(table)) == table)
+
+    cb = LAUNCH(look)
+    fake.fake_on_launch(cb)
+    with closing(m.stream_open(2, 8, 3)) as g:
+        for step in range(16):
+            last = step == 10                                # a short chunk that ends an utterance; the stream goes on
+            g.step(np.zeros((2, 9 if last else g.need(), 80), np.float32), last)
+    assert len(replays) >= 8 and all(replays), replays
 
 
 if __name__ == "__main__":
