@@ -61,12 +61,14 @@ public:
         h->busy[(size_t)idx_] = 1;
     }
     ~Lease() {
-        model().settle();
+        if (!idle_) model().settle();
         { std::lock_guard<std::mutex> lk(h_->pool_mu); h_->busy[(size_t)idx_] = 0; }
         h_->pool_cv.notify_all();
     }
     Model &model() { return h_->ctx(idx_); }
     int index() const { return idx_; }
+    // the call's last act was to wait, with success, for everything it issued: no need to ask the streams (3 us)
+    void idle() { idle_ = true; }
     Lease(const Lease &) = delete;
     Lease &operator=(const Lease &) = delete;
 
@@ -88,6 +90,7 @@ private:
     }
     mynah_b200_model *h_;
     int idx_ = -1;
+    bool idle_ = false;
 };
 
 // Runs fn on every context while none of them is in a call.
@@ -893,6 +896,7 @@ int mynah_b200_encoder_forward_batch(mynah_b200_model *h, const float *const *fe
         off += lens[b];
     }
     MB_CUDA(cudaStreamSynchronize(m.stream));
+    lease.idle();
     return 0;
 }
 
@@ -917,6 +921,7 @@ static float *forward_one(mynah_b200_model *h, const float *feats, int t_mel, in
     if (!out) { set_error("out of host memory"); return nullptr; }
     MB_CUDA_NULL(cudaMemcpyAsync(out, raw ? x : y, M * wout * 4, cudaMemcpyDeviceToHost, m.stream));
     MB_CUDA_NULL(cudaStreamSynchronize(m.stream));
+    lease.idle();
     *t_out = (int)M;
     return out;
 }
@@ -1099,6 +1104,7 @@ int mynah_b200_stream_step_device(mynah_b200_stream_group *g, const float *mel_d
     m.ws.reset();
     const int q = m.stream_step(g->st, mel_dev, n_mel, is_last, out_dev);
     if (q < 0 || m.check_status("stream_step")) return -1;
+    lease.idle();
     return q;
 }
 
@@ -1118,6 +1124,7 @@ int mynah_b200_stream_step(mynah_b200_stream_group *g, const float *mel, int n_m
     MB_CUDA(cudaMemcpyAsync(out, od, S * q * m.d_out * 4, cudaMemcpyDeviceToHost, m.stream));
     MB_CUDA(cudaStreamSynchronize(m.stream));
     if (m.check_status("stream_step")) return -1;
+    lease.idle();
     return q;
 }
 
@@ -1149,6 +1156,7 @@ int mynah_b200_stream_step_decode(mynah_b200_stream_group *g, const float *mel, 
     if (q < 0) return -1;
     std::vector<std::vector<int>> tk, fr;
     if (m.stream_decode(g->st, od, q, tk, fr) || m.check_status("stream_step_decode")) return -1;
+    lease.idle();
     for (size_t s = 0; s < S; s++) {
         n_tokens[s] = (int)tk[s].size();
         tokens[s] = (int *)malloc((tk[s].size() ? tk[s].size() : 1) * sizeof(int));
@@ -1286,6 +1294,7 @@ int mynah_b200_transcribe_batch_prompts(mynah_b200_model *h, const float *const 
     {
         Lease lease(h);
         rc = run_batch_locked(lease.model(), &bt, nullptr, audio, decoder);
+        if (rc == 0) lease.idle();
     }
     if (rc == 0) rc = mynah_b200_batch_fetch(h, &bt, tokens, frames, n_tokens);
     return rc;
@@ -1302,6 +1311,7 @@ int mynah_b200_transcribe_batch_aed(mynah_b200_model *h, const float *const *aud
     {
         Lease lease(h);
         rc = run_batch_locked(lease.model(), &bt, nullptr, audio, 2);
+        if (rc == 0) lease.idle();
     }
     if (rc == 0) rc = mynah_b200_batch_fetch(h, &bt, tokens, nullptr, n_tokens);
     return rc;

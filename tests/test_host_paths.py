@@ -183,9 +183,11 @@ def error_is_reported_once(pkg, synth, fake):
 
 @scenario
 def failed_call_waits(pkg, synth, fake):
-    """A call that fails anywhere returns with nothing in flight: neither copies out of the caller's memory nor kernels on
-    the workspace that the next call lays out anew."""
+    """A call returns with nothing in flight, also one that fails on the way: neither copies out of the caller's memory nor
+    kernels on the workspace that the next call lays out anew."""
     def idle(what, call):
+        assert fake.fake_pending() == 0, what
+        call()
         assert fake.fake_pending() == 0, what
 
     _each_failure(pkg, synth, fake, ASYNC, idle)
