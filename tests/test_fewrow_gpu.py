@@ -74,3 +74,31 @@ def test_streams_go_on_after_a_short_chunk(gpu_pkg, synth):
             outs.append(got)
     assert outs[0][7].shape[1] < outs[0][6].shape[1]
     assert all(np.array_equal(a, b) for a, b in zip(*outs))
+
+
+@pytest.mark.parametrize("d", [128, 192])
+def test_layernorm_of_rows_far_from_zero(gpu_pkg, synth, d):
+    """Rows of one large value c with as many elements one step above it as below: their mean is c. Squares take 48 bits, the
+    sum of K of them more than the 53 of a double, so K c^2 is lost to the last units, and the variance of 2 / K or 6 / K
+    steps^2 with it (d = 128: sums of squares give 0 and 8 / K) unless the sums are of differences."""
+    cfg = synth.config("far", d_model=128, n_layers=1, n_heads=4, ffn_dim=256, n_mels=80, decoder="aed", vocab=211, aed_d=d,
+                       aed_layers=2, aed_heads=2, aed_ffn=256, aed_max_seq=48, wtype="q8_0")
+    tensors = synth.make_model(cfg, seed=4)
+    tables = {n: tensors[n].raw.view(np.float32).reshape(tensors[n].shape).copy() for n in ("aed.embedding.weight", "aed.pos_enc")}
+    emb, pos = tables.values()
+    prompt = (3, 4, 5, 6)
+    for tok, c, pairs in zip(prompt, (16777214.0, 16777213.0, 16777214.0 * 128, -16777212.0), (1, 3, 1, 3)):
+        step = abs(c) - np.float64(np.nextafter(np.float32(abs(c)), np.float32(0)))
+        emb[tok] = c
+        for i in range(pairs):
+            emb[tok, (7 * i) % d] = c + step                 # (the row's first value is one of them)
+            emb[tok, d - 2 - 11 * i] = c - step
+    pos[:len(prompt)] = 0
+    for n, a in tables.items():
+        tensors[n] = synth.Tensor(n, tensors[n].ggml_type, tensors[n].shape, a.reshape(-1).view(np.uint8))
+    A = model_io.oracle_model(cfg, tensors)["aed"]
+    enc = np.random.default_rng(2).standard_normal((11, cfg.d_model), dtype=np.float32)
+    with closing(cases.device_model(gpu_pkg, synth, cfg, tensors, aed_heads=cfg.aed_heads)) as dm:
+        for n in range(1, 5):
+            for p in (prompt[:n], prompt[n - 1:n]):
+                assert dm.aed_decode(enc, p, -1, 12).tolist() == O.aed_decode(A, enc, p, -1, 12).tolist(), p
