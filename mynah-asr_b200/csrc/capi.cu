@@ -118,12 +118,17 @@ struct mynah_b200_qmat {
     uint64_t id = 0;                     // never used again, unlike an address or a stream
     mutable std::mutex mu;
     mutable uint8_t *host = nullptr;     // the block's pinned twin, once a graph names it; until then a call borrows one
-    // A small call repeated with the same rows and flags is one graph (copy in, kernels, copy out): issuing its four or five
-    // pieces one by one took longer than running them. Recorded on the second such call, kept for the last few.
+    // A small call repeated with the same rows and flags is one graph (copy in, kernels, copy out) instead of four or five
+    // pieces: 29.5 us against 34.4 for one row of [4096 x 1024], 51 against 57 for 32 of [1024 x 1024]. Recording takes 70 us, so
+    // it waits for the second such call. Four of them, for a program that alternates between a few row counts; a fifth takes the
+    // oldest one's place and runs in pieces until it comes again.
     struct Graph { int T = 0, flags = 0, uses = 0, launches = 0; cudaGraphExec_t exec = nullptr; };
     mutable Graph graphs[4];
     mutable int graph_next = 0;
 };
+// Rows or results up to QMAT_SMALL bytes go through the block. With 32 rows of [1024 x 1024], 128 KB each way, a product takes
+// 51 us that way and 65 by copies of their own from pageable memory. It would still take 101 against 118 us at 512 KB: the
+// line is what every handle of a model holds for it, three times this on the device.
 static constexpr size_t QMAT_HEAD = 256, QMAT_SMALL = 128 << 10;
 static constexpr size_t QMAT_TEMP_AT = QMAT_HEAD + 2 * QMAT_SMALL, QMAT_TEMP = QMAT_SMALL + 512;   // two fp16 planes of x, aligned
 static constexpr size_t QMAT_PINNED = QMAT_TEMP_AT, QMAT_BLOCK = QMAT_TEMP_AT + QMAT_TEMP;

@@ -420,6 +420,8 @@ qgemv_a8_kernel(const uint8_t *__restrict__ raw, const float *__restrict__ scale
 
 int act_quant_rows(const float *x, int8_t *qx, float *sx, int T, int k, cudaStream_t st, bool chain) {
     if (T <= 0) return 0;
+    // Rows in registers for the model and FFN widths of the configurations, which are the only ones timed: an encoder of 24
+    // layers takes 3.23 ms with them and 3.76 with the scalar kernel (one utterance of 5 s), 12.9 and 13.2 (eight of 30 s).
     const bool al = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(qx) & 3) == 0;
 #define AQ_VEC(W, NV) MB_CUDA(launch_kernel(act_quant_vec_kernel<W, NV>, dim3(cdiv(T, 8 / W)), dim3(256), 0, st, chain, 1, x, qx, sx, T))
     if (al && k == 512) AQ_VEC(1, 4);
