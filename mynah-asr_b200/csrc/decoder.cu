@@ -19,8 +19,9 @@
 //           update; layers are separated by a grid barrier
 //   proj    g[b] = decoder_projector(h_last[b])
 // What bounds it is latency: 49 MB of weights per emitting step come from L2 in 9 us, the four phases take 19 us with one
-// utterance and 33 with sixteen (26 and 40 with the selection as a phase of its own, weights asked for only behind the
-// barriers and the cells of a row block updated by one warp).
+// utterance (36 k cycles) and 28 with sixteen (53 k; 35 behind the contractions of a large batch, which leave the clock at the
+// power cap). 26 and 40 with the selection as a phase of its own, weights asked for only behind the barriers and the cells of a
+// row block updated by one warp.
 // The matvecs run on the warp-level tensor-core path with the utterances as the N
 // dimension: weights as fp16 (hi, lo) planes (a decoded Q4_0/Q8_0 weight is exact in
 // that form), activations split the same way, three MMAs per k-step, f32 accumulate —

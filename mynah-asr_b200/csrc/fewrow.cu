@@ -3,7 +3,7 @@
 // A streaming step or an AED position is a few hundred dependent operations of at most 128 rows. As launches, chained and
 // replayed from a graph, each of them costs 9-11 us (set-up, tensor-memory allocation, slice sums over a cluster, LayerNorm
 // by the last warp to arrive) where its bytes would need one. Here one cooperative launch walks the whole chain; what
-// separates two operations is a barrier over the CTAs of a row tile (about 1.3 us):
+// separates two operations is a barrier over the CTAs of a row tile (about 1.6 us, the next weights asked for within it):
 //   * a CTA keeps its place: a row tile of at most sixteen rows and every ngroups-th unit of eight weight rows. It sums a
 //     unit over all of K itself (sixteen warps take 64-wide pieces of K, added in warp order), so nothing is exchanged
 //     between CTAs inside an operation, and a row's bits do not depend on how many other rows there are;
@@ -15,8 +15,11 @@
 //     with N = 1024 and no exchange of partial sums.)
 //   * the LayerNorms are computed where their result is staged, by every CTA. The conv module's middle sits in the epilogue
 //     of the contraction before it.
-// Measured: a step of 24 layers of d = 1024 takes 1.16 ms for one stream (2.74 as launches), 2.25 for 22, 3.7 for 64 with
-// decoding (4.8), 4.9 for 120 (5.9); AED with 32 + 8 layers takes 27.5 ms for one sentence (48.7), 53 for eight (78).
+// Measured: a step of 24 layers of d = 1024 takes 1.17 ms for one stream (2.74 as launches), 2.25 for 22, 3.7 for 64 with
+// decoding (4.8), 4.85 for 120 (5.9); AED of the Canary shape (32 encoder layers, 4 decoder layers: 33 operations a position)
+// takes 34 ms for one sentence of 10 s (180 positions), 44.5 for eight; 64 positions of the decoder alone 10.9 ms (19.3 as
+// launches, with f32 weights), 13.3 for eight (20.1), 22.8 for 32 (25.1). An operation is 9.5 k cycles with one row, 11.2 to
+// 11.4 k with eight and 15 to 16 k with sixteen, of which the barrier is 3 k.
 // Values that other CTAs write are read past the L1 (ld.cg, cp.async.cg). All waits are bounded: one that runs out sets the
 // status word and the abort flag, and every CTA leaves.
 #include "fewrow.h"
