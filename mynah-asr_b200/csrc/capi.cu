@@ -224,6 +224,7 @@ public:
     }
     // Workspace::p is null on failure
     Workspace take(size_t bytes, uint64_t user, cudaStream_t st) {
+        RelaxedCapture relaxed;
         Workspace w;
         w.device = current();
         {
@@ -271,7 +272,7 @@ public:
 private:
     static constexpr int KEEP_BLOCKS = 4;
     static int current() { int d = 0; if (cudaGetDevice(&d) != cudaSuccess) cudaGetLastError(); return d; }
-    static void destroy(Workspace &w) { cudaEventSynchronize(w.done); cudaEventDestroy(w.done); cudaFree(w.p); cudaGetLastError(); }
+    static void destroy(Workspace &w) { RelaxedCapture relaxed; cudaEventSynchronize(w.done); cudaEventDestroy(w.done); cudaFree(w.p); cudaGetLastError(); }
     std::mutex mu_;
     std::vector<Workspace> free_;
     std::map<int, int> handles_;

@@ -33,6 +33,16 @@ const char *last_error();
         }                                                                                \
     } while (0)
 
+// While one lives, its thread's queries, allocations and frees leave a recording alone that another thread of the process
+// makes in the global capture mode (they would end it with an error).
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture &) = delete;
+    RelaxedCapture &operator=(const RelaxedCapture &) = delete;
+};
+
 // CUDA keeps function attributes and the SM count per device; a process may drive several devices.
 // PerDevice remembers, for every device, the largest value configured so far (0 = nothing yet).
 static constexpr int MB_MAX_DEVICES = 64;

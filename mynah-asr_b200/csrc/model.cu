@@ -93,6 +93,7 @@ int Model::lanes_join(int lanes) {
     return 0;
 }
 void Model::settle() {
+    RelaxedCapture relaxed;
     bool left = false;
     auto wait = [&](cudaStream_t s) { if (s && cudaStreamQuery(s) != cudaSuccess) { cudaStreamSynchronize(s); left = true; } };
     wait(copy);

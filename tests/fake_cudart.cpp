@@ -10,6 +10,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace {
@@ -39,6 +40,11 @@ typedef void (*hook_cb)();
 launch_cb on_launch = nullptr;
 hook_cb on_capture = nullptr;
 thread_local cudaError_t last_error = cudaSuccess;
+thread_local cudaStreamCaptureMode capture_mode = cudaStreamCaptureModeGlobal;
+bool foreign_capture = false;                            // another library of the process records in global mode
+long long broken_captures = 0;
+// calls that end such a recording unless their thread has asked for the relaxed mode
+void unsafe_call() { if (foreign_capture && capture_mode != cudaStreamCaptureModeRelaxed) broken_captures++; }
 thread_local dim3 cfg_grid, cfg_block;
 thread_local size_t cfg_smem;
 thread_local cudaStream_t cfg_stream;
@@ -102,6 +108,9 @@ size_t fake_room(const void *p) {                        // bytes from p to the 
 void fake_on_launch(launch_cb cb) { Lock l(mu); on_launch = cb; }
 void fake_on_capture(hook_cb cb) { Lock l(mu); on_capture = cb; }
 
+void fake_foreign_capture(int on) { Lock l(mu); foreign_capture = on; broken_captures = 0; }
+long long fake_broken_captures() { Lock l(mu); return broken_captures; }
+
 // ---- registration
 void **__cudaRegisterFatBinary(void *) { static void *h; return &h; }
 void __cudaRegisterFatBinaryEnd(void **) {}
@@ -134,6 +143,7 @@ cudaError_t cudaGetDriverEntryPoint(const char *, void **p, unsigned long long, 
 // ---- memory
 cudaError_t cudaMalloc(void **p, size_t n) {
     Lock l(mu);
+    unsafe_call();
     if (fails("cudaMalloc")) return cudaErrorMemoryAllocation;
     *p = calloc(1, n);
     dev_mem[*p] = n;
@@ -144,6 +154,7 @@ cudaError_t cudaMalloc(void **p, size_t n) {
 cudaError_t cudaFree(void *p) {                          // waits for the device, as the real one does
     Lock l(mu);
     calls["cudaFree"]++;
+    unsafe_call();
     if (!p) return cudaSuccess;
     if (!dev_mem.count(p)) return cudaErrorInvalidValue;
     wait_all();
@@ -178,7 +189,7 @@ cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t st) {
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { Lock l(mu); if (fails("cudaStreamCreate")) return cudaErrorMemoryAllocation; *s = handle<cudaStream_t>(); return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { Lock l(mu); streams.erase(s); stream_behind.erase(s); return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { Lock l(mu); calls["cudaStreamSynchronize"]++; wait_stream(s); return cudaSuccess; }
-cudaError_t cudaStreamQuery(cudaStream_t s) { Lock l(mu); return streams[s].done < streams[s].issued ? cudaErrorNotReady : cudaSuccess; }
+cudaError_t cudaStreamQuery(cudaStream_t s) { Lock l(mu); unsafe_call(); return streams[s].done < streams[s].issued ? cudaErrorNotReady : cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) { Lock l(mu); calls["cudaStreamWaitEvent"]++; merge(stream_behind[s], event_behind[e]); return work(s, [] {}); }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { Lock l(mu); if (fails("cudaEventCreate")) return cudaErrorMemoryAllocation; *e = handle<cudaEvent_t>(); return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return cudaEventCreate(e); }
@@ -192,6 +203,7 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
 }
 cudaError_t cudaEventQuery(cudaEvent_t e) {
     Lock l(mu);
+    unsafe_call();
     for (auto &b : event_behind[e]) if (streams.count(b.first) && streams[b.first].done < b.second) return cudaErrorNotReady;
     return cudaSuccess;
 }
@@ -206,6 +218,7 @@ cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { *ms = 1.
 cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **args, size_t, cudaStream_t st) { return launch(f, args, st); }
 cudaError_t cudaLaunchCooperativeKernel(const void *f, dim3, dim3, void **args, size_t, cudaStream_t st) { return launch(f, args, st); }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **args) { return launch(f, args, c->stream); }
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode *m) { std::swap(*m, capture_mode); return cudaSuccess; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t s, cudaStreamCaptureMode) { Lock l(mu); capturing[s]; return cudaSuccess; }
 cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t *g) {
     Lock l(mu);

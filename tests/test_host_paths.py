@@ -34,7 +34,7 @@ def fake_runtime(tmp_path_factory, pkg):
 
 @pytest.mark.parametrize("name", [
     "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads", "qmat_workspace_is_shared",
-    "chain_table_copy_fails", "chain_graph_reads_its_own_table",
+    "foreign_capture_survives", "chain_table_copy_fails", "chain_graph_reads_its_own_table",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -47,7 +47,7 @@ def _fake():
     L = C.CDLL("libcudart.so.12")
     for f in ("fake_device_bytes", "fake_device_peak", "fake_room"):
         getattr(L, f).restype = C.c_size_t
-    L.fake_calls.restype = C.c_longlong
+    L.fake_calls.restype = L.fake_broken_captures.restype = C.c_longlong
     L.fake_calls.argtypes = [C.c_char_p]
     L.fake_fail.argtypes = [C.c_char_p, C.c_longlong]
     L.fake_room.argtypes = [C.c_void_p]
@@ -287,6 +287,30 @@ def qmat_workspace_is_shared(pkg, synth, fake):
     for i, q in enumerate(handles):
         q.close()
     assert fake.fake_device_bytes() == 0
+
+
+@scenario
+def foreign_capture_survives(pkg, synth, fake):
+    """Queries of events and streams, allocations and frees end a recording that another thread of the process makes in the
+    global mode. Calls whose buffers are there already issue none that would, and neither does a product that has to grow."""
+    calls = _small_calls(pkg, synth)
+    calls = {k: v for k, v in calls.items() if k != "stream"}    # (opening a group allocates)
+    import cases
+    cfg, tensors = cases.build(synth, "ctc_q8")
+    m = cases.device_model(pkg, synth, cfg, tensors)
+    calls["log_mel"] = lambda: m.log_mel(np.zeros(16000, np.float32))
+    handles = [pkg.QMat(pkg.F32, np.ones((128, 512), np.float32), 128, 512) for _ in range(3)]
+    calls["products"] = lambda: [q.mul(np.ones((600, 512), np.float32)) for q in handles]
+    for what, call in calls.items():
+        call()
+        fake.fake_foreign_capture(1)
+        call()
+        assert fake.fake_broken_captures() == 0, what
+        fake.fake_foreign_capture(0)
+    fake.fake_foreign_capture(1)
+    handles[0].mul(np.ones((3000, 512), np.float32))
+    assert fake.fake_broken_captures() == 0
+    fake.fake_foreign_capture(0)
 
 
 def _chain_model(pkg, synth):
