@@ -291,15 +291,19 @@ int gemm_i8(const int8_t *a, int lda, const float *row_scale, const int8_t *b, i
     if (K <= 0 || K % I8_BK != 0) { set_error("gemm_i8: K=%d must be a positive multiple of %d", K, I8_BK); return -1; }
     if (!row_scale || !col_scale) { set_error("gemm_i8: scales missing"); return -1; }
     const int sms = device_sm_count();
-    // tile width by waves x time of one tile (an output element sees the same integers whatever the width). The fp16
-    // contraction also counts K and the strips of a last wave (gemm_tc.cu). Here that takes 24 layers of d = 1024 from 12.9 to
-    // 10.4 ms for eight utterances of 21 to 30 s, from 8.8 to 8.1 for five, and leaves most other batches as they are (12.9 to
-    // 15.9 ms for twelve, either way): not done yet.
-    const int tm = cdiv(M, GEMM_BM);
+    // Tile width by waves x time of one tile, as in gemm_tc.cu (an output element sees the same integers whatever the width): what a
+    // last partial wave is cut into counts with its strips' width, prologue and epilogue as much as 48 columns of K = 1024. Without
+    // the strips and K in the cost 24 layers of d = 1024 took 13.1 ms instead of 10.4 for eight utterances of 21 to 30 s, 14.8
+    // instead of 11.7 for twelve of 5 to 40, 5.8 instead of 5.4 for four of 5 to 20; twelve of 20 to 40 s and what fits one wave take
+    // the same. With twice the fixed part most of that is lost (11.7, 13.0, 5.8); with the strips counted below one wave, too, one
+    // utterance of 30 s takes 5.5 ms instead of 4.65 (a strip still reads its tile's whole operands).
+    const int tm = cdiv(M, GEMM_BM), fixed = K >= 49152 ? 1 : 49152 / K;
     int bn = 256;
     long best = -1;
     for (int cand = 256; cand >= 32; cand >>= 1) {
-        const long cost = (long)cdiv(tm * cdiv(N, cand), sms) * (cand + 48);
+        const int tiles = tm * cdiv(N, cand), rem = tiles % sms;
+        const int split = tiles < sms ? 1 : rem * 4 <= sms && cand % 128 == 0 ? 4 : rem * 2 <= sms && cand % 64 == 0 ? 2 : 1;
+        const long cost = (long)(tiles / sms) * (cand + fixed) + (rem ? cand / split + fixed : 0);
         if (best < 0 || cost < best) { best = cost; bn = cand; }
     }
     if (bn == 256) return i8_launch<256>(a, lda, row_scale, b, ldb, col_scale, ep, M, N, K, status, stream, chain);

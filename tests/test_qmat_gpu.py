@@ -304,3 +304,17 @@ def test_a8_many_rows_on_the_tensor_cores_bit_exact(gpu_pkg):
             assert np.array_equal(m.mul(x[:T], gpu_pkg.A8), want[:T]), (n, k, T)
         assert np.array_equal(m.mul(x[:9], gpu_pkg.A8), want[:9])          # the row-dot kernel below 17 rows agrees too
         m.close()
+
+
+@pytest.mark.parametrize("rows,n,k", [(1409, 4096, 256), (1665, 3000, 256), (1793, 1024, 1024)])
+def test_a8_last_wave_in_strips_bit_exact(gpu_pkg, rows, n, k):
+    """Sizes whose last partial wave of tiles is cut into two and four column strips, some of them past the last column, and one
+    just past a wave of narrow tiles: the same integers, so the same bits."""
+    rng = np.random.default_rng(rows)
+    q8, s8 = O.quantize_int8(rng.uniform(-1, 1, (n, k)).astype(np.float32))
+    x = (rng.standard_normal((rows, k)) * rng.uniform(0.1, 30, (rows, 1))).astype(np.float32)
+    qx, sx = O.quantize_act_int8(x)
+    dots = (qx.astype(np.float64) @ q8.astype(np.float64).T).astype(np.float32)      # integers below 2^53: exact
+    m = gpu_pkg.QMat(gpu_pkg.MYNAH_Q8, q8, n, k, scales=s8)
+    assert np.array_equal(m.mul(x, gpu_pkg.A8), (dots * s8[None, :].astype(np.float32)) * sx[:, None])
+    m.close()
