@@ -227,13 +227,21 @@ def _at(a):
     return a.__array_interface__["data"][0]
 
 
+class _Malloced:
+    """Memory that the library allocated for a result: lives as long as an array over it."""
+
+    def __init__(self, ptr, shape):
+        self.ptr, self._free = ptr, _libc.free
+        self.__array_interface__ = {"shape": tuple(shape), "typestr": "<f4", "data": (ptr, False), "version": 3}
+
+    def __del__(self):
+        self._free(self.ptr)
+
+
 def _take_f32(ptr, shape):
     if not ptr:
         raise BackendError(_err())
-    n = int(np.prod(shape))
-    out = np.ctypeslib.as_array(C.cast(ptr, c_fp), shape=(max(n, 1),))[:n].copy().reshape(shape)
-    _libc.free(ptr)
-    return out
+    return np.asarray(_Malloced(ptr if isinstance(ptr, int) else C.cast(ptr, C.c_void_p).value, shape))
 
 
 def _take_i32(ptr, n):

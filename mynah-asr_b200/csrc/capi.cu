@@ -9,6 +9,7 @@
 #include <condition_variable>
 #include <memory>
 
+#include "hostcopy.h"
 #include "model.h"
 
 using namespace mb;
@@ -21,6 +22,7 @@ namespace mb { long long launch_count(bool reset); }
 // same weights — the counterpart of the reference's per-thread cuBLAS handle / stream / buffers over a shared
 // weight cache (src/cuda_gemm.cu:50-60,92-130).
 struct mynah_b200_model {
+    CopyUser copies;
     Model m;
     std::vector<std::unique_ptr<Model>> extra;      // contexts 1..
     std::vector<char> busy{0};                      // per context
@@ -110,6 +112,7 @@ void with_all_contexts_idle(mynah_b200_model *h, F fn) {
 // of [1024 x 4096]: 680 us instead of 309).
 // One lock per handle: products of one weight share the block and run one after the other on the handle's stream.
 struct mynah_b200_qmat {
+    CopyUser copies;
     QWeight w;
     std::vector<void *> owned;
     cudaStream_t stream = nullptr;
@@ -894,13 +897,15 @@ int mynah_b200_encoder_forward_batch(mynah_b200_model *h, const float *const *fe
     if (m.front_end(nullptr, nullptr, feats, t_mel, batch, true, x, lens) || m.encoder_layers(x, lens, left, right, 0, m.n_layers)) return -1;
     if (m.encoder_post(x, lens, prompt_ids, y) || m.check_status("encoder_forward_batch")) return -1;
     size_t off = 0;
+    std::vector<CopyOut> parts;
     for (int b = 0; b < batch; b++) {
         t_outs[b] = lens[b];
         outs[b] = (float *)malloc((size_t)(lens[b] ? lens[b] : 1) * m.d_out * sizeof(float));
         if (!outs[b]) { set_error("out of host memory"); return -1; }
-        MB_CUDA(cudaMemcpyAsync(outs[b], y + off * m.d_out, (size_t)lens[b] * m.d_out * 4, cudaMemcpyDeviceToHost, m.stream));
+        parts.push_back(CopyOut{outs[b], y + off * m.d_out, (size_t)lens[b] * m.d_out * 4});
         off += lens[b];
     }
+    if (copy_out(parts, m.stream)) return -1;
     MB_CUDA(cudaStreamSynchronize(m.stream));
     lease.idle();
     return 0;
@@ -925,7 +930,7 @@ static float *forward_one(mynah_b200_model *h, const float *feats, int t_mel, in
     if (m.check_status("encoder_forward")) return nullptr;
     float *out = (float *)malloc(M * wout * sizeof(float));
     if (!out) { set_error("out of host memory"); return nullptr; }
-    MB_CUDA_NULL(cudaMemcpyAsync(out, raw ? x : y, M * wout * 4, cudaMemcpyDeviceToHost, m.stream));
+    if (copy_out(out, raw ? x : y, M * wout * 4, m.stream)) return nullptr;
     MB_CUDA_NULL(cudaStreamSynchronize(m.stream));
     lease.idle();
     *t_out = (int)M;
@@ -1124,10 +1129,10 @@ int mynah_b200_stream_step(mynah_b200_stream_group *g, const float *mel, int n_m
     m.ws.reset();
     float *md = m.ws.get<float>(nin), *od = m.ws.get<float>(nout);
     if (!md || !od) return -1;
-    MB_CUDA(cudaMemcpyAsync(md, mel, nin * 4, cudaMemcpyHostToDevice, m.stream));
+    if (copy_in(md, mel, nin * 4, m.stream)) return -1;
     const int q = m.stream_step(g->st, md, n_mel, is_last, od);
     if (q < 0) return -1;
-    MB_CUDA(cudaMemcpyAsync(out, od, S * q * m.d_out * 4, cudaMemcpyDeviceToHost, m.stream));
+    if (copy_out(out, od, S * q * m.d_out * 4, m.stream)) return -1;
     MB_CUDA(cudaStreamSynchronize(m.stream));
     if (m.check_status("stream_step")) return -1;
     lease.idle();
@@ -1157,7 +1162,7 @@ int mynah_b200_stream_step_decode(mynah_b200_stream_group *g, const float *mel, 
     m.ws.reset();
     float *md = m.ws.get<float>(nin), *od = m.ws.get<float>(nout);
     if (!md || !od) return -1;
-    MB_CUDA(cudaMemcpyAsync(md, mel, nin * 4, cudaMemcpyHostToDevice, m.stream));
+    if (copy_in(md, mel, nin * 4, m.stream)) return -1;
     const int q = m.stream_step(g->st, md, n_mel, is_last, od);
     if (q < 0) return -1;
     std::vector<std::vector<int>> tk, fr;
@@ -1474,10 +1479,10 @@ int mynah_b200_qmat_mul(const mynah_b200_qmat *q, const float *x, float *out, in
     const void *src = x;
     if (small_x) src = memcpy(host + QMAT_HEAD + QMAT_SMALL, x, nx);
     auto issue = [&]() -> int {
-        if (cudaMemcpyAsync(xd, src, nx, cudaMemcpyHostToDevice, q->stream) != cudaSuccess) { cudaGetLastError(); set_error("qmat_mul: H2D copy failed"); return -1; }
+        if (copy_in(xd, src, nx, q->stream)) return -1;
         if (qmat_mul_locked(q, xd, od, T, flags, temp)) return -1;
-        bool ok = small_out || cudaMemcpyAsync(out, od, no, cudaMemcpyDeviceToHost, q->stream) == cudaSuccess;
-        ok = cudaMemcpyAsync(host, block, QMAT_HEAD + (small_out ? no : 0), cudaMemcpyDeviceToHost, q->stream) == cudaSuccess && ok;
+        const bool ok = cudaMemcpyAsync(host, block, QMAT_HEAD + (small_out ? no : 0), cudaMemcpyDeviceToHost, q->stream) == cudaSuccess;
+        if (!small_out && copy_out(out, od, no, q->stream)) return -1;
         if (!ok) { cudaGetLastError(); set_error("qmat_mul: D2H copy failed"); return -1; }
         return 0;
     };

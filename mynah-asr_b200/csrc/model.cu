@@ -10,6 +10,8 @@
 
 #include <atomic>
 
+#include "hostcopy.h"
+
 namespace mb {
 
 static std::atomic<long long> g_launches{0};
@@ -421,8 +423,7 @@ int Model::front_end(const float *const *audio, const size_t *n_samples, const f
             for (int u = g.b0; u < g.b1; u++) {
                 if (t_mel[u] <= 0) continue;
                 const FrontItem &it = items[i++];
-                if (audio) MB_CUDA(cudaMemcpyAsync(const_cast<float *>(it.audio), audio[u], n_samples[u] * 4, cudaMemcpyHostToDevice, copy));
-                else MB_CUDA(cudaMemcpyAsync(it.feats, feats[u], (size_t)it.t_mel * cfg.n_mels * 4, cudaMemcpyHostToDevice, copy));
+                if (audio ? copy_in(const_cast<float *>(it.audio), audio[u], n_samples[u] * 4, copy) : copy_in(it.feats, feats[u], (size_t)it.t_mel * cfg.n_mels * 4, copy)) return -1;
             }
             if (gi >= copy_ev.size()) {
                 cudaEvent_t e = nullptr;

@@ -168,6 +168,7 @@ cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return cudaFree(p); }
 cudaError_t cudaMallocHost(void **p, size_t n) { Lock l(mu); if (fails("cudaMallocHost")) return cudaErrorMemoryAllocation; *p = calloc(1, n); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { Lock l(mu); if (fails("cudaHostAlloc")) return cudaErrorMemoryAllocation; *p = calloc(1, n); return cudaSuccess; }
 cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) { memset(a, 0, sizeof(*a)); a->type = cudaMemoryTypeUnregistered; return cudaSuccess; }
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemset(void *p, int v, size_t n) { memset(p, v, n); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st) {
