@@ -21,7 +21,7 @@ namespace mb {
 namespace {
 
 constexpr size_t PIECE = 512 << 10, PART = 128 << 10;
-constexpr int SLOTS = 12;                                        // page-locked pieces: 6 MB
+constexpr int SLOTS = 4;                                         // page-locked pieces: 2 MB (page-locking takes 1 ms per MB, once)
 constexpr int HELPERS = 3;
 // Below this the driver's way is as fast: 0.75 MB take 62 us in and 77 out there, 40 to 50 by way of the pieces with the helpers
 // still asleep.

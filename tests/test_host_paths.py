@@ -35,6 +35,7 @@ def fake_runtime(tmp_path_factory, pkg):
 @pytest.mark.parametrize("name", [
     "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads", "qmat_workspace_is_shared",
     "foreign_capture_survives", "chain_table_copy_fails", "chain_graph_reads_its_own_table",
+    "copies_by_pieces",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -380,6 +381,60 @@ def chain_graph_reads_its_own_table(pkg, synth, fake):
             last = step == 10                                # a short chunk that ends an utterance; the stream goes on
             g.step(np.zeros((2, 9 if last else g.need(), 80), np.float32), last)
     assert len(replays) >= 8 and all(replays), replays
+
+
+@scenario
+def copies_by_pieces(pkg, synth, fake):
+    """Rows and results of more pieces than there are places for arrive whole, from several threads at once, while calls of
+    the transfers fail, and after the last handle has given threads and pieces back."""
+    import threading
+    n, k, rows = 640, 1024, 1500                             # 6.1 MB in, 3.8 MB out
+    rng = np.random.default_rng(0)
+    seen, errors = [], []
+
+    def look(name, args, recorded):                          # the split reads the product's input
+        if b"split_kernel" in name and _arg(args, 3, C.c_size_t) == rows * k // 4:
+            at = _arg(args, 0, C.c_void_p)
+            got = np.ctypeslib.as_array(C.cast(at, C.POINTER(C.c_float)), shape=(rows, k))
+            seen.append(any(np.array_equal(got, x) for x in xs))
+
+    xs = [rng.standard_normal((rows, k)).astype(np.float32) for _ in range(4)]
+
+    def guarded(name, args, recorded):
+        try:
+            look(name, args, recorded)
+        except BaseException as e:
+            errors.append(repr(e))
+
+    cb = LAUNCH(guarded)
+    fake.fake_on_launch(cb)
+    w = np.ones((n, k), np.float32)
+    for life in range(2):
+        handles = [pkg.QMat(pkg.F32, w, n, k) for _ in xs]
+        failed = 0
+        for f in (b"cudaMemcpyAsync", b"cudaEventRecord", b"cudaHostAlloc"):
+            for at in (1, 2, 7, 13, 16, 20):
+                fake.fake_fail(f, at)
+                try:
+                    handles[0].mul(xs[0])
+                except pkg.BackendError:
+                    failed += 1
+                fake.fake_fail(b"", 0)
+                handles[1].mul(xs[1])
+        assert failed >= 8, failed
+
+        def many(i):
+            for _ in range(20):
+                handles[i].mul(xs[i])
+
+        threads = [threading.Thread(target=many, args=(i,)) for i in range(len(xs))]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for q in handles:
+            q.close()
+    assert len(seen) > 160 and all(seen) and not errors, (len(seen), sum(seen), errors[:3])
 
 
 if __name__ == "__main__":

@@ -318,3 +318,17 @@ def test_a8_last_wave_in_strips_bit_exact(gpu_pkg, rows, n, k):
     m = gpu_pkg.QMat(gpu_pkg.MYNAH_Q8, q8, n, k, scales=s8)
     assert np.array_equal(m.mul(x, gpu_pkg.A8), (dots * s8[None, :].astype(np.float32)) * sx[:, None])
     m.close()
+
+
+@pytest.mark.parametrize("rows", [128, 129, 500, 1563, 3200])
+def test_copies_by_pieces(gpu_pkg, rows):
+    """Host rows and results around one page-locked piece (512 KB), with ragged ends and more pieces than there are places for
+    (the transfers that start the pieces, too), give the bits of few rows, which the driver copies."""
+    rng = np.random.default_rng(rows)
+    n, k = 1032, 1024
+    m = gpu_pkg.QMat(gpu_pkg.F32, (rng.standard_normal((n, k)) * 0.02).astype(np.float32), n, k)
+    x = rng.standard_normal((rows, k)).astype(np.float32)
+    want = np.concatenate([m.mul(x[i:i + 100]) for i in range(0, rows, 100)])
+    for _ in range(3):
+        assert np.array_equal(m.mul(x), want)
+    m.close()
