@@ -478,7 +478,7 @@ __device__ __forceinline__ void fr_epilogue(const FrArgs &a, const FrOp &op, con
     if (!o.on) return;
     const int m = c.row0 + o.row;
     bool fits = true;
-    if (op.act == ACT_SILU) v = v * __frcp_rn(1.0f + __expf(-v));
+    if (op.act == ACT_SILU) v = silu_f(v);
     else if (op.act == ACT_RELU) v = fmaxf(v, 0.0f);
     if (op.epi == FR_EPI_PLANES) {
         __half h, l;
