@@ -83,13 +83,14 @@ struct GemmUnits {
     }
 };
 
-// Fused tail for 32 consecutive columns [nb, nb+32) of output row m.
+// Fused tail for COLS (16 or 32) consecutive columns from nb on of output row m.
 // Returns false if a value written as fp16 planes was out of their range (see split_h16).
-__device__ __forceinline__ bool gemm_epilogue_row(const GemmEpilogue &ep, float (&v)[32], int m, int nb, int N) {
+template <int COLS>
+__device__ __forceinline__ bool gemm_epilogue_row(const GemmEpilogue &ep, float (&v)[COLS], int m, int nb, int N) {
     bool fits = true;
-    const int nvalid = N - nb < 32 ? N - nb : 32, mode = gemm_mode(ep, nb), nh = gemm_plane_col(ep, nb);
+    const int nvalid = N - nb < COLS ? N - nb : COLS, mode = gemm_mode(ep, nb), nh = gemm_plane_col(ep, nb);
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
+    for (int j = 0; j < COLS; j++) {
         float x = v[j];
         if (ep.bias && j < nvalid) x += ep.bias[nb + j];
         if (ep.act == ACT_SILU) x = silu_f(x);
@@ -98,11 +99,11 @@ __device__ __forceinline__ bool gemm_epilogue_row(const GemmEpilogue &ep, float 
     }
     if (mode != OUT_H16) {
         float *o = ep.out + (size_t)m * ep.ldo + nb;
-        const bool vec = nvalid == 32 && ((reinterpret_cast<uintptr_t>(o) & 15) == 0);
+        const bool vec = nvalid == COLS && ((reinterpret_cast<uintptr_t>(o) & 15) == 0);
         if (mode == OUT_RESID) {
             if (vec) {
 #pragma unroll
-                for (int j = 0; j < 32; j += 4) {
+                for (int j = 0; j < COLS; j += 4) {
                     float4 r = *reinterpret_cast<float4 *>(o + j);
                     r.x += ep.alpha * v[j]; r.y += ep.alpha * v[j + 1];
                     r.z += ep.alpha * v[j + 2]; r.w += ep.alpha * v[j + 3];
@@ -110,26 +111,26 @@ __device__ __forceinline__ bool gemm_epilogue_row(const GemmEpilogue &ep, float 
                 }
             } else {
 #pragma unroll
-                for (int j = 0; j < 32; j++) if (j < nvalid) o[j] += ep.alpha * v[j];
+                for (int j = 0; j < COLS; j++) if (j < nvalid) o[j] += ep.alpha * v[j];
             }
         } else {
             if (vec) {
 #pragma unroll
-                for (int j = 0; j < 32; j += 4)
+                for (int j = 0; j < COLS; j += 4)
                     *reinterpret_cast<float4 *>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             } else {
 #pragma unroll
-                for (int j = 0; j < 32; j++) if (j < nvalid) o[j] = v[j];
+                for (int j = 0; j < COLS; j++) if (j < nvalid) o[j] = v[j];
             }
         }
     }
     if (mode == OUT_H16 || mode == OUT_F32_H16) {
         __half *ph = ep.out_hi + (size_t)m * ep.ldh + nh;
         __half *pl = ep.out_lo ? ep.out_lo + (size_t)m * ep.ldh + nh : nullptr;
-        const bool vec = nvalid == 32 && ((reinterpret_cast<uintptr_t>(ph) & 15) == 0);
+        const bool vec = nvalid == COLS && ((reinterpret_cast<uintptr_t>(ph) & 15) == 0);
         if (vec) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
+            for (int j = 0; j < COLS; j += 8) {
                 __align__(16) __half h[8], l[8];
 #pragma unroll
                 for (int i = 0; i < 8; i++) fits &= split_h16(v[j + i], h[i], l[i]);
@@ -138,7 +139,7 @@ __device__ __forceinline__ bool gemm_epilogue_row(const GemmEpilogue &ep, float 
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
+            for (int j = 0; j < COLS; j++) {
                 if (j < nvalid) {
                     __half h, l;
                     fits &= split_h16(v[j], h, l);
