@@ -191,9 +191,10 @@ __device__ __forceinline__ void gemm_block_stage(const float (&v)[16], int h, fl
     for (int j = 0; j < 4; j++) s4[lane * 8 + ((4 * h + j) ^ (lane & 7))] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
 }
 
-// after both halves were staged: the fused tail and the stores
+// after both halves were staged: the fused tail and the stores. pre(t, i): what comes before the bias at this lane's i-th place.
+template <typename F>
 __device__ __forceinline__ bool gemm_block_store(const GemmEpilogue &ep, const float4 (&res)[8], int m_base, int M,
-                                                 int nb, float *stage, int lane) {
+                                                 int nb, float *stage, int lane, F pre) {
     float4 *s4 = reinterpret_cast<float4 *>(stage);
     __syncwarp();
     const int q = lane & 7, r0 = lane >> 3, col = nb + q * 4, mode = gemm_mode(ep, nb), hcol = gemm_plane_col(ep, nb) + q * 4;
@@ -202,7 +203,7 @@ __device__ __forceinline__ bool gemm_block_store(const GemmEpilogue &ep, const f
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int r = i * 4 + r0, m = m_base + r;
-        float4 t = s4[r * 8 + (q ^ (r & 7))];
+        float4 t = pre(s4[r * 8 + (q ^ (r & 7))], i);
         if (ep.bias) { t.x += b.x; t.y += b.y; t.z += b.z; t.w += b.w; }
         t.x = gemm_act(ep, t.x); t.y = gemm_act(ep, t.y); t.z = gemm_act(ep, t.z); t.w = gemm_act(ep, t.w);
         if (m >= M) continue;

@@ -247,7 +247,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
                             }
                             gemm_block_stage(v, h, stage, lane);
                         }
-                        fits &= gemm_block_store(ep, res, m0 + lg * 32, M, nb, stage, lane);
+                        fits &= gemm_block_store(ep, res, m0 + lg * 32, M, nb, stage, lane, [](float4 t, int) { return t; });
                         continue;
                     }
                     float v[32];
