@@ -121,6 +121,19 @@ __device__ __forceinline__ bool split_h16(float v, __half &hi, __half &lo) {
     return fabsf(v) < H16_MAX;
 }
 
+// The same for two values, and for four: neighbours share the conversions.
+__device__ __forceinline__ bool split_h16x2(float x, float y, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn((x - f.x) * H16_LO_SCALE, (y - f.y) * H16_LO_SCALE);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = *reinterpret_cast<const uint32_t *>(&l);
+    return (fabsf(x) < H16_MAX) & (fabsf(y) < H16_MAX);
+}
+__device__ __forceinline__ bool split_h16x4(float4 v, uint2 &hi, uint2 &lo) {
+    return split_h16x2(v.x, v.y, hi.x, lo.x) & split_h16x2(v.z, v.w, hi.y, lo.y);
+}
+
 // Stable sigmoid: never exponentiates a positive argument (the reference's
 // mynah_asr_sigmoid, src/qmat.h:31-35).
 __device__ __forceinline__ float sigmoid_stable(float x) {

@@ -75,10 +75,12 @@ ln_reg_kernel(const float *__restrict__ x, const float *__restrict__ w, const fl
               float *__restrict__ out, __half *__restrict__ hi, __half *__restrict__ lo, int8_t *__restrict__ q8,
               float *__restrict__ sx8, int T, int act) {
     chain_trigger();
-    chain_wait();
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    LnVectors<NV> p;                        // constants: they arrive while the kernels in front end
+    p.load(w, b, lane);
+    chain_wait();
     if (row >= T) return;
-    ln_row<NV, false>(x, w, b, out, hi, lo, q8, sx8, row, act, lane);
+    ln_row<NV, false>(x, p, out, hi, lo, q8, sx8, row, act, lane);
 }
 
 int layer_norm(const float *x, const float *w, const float *b, float *out_f32, H16 out_h, int T, int d, int act,
@@ -187,11 +189,10 @@ glu_dw_kernel(const float *__restrict__ h2, const float *__restrict__ dw_w, cons
             const float y[4] = {silu_f(acc[i].x * sc.x + sh.x), silu_f(acc[i].y * sc.y + sh.y), silu_f(acc[i].z * sc.z + sh.z),
                                 silu_f(acc[i].w * sc.w + sh.w)};
             if (hi) {
-                __align__(8) __half h[4], l[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) split_h16(y[e], h[e], l[e]);
-                *reinterpret_cast<uint2 *>(hi + o) = *reinterpret_cast<const uint2 *>(h);
-                if (lo) *reinterpret_cast<uint2 *>(lo + o) = *reinterpret_cast<const uint2 *>(l);
+                uint2 h, l;
+                split_h16x4(make_float4(y[0], y[1], y[2], y[3]), h, l);
+                *reinterpret_cast<uint2 *>(hi + o) = h;
+                if (lo) *reinterpret_cast<uint2 *>(lo + o) = l;
             }
             if (out) *reinterpret_cast<float4 *>(out + o) = make_float4(y[0], y[1], y[2], y[3]);
         } else {

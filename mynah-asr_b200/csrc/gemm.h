@@ -145,11 +145,11 @@ __device__ __forceinline__ bool gemm_epilogue_row(const GemmEpilogue &ep, float 
         if (vec) {
 #pragma unroll
             for (int j = 0; j < COLS; j += 8) {
-                __align__(16) __half h[8], l[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) fits &= split_h16(v[j + i], h[i], l[i]);
-                *reinterpret_cast<uint4 *>(ph + j) = *reinterpret_cast<uint4 *>(h);
-                if (pl) *reinterpret_cast<uint4 *>(pl + j) = *reinterpret_cast<uint4 *>(l);
+                uint4 h, l;
+                fits &= split_h16x2(v[j], v[j + 1], h.x, l.x) & split_h16x2(v[j + 2], v[j + 3], h.y, l.y) &
+                        split_h16x2(v[j + 4], v[j + 5], h.z, l.z) & split_h16x2(v[j + 6], v[j + 7], h.w, l.w);
+                *reinterpret_cast<uint4 *>(ph + j) = h;
+                if (pl) *reinterpret_cast<uint4 *>(pl + j) = l;
             }
         } else {
 #pragma unroll
@@ -252,16 +252,12 @@ __device__ __forceinline__ bool gemm_block_store(const GemmEpilogue &ep, const f
         const size_t off = (size_t)(m_base + r0) * ep.ldh + hcol;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            __half h0, h1, h2, h3, l0, l1, l2, l3;
-            bool f = split_h16(t[i].x, h0, l0);
-            f &= split_h16(t[i].y, h1, l1);
-            f &= split_h16(t[i].z, h2, l2);
-            f &= split_h16(t[i].w, h3, l3);
+            uint2 h, l;
+            const bool f = split_h16x4(t[i], h, l);
             if (i * 4 >= left) continue;
             fits &= f;
-            const __half2 ha = __halves2half2(h0, h1), hb = __halves2half2(h2, h3), la = __halves2half2(l0, l1), lb = __halves2half2(l2, l3);
-            *reinterpret_cast<uint2 *>(ep.out_hi + off + (size_t)(i * 4) * ep.ldh) = make_uint2(*reinterpret_cast<const uint32_t *>(&ha), *reinterpret_cast<const uint32_t *>(&hb));
-            if (ep.out_lo) *reinterpret_cast<uint2 *>(ep.out_lo + off + (size_t)(i * 4) * ep.ldh) = make_uint2(*reinterpret_cast<const uint32_t *>(&la), *reinterpret_cast<const uint32_t *>(&lb));
+            *reinterpret_cast<uint2 *>(ep.out_hi + off + (size_t)(i * 4) * ep.ldh) = h;
+            if (ep.out_lo) *reinterpret_cast<uint2 *>(ep.out_lo + off + (size_t)(i * 4) * ep.ldh) = l;
         }
     }
     __syncwarp();                                                   // the stage is free for the next block

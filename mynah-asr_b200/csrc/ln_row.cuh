@@ -39,52 +39,71 @@ __device__ __forceinline__ void ln_stats(const float4 (&v)[NV], int K, float &mu
     inv = (float)rsqrt(ve);
 }
 
+// weight and bias of a lane's columns
+template <int NV>
+struct LnVectors {
+    float4 w[NV], b[NV];
+    __device__ __forceinline__ void load(const float *__restrict__ pw, const float *__restrict__ pb, int lane) {
+#pragma unroll
+        for (int j = 0; j < NV; j++) { w[j] = reinterpret_cast<const float4 *>(pw)[lane + 32 * j]; b[j] = reinterpret_cast<const float4 *>(pb)[lane + 32 * j]; }
+    }
+};
+
+// Every step over the whole row before the next one, the choice of outputs outside of the loops, neighbours converted in pairs,
+// and (ln_reg_kernel) weight and bias on their way before the kernels in front have ended: with the outputs chosen value by
+// value a voice command took 1.940 ms instead of 1.837 (85 of its 267 launches are LayerNorms), 15 s on 24 layers 6.09 instead
+// of 5.74, eight utterances with int8 activations 5.80 instead of 5.40.
+template <int NV, bool L2>
+__device__ __forceinline__ void ln_row(const float *__restrict__ x, const LnVectors<NV> &p, float *__restrict__ out, __half *__restrict__ hi,
+                                       __half *__restrict__ lo, int8_t *__restrict__ q8, float *__restrict__ sx8, int row, int act, int lane) {
+    constexpr int d = NV * 128;
+    const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)row * d) + lane;
+    float4 v[NV];
+#pragma unroll
+    for (int j = 0; j < NV; j++) v[j] = L2 ? __ldcg(xr + 32 * j) : xr[32 * j];
+    float muf, inv;
+    ln_stats<NV>(v, d, muf, inv);
+#pragma unroll
+    for (int j = 0; j < NV; j++)            // the finished values replace the inputs in the registers
+        v[j] = make_float4(((v[j].x - muf) * inv) * p.w[j].x + p.b[j].x, ((v[j].y - muf) * inv) * p.w[j].y + p.b[j].y,
+                           ((v[j].z - muf) * inv) * p.w[j].z + p.b[j].z, ((v[j].w - muf) * inv) * p.w[j].w + p.b[j].w);
+    if (act == ACT_SILU)
+#pragma unroll
+        for (int j = 0; j < NV; j++) v[j] = make_float4(silu_f(v[j].x), silu_f(v[j].y), silu_f(v[j].z), silu_f(v[j].w));
+    if (q8) {
+        float amax = 0.0f;
+#pragma unroll
+        for (int j = 0; j < NV; j++) amax = fmaxf(fmaxf(amax, fmaxf(fabsf(v[j].x), fabsf(v[j].y))), fmaxf(fabsf(v[j].z), fabsf(v[j].w)));
+        amax = warp_max(amax);
+        const float qinv = amax > 0.0f ? 127.0f / amax : 0.0f;
+        if (lane == 0) sx8[row] = amax > 0.0f ? amax / 127.0f : 0.0f;
+        char4 *o = reinterpret_cast<char4 *>(q8 + (size_t)row * d) + lane;
+#pragma unroll
+        for (int j = 0; j < NV; j++) o[32 * j] = make_char4(act_q8(v[j].x, qinv), act_q8(v[j].y, qinv), act_q8(v[j].z, qinv), act_q8(v[j].w, qinv));
+    }
+    if (out) {
+        float4 *o = reinterpret_cast<float4 *>(out + (size_t)row * d) + lane;
+#pragma unroll
+        for (int j = 0; j < NV; j++) o[32 * j] = v[j];
+    }
+    if (!hi) return;
+    uint2 *ph = reinterpret_cast<uint2 *>(hi + (size_t)row * d) + lane, *pl = reinterpret_cast<uint2 *>(lo + (size_t)row * d) + lane;
+    uint2 h[NV], l[NV];
+#pragma unroll
+    for (int j = 0; j < NV; j++) split_h16x4(v[j], h[j], l[j]);
+#pragma unroll
+    for (int j = 0; j < NV; j++) ph[32 * j] = h[j];
+    if (lo)
+#pragma unroll
+        for (int j = 0; j < NV; j++) pl[32 * j] = l[j];
+}
 template <int NV, bool L2>
 __device__ __forceinline__ void ln_row(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ b,
                                        float *__restrict__ out, __half *__restrict__ hi, __half *__restrict__ lo, int8_t *__restrict__ q8,
                                        float *__restrict__ sx8, int row, int act, int lane) {
-    constexpr int d = NV * 128;
-    const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)row * d);
-    float4 v[NV];
-#pragma unroll
-    for (int j = 0; j < NV; j++) v[j] = L2 ? __ldcg(xr + lane + 32 * j) : xr[lane + 32 * j];
-    float muf, inv;
-    ln_stats<NV>(v, d, muf, inv);
-    float amax = 0.0f;
-#pragma unroll
-    for (int j = 0; j < NV; j++) {          // the finished values replace the inputs in the registers
-        const int i = lane + 32 * j;
-        const float4 ww = reinterpret_cast<const float4 *>(w)[i];
-        const float4 bb = reinterpret_cast<const float4 *>(b)[i];
-        float y[4] = {((v[j].x - muf) * inv) * ww.x + bb.x, ((v[j].y - muf) * inv) * ww.y + bb.y,
-                      ((v[j].z - muf) * inv) * ww.z + bb.z, ((v[j].w - muf) * inv) * ww.w + bb.w};
-        if (act == ACT_SILU) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) y[e] = silu_f(y[e]);
-        }
-        v[j] = make_float4(y[0], y[1], y[2], y[3]);
-        amax = fmaxf(fmaxf(amax, fmaxf(fabsf(y[0]), fabsf(y[1]))), fmaxf(fabsf(y[2]), fabsf(y[3])));
-    }
-    float qinv = 0.0f;
-    if (q8) {
-        amax = warp_max(amax);
-        qinv = amax > 0.0f ? 127.0f / amax : 0.0f;
-        if (lane == 0) sx8[row] = amax > 0.0f ? amax / 127.0f : 0.0f;
-    }
-#pragma unroll
-    for (int j = 0; j < NV; j++) {
-        const int i = lane + 32 * j;
-        const float y[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-        if (q8) reinterpret_cast<char4 *>(q8 + (size_t)row * d)[i] = make_char4(act_q8(y[0], qinv), act_q8(y[1], qinv), act_q8(y[2], qinv), act_q8(y[3], qinv));
-        if (out) reinterpret_cast<float4 *>(out + (size_t)row * d)[i] = make_float4(y[0], y[1], y[2], y[3]);
-        if (hi) {
-            __align__(8) __half h[4], l[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) split_h16(y[e], h[e], l[e]);
-            reinterpret_cast<uint2 *>(hi + (size_t)row * d)[i] = *reinterpret_cast<uint2 *>(h);
-            if (lo) reinterpret_cast<uint2 *>(lo + (size_t)row * d)[i] = *reinterpret_cast<uint2 *>(l);
-        }
-    }
+    LnVectors<NV> p;
+    p.load(w, b, lane);
+    ln_row<NV, L2>(x, p, out, hi, lo, q8, sx8, row, act, lane);
 }
 
 }  // namespace mb
