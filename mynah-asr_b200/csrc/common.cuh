@@ -207,6 +207,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
     return true;
 }
 
+// The same by a whole warp, with one answer for all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+        if (__any_sync(0xffffffffu, clock64() - t0 > (1ll << 31))) return false;
+    }
+    return true;
+}
+
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
 }
@@ -216,6 +226,15 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *m, int
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
+}
+
+// The warp's number as a value that the compiler knows to be the same in all lanes, and one lane of a converged warp: what a warp
+// computes for an instruction that one lane issues then stays in uniform registers, which tcgen05 and TMA take their operands from.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t on;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(on));
+    return on != 0;
 }
 
 // ------------------------------------------------------------------- tcgen05

@@ -74,7 +74,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint64_t *acc_empty = acc_full + 2;                // [2] epilogue -> MMA
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int num_k = K / I8_BK;
     const GemmUnits units(M, N, BN, gridDim.x);
     const int total = units.total;
@@ -93,43 +93,50 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t tmem_base = *tmem_slot;
     chain_trigger();       // not before the allocation: a successor placed on this SM must not be first to take tensor memory
 
-    if (warp == 0 && lane == 0) {
-        // ---------------------------------------------------------- TMA producer
-        int it = 0;
+    if (warp == 0) {
+        // ---------------------------------------------------------- TMA producer (one lane; the warp goes along)
+        int s = 0, filled = 0;                         // ring position, k-blocks issued so far
+        uint32_t ph = 1;
         bool ok = true;
         int ahead = 0;                                 // B tiles (weights) asked for before the kernels in front have finished
         if (blockIdx.x < total) {
             int m0, n0, width;
             units.at(blockIdx.x, BN, m0, n0, width);
             ahead = num_k < Cfg::STAGES ? num_k : Cfg::STAGES;
-            for (int s = 0; s < ahead; s++) {
-                mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
-                tma_load_2d(tiles + s * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmB, s * I8_BK, n0, &full_bar[s]);
-            }
+            if (elect_one())
+                for (int i = 0; i < ahead; i++) {
+                    mbar_expect_tx(&full_bar[i], Cfg::STAGE_BYTES);
+                    tma_load_2d(tiles + i * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmB, i * I8_BK, n0, &full_bar[i]);
+                }
+            __syncwarp();
         }
         chain_wait();
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
             int m0, n0, width;
             units.at(tile, BN, m0, n0, width);               // a strip still loads BN rows of B: the MMAs read the first `width`
-            for (int kb = 0; kb < num_k; kb++, it++) {
-                const int s = it % Cfg::STAGES;
-                const uint32_t ph = (it / Cfg::STAGES) & 1;
-                if (!mbar_wait(&empty_bar[s], ph ^ 1)) { ok = false; break; }
-                uint8_t *st = tiles + s * Cfg::STAGE_BYTES;
-                if (it >= ahead) mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
-                tma_load_2d(st, &tmA, kb * I8_BK, m0, &full_bar[s]);
-                if (it >= ahead) tma_load_2d(st + Cfg::A_BYTES, &tmB, kb * I8_BK, n0, &full_bar[s]);
+            for (int kb = 0; kb < num_k; kb++, filled++) {
+                ok = mbar_wait_warp(&empty_bar[s], ph);
+                if (!ok) break;
+                if (elect_one()) {
+                    uint8_t *st = tiles + s * Cfg::STAGE_BYTES;
+                    if (filled >= ahead) mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
+                    tma_load_2d(st, &tmA, kb * I8_BK, m0, &full_bar[s]);
+                    if (filled >= ahead) tma_load_2d(st + Cfg::A_BYTES, &tmB, kb * I8_BK, n0, &full_bar[s]);
+                }
+                __syncwarp();
+                if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
             }
         }
         if (!ok) {
-            atomicExch(status, ST_TIMEOUT_PRODUCER);
+            if (lane == 0) atomicExch(status, ST_TIMEOUT_PRODUCER);
             // let copies already in flight land before the CTA's shared memory goes away
-            for (int j = it > Cfg::STAGES ? it - Cfg::STAGES : 0; j < it; j++)
-                mbar_wait(&full_bar[j % Cfg::STAGES], (j / Cfg::STAGES) & 1);
+            for (int j = filled > Cfg::STAGES ? filled - Cfg::STAGES : 0; j < filled; j++)
+                mbar_wait_warp(&full_bar[j % Cfg::STAGES], (j / Cfg::STAGES) & 1);
         }
-    } else if (warp == 1 && lane == 0) {
-        // ------------------------------------------------------------ MMA issuer
-        int it = 0, lt = 0;
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer (one lane; the warp goes along)
+        int s = 0, lt = 0;
+        uint32_t ph = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, lt++) {
             int m0, n0, width;
@@ -137,25 +144,27 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const uint32_t idesc = umma_idesc_i8(GEMM_BM, width);
             const int buf = lt & 1;
             const uint32_t acc = tmem_base + buf * BN;
-            if (!mbar_wait(&acc_empty[buf], ((lt >> 1) & 1) ^ 1)) { ok = false; break; }
+            ok = mbar_wait_warp(&acc_empty[buf], ((lt >> 1) & 1) ^ 1);
+            if (!ok) break;
             tc_fence_after();
-            for (int kb = 0; kb < num_k; kb++, it++) {
-                const int s = it % Cfg::STAGES;
-                const uint32_t ph = (it / Cfg::STAGES) & 1;
-                if (!mbar_wait(&full_bar[s], ph)) { ok = false; break; }
+            for (int kb = 0; kb < num_k; kb++) {
+                ok = mbar_wait_warp(&full_bar[s], ph);
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t a = smem_u32(tiles + s * Cfg::STAGE_BYTES);
-                const uint32_t b = a + Cfg::A_BYTES;
+                if (elect_one()) {
+                    const uint32_t t = smem_u32(tiles + s * Cfg::STAGE_BYTES);
+                    const uint64_t a = umma_desc_sw128(t), b = umma_desc_sw128(t + Cfg::A_BYTES);
 #pragma unroll
-                for (int kk = 0; kk < I8_BK / 32; kk++) {
-                    const uint32_t off = kk * 32;   // 32 int8 = 32 bytes inside the swizzle atom
-                    tc_mma_i8(acc, umma_desc_sw128(a + off), umma_desc_sw128(b + off), idesc, (kb | kk) != 0);
+                    for (int kk = 0; kk < I8_BK / 32; kk++)  // 32 int8 = 32 bytes inside the swizzle atom, in units of 16
+                        tc_mma_i8(acc, a + kk * 2, b + kk * 2, idesc, kk > 0 || kb > 0);
+                    tc_commit(&empty_bar[s]);                // frees the stage once these MMAs have read it
+                    if (kb + 1 == num_k) tc_commit(&acc_full[buf]);
                 }
-                tc_commit(&empty_bar[s]);           // frees the stage once these MMAs have read it
+                __syncwarp();
+                if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
             }
-            tc_commit(&acc_full[buf]);              // accumulator complete (or abandoned)
         }
-        if (!ok) atomicExch(status, ST_TIMEOUT_MMA);
+        if (!ok && lane == 0) atomicExch(status, ST_TIMEOUT_MMA);
     } else if (warp >= 2) {
         // -------------------------------------------------------------- epilogue
         const int lg = warp & 3;                       // TMEM lane group this warp may read

@@ -13,6 +13,12 @@
 //     epilogue adds the second accumulator back times 2^-11), so the product carries
 //     ~22 significant bits per operand (f32-grade parity with the reference's sgemm);
 //     with NTERMS=1 only hi*hi (fast mode);
+//   * the issuing warps walk their loops whole and elect the lane that issues (warp_index, elect_one): operands of tcgen05 and TMA
+//     then are uniform registers. As code of one lane of a diverged warp every MMA waited for its operands to be moved there:
+//     [12000 x 1024 x 4096] took 223 us instead of 202, 47 rows of it 33 instead of 25; a voice command on 17 layers 1.83 ms
+//     instead of 1.60, 15 s on 24 layers 5.73 instead of 5.06, sixteen minutes 60.6 instead of 58.7. What bounds a k-step now is
+//     shared memory (TMA's writes and the MMAs' reads at 128 bytes a cycle): 128 x 128 columns 295 cycles of 312 so computed, 32
+//     columns 127 of 133;
 //   * the kernel is persistent (one CTA per SM walks the output tiles) and the
 //     accumulators are double-buffered in TMEM, so the epilogue of one tile overlaps
 //     the MMAs of the next; eight epilogue warps read the accumulator with tcgen05.ld
@@ -77,7 +83,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
     uint64_t *acc_empty = acc_full + 2;                // [2] epilogue -> MMA
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int num_k = K / BK;
     const GemmUnits units(M, N, BN, gridDim.x);
     const int total = units.total;
@@ -97,50 +103,54 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
     const uint32_t tmem_base = *tmem_slot;
     chain_trigger();       // not before the allocation: a successor placed on this SM must not be first to take tensor memory
 
-    if (warp == 0 && lane == 0) {
-        // ---------------------------------------------------------- TMA producer
-        int it = 0;                                    // k-blocks issued so far (ring position)
+    if (warp == 0) {
+        // ---------------------------------------------------------- TMA producer (one lane; the warp goes along)
+        int s = 0, filled = 0;                         // ring position, k-blocks issued so far
+        uint32_t ph = 1;
         bool ok = true;
+        auto load_b = [&](int s, int kb, int n0) {
+            uint8_t *bt = tiles + s * Cfg::STAGE_BYTES + Cfg::NPLANES * Cfg::A_BYTES;
+            tma_load_2d(bt, &tmB_hi, kb * BK, n0, &full_bar[s]);
+            if (NTERMS > 1) tma_load_2d(bt + Cfg::B_BYTES, &tmB_lo, kb * BK, n0, &full_bar[s]);
+        };
         // the first ring of B tiles (weights) is asked for before the kernels in front have finished
         int ahead = 0;
         if (blockIdx.x < total) {
             int m0, n0, width;
             units.at(blockIdx.x, BN, m0, n0, width);
             ahead = num_k < Cfg::STAGES ? num_k : Cfg::STAGES;
-            for (int s = 0; s < ahead; s++) {
-                uint8_t *bt = tiles + s * Cfg::STAGE_BYTES + Cfg::NPLANES * Cfg::A_BYTES;
-                mbar_expect_tx(&full_bar[s], stage_tx);
-                tma_load_2d(bt, &tmB_hi, s * BK, n0, &full_bar[s]);
-                if (NTERMS > 1) tma_load_2d(bt + Cfg::B_BYTES, &tmB_lo, s * BK, n0, &full_bar[s]);
-            }
+            if (elect_one())
+                for (int i = 0; i < ahead; i++) { mbar_expect_tx(&full_bar[i], stage_tx); load_b(i, i, n0); }
+            __syncwarp();
         }
         chain_wait();
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
             int m0, n0, width;
             units.at(tile, BN, m0, n0, width);               // a strip still loads BN rows of B: the MMAs read the first `width`
-            for (int kb = 0; kb < num_k; kb++, it++) {
-                const int s = it % Cfg::STAGES;
-                const uint32_t ph = (it / Cfg::STAGES) & 1;
-                if (!mbar_wait(&empty_bar[s], ph ^ 1)) { ok = false; break; }
-                uint8_t *st = tiles + s * Cfg::STAGE_BYTES;
-                if (it >= ahead) mbar_expect_tx(&full_bar[s], stage_tx);
-                tma_load_2d(st, &tmA_hi, kb * BK, m0, &full_bar[s]);
-                if (NTERMS > 1) tma_load_2d(st + Cfg::A_BYTES, &tmA_lo, kb * BK, m0, &full_bar[s]);
-                if (it < ahead) continue;
-                uint8_t *bt = st + Cfg::NPLANES * Cfg::A_BYTES;
-                tma_load_2d(bt, &tmB_hi, kb * BK, n0, &full_bar[s]);
-                if (NTERMS > 1) tma_load_2d(bt + Cfg::B_BYTES, &tmB_lo, kb * BK, n0, &full_bar[s]);
+            for (int kb = 0; kb < num_k; kb++, filled++) {
+                ok = mbar_wait_warp(&empty_bar[s], ph);
+                if (!ok) break;
+                if (elect_one()) {
+                    uint8_t *st = tiles + s * Cfg::STAGE_BYTES;
+                    if (filled >= ahead) mbar_expect_tx(&full_bar[s], stage_tx);
+                    tma_load_2d(st, &tmA_hi, kb * BK, m0, &full_bar[s]);
+                    if (NTERMS > 1) tma_load_2d(st + Cfg::A_BYTES, &tmA_lo, kb * BK, m0, &full_bar[s]);
+                    if (filled >= ahead) load_b(s, kb, n0);
+                }
+                __syncwarp();
+                if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
             }
         }
         if (!ok) {
-            atomicExch(status, ST_TIMEOUT_PRODUCER);
+            if (lane == 0) atomicExch(status, ST_TIMEOUT_PRODUCER);
             // let copies already in flight land before the CTA's shared memory goes away
-            for (int j = it > Cfg::STAGES ? it - Cfg::STAGES : 0; j < it; j++)
-                mbar_wait(&full_bar[j % Cfg::STAGES], (j / Cfg::STAGES) & 1);
+            for (int j = filled > Cfg::STAGES ? filled - Cfg::STAGES : 0; j < filled; j++)
+                mbar_wait_warp(&full_bar[j % Cfg::STAGES], (j / Cfg::STAGES) & 1);
         }
-    } else if (warp == 1 && lane == 0) {
-        // ------------------------------------------------------------ MMA issuer
-        int it = 0, lt = 0;
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer (one lane; the warp goes along)
+        int s = 0, lt = 0;
+        uint32_t ph = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, lt++) {
             int m0, n0, width;
@@ -149,42 +159,45 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
             const int buf = lt & 1;
             const uint32_t acc = tmem_base + buf * Cfg::ACC_COLS;
             // the epilogue must have drained this accumulator (two tiles ago)
-            if (!mbar_wait(&acc_empty[buf], ((lt >> 1) & 1) ^ 1)) { ok = false; break; }
+            ok = mbar_wait_warp(&acc_empty[buf], ((lt >> 1) & 1) ^ 1);
+            if (!ok) break;
             tc_fence_after();
-            for (int kb = 0; kb < num_k; kb++, it++) {
-                const int s = it % Cfg::STAGES;
-                const uint32_t ph = (it / Cfg::STAGES) & 1;
-                if (!mbar_wait(&full_bar[s], ph)) { ok = false; break; }
+            for (int kb = 0; kb < num_k; kb++) {
+                ok = mbar_wait_warp(&full_bar[s], ph);
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t a_hi = smem_u32(tiles + s * Cfg::STAGE_BYTES);
-                const uint32_t a_lo = a_hi + Cfg::A_BYTES;
-                const uint32_t b_hi = a_hi + Cfg::NPLANES * Cfg::A_BYTES;
-                const uint32_t b_lo = b_hi + Cfg::B_BYTES;
+                if (elect_one()) {
+                    const uint32_t a = smem_u32(tiles + s * Cfg::STAGE_BYTES);
+                    const uint64_t a_hi = umma_desc_sw128(a), a_lo = umma_desc_sw128(a + Cfg::A_BYTES);
+                    const uint64_t b_hi = umma_desc_sw128(a + Cfg::NPLANES * Cfg::A_BYTES), b_lo = umma_desc_sw128(a + Cfg::NPLANES * Cfg::A_BYTES + Cfg::B_BYTES);
 #pragma unroll
-                for (int kk = 0; kk < BK / 16; kk++) {
-                    const uint32_t off = kk * 32;   // 16 fp16 = 32 bytes inside the swizzle atom
-                    const uint64_t da = umma_desc_sw128(a_hi + off), db = umma_desc_sw128(b_hi + off);
-                    if (NTERMS == 1) {
-                        tc_mma_f16(acc, da, db, idesc, (kb | kk) != 0);
-                        continue;
+                    for (int kk = 0; kk < BK / 16; kk++) {
+                        const uint64_t k = kk * 2;           // 16 fp16 = 32 bytes inside the swizzle atom, in units of 16
+                        const uint32_t more = kk > 0 || kb > 0;
+                        if (NTERMS == 1) {
+                            tc_mma_f16(acc, a_hi + k, b_hi + k, idesc, more);
+                            continue;
+                        }
+                        // The hi and the lo rows of B lie one below the other, as the two accumulators lie side by side: hi*hi and
+                        // hi*lo can be one MMA of twice the width. With narrow tiles the MMA's fixed time is what counts (3.7 s of
+                        // audio through 17 layers of 512: 2.24 -> 2.14 ms); from 64 columns on every MMA then waits for both
+                        // accumulators of the one before it, which costs more than the second read of A (a minute through 24
+                        // layers of 1024: 14.4 -> 15.1 ms). The first step has to clear both accumulators, and a strip's hi and lo
+                        // rows do not touch.
+                        const bool both = BN == 32 && width == BN && more;
+                        if (!both) tc_mma_f16(acc, a_hi + k, b_hi + k, idesc, more);
+                        tc_mma_f16(acc + BN, a_lo + k, b_hi + k, idesc, more);
+                        if (both) tc_mma_f16(acc, a_hi + k, b_hi + k, idesc_both, 1);
+                        else tc_mma_f16(acc + BN, a_hi + k, b_lo + k, idesc, 1);
                     }
-                    // The hi and the lo rows of B lie one below the other, as the two accumulators lie side by side: hi*hi and
-                    // hi*lo can be one MMA of twice the width. With narrow tiles the MMA's fixed time is what counts (3.7 s of
-                    // audio through 17 layers of 512: 2.24 -> 2.14 ms); from 64 columns on every MMA then waits for both
-                    // accumulators of the one before it, which costs more than the second read of A (a minute through 24
-                    // layers of 1024: 14.4 -> 15.1 ms). The first step has to clear both accumulators, and a strip's hi and lo
-                    // rows do not touch.
-                    const bool both = BN == 32 && width == BN && (kb | kk) != 0;
-                    if (!both) tc_mma_f16(acc, da, db, idesc, (kb | kk) != 0);
-                    tc_mma_f16(acc + BN, umma_desc_sw128(a_lo + off), db, idesc, (kb | kk) != 0);
-                    if (both) tc_mma_f16(acc, da, db, idesc_both, 1);
-                    else tc_mma_f16(acc + BN, da, umma_desc_sw128(b_lo + off), idesc, 1);
+                    tc_commit(&empty_bar[s]);                // frees the stage once these MMAs have read it
+                    if (kb + 1 == num_k) tc_commit(&acc_full[buf]);
                 }
-                tc_commit(&empty_bar[s]);           // frees the stage once these MMAs have read it
+                __syncwarp();
+                if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
             }
-            tc_commit(&acc_full[buf]);              // accumulator complete (or abandoned)
         }
-        if (!ok) atomicExch(status, ST_TIMEOUT_MMA);
+        if (!ok && lane == 0) atomicExch(status, ST_TIMEOUT_MMA);
     } else if (warp >= 2) {
         // -------------------------------------------------------------- epilogue
         const int lg = warp & 3;                       // TMEM lane group this warp may read
