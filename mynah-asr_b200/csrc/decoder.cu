@@ -216,6 +216,18 @@ __device__ __forceinline__ void stage_planes(__half *xhi, __half *xlo, int xs, i
     }
 }
 
+// sigmoid_stable without its branch and the division's, so that a cell's gates overlap: one exponential, a reciprocal approximation
+// with Newton's step, and the quotient's rounding step. Its error against double is that of sigmoid_stable (2.45e-7 at most,
+// 3.1e-8 in the mean over +-87). 244 steps of one utterance (a minute of audio): 10.70 ms a call become 10.48.
+__device__ __forceinline__ float dec_sigmoid(float x) {
+    const float e = expf(-fabsf(x)), num = x >= 0.0f ? 1.0f : e, den = 1.0f + e;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den));
+    r = fmaf(r, fmaf(-den, r, 1.0f), r);
+    const float y = num * r;
+    return fmaf(fmaf(-den, y, num), r, y);
+}
+
 // What every CTA knows of the utterances, kept in step by applying the same rule to the same maxima
 struct GreedyShared {
     int t[DEC_MAX_B], len[DEC_MAX_B], off[DEC_MAX_B];            // frame, frames, first row in enc
@@ -348,10 +360,10 @@ __device__ __forceinline__ void lstm_phase(const GreedyDev &p, const GreedyShare
             }
             const size_t o = (size_t)b * H + unit;
             if (sh.emit[b]) {
-                const float cn = sigmoid_stable(z[1]) * cprev + sigmoid_stable(z[0]) * tanhf(z[2]);
+                const float cn = dec_sigmoid(z[1]) * cprev + dec_sigmoid(z[0]) * tanhf(z[2]);
                 cc[o] = cn;
                 __half hh, hl;
-                split_h16(sigmoid_stable(z[3]) * tanhf(cn), hh, hl);
+                split_h16(dec_sigmoid(z[3]) * tanhf(cn), hh, hl);
                 hnew_hi[o] = hh; hnew_lo[o] = hl;
             } else {
                 hnew_hi[o] = hold_hi[o]; hnew_lo[o] = hold_lo[o];
