@@ -142,16 +142,18 @@ __device__ __forceinline__ float sigmoid_stable(float x) {
     return e / (1.0f + e);
 }
 // The same function for the bulk element-wise passes (GLU, SiLU after the conv norm, the contractions' epilogues): one ex2, one
-// reciprocal approximation and Newton's step on it, no branch. Below -87 the result stays that of -87, 1.6e-38: the reciprocal
-// would leave the normal range. NaN stays NaN. Relative error against double 1.4e-7 for x >= 0 and 3.8e-6 below (the exponential's),
-// the same value as __frcp_rn(1 + exp(-x)) for every x within +-87; but that has a branch for special operands, which keeps the
-// values of a thread from interleaving: the encoder over twelve ragged utterances in the single-product mode took 4.47 ms
-// instead of 4.23, over eight with int8 activations 7.05 instead of 6.40, one minute on 24 layers 11.90 instead of 11.70.
+// reciprocal approximation and Newton's step on it, no branch. Below -87 (1.6e-38) it is 0: the reciprocal would leave the normal
+// range, and x * sigmoid(x) has to vanish for large x, too. NaN stays NaN. Relative error against double 1.4e-7 for x >= 0 and
+// 3.8e-6 below (the exponential's), the same value as __frcp_rn(1 + exp(-x)) for every x within +-87; but that has a branch for
+// special operands, which keeps the values of a thread from interleaving: the encoder over twelve ragged utterances in the
+// single-product mode took 4.47 ms instead of 4.23, over eight with int8 activations 7.05 instead of 6.40, one minute on 24 layers
+// 11.90 instead of 11.70.
 __device__ __forceinline__ float sigmoid_fast(float x) {
-    const float d = 1.0f + __expf(-x > 87.0f ? 87.0f : -x);
+    const float d = 1.0f + __expf(-x);
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    return fmaf(r, fmaf(-d, r, 1.0f), r);
+    r = fmaf(r, fmaf(-d, r, 1.0f), r);
+    return x < -87.0f ? 0.0f : r;
 }
 __device__ __forceinline__ float silu_f(float x) { return x * sigmoid_fast(x); }
 

@@ -181,3 +181,24 @@ def test_tcgen05_attention_long_segments(gpu_pkg, synth):
         assert rel(o, plain.encoder_forward(f)) < 1e-4
     for m in (tc, plain, tiled):
         m.close()
+
+
+def test_silu_vanishes_below(gpu_pkg, synth):
+    """x * sigmoid(x) of every negative number that float32 has: 0 from -104 on, in the feed-forward contraction and behind the
+    conv norm, so that shifts of -200 and of -3e38 give the same bits."""
+    cfg, tensors = cases.build(synth, "ctc_bias")
+    x = np.random.default_rng(5).standard_normal((31, cfg.d_model), dtype=np.float32)
+    outs = []
+    for shift in (-200.0, -3e38):
+        shifted, names = {}, 0
+        for name, t in tensors.items():
+            if name.endswith(("feed_forward1.linear1.bias", "conv.norm.bias")):
+                data = t.raw.view(np.float32).copy()
+                data[::7] = shift
+                t, names = synth.Tensor(t.name, t.ggml_type, t.shape, data), names + 1
+            shifted[name] = t
+        assert names == 2
+        dm = cases.device_model(gpu_pkg, synth, cfg, shifted)
+        outs.append(dm.encoder_layer(0, x))
+        dm.close()
+    assert np.isfinite(outs[0]).all() and np.array_equal(*outs)
