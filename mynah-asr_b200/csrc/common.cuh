@@ -134,14 +134,7 @@ __device__ __forceinline__ bool split_h16x4(float4 v, uint2 &hi, uint2 &lo) {
     return split_h16x2(v.x, v.y, hi.x, lo.x) & split_h16x2(v.z, v.w, hi.y, lo.y);
 }
 
-// Stable sigmoid: never exponentiates a positive argument (the reference's
-// mynah_asr_sigmoid, src/qmat.h:31-35).
-__device__ __forceinline__ float sigmoid_stable(float x) {
-    if (x >= 0.0f) return 1.0f / (1.0f + expf(-x));
-    const float e = expf(x);
-    return e / (1.0f + e);
-}
-// The same function for the bulk element-wise passes (GLU, SiLU after the conv norm, the contractions' epilogues): one ex2, one
+// Sigmoid for the bulk element-wise passes (GLU, SiLU after the conv norm, the contractions' epilogues): one ex2, one
 // reciprocal approximation and Newton's step on it, no branch. Below -87 (1.6e-38) it is 0: the reciprocal would leave the normal
 // range, and x * sigmoid(x) has to vanish for large x, too. NaN stays NaN. Relative error against double 1.4e-7 for x >= 0 and
 // 3.8e-6 below (the exponential's), the same value as __frcp_rn(1 + exp(-x)) for every x within +-87; but that has a branch for

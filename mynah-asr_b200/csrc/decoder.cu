@@ -216,9 +216,10 @@ __device__ __forceinline__ void stage_planes(__half *xhi, __half *xlo, int xs, i
     }
 }
 
-// sigmoid_stable without its branch and the division's, so that a cell's gates overlap: one exponential, a reciprocal approximation
-// with Newton's step, and the quotient's rounding step. Its error against double is that of sigmoid_stable (2.45e-7 at most,
-// 3.1e-8 in the mean over +-87). 244 steps of one utterance (a minute of audio): 10.70 ms a call become 10.48.
+// Sigmoid that never exponentiates a positive argument (the reference's mynah_asr_sigmoid, src/qmat.h:31-35), without a branch on the
+// sign or the division's, so that a cell's gates overlap: one exponential, a reciprocal approximation with Newton's step, and the
+// quotient's rounding step. Error against double as with the branches: 2.45e-7 at most, 3.1e-8 in the mean over +-87. 244 steps of
+// one utterance (a minute of audio): 10.70 ms a call become 10.48.
 __device__ __forceinline__ float dec_sigmoid(float x) {
     const float e = expf(-fabsf(x)), num = x >= 0.0f ? 1.0f : e, den = 1.0f + e;
     float r;
