@@ -28,6 +28,17 @@ constexpr int HELPERS = 3;
 constexpr size_t LEAST = 512 << 10;
 constexpr int PARTS = (int)(PIECE / PART);
 
+// what a thread does between two looks at a word that another one writes
+inline void cpu_relax() {
+#if defined(__x86_64__) || defined(__i386__)
+    __builtin_ia32_pause();
+#elif defined(__aarch64__)
+    asm volatile("yield" ::: "memory");
+#else
+    std::this_thread::yield();
+#endif
+}
+
 // A transfer as parts of at most PART bytes in the order of the pieces. Parts below `open` may be taken.
 struct Part { void *to; const void *from; size_t n; int piece; };
 struct Job {
@@ -133,7 +144,7 @@ private:
             if (--inside_ == 0) idle_.notify_all();
         }
     }
-    static void pause() { for (int i = 0; i < 8; i++) __builtin_ia32_pause(); }
+    static void pause() { for (int i = 0; i < 8; i++) cpu_relax(); }
 
     std::mutex mu_;
     std::condition_variable wake_, idle_;
@@ -172,7 +183,7 @@ struct Transfer {
         j.next.store((int)j.parts.size(), std::memory_order_relaxed);       // (nothing is left unless an error came between)
         c.end();
     }
-    void finish(int piece) { while (!j.ready(piece)) if (!j.take()) __builtin_ia32_pause(); }
+    void finish(int piece) { while (!j.ready(piece)) if (!j.take()) cpu_relax(); }
 };
 
 }  // namespace
