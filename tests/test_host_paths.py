@@ -35,12 +35,31 @@ def fake_runtime(tmp_path_factory, pkg):
 @pytest.mark.parametrize("name", [
     "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads", "qmat_workspace_is_shared",
     "foreign_capture_survives", "chain_table_copy_fails", "chain_graph_reads_its_own_table",
-    "copies_by_pieces",
+    "copies_by_pieces", "copies_on_few_cores", "copies_of_other_classes", "copies_under_a_quota",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
+    if name == "copies_under_a_quota":
+        env["LD_PRELOAD"] = _quota_shim(fake_runtime)
     r = subprocess.run([sys.executable, os.path.abspath(__file__), name], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def _quota_shim(folder):
+    """A control group of this process's own: its cpu.max is the file beside the shim."""
+    src, lib = os.path.join(folder, "quota.c"), os.path.join(folder, "quota.so")
+    with open(src, "w") as f:
+        f.write("""#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stdio.h>
+#include <string.h>
+FILE *fopen(const char *path, const char *mode) {
+    FILE *(*real)(const char *, const char *) = dlsym(RTLD_NEXT, "fopen");
+    return real(strcmp(path, "/sys/fs/cgroup/cpu.max") ? path : "%s/cpu.max", mode);
+}
+""" % folder)
+    subprocess.run(["gcc", "-O1", "-fPIC", "-shared", src, "-o", lib, "-ldl"], check=True)
+    return lib
 
 
 # ------------------------------------------------------------------------------------------- in the child process
@@ -435,6 +454,72 @@ def copies_by_pieces(pkg, synth, fake):
         for q in handles:
             q.close()
     assert len(seen) > 160 and all(seen) and not errors, (len(seen), sum(seen), errors[:3])
+
+
+def _product(pkg, fake):
+    """A product of 6.1 MB in and 3.8 MB out: () -> (threads that the process has gained since now, copies of one call)."""
+    def threads():
+        return len(os.listdir("/proc/self/task"))
+
+    q = pkg.QMat(pkg.F32, np.ones((640, 1024), np.float32), 640, 1024)
+    x = np.ones((1500, 1024), np.float32)
+    before = threads()
+
+    def call():
+        q.mul(x)
+        fake.fake_reset()
+        q.mul(x)
+        return threads() - before, fake.fake_calls(b"cudaMemcpyAsync")
+
+    call.close = q.close
+    return call
+
+
+@scenario
+def copies_on_few_cores(pkg, synth, fake):
+    """Helpers are counted by the cores that the process may use: on one core none, and no pieces."""
+    cores = sorted(os.sched_getaffinity(0))
+    os.sched_setaffinity(0, cores[:1])
+    call = _product(pkg, fake)
+    threads, copies = call()
+    assert threads == 0 and copies <= 3, (threads, copies)
+    for n in (2, 3, 4, 5):
+        if len(cores) >= n:
+            os.sched_setaffinity(0, cores[:n])
+            threads, copies = call()
+            assert threads == min(n - 1, 3) and copies > 16, (n, threads, copies)
+    os.sched_setaffinity(0, cores[:1])
+    assert call()[1] <= 3
+
+
+@scenario
+def copies_of_other_classes(pkg, synth, fake):
+    """A real-time or idle thread starts no helpers, which would inherit its class, and waits for none."""
+    for policy, priority in ((os.SCHED_IDLE, 0), (os.SCHED_FIFO, 1), (os.SCHED_RR, 1)):
+        with closing(_product(pkg, fake)) as call:
+            try:
+                os.sched_setscheduler(0, policy, os.sched_param(priority))
+            except PermissionError:
+                continue
+            threads, copies = call()
+            assert threads == 0 and copies <= 3, (policy, threads, copies)
+            try:
+                os.sched_setscheduler(0, os.SCHED_OTHER, os.sched_param(0))
+            except PermissionError:                          # out of the idle class
+                break
+
+
+@scenario
+def copies_under_a_quota(pkg, synth, fake):
+    """A control group's share of processor time counts as its cores."""
+    cores = len(os.sched_getaffinity(0))
+    for text, want in (("150000 100000", 1), ("50000 100000", 1), ("max 100000", cores), ("200000 100000", 2), ("350000 100000", 3)):
+        with open(os.path.join(os.path.dirname(os.environ["LD_PRELOAD"]), "cpu.max"), "w") as f:
+            f.write(text + "\n")
+        with closing(_product(pkg, fake)) as call:           # (read when the first handle comes)
+            threads, copies = call()
+            want = min(want, cores, 4)
+            assert threads == want - 1 and (copies > 16 if want > 1 else copies <= 3), (text, threads, copies)
 
 
 if __name__ == "__main__":
