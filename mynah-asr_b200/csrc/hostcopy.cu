@@ -2,11 +2,12 @@
 //
 // The driver copies pageable memory through a buffer of its own with one thread: 3 MB in 200 us, 24 MB in 1.2 to 1.4 ms, either
 // way, where the link needs 55 us and 430 (page-locked memory). One core's memcpy is the limit (18 GB/s). Here the caller and up
-// to three helpers copy parts of pieces of 512 KB, and a piece is on the link while the next ones are being filled.
+// to two helpers copy parts of pieces of 512 KB, and a piece is on the link while the next ones are being filled.
 //
 // One transfer at a time has the pieces: another thread's, meanwhile, takes the driver's way, and so do small and page-locked
 // ones (all that is ever recorded into a graph here is small) and those of a caller that has no second core for a helper. Nothing
 // waits for a helper that has not taken a part yet: without helpers (none could be started, a forked child) the caller copies all of it.
+// Threads that wait for one another look for a bounded time, then they sleep: the one that is waited for may need their core.
 #include "hostcopy.h"
 
 #include <sched.h>
@@ -15,16 +16,26 @@
 #include <unistd.h>
 
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
+#include <memory>
 #include <mutex>
 #include <thread>
 
 namespace mb {
 namespace {
 
-constexpr size_t PIECE = 512 << 10, PART = 128 << 10;
+constexpr size_t PIECE = 512 << 10, PART = 64 << 10;
 constexpr int SLOTS = 4;                                         // page-locked pieces: 2 MB (page-locking takes 1 ms per MB, once)
-constexpr int HELPERS = 3;
+// us of a call with 3 MB of rows and 0.8 MB of results (and of processor time): one helper 255 (470), two 231 (630), three 217 (750);
+// the driver's way 302 (305).
+constexpr int HELPERS = 2;
+// Waking a thread takes 17 us there, and a part 3.5: a helper that sleeps is not woken for the last FRESH parts.
+constexpr int FRESH = 3;
+// How long a thread looks within a transfer before it sleeps (four processes that share the device, 24 MB each: 25 us 7.9 ms a call,
+// 200 us 2.5), and how long a helper looks out for the next transfer: they often come in pairs, rows in, result out. The same call with
+// 2 ms of pause in front: 10 us 390, 25 us 310, 60 us 258, 100 us 260.
+constexpr auto PATIENCE = std::chrono::microseconds(200), LOOK = std::chrono::microseconds(60);
 // Below this the driver's way is as fast: 0.75 MB take 62 us in and 77 out there, 40 to 50 by way of the pieces with the helpers
 // still asleep.
 constexpr size_t LEAST = 512 << 10;
@@ -39,6 +50,16 @@ inline void cpu_relax() {
 #else
     std::this_thread::yield();
 #endif
+}
+template <typename F> bool spin(std::chrono::microseconds limit, F ready) {
+    const auto until = std::chrono::steady_clock::now() + limit;
+    do
+        for (int i = 0; i < 16; i++) {
+            if (ready()) return true;
+            cpu_relax();
+        }
+    while (std::chrono::steady_clock::now() < until);
+    return false;
 }
 
 // Cores' worth of time that the control group of the process may use.
@@ -76,18 +97,22 @@ struct Job {
     std::vector<Part> parts;
     std::vector<int> left;                                       // per piece: parts in it
     std::vector<std::atomic<int>> done;                          // ... copied
-    std::atomic<int> open{0}, next{0};
-    explicit Job(size_t pieces) : left(pieces, 0), done(pieces) { for (auto &d : done) d.store(0, std::memory_order_relaxed); }
+    std::atomic<int> open{0}, next{0}, copied{0};
+    explicit Job(size_t pieces) : left(pieces, 0), done(pieces) { for (auto &d : done) d.store(0); }
+    bool some() const { return next.load() < open.load(); }
+    bool left_over() const { return next.load() < (int)parts.size(); }
+    bool worth_waking() const { return some() && next.load() + FRESH < (int)parts.size(); }
     bool take() {
         int i = next.load(std::memory_order_relaxed);
-        do if (i >= open.load(std::memory_order_acquire)) return false;
-        while (!next.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
+        do if (i >= open.load()) return false;
+        while (!next.compare_exchange_weak(i, i + 1));
         const Part &p = parts[(size_t)i];
         memcpy(p.to, p.from, p.n);
-        done[(size_t)p.piece].fetch_add(1, std::memory_order_release);
+        done[(size_t)p.piece].fetch_add(1);
+        copied.fetch_add(1);
         return true;
     }
-    bool ready(int piece) const { return done[(size_t)piece].load(std::memory_order_acquire) == left[(size_t)piece]; }
+    bool ready(int piece) const { return done[(size_t)piece].load() == left[(size_t)piece]; }
 };
 
 class Copier {
@@ -142,49 +167,72 @@ public:
         *events = per.data();
         return base_;
     }
-    void begin(Job *j) {
+    void begin(std::shared_ptr<Job> j) {
         std::lock_guard<std::mutex> lk(mu_);
-        job_ = j;
-        asked_.fetch_add(1, std::memory_order_release);
+        job_ = std::move(j);
+        asked_.fetch_add(1);
+        asleep_ = 0;
         wake_.notify_all();
     }
-    // no helper looks at the job any more
-    void end() {
+    // parts up to there may be taken (a helper says that it sleeps before it looks for the last time)
+    void open(Job &j, int upto) {
+        j.open.store(upto);
+        if (asleep_.load() == 0) return;
+        std::lock_guard<std::mutex> lk(mu_);
+        asleep_ = 0;
+        wake_.notify_all();
+    }
+    // the caller's wait for the helpers' parts (a helper looks for a sleeping caller behind each of its parts)
+    template <typename F> void await(F ready) {
+        if (spin(PATIENCE, ready)) return;
         std::unique_lock<std::mutex> lk(mu_);
+        caller_sleeps_ = true;
+        while (!ready()) done_.wait(lk);
+        caller_sleeps_ = false;
+    }
+    void end() {
+        std::lock_guard<std::mutex> lk(mu_);
         job_ = nullptr;
-        if (pid_ == getpid()) idle_.wait(lk, [this] { return inside_ == 0; });
     }
 
 private:
     void help() {
+        sched_param none{};
+        sched_setscheduler(0, SCHED_BATCH, &none);               // a woken helper does not take another process's core from it
         unsigned seen = 0;
         for (;;) {
-            // transfers often come in pairs (rows in, result out): look out for the next one for 100 us before going to sleep
-            for (int i = 0; i < 2000 && asked_.load(std::memory_order_acquire) == seen; i++) pause();
-            Job *j = nullptr;
+            std::shared_ptr<Job> j;
             {
                 std::unique_lock<std::mutex> lk(mu_);
-                wake_.wait(lk, [&] { return leave_ || asked_.load(std::memory_order_relaxed) != seen; });
-                if (leave_) return;
-                seen = asked_.load(std::memory_order_relaxed);
+                for (;;) {
+                    asleep_++;
+                    if (leave_) return;
+                    // a transfer that is about to begin, or parts enough
+                    if (job_ && ((asked_.load() != seen && job_->open.load() == 0) || job_->worth_waking())) break;
+                    wake_.wait(lk);
+                }
+                asleep_--;
+                seen = asked_.load();
                 j = job_;
-                if (j) inside_++;
             }
-            if (!j) continue;
-            while (j->next.load(std::memory_order_relaxed) < (int)j->parts.size())
-                if (!j->take()) pause();
-            std::lock_guard<std::mutex> lk(mu_);
-            if (--inside_ == 0) idle_.notify_all();
+            do
+                while (j->take())
+                    if (caller_sleeps_.load()) {
+                        std::lock_guard<std::mutex> lk(mu_);
+                        done_.notify_one();
+                    }
+            while (spin(j->left_over() ? PATIENCE : LOOK, [&] { return j->some() || asked_.load() != seen; }) && asked_.load() == seen);
         }
     }
-    static void pause() { for (int i = 0; i < 8; i++) cpu_relax(); }
 
     std::mutex mu_;
-    std::condition_variable wake_, idle_;
-    std::atomic<unsigned> asked_{0};
+    std::condition_variable wake_, done_;
+    std::atomic<unsigned> asked_{0};                             // transfers so far
+    std::atomic<int> asleep_{0};                                 // helpers that nobody has woken yet
+    std::atomic<bool> caller_sleeps_{false};
     std::atomic<int> quota_{1};
-    Job *job_ = nullptr;
-    int inside_ = 0, users_ = 0;
+    std::shared_ptr<Job> job_;
+    int users_ = 0;
     bool leave_ = false;
     pid_t pid_ = 0;
     std::vector<std::thread> helpers_;
@@ -205,19 +253,22 @@ int failed(const char *what, cudaError_t e) {
     return -1;
 }
 
-// The caller's side of a transfer. Whatever happens, it ends with no helper in the job, and with no piece on the link.
+// The caller's side of a transfer. Whatever happens, it ends with no helper at a part (a helper may still look at the job, which
+// lives as long as it is looked at).
 struct Transfer {
     Copier &c;
     Job &j;
-    cudaStream_t st;
-    cudaEvent_t *ev;
-    int used = 0;                                                // events recorded so far
-    Transfer(Copier &c_, Job &j_, cudaStream_t s, cudaEvent_t *e) : c(c_), j(j_), st(s), ev(e) { c.begin(&j); }
+    Transfer(Copier &c_, const std::shared_ptr<Job> &j_) : c(c_), j(*j_) { c.begin(j_); }
     ~Transfer() {
-        j.next.store((int)j.parts.size(), std::memory_order_relaxed);       // (nothing is left unless an error came between)
         c.end();
+        const int taken = j.next.exchange((int)j.parts.size());  // all of them, unless an error came between
+        c.await([&] { return j.copied.load() == taken; });
     }
-    void finish(int piece) { while (!j.ready(piece)) if (!j.take()) cpu_relax(); }
+    void open(int upto) { c.open(j, upto); }
+    void finish(int piece) {
+        while (!j.ready(piece) && j.take()) {}
+        c.await([&] { return j.ready(piece); });
+    }
 };
 
 }  // namespace
@@ -239,7 +290,8 @@ int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st) {
         return e == cudaSuccess ? 0 : failed("copy to the device", e);
     }
     const int n = (int)((bytes + PIECE - 1) / PIECE);
-    Job j((size_t)n);
+    const auto job = std::make_shared<Job>((size_t)n);
+    Job &j = *job;
     for (size_t at = 0; at < bytes; at += PART) {
         const int p = (int)(at / PIECE);
         j.parts.push_back(Part{base + (size_t)(p % SLOTS) * PIECE + at % PIECE, (const uint8_t *)host + at, bytes - at < PART ? bytes - at : PART, p});
@@ -247,8 +299,8 @@ int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st) {
     }
     cudaError_t e = cudaSuccess;
     {
-        Transfer t(c, j, st, ev);
-        j.open.store(n <= SLOTS ? (int)j.parts.size() : SLOTS * PARTS, std::memory_order_release);
+        Transfer t(c, job);
+        t.open(n <= SLOTS ? (int)j.parts.size() : SLOTS * PARTS);
         for (int p = 0; p < n && e == cudaSuccess; p++) {
             t.finish(p);
             const size_t at = (size_t)p * PIECE;
@@ -259,7 +311,7 @@ int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st) {
             if (e == cudaSuccess && old >= 0 && old + SLOTS < n) {
                 e = cudaEventSynchronize(ev[old % SLOTS]);
                 const int open = (old + SLOTS + 1) * PARTS;
-                if (e == cudaSuccess) j.open.store(open < (int)j.parts.size() ? open : (int)j.parts.size(), std::memory_order_release);
+                if (e == cudaSuccess) t.open(open < (int)j.parts.size() ? open : (int)j.parts.size());
             }
         }
     }
@@ -296,7 +348,8 @@ int copy_out(const std::vector<CopyOut> &parts, cudaStream_t st) {
     for (const CopyOut &o : parts)
         for (size_t at = 0; at < o.bytes; at += PIECE) pieces.push_back(Piece{(const uint8_t *)o.dev + at, o.bytes - at < PIECE ? o.bytes - at : PIECE, 0});
     const int n = (int)pieces.size();
-    Job j((size_t)n);
+    const auto job = std::make_shared<Job>((size_t)n);
+    Job &j = *job;
     int p = 0;
     for (const CopyOut &o : parts)
         for (size_t at = 0; at < o.bytes; at += PIECE, p++)
@@ -304,7 +357,7 @@ int copy_out(const std::vector<CopyOut> &parts, cudaStream_t st) {
                 j.parts.push_back(Part{(uint8_t *)o.host + at + in, base + (size_t)(p % SLOTS) * PIECE + in, pieces[(size_t)p].n - in < PART ? pieces[(size_t)p].n - in : PART, p});
     cudaError_t e = cudaSuccess;
     {
-        Transfer t(c, j, st, ev);
+        Transfer t(c, job);
         int asked = 0, open = 0;
         for (int q = 0; q < n && e == cudaSuccess; q++) {
             for (; asked < n && asked < q + SLOTS && e == cudaSuccess; asked++) {
@@ -314,7 +367,7 @@ int copy_out(const std::vector<CopyOut> &parts, cudaStream_t st) {
             }
             if (e == cudaSuccess) e = cudaEventSynchronize(ev[q % SLOTS]);
             open += j.left[(size_t)q];
-            if (e == cudaSuccess) j.open.store(open, std::memory_order_release);
+            if (e == cudaSuccess) t.open(open);
         }
         for (int q = 0; q < n && e == cudaSuccess; q++) t.finish(q);
     }

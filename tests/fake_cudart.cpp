@@ -5,6 +5,7 @@
 #include <cuda_runtime_api.h>
 #include <stdlib.h>
 #include <string.h>
+#include <unistd.h>
 
 #include <functional>
 #include <map>
@@ -35,6 +36,16 @@ std::map<cudaStream_t, std::vector<std::function<void()>>> capturing;
 std::map<std::string, long long> calls;
 std::string fail_name;                                   // the fail_at-th call of this function from now on fails
 long long fail_at = 0;
+long long slow_at = 0;                                   // the slow_at-th wait of the host from now on takes slow_ms
+int slow_ms = 0;
+void take_time() {                                       // (outside the lock: the thread waits, the others go on)
+    int ms = 0;
+    {
+        Lock l(mu);
+        if (slow_at && --slow_at == 0) ms = slow_ms;
+    }
+    if (ms) usleep(1000 * ms);
+}
 typedef void (*launch_cb)(const char *kernel, void **args, int recorded);   // kernel "": a graph is launched
 typedef void (*hook_cb)();
 launch_cb on_launch = nullptr;
@@ -90,6 +101,7 @@ extern "C" {
 // ---- driven by the test
 void fake_reset() { Lock l(mu); calls.clear(); fail_name.clear(); fail_at = 0; dev_peak = dev_bytes; }
 void fake_fail(const char *name, long long nth) { Lock l(mu); fail_name = name; fail_at = nth; }
+void fake_slow(long long nth, int ms) { Lock l(mu); slow_at = nth; slow_ms = ms; }
 int fake_failed() { Lock l(mu); return fail_name.empty(); }
 long long fake_calls(const char *name) { Lock l(mu); return calls[name]; }
 int fake_pending() {                                     // streams with work nobody has waited for
@@ -189,7 +201,7 @@ cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t st) {
 // ---- streams and events
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { Lock l(mu); if (fails("cudaStreamCreate")) return cudaErrorMemoryAllocation; *s = handle<cudaStream_t>(); return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { Lock l(mu); streams.erase(s); stream_behind.erase(s); return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { Lock l(mu); calls["cudaStreamSynchronize"]++; wait_stream(s); return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { take_time(); Lock l(mu); calls["cudaStreamSynchronize"]++; wait_stream(s); return cudaSuccess; }
 cudaError_t cudaStreamQuery(cudaStream_t s) { Lock l(mu); unsafe_call(); return streams[s].done < streams[s].issued ? cudaErrorNotReady : cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) { Lock l(mu); calls["cudaStreamWaitEvent"]++; merge(stream_behind[s], event_behind[e]); return work(s, [] {}); }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { Lock l(mu); if (fails("cudaEventCreate")) return cudaErrorMemoryAllocation; *e = handle<cudaEvent_t>(); return cudaSuccess; }
@@ -209,6 +221,7 @@ cudaError_t cudaEventQuery(cudaEvent_t e) {
     return cudaSuccess;
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    take_time();
     Lock l(mu);
     for (auto &b : event_behind[e]) if (streams.count(b.first) && streams[b.first].done < b.second) streams[b.first].done = b.second;
     return cudaSuccess;
