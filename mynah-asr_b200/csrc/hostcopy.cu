@@ -4,10 +4,12 @@
 // way, where the link needs 55 us and 430 (page-locked memory). One core's memcpy is the limit (18 GB/s). Here the caller and up
 // to two helpers copy parts of pieces of 512 KB, and a piece is on the link while the next ones are being filled.
 //
-// One transfer at a time has the pieces: another thread's, meanwhile, takes the driver's way, and so do small and page-locked
-// ones (all that is ever recorded into a graph here is small) and those of a caller that has no second core for a helper. Nothing
-// waits for a helper that has not taken a part yet: without helpers (none could be started, a forked child) the caller copies all of it.
-// Threads that wait for one another look for a bounded time, then they sleep: the one that is waited for may need their core.
+// A transfer holds a set of pieces from the first copy that is queued on, and the helpers only while there is something to copy: what
+// the stream still computes in front of a result keeps nobody busy. One transfer at a time has the helpers; others, meanwhile, copy
+// their pieces alone. Small copies (all that is ever recorded into a graph here is small), page-locked memory, callers that have no
+// second core for a helper, and whoever finds all sets held take the driver's way. Nothing waits for a helper that has not taken a part
+// yet: without helpers (none could be started, a forked child) the caller copies all of it. Threads that wait for one another look
+// for a bounded time, then they sleep: the one that is waited for may need their core.
 #include "hostcopy.h"
 
 #include <sched.h>
@@ -26,7 +28,8 @@ namespace mb {
 namespace {
 
 constexpr size_t PIECE = 512 << 10, PART = 64 << 10;
-constexpr int SLOTS = 4;                                         // page-locked pieces: 2 MB (page-locking takes 1 ms per MB, once)
+constexpr int SLOTS = 4;                                         // page-locked pieces of a set: 2 MB (page-locking takes 1 ms per MB, once)
+constexpr int SETS = 4;                                          // made when as many transfers are under way at once
 // us of a call with 3 MB of rows and 0.8 MB of results (and of processor time): one helper 255 (470), two 231 (630), three 217 (750);
 // the driver's way 302 (305).
 constexpr int HELPERS = 2;
@@ -115,15 +118,47 @@ struct Job {
     bool ready(int piece) const { return done[(size_t)piece].load() == left[(size_t)piece]; }
 };
 
+// Page-locked pieces, and per device the events behind their copies.
+struct Set {
+    bool held = false;
+    uint8_t *base = nullptr;
+    cudaEvent_t on_link = nullptr;                               // behind the last piece of a transfer to the device: free once it has left
+    std::vector<cudaEvent_t> events[MB_MAX_DEVICES];
+    cudaEvent_t *ev = nullptr;                                   // the current device's
+    bool prepare() {
+        int dev = 0;
+        bool ok = !on_link || cudaEventSynchronize(on_link) == cudaSuccess;
+        on_link = nullptr;
+        ok = ok && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < MB_MAX_DEVICES;
+        if (ok && !base && cudaHostAlloc((void **)&base, PIECE * SLOTS, cudaHostAllocPortable) != cudaSuccess) { base = nullptr; ok = false; }
+        while (ok && events[dev].size() < (size_t)SLOTS + 1) {
+            cudaEvent_t e = nullptr;
+            ok = cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+            if (ok) events[dev].push_back(e);
+        }
+        if (!ok) { cudaGetLastError(); return false; }
+        ev = events[dev].data();
+        return true;
+    }
+    void give_back() {
+        if (on_link) cudaEventSynchronize(on_link);
+        on_link = nullptr;
+        for (auto &per : events) { for (cudaEvent_t e : per) cudaEventDestroy(e); per.clear(); }
+        if (base) cudaFreeHost(base);
+        base = nullptr;
+        cudaGetLastError();
+    }
+};
+
 class Copier {
 public:
-    std::mutex busy;                                             // held by the transfer that has the pieces
+    std::mutex helped;                                           // held by the transfer that has the helpers
 
     void user(int d) {
-        std::lock_guard<std::mutex> b(busy);                     // no transfer under way
+        std::lock_guard<std::mutex> pl(pool_);
         if (users_ == 0) quota_.store(quota_cores(), std::memory_order_relaxed);
         users_ += d;
-        if (users_ > 0) return;
+        if (users_ > 0) return;                                  // (a transfer under way has a user)
         {
             std::lock_guard<std::mutex> lk(mu_);
             leave_ = true;
@@ -134,39 +169,34 @@ public:
         helpers_.clear();
         leave_ = false;
         RelaxedCapture relaxed;
-        if (on_link_) cudaEventSynchronize(on_link_);
-        on_link_ = nullptr;
-        for (auto &per : events_) { for (cudaEvent_t e : per) cudaEventDestroy(e); per.clear(); }
-        if (base_) cudaFreeHost(base_);
-        base_ = nullptr;
-        cudaGetLastError();
+        for (Set &s : sets_) s.give_back();
     }
-    // the last piece of a transfer to the device, still on the link: the pieces are free once it has left
-    void on_link(cudaEvent_t e) { on_link_ = e; }
     int cores() const { return caller_cores(quota_.load(std::memory_order_relaxed)); }
-    // with `busy` held: the pieces, free again, the helpers for a caller with that many cores and the current device's events;
-    // null where there are none
-    uint8_t *pieces(int cores, cudaEvent_t **events) {
-        if (on_link_ && cudaEventSynchronize(on_link_) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        on_link_ = nullptr;
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MB_MAX_DEVICES) { cudaGetLastError(); return nullptr; }
-        if (!base_ && cudaHostAlloc((void **)&base_, PIECE * SLOTS, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); base_ = nullptr; return nullptr; }
-        std::vector<cudaEvent_t> &per = events_[dev];
-        while (per.size() < (size_t)SLOTS) {
-            cudaEvent_t e = nullptr;
-            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-            per.push_back(e);
+    // a set of pieces, free again, and helpers for a caller with that many cores; null where there are none
+    Set *take(int cores) {
+        Set *s = nullptr;
+        {
+            std::lock_guard<std::mutex> pl(pool_);
+            if (helpers_.empty()) pid_ = getpid();
+            if (pid_ == getpid()) {
+                try {
+                    while ((int)helpers_.size() < HELPERS && (int)helpers_.size() + 1 < cores) helpers_.emplace_back([this] { help(); });
+                } catch (...) {}                                 // fewer of them
+            }
+            auto rank = [](const Set &t) { return !t.base ? 0 : t.on_link ? 1 : 2; };
+            for (Set &t : sets_) if (!t.held && (!s || rank(t) > rank(*s))) s = &t;
+            if (!s) return nullptr;
+            s->held = true;
         }
-        if (helpers_.empty()) pid_ = getpid();
-        if (pid_ == getpid()) {
-            try {
-                while ((int)helpers_.size() < HELPERS && (int)helpers_.size() + 1 < cores) helpers_.emplace_back([this] { help(); });
-            } catch (...) {}                                     // fewer of them
-        }
-        *events = per.data();
-        return base_;
+        if (s->prepare()) return s;
+        give(s);
+        return nullptr;
     }
+    void give(Set *s) {
+        std::lock_guard<std::mutex> pl(pool_);
+        s->held = false;
+    }
+    // with `helped`, from here on
     void begin(std::shared_ptr<Job> j) {
         std::lock_guard<std::mutex> lk(mu_);
         job_ = std::move(j);
@@ -225,20 +255,20 @@ private:
         }
     }
 
-    std::mutex mu_;
+    std::mutex mu_;                                              // the helpers' sleep
     std::condition_variable wake_, done_;
     std::atomic<unsigned> asked_{0};                             // transfers so far
     std::atomic<int> asleep_{0};                                 // helpers that nobody has woken yet
     std::atomic<bool> caller_sleeps_{false};
-    std::atomic<int> quota_{1};
     std::shared_ptr<Job> job_;
-    int users_ = 0;
     bool leave_ = false;
+
+    std::mutex pool_;                                            // what follows
+    Set sets_[SETS];
+    int users_ = 0;
     pid_t pid_ = 0;
     std::vector<std::thread> helpers_;
-    uint8_t *base_ = nullptr;
-    cudaEvent_t on_link_ = nullptr;
-    std::vector<cudaEvent_t> events_[MB_MAX_DEVICES];
+    std::atomic<int> quota_{1};
 };
 Copier &copier() { static Copier *c = new Copier(); return *c; }  // alive until the process ends
 
@@ -254,17 +284,28 @@ int failed(const char *what, cudaError_t e) {
 }
 
 // The caller's side of a transfer. Whatever happens, it ends with no helper at a part (a helper may still look at the job, which
-// lives as long as it is looked at).
+// lives as long as it is looked at), and with the pieces given back.
 struct Transfer {
     Copier &c;
+    Set *s;
+    const std::shared_ptr<Job> job;
     Job &j;
-    Transfer(Copier &c_, const std::shared_ptr<Job> &j_) : c(c_), j(*j_) { c.begin(j_); }
+    std::unique_lock<std::mutex> helped;
+    Transfer(Copier &c_, Set *s_, size_t pieces) : c(c_), s(s_), job(std::make_shared<Job>(pieces)), j(*job), helped(c_.helped, std::defer_lock) {}
     ~Transfer() {
-        c.end();
         const int taken = j.next.exchange((int)j.parts.size());  // all of them, unless an error came between
-        c.await([&] { return j.copied.load() == taken; });
+        if (helped.owns_lock()) {
+            c.end();
+            c.await([&] { return j.copied.load() == taken; });
+            helped.unlock();
+        }
+        c.give(s);
     }
-    void open(int upto) { c.open(j, upto); }
+    void ask_helpers() { if (helped.try_lock()) c.begin(job); }
+    void open(int upto) {
+        if (helped.owns_lock()) c.open(j, upto);
+        else j.open.store(upto);
+    }
     void finish(int piece) {
         while (!j.ready(piece) && j.take()) {}
         c.await([&] { return j.ready(piece); });
@@ -278,64 +319,52 @@ void copy_user_gone() { copier().user(-1); }
 
 int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st) {
     Copier &c = copier();
-    std::unique_lock<std::mutex> lk(c.busy, std::defer_lock);
-    cudaEvent_t *ev = nullptr;
-    uint8_t *base = nullptr;
     RelaxedCapture relaxed;
     const int cores = bytes >= LEAST ? c.cores() : 1;
-    if (cores > 1 && pageable(host) && lk.try_lock()) base = c.pieces(cores, &ev);
-    if (!base) {
-        if (lk.owns_lock()) lk.unlock();
+    Set *s = cores > 1 && pageable(host) ? c.take(cores) : nullptr;
+    if (!s) {
         const cudaError_t e = cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
         return e == cudaSuccess ? 0 : failed("copy to the device", e);
     }
     const int n = (int)((bytes + PIECE - 1) / PIECE);
-    const auto job = std::make_shared<Job>((size_t)n);
-    Job &j = *job;
+    Transfer t(c, s, (size_t)n);
+    Job &j = t.j;
     for (size_t at = 0; at < bytes; at += PART) {
         const int p = (int)(at / PIECE);
-        j.parts.push_back(Part{base + (size_t)(p % SLOTS) * PIECE + at % PIECE, (const uint8_t *)host + at, bytes - at < PART ? bytes - at : PART, p});
+        j.parts.push_back(Part{s->base + (size_t)(p % SLOTS) * PIECE + at % PIECE, (const uint8_t *)host + at, bytes - at < PART ? bytes - at : PART, p});
         j.left[(size_t)p]++;
     }
+    t.ask_helpers();
+    t.open(n <= SLOTS ? (int)j.parts.size() : SLOTS * PARTS);
     cudaError_t e = cudaSuccess;
-    {
-        Transfer t(c, job);
-        t.open(n <= SLOTS ? (int)j.parts.size() : SLOTS * PARTS);
-        for (int p = 0; p < n && e == cudaSuccess; p++) {
-            t.finish(p);
-            const size_t at = (size_t)p * PIECE;
-            e = cudaMemcpyAsync((uint8_t *)dev + at, base + (size_t)(p % SLOTS) * PIECE, bytes - at < PIECE ? bytes - at : PIECE, cudaMemcpyHostToDevice, st);
-            if (e == cudaSuccess) e = cudaEventRecord(ev[p % SLOTS], st);
-            // the place of a piece that has left is opened for the piece SLOTS behind it, half the places ahead of need
-            const int old = p - SLOTS / 2;
-            if (e == cudaSuccess && old >= 0 && old + SLOTS < n) {
-                e = cudaEventSynchronize(ev[old % SLOTS]);
-                const int open = (old + SLOTS + 1) * PARTS;
-                if (e == cudaSuccess) t.open(open < (int)j.parts.size() ? open : (int)j.parts.size());
-            }
+    for (int p = 0; p < n && e == cudaSuccess; p++) {
+        t.finish(p);
+        const size_t at = (size_t)p * PIECE;
+        e = cudaMemcpyAsync((uint8_t *)dev + at, s->base + (size_t)(p % SLOTS) * PIECE, bytes - at < PIECE ? bytes - at : PIECE, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaEventRecord(s->ev[p % SLOTS], st);
+        // the place of a piece that has left is opened for the piece SLOTS behind it, half the places ahead of need
+        const int old = p - SLOTS / 2;
+        if (e == cudaSuccess && old >= 0 && old + SLOTS < n) {
+            e = cudaEventSynchronize(s->ev[old % SLOTS]);
+            const int open = (old + SLOTS + 1) * PARTS;
+            if (e == cudaSuccess) t.open(open < (int)j.parts.size() ? open : (int)j.parts.size());
         }
     }
-    if (e == cudaSuccess) { c.on_link(ev[(n - 1) % SLOTS]); return 0; }
+    if (e == cudaSuccess) { s->on_link = s->ev[(n - 1) % SLOTS]; return 0; }
     cudaStreamSynchronize(st);
     return failed("copy to the device", e);
 }
 
 int copy_out(const std::vector<CopyOut> &parts, cudaStream_t st) {
     size_t total = 0;
-    bool page = true;
     for (const CopyOut &o : parts) total += o.bytes;
     Copier &c = copier();
-    std::unique_lock<std::mutex> lk(c.busy, std::defer_lock);
-    cudaEvent_t *ev = nullptr;
-    uint8_t *base = nullptr;
     RelaxedCapture relaxed;
     const int cores = total >= LEAST ? c.cores() : 1;
-    if (cores > 1) {
-        for (const CopyOut &o : parts) page = page && (!o.bytes || pageable(o.host));
-        if (page && lk.try_lock()) base = c.pieces(cores, &ev);
-    }
-    if (!base) {
-        if (lk.owns_lock()) lk.unlock();
+    bool page = cores > 1;
+    for (const CopyOut &o : parts) page = page && (!o.bytes || pageable(o.host));
+    Set *s = page ? c.take(cores) : nullptr;
+    if (!s) {
         for (const CopyOut &o : parts) {
             const cudaError_t e = o.bytes ? cudaMemcpyAsync(o.host, o.dev, o.bytes, cudaMemcpyDeviceToHost, st) : cudaSuccess;
             if (e != cudaSuccess) return failed("copy to the host", e);
@@ -343,34 +372,37 @@ int copy_out(const std::vector<CopyOut> &parts, cudaStream_t st) {
         return 0;
     }
     // pieces end with their part of the caller's memory
-    struct Piece { const void *dev; size_t n; int parts; };
+    struct Piece { const void *dev; size_t n; };
     std::vector<Piece> pieces;
     for (const CopyOut &o : parts)
-        for (size_t at = 0; at < o.bytes; at += PIECE) pieces.push_back(Piece{(const uint8_t *)o.dev + at, o.bytes - at < PIECE ? o.bytes - at : PIECE, 0});
+        for (size_t at = 0; at < o.bytes; at += PIECE) pieces.push_back(Piece{(const uint8_t *)o.dev + at, o.bytes - at < PIECE ? o.bytes - at : PIECE});
     const int n = (int)pieces.size();
-    const auto job = std::make_shared<Job>((size_t)n);
-    Job &j = *job;
+    Transfer t(c, s, (size_t)n);
+    Job &j = t.j;
     int p = 0;
     for (const CopyOut &o : parts)
         for (size_t at = 0; at < o.bytes; at += PIECE, p++)
             for (size_t in = 0; in < pieces[(size_t)p].n; in += PART, j.left[(size_t)p]++)
-                j.parts.push_back(Part{(uint8_t *)o.host + at + in, base + (size_t)(p % SLOTS) * PIECE + in, pieces[(size_t)p].n - in < PART ? pieces[(size_t)p].n - in : PART, p});
-    cudaError_t e = cudaSuccess;
-    {
-        Transfer t(c, job);
-        int asked = 0, open = 0;
-        for (int q = 0; q < n && e == cudaSuccess; q++) {
-            for (; asked < n && asked < q + SLOTS && e == cudaSuccess; asked++) {
-                if (asked >= SLOTS) t.finish(asked - SLOTS);
-                e = cudaMemcpyAsync(base + (size_t)(asked % SLOTS) * PIECE, pieces[(size_t)asked].dev, pieces[(size_t)asked].n, cudaMemcpyDeviceToHost, st);
-                if (e == cudaSuccess) e = cudaEventRecord(ev[asked % SLOTS], st);
-            }
-            if (e == cudaSuccess) e = cudaEventSynchronize(ev[q % SLOTS]);
-            open += j.left[(size_t)q];
-            if (e == cudaSuccess) t.open(open);
+                j.parts.push_back(Part{(uint8_t *)o.host + at + in, s->base + (size_t)(p % SLOTS) * PIECE + in, pieces[(size_t)p].n - in < PART ? pieces[(size_t)p].n - in : PART, p});
+    int asked = 0, open = 0;
+    cudaError_t e = cudaEventRecord(s->ev[SLOTS], st);
+    for (int q = 0; q < n && e == cudaSuccess; q++) {
+        for (; asked < n && asked < q + SLOTS && e == cudaSuccess; asked++) {
+            if (asked >= SLOTS) t.finish(asked - SLOTS);
+            e = cudaMemcpyAsync(s->base + (size_t)(asked % SLOTS) * PIECE, pieces[(size_t)asked].dev, pieces[(size_t)asked].n, cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaEventRecord(s->ev[asked % SLOTS], st);
         }
-        for (int q = 0; q < n && e == cudaSuccess; q++) t.finish(q);
+        if (e == cudaSuccess && q == 0) {
+            // what came before is done: the helpers wake up while the first piece is on the link (with them asleep 3 MB in and
+            // 0.8 MB out take 320 us instead of 340)
+            e = cudaEventSynchronize(s->ev[SLOTS]);
+            t.ask_helpers();
+        }
+        if (e == cudaSuccess) e = cudaEventSynchronize(s->ev[q % SLOTS]);
+        open += j.left[(size_t)q];
+        if (e == cudaSuccess) t.open(open);
     }
+    for (int q = 0; q < n && e == cudaSuccess; q++) t.finish(q);
     if (e == cudaSuccess) return 0;
     cudaStreamSynchronize(st);
     return failed("copy to the host", e);

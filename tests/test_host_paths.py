@@ -35,7 +35,7 @@ def fake_runtime(tmp_path_factory, pkg):
 @pytest.mark.parametrize("name", [
     "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads", "qmat_workspace_is_shared",
     "foreign_capture_survives", "chain_table_copy_fails", "chain_graph_reads_its_own_table",
-    "copies_by_pieces", "copies_on_few_cores", "copies_of_other_classes", "copies_under_a_quota", "waits_of_copies_end_in_sleep",
+    "copies_by_pieces", "copies_on_few_cores", "copies_of_other_classes", "copies_under_a_quota", "waits_of_copies_end_in_sleep", "copies_leave_others_alone",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -564,6 +564,31 @@ def waits_of_copies_end_in_sleep(pkg, synth, fake):
         cpu, t = time.process_time() - cpu, time.perf_counter() - t
         assert t > 0.3, (at, t)
         assert cpu < 0.15, (at, cpu, t)
+
+
+@scenario
+def copies_leave_others_alone(pkg, synth, fake):
+    """While a product is being computed whose result is large, other threads make and free handles, and copy by pieces."""
+    import threading
+    import time
+    if len(os.sched_getaffinity(0)) < 2:
+        return
+    slow = pkg.QMat(pkg.F32, np.ones((4096, 64), np.float32), 4096, 64)
+    x = np.ones((400, 64), np.float32)                       # 0.1 MB in, 6.5 MB out
+    slow.mul(x)
+    with closing(_product(pkg, fake)) as call:
+        threads, copies = call()
+        fake.fake_slow(1, 600)                               # the first wait of the product
+        done = []
+        thread = threading.Thread(target=lambda: (slow.mul(x), done.append(1)))
+        thread.start()
+        time.sleep(0.1)
+        t = time.perf_counter()
+        pkg.QMat(pkg.F32, np.ones((64, 64), np.float32), 64, 64).close()
+        beside = call()[1]
+        t = time.perf_counter() - t
+        assert not done and t < 0.4 and beside == copies > 16, (done, t, beside, copies)
+        thread.join()
 
 
 if __name__ == "__main__":
