@@ -39,9 +39,11 @@ constexpr int FRESH = 3;
 // 200 us 2.5), and how long a helper looks out for the next transfer: they often come in pairs, rows in, result out. The same call with
 // 2 ms of pause in front: 10 us 390, 25 us 310, 60 us 258, 100 us 260.
 constexpr auto PATIENCE = std::chrono::microseconds(200), LOOK = std::chrono::microseconds(60);
-// Below this the driver's way is as fast: 0.75 MB take 62 us in and 77 out there, 40 to 50 by way of the pieces with the helpers
-// still asleep.
-constexpr size_t LEAST = 512 << 10;
+// Below these the driver's way is as fast, or faster when the helpers are asleep. Us of a product whose rows (results) are so large,
+// new memory each time, driver and pieces, with no pause between calls and with 2 ms:
+//   in   0.5 MB  91, 93; 97, 107    0.75 MB  111, 112; 118, 126    1 MB  138, 125; 145, 138    1.5 MB  157, 157; 163, 167
+//   out  0.5 MB  78, 58; 80, 80     0.75 MB   92, 69;  96, 95      1 MB  111, 85;  118, 110    1.5 MB  142, 108; 150, 133
+constexpr size_t LEAST_IN = 1 << 20, LEAST_OUT = 512 << 10;
 constexpr int PARTS = (int)(PIECE / PART);
 
 // what a thread does between two looks at a word that another one writes
@@ -320,7 +322,7 @@ void copy_user_gone() { copier().user(-1); }
 int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st) {
     Copier &c = copier();
     RelaxedCapture relaxed;
-    const int cores = bytes >= LEAST ? c.cores() : 1;
+    const int cores = bytes >= LEAST_IN ? c.cores() : 1;
     Set *s = cores > 1 && pageable(host) ? c.take(cores) : nullptr;
     if (!s) {
         const cudaError_t e = cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
@@ -360,7 +362,7 @@ int copy_out(const std::vector<CopyOut> &parts, cudaStream_t st) {
     for (const CopyOut &o : parts) total += o.bytes;
     Copier &c = copier();
     RelaxedCapture relaxed;
-    const int cores = total >= LEAST ? c.cores() : 1;
+    const int cores = total >= LEAST_OUT ? c.cores() : 1;
     bool page = cores > 1;
     for (const CopyOut &o : parts) page = page && (!o.bytes || pageable(o.host));
     Set *s = page ? c.take(cores) : nullptr;

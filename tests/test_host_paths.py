@@ -35,7 +35,7 @@ def fake_runtime(tmp_path_factory, pkg):
 @pytest.mark.parametrize("name", [
     "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads", "qmat_workspace_is_shared",
     "foreign_capture_survives", "chain_table_copy_fails", "chain_graph_reads_its_own_table",
-    "copies_by_pieces", "copies_on_few_cores", "copies_of_other_classes", "copies_under_a_quota", "waits_of_copies_end_in_sleep", "copies_leave_others_alone",
+    "copies_by_pieces", "copies_on_few_cores", "copies_of_other_classes", "copies_under_a_quota", "waits_of_copies_end_in_sleep", "copies_leave_others_alone", "small_copies_go_the_drivers_way",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -589,6 +589,21 @@ def copies_leave_others_alone(pkg, synth, fake):
         t = time.perf_counter() - t
         assert not done and t < 0.4 and beside == copies > 16, (done, t, beside, copies)
         thread.join()
+
+
+@scenario
+def small_copies_go_the_drivers_way(pkg, synth, fake):
+    """Pieces from 1 MB of rows and 512 KB of results on: below, waking the helpers costs more than they save."""
+    if len(os.sched_getaffinity(0)) < 2:
+        return
+    for n, k, rows, copies in ((64, 1024, 255, 2), (64, 1024, 256, 3), (64, 1024, 257, 4),        # rows, and result with status
+                               (1024, 64, 127, 3), (1024, 64, 128, 3), (1024, 64, 129, 4)):       # rows, status, result
+        with closing(pkg.QMat(pkg.F32, np.ones((n, k), np.float32), n, k)) as q:
+            x = np.ones((rows, k), np.float32)
+            q.mul(x)
+            fake.fake_reset()
+            q.mul(x)
+            assert fake.fake_calls(b"cudaMemcpyAsync") == copies, (n, k, rows, fake.fake_calls(b"cudaMemcpyAsync"))
 
 
 if __name__ == "__main__":
