@@ -362,6 +362,8 @@ void mynah_b200_profile_bytes(mynah_b200_model *m, double *bytes, int ncat);
  * on: head, head barrier, select + barrier, LSTM layers + barriers, projector + barrier, then the
  * number of steps and of steps in which some utterance emitted. */
 void mynah_b200_decoder_clocks(mynah_b200_model *m, long long *out8);
+/* out[i] = sigmoid(x[i]), i < n, as the element-wise passes (cell = 0) or the greedy decoder's cells (cell = 1) compute it. */
+int mynah_b200_sigmoid(const float *x, float *out, int n, int cell);
 /* Times one large-T contraction with device-resident operands: returns the average milliseconds
  * of `iters` launches of out[T,n] = x[T,k] W^T (CUDA events on the launching stream). */
 double mynah_b200_qmat_time(const mynah_b200_qmat *m, int T, int flags, int iters);

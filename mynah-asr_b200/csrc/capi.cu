@@ -1675,6 +1675,18 @@ void mynah_b200_decoder_clocks(mynah_b200_model *h, long long *out8) {
     for (int i = 0; i < 8; i++) out8[i] = h ? h->m.dec_dbg[i] : 0;
 }
 
+int mynah_b200_sigmoid(const float *x, float *out, int n, int cell) {
+    if (!x || !out || n <= 0) { set_error("sigmoid: bad argument"); return -1; }
+    float *d = nullptr;
+    MB_CUDA(cudaMalloc(&d, (size_t)n * 4));
+    int rc = cudaMemcpy(d, x, (size_t)n * 4, cudaMemcpyHostToDevice) == cudaSuccess ? sigmoids(d, d, n, cell, nullptr) : -1;
+    if (rc == 0) note_launch();
+    if (rc == 0 && cudaMemcpy(out, d, (size_t)n * 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = -1;
+    if (rc) { cudaGetLastError(); set_error("sigmoid: a copy or kernel failed"); }
+    cudaFree(d);
+    return rc;
+}
+
 double mynah_b200_qmat_time(const mynah_b200_qmat *q, int T, int flags, int iters) {
     if (!q || T <= 0 || iters <= 0) { set_error("qmat_time: bad argument"); return -1.0; }
     const QWeight &w = q->w;

@@ -310,6 +310,7 @@ struct GreedyDev {
 
 // blocks: CTAs of the cooperative grid (0 = one per SM); at least p.B
 int greedy_launch(const GreedyDev &p, cudaStream_t st, int blocks = 0);
+int sigmoids(const float *x, float *out, int n, int cell, cudaStream_t st);     // the decoder's cells' (1) or the element-wise passes' (0)
 void set_load_seconds(mynah_b200_model *h, double seconds);     // capi.cu: the loader reports its whole wall time
 
 }  // namespace mb

@@ -183,6 +183,39 @@ def test_tcgen05_attention_long_segments(gpu_pkg, synth):
         m.close()
 
 
+def test_sigmoids_against_float64(gpu_pkg):
+    """Both sigmoids over every magnitude that float32 has. Bounds from the documented ones of the exponentials: __expf 2 + 1.173 |x|
+    units of the last place (up to 2^-23 each), expf one; a sigmoid passes on sigmoid(-x) of its exponential's relative error. To
+    that come the roundings of 1 + e, of the reciprocal and of the quotient, 2^-24 each, and one more."""
+    rng = np.random.default_rng(0)
+    x = np.concatenate([np.asarray(part, np.float32) for part in (
+        np.linspace(-110, 110, 1 << 20), rng.uniform(-20, 20, 1 << 20), rng.standard_normal(1 << 20) * np.exp(rng.uniform(-100, 4, 1 << 20)),
+        [0.0, -0.0, 87.0, -87.0, np.nextafter(np.float32(-87), np.float32(-88)), 88.8, -88.8, 3.4e38, -3.4e38, np.inf, -np.inf, np.nan],
+        rng.integers(0, 1 << 32, 1 << 20, dtype=np.uint64).astype(np.uint32).view(np.float32),
+    )])
+    x64 = x.astype(np.float64)
+    with np.errstate(over="ignore", invalid="ignore"):
+        e = np.exp(-np.abs(x64))
+        want = np.where(x64 >= 0, 1.0, e) / (1 + e)
+        other = np.where(x64 >= 0, e, 1.0) / (1 + e)         # sigmoid(-x)
+    nan = np.isnan(x)
+    for cell in (0, 1):
+        got = np.empty_like(x)
+        gpu_pkg._check(gpu_pkg.lib().mynah_b200_sigmoid(gpu_pkg._fp(x), gpu_pkg._fp(got), x.size, cell), "sigmoid")
+        assert np.isnan(got[nan]).all() and not np.isnan(got[~nan]).any()
+        ulps = np.where(np.abs(x64) < 1e3, 2 + 1.173 * np.abs(x64), 0) if cell == 0 else 1
+        bound = want * (other * ulps * 2.0 ** -23 + 4 * 2.0 ** -24)
+        low = ~nan & (x < -87)
+        if cell == 0:
+            assert (got[low] == 0).all()
+        else:                                                # the exponential leaves the normal range: one more of its steps
+            assert (np.abs(got - want)[low] <= bound[low] + 2.0 ** -149).all()
+        ok = ~nan & (x >= -87)
+        rel = np.abs(got[ok] - want[ok]) / want[ok]
+        print(cell, rel[x[ok] >= 0].max(), rel[x[ok] < 0].max(), rel[np.abs(x[ok]) <= 87].mean())
+        assert (np.abs(got - want)[ok] <= bound[ok]).all()
+
+
 def test_silu_vanishes_below(gpu_pkg, synth):
     """x * sigmoid(x) of every negative number that float32 has: 0 from -104 on, in the feed-forward contraction and behind the
     conv norm, so that shifts of -200 and of -3e38 give the same bits."""
