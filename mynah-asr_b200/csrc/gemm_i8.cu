@@ -163,6 +163,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 __syncwarp();
                 if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
             }
+            if (!ok && elect_one()) tc_commit(&acc_full[buf]);   // abandoned: the epilogue need not serve a wait of its own for it
         }
         if (!ok && lane == 0) atomicExch(status, ST_TIMEOUT_MMA);
     } else if (warp >= 2) {
