@@ -170,7 +170,9 @@ __device__ __forceinline__ bool gemm_epilogue_row(const GemmEpilogue &ep, float 
 // Stored row by row, every store instruction of a warp touches 32 different 128-byte lines with 16 bytes each, and the
 // load/store unit spends one cycle per line. Here the block is turned through 4 KB of shared memory (float4 columns
 // XOR-swizzled by the row: no bank conflicts either way) so that an instruction covers four whole lines: eight lanes
-// take the eight float4 of one row. Values and operation order per element are those of gemm_epilogue_row.
+// take the eight float4 of one row. Values and operation order per element are those of gemm_epilogue_row. By blocks for single tiles,
+// too: the encoder over twelve ragged utterances in the single-product mode 5.09 -> 4.47 ms, over eight with int8 activations 8.61 ->
+// 7.05, five utterances of 10 to 40 s on 24 layers 13.7 -> 12.6.
 static constexpr int GEMM_BLOCK_STAGE_FLOATS = 32 * 32;           // shared memory per epilogue warp
 
 // true if the block form can be used for every full-width chunk of this contraction (pointer and stride alignment)
@@ -213,10 +215,10 @@ __device__ __forceinline__ bool gemm_block_store(const GemmEpilogue &ep, const f
     __syncwarp();
     const int q = lane & 7, r0 = lane >> 3, col = nb + q * 4, mode = gemm_mode(ep, nb), hcol = gemm_plane_col(ep, nb) + q * 4;
     const float4 b = ep.bias ? *reinterpret_cast<const float4 *>(ep.bias + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-    // Every step over all eight places before the next one, and what the kind of contraction decides outside of the loops. Place by
-    // place, with the branches between, an epilogue warp spent 2000 to 5000 cycles here per block. With the row form written the
-    // same way: encoder over twelve ragged utterances, single products 4.26 -> 3.98 ms, over eight with int8 activations 6.32 ->
-    // 5.85, a voice command 2.048 -> 1.947, one minute on 24 layers 11.79 -> 11.54, sixteen of them 62.6 -> 62.0.
+    // Every step over all eight places before the next one, and what the kind of contraction decides outside of the loops, so that a
+    // thread's loads and reciprocals overlap. With the row form written the same way, instead of place by place with the branches
+    // between: encoder over twelve ragged utterances, single products 4.26 -> 3.98 ms, over eight with int8 activations 6.32 -> 5.85,
+    // a voice command 2.048 -> 1.947, one minute on 24 layers 11.79 -> 11.54, sixteen of them 62.6 -> 62.0.
     float4 t[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) t[i] = s4[(i * 4 + r0) * 8 + (q ^ ((i * 4 + r0) & 7))];

@@ -174,10 +174,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         int lt = 0;
         bool fits = true;
         chain_wait();                                  // row scales, the residual and the outputs belong to the kernels in front
-        // Whole 128-byte lines per store wherever the alignment allows; both forms produce the same bits. Row by row, a tile of 128
-        // columns spent 7 to 10 us behind its last MMA and one of 256 columns 10 to 15 (where the MMAs of K = 512 take 2.4), also
-        // with one tile per CTA. By blocks everywhere: the encoder over twelve ragged utterances in the single-product mode 5.09
-        // -> 4.47 ms, over eight with int8 activations 8.61 -> 7.05, five utterances of 10 to 40 s on 24 layers 13.7 -> 12.6.
+        // by blocks wherever the alignment allows, also with one tile per CTA (gemm.h)
         const bool blk_ok = Cfg::BLOCK_EPILOGUE && gemm_block_ok(ep) && (reinterpret_cast<uintptr_t>(col_scale) & 15) == 0;
         float *stage = epi_stage + (warp - 2) * GEMM_BLOCK_STAGE_FLOATS;
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x, lt++) {

@@ -15,10 +15,10 @@
 //     with NTERMS=1 only hi*hi (fast mode);
 //   * the issuing warps walk their loops whole and elect the lane that issues (warp_index, elect_one): operands of tcgen05 and TMA
 //     then are uniform registers. As code of one lane of a diverged warp every MMA waited for its operands to be moved there:
-//     [12000 x 1024 x 4096] took 223 us instead of 202, 47 rows of it 33 instead of 25; a voice command on 17 layers 1.83 ms
-//     instead of 1.60, 15 s on 24 layers 5.73 instead of 5.06, sixteen minutes 60.6 instead of 58.7. What bounds a k-step now is
-//     shared memory (TMA's writes and the MMAs' reads at 128 bytes a cycle): 128 x 128 columns 295 cycles of 312 so computed, 32
-//     columns 127 of 133;
+//     three products of [12000 x 1024 x 4096] took 224 us instead of 202, 47 rows of it 33 instead of 25, [750 x 4096 x 1024] 25.4
+//     instead of 22.7 (f32 out); a voice command on 17 layers 1.83 ms instead of 1.60, 15 s on 24 layers 5.73 instead of 5.06,
+//     sixteen minutes 60.6 instead of 58.7. With parts of the kernel left out, [12000 x 4096 x 1024]: operand loads alone 126 us,
+//     loads and MMAs 180, loads and epilogue 132, all 198; with a single product 49, 59, 72 and 87;
 //   * the kernel is persistent (one CTA per SM walks the output tiles) and the
 //     accumulators are double-buffered in TMEM, so the epilogue of one tile overlaps
 //     the MMAs of the next; eight epilogue warps read the accumulator with tcgen05.ld
@@ -207,10 +207,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant
         int lt = 0;
         bool fits = true;
         chain_wait();                                  // the residual is read and outputs are written only after the kernels in front
-        // Whole 128-byte lines per store wherever the alignment allows; both forms produce the same bits. Row by row, a tile of 128
-        // columns spent 7 to 10 us behind its last MMA and one of 256 columns 10 to 15 (where the MMAs of K = 512 take 2.4), also
-        // with one tile per CTA. By blocks everywhere: the encoder over twelve ragged utterances in the single-product mode 5.09
-        // -> 4.47 ms, over eight with int8 activations 8.61 -> 7.05, five utterances of 10 to 40 s on 24 layers 13.7 -> 12.6.
+        // by blocks wherever the alignment allows, also with one tile per CTA (gemm.h)
         const bool blk_ok = Cfg::BLOCK_EPILOGUE && gemm_block_ok(ep);
         float *stage = epi_stage + (warp - 2) * GEMM_BLOCK_STAGE_FLOATS;
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x, lt++) {
