@@ -2,7 +2,7 @@
 //
 // The driver copies pageable memory through a buffer of its own with one thread: 3 MB in 200 us, 24 MB in 1.2 to 1.4 ms, either
 // way, where the link needs 55 us and 430 (page-locked memory). One core's memcpy is the limit (18 GB/s). Here the caller and up
-// to two helpers copy parts of pieces of 512 KB, and a piece is on the link while the next ones are being filled.
+// to three helpers copy parts of pieces of 512 KB, and a piece is on the link while the next ones are being filled.
 //
 // A transfer holds a set of pieces from the first copy that is queued on, and the helpers only while there is something to copy: what
 // the stream still computes in front of a result keeps nobody busy. One transfer at a time has the helpers; others, meanwhile, copy
@@ -16,6 +16,9 @@
 #include <stdio.h>
 #include <string.h>
 #include <unistd.h>
+#if defined(__SSE2__)
+#include <emmintrin.h>
+#endif
 
 #include <atomic>
 #include <chrono>
@@ -30,20 +33,20 @@ namespace {
 constexpr size_t PIECE = 512 << 10, PART = 64 << 10;
 constexpr int SLOTS = 4;                                         // page-locked pieces of a set: 2 MB (page-locking takes 1 ms per MB, once)
 constexpr int SETS = 4;                                          // made when as many transfers are under way at once
-// us of a call with 3 MB of rows and 0.8 MB of results (and of processor time): one helper 255 (470), two 231 (630), three 217 (750);
-// the driver's way 302 (305).
-constexpr int HELPERS = 2;
+// Us of a call with 3 MB of rows and 0.8 MB of results (and of processor time): two helpers 192 (440), three 183 (510), the driver's way
+// 305 (310); with 24 and 6 MB 1226 (3480), 1030 (3780), 2650 (2680).
+constexpr int HELPERS = 3;
 // Waking a thread takes 17 us there, and a part 3.5: a helper that sleeps is not woken for the last FRESH parts.
 constexpr int FRESH = 3;
-// How long a thread looks within a transfer before it sleeps (four processes that share the device, 24 MB each: 25 us 7.9 ms a call,
-// 200 us 2.5), and how long a helper looks out for the next transfer: they often come in pairs, rows in, result out. The same call with
-// 2 ms of pause in front: 10 us 390, 25 us 310, 60 us 258, 100 us 260.
-constexpr auto PATIENCE = std::chrono::microseconds(200), LOOK = std::chrono::microseconds(60);
+// How long a thread looks within a transfer before it sleeps (with 25 us instead, four processes that shared a device took 8 ms instead of
+// 2.5 for a call of 24 and 6 MB: their pieces wait for one another on the link), and how long a helper looks out for the next
+// transfer (the smaller call, with 2 ms in front: 5 us 210, 10 us 199, 20 us 199, at 537, 531 and 592 us of processor time).
+constexpr auto PATIENCE = std::chrono::microseconds(200), LOOK = std::chrono::microseconds(10);
 // Below these the driver's way is as fast, or faster when the helpers are asleep. Us of a product whose rows (results) are so large,
 // new memory each time, driver and pieces, with no pause between calls and with 2 ms:
-//   in   0.5 MB  91, 93; 97, 107    0.75 MB  111, 112; 118, 126    1 MB  138, 125; 145, 138    1.5 MB  157, 157; 163, 167
-//   out  0.5 MB  78, 58; 80, 80     0.75 MB   92, 69;  96, 95      1 MB  111, 85;  118, 110    1.5 MB  142, 108; 150, 133
-constexpr size_t LEAST_IN = 1 << 20, LEAST_OUT = 512 << 10;
+//   in   0.5 MB  91, 85; 96, 101    0.63 MB  102, 97; 106, 108    0.75 MB  110, 100; 115, 112    1 MB  139, 110; 144, 121
+//   out  0.5 MB  81, 56; 84,  81    0.63 MB   90, 62;  90,  94    0.75 MB   96,  68;  96,  97    1 MB  113,  86; 120, 115
+constexpr size_t LEAST_IN = 640 << 10, LEAST_OUT = 512 << 10;
 constexpr int PARTS = (int)(PIECE / PART);
 
 // what a thread does between two looks at a word that another one writes
@@ -96,9 +99,31 @@ int caller_cores(int quota) {
     return n < quota ? n : quota;
 }
 
+// Into a piece (16-byte aligned) that the link reads next, past the caches: out of the caches of cores that have gone to sleep
+// meanwhile it reads slowly. A call with 2 MB of rows, 2 ms after the one before: 250 us when the helpers slept 25 us after they had
+// copied, 179 when they stayed awake for 250; past the caches 138, and 125 instead of 160 without the pause.
+inline void copy_past_caches(void *to, const void *from, size_t n) {
+#if defined(__SSE2__)
+    __m128i *d = (__m128i *)to;
+    const __m128i *f = (const __m128i *)from;
+    for (; n >= 64; n -= 64, d += 4, f += 4) {
+        const __m128i a = _mm_loadu_si128(f), b = _mm_loadu_si128(f + 1), c = _mm_loadu_si128(f + 2), e = _mm_loadu_si128(f + 3);
+        _mm_stream_si128(d, a);
+        _mm_stream_si128(d + 1, b);
+        _mm_stream_si128(d + 2, c);
+        _mm_stream_si128(d + 3, e);
+    }
+    memcpy(d, f, n);
+    _mm_sfence();                                                // before the part counts as copied
+#else
+    memcpy(to, from, n);
+#endif
+}
+
 // A transfer as parts of at most PART bytes in the order of the pieces. Parts below `open` may be taken.
 struct Part { void *to; const void *from; size_t n; int piece; };
 struct Job {
+    bool to_link = false;                                        // the parts go into pieces
     std::vector<Part> parts;
     std::vector<int> left;                                       // per piece: parts in it
     std::vector<std::atomic<int>> done;                          // ... copied
@@ -112,7 +137,8 @@ struct Job {
         do if (i >= open.load()) return false;
         while (!next.compare_exchange_weak(i, i + 1));
         const Part &p = parts[(size_t)i];
-        memcpy(p.to, p.from, p.n);
+        if (to_link) copy_past_caches(p.to, p.from, p.n);
+        else memcpy(p.to, p.from, p.n);
         done[(size_t)p.piece].fetch_add(1);
         copied.fetch_add(1);
         return true;
@@ -331,6 +357,7 @@ int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st) {
     const int n = (int)((bytes + PIECE - 1) / PIECE);
     Transfer t(c, s, (size_t)n);
     Job &j = t.j;
+    j.to_link = true;
     for (size_t at = 0; at < bytes; at += PART) {
         const int p = (int)(at / PIECE);
         j.parts.push_back(Part{s->base + (size_t)(p % SLOTS) * PIECE + at % PIECE, (const uint8_t *)host + at, bytes - at < PART ? bytes - at : PART, p});
@@ -395,8 +422,8 @@ int copy_out(const std::vector<CopyOut> &parts, cudaStream_t st) {
             if (e == cudaSuccess) e = cudaEventRecord(s->ev[asked % SLOTS], st);
         }
         if (e == cudaSuccess && q == 0) {
-            // what came before is done: the helpers wake up while the first piece is on the link (with them asleep 3 MB in and
-            // 0.8 MB out take 320 us instead of 340)
+            // what came before is done: the helpers wake up while the first piece is on the link (20 us of a call that found them
+            // asleep)
             e = cudaEventSynchronize(s->ev[SLOTS]);
             t.ask_helpers();
         }

@@ -35,7 +35,7 @@ def fake_runtime(tmp_path_factory, pkg):
 @pytest.mark.parametrize("name", [
     "vad_allocation_fails", "vad_gives_back", "error_is_reported_once", "failed_call_waits", "launches_of_other_threads", "qmat_workspace_is_shared",
     "foreign_capture_survives", "chain_table_copy_fails", "chain_graph_reads_its_own_table",
-    "copies_by_pieces", "copies_on_few_cores", "copies_of_other_classes", "copies_under_a_quota", "waits_of_copies_end_in_sleep", "copies_leave_others_alone", "small_copies_go_the_drivers_way",
+    "copies_by_pieces", "copies_on_few_cores", "copies_of_other_classes", "copies_under_a_quota", "waits_of_copies_end_in_sleep", "copies_leave_others_alone", "small_copies_go_the_drivers_way", "ragged_audio_arrives_whole",
 ])
 def test_host_path(fake_runtime, name):
     env = dict(os.environ, LD_LIBRARY_PATH=fake_runtime + ":" + os.environ.get("LD_LIBRARY_PATH", ""), OMP_NUM_THREADS="1")
@@ -488,7 +488,7 @@ def copies_on_few_cores(pkg, synth, fake):
         if len(cores) >= n:
             os.sched_setaffinity(0, cores[:n])
             threads, copies = call()
-            assert threads == min(n - 1, 2) and copies > 16, (n, threads, copies)
+            assert threads == min(n - 1, 3) and copies > 16, (n, threads, copies)
     os.sched_setaffinity(0, cores[:1])
     assert call()[1] <= 3
 
@@ -519,7 +519,7 @@ def copies_under_a_quota(pkg, synth, fake):
             f.write(text + "\n")
         with closing(_product(pkg, fake)) as call:           # (read when the first handle comes)
             threads, copies = call()
-            want = min(want, cores, 3)
+            want = min(want, cores, 4)
             assert threads == want - 1 and (copies > 16 if want > 1 else copies <= 3), (text, threads, copies)
 
 
@@ -593,10 +593,10 @@ def copies_leave_others_alone(pkg, synth, fake):
 
 @scenario
 def small_copies_go_the_drivers_way(pkg, synth, fake):
-    """Pieces from 1 MB of rows and 512 KB of results on: below, waking the helpers costs more than they save."""
+    """Pieces from 640 KB of rows and 512 KB of results on: below, waking the helpers costs more than they save."""
     if len(os.sched_getaffinity(0)) < 2:
         return
-    for n, k, rows, copies in ((64, 1024, 255, 2), (64, 1024, 256, 3), (64, 1024, 257, 4),        # rows, and result with status
+    for n, k, rows, copies in ((64, 1024, 159, 2), (64, 1024, 160, 3), (64, 1024, 257, 4),        # rows, and result with status
                                (1024, 64, 127, 3), (1024, 64, 128, 3), (1024, 64, 129, 4)):       # rows, status, result
         with closing(pkg.QMat(pkg.F32, np.ones((n, k), np.float32), n, k)) as q:
             x = np.ones((rows, k), np.float32)
@@ -604,6 +604,30 @@ def small_copies_go_the_drivers_way(pkg, synth, fake):
             fake.fake_reset()
             q.mul(x)
             assert fake.fake_calls(b"cudaMemcpyAsync") == copies, (n, k, rows, fake.fake_calls(b"cudaMemcpyAsync"))
+
+
+@scenario
+def ragged_audio_arrives_whole(pkg, synth, fake):
+    """Signals of every length modulo the 64 bytes that a copy past the caches moves at once, from any address, and signals that
+    end with a piece or a part."""
+    import cases
+    cfg, tensors = cases.build(synth, "ctc_q8")
+    m = cases.device_model(pkg, synth, cfg, tensors)
+    rng = np.random.default_rng(3)
+    signal = rng.standard_normal(700000).astype(np.float32)
+    seen = []
+
+    def look(name, args, recorded):
+        if b"mel_frame_kernel" in name:
+            item = C.cast(_arg(args, 19, C.c_void_p), C.POINTER(C.c_void_p * 2)).contents     # (audio, n_samples, ..)
+            seen.append(np.ctypeslib.as_array(C.cast(item[0], C.POINTER(C.c_float)), shape=(item[1],)).copy())
+
+    cb = LAUNCH(look)
+    fake.fake_on_launch(cb)
+    for n in [163840 + i for i in range(17)] + [262143, 262144, 262145, 278528, 655359]:
+        x = signal[n % 7:n % 7 + n]
+        m.transcribe_batch([x], decoder=1)
+        assert len(seen) == 1 and np.array_equal(seen.pop(), x), n
 
 
 if __name__ == "__main__":
