@@ -193,8 +193,8 @@ def test_sigmoids_against_float64(gpu_pkg):
         [0.0, -0.0, 87.0, -87.0, np.nextafter(np.float32(-87), np.float32(-88)), 88.8, -88.8, 3.4e38, -3.4e38, np.inf, -np.inf, np.nan],
         rng.integers(0, 1 << 32, 1 << 20, dtype=np.uint64).astype(np.uint32).view(np.float32),
     )])
-    x64 = x.astype(np.float64)
-    with np.errstate(over="ignore", invalid="ignore"):
+    with np.errstate(over="ignore", invalid="ignore"):       # (signalling NaNs among the bit patterns)
+        x64 = x.astype(np.float64)
         e = np.exp(-np.abs(x64))
         want = np.where(x64 >= 0, 1.0, e) / (1 + e)
         other = np.where(x64 >= 0, e, 1.0) / (1 + e)         # sigmoid(-x)
